@@ -87,15 +87,26 @@ __device__ inline void cfms(float2& acc, float2 a, float2 b) {
 __device__ inline double cabs1(double2 a) { return fabs(a.x) + fabs(a.y); }
 __device__ inline float cabs1(float2 a) { return fabsf(a.x) + fabsf(a.y); }
 
-// 1/z with Smith's scaling (avoids overflow of |z|^2 for large entries)
-__device__ inline double2 crecip(double2 z) {
-  if (fabs(z.x) >= fabs(z.y)) {
-    double r = z.y / z.x, d = z.x + z.y * r;
-    return make_double2(1.0 / d, -r / d);
-  }
-  double r = z.x / z.y, d = z.y + z.x * r;
-  return make_double2(r / d, -1.0 / d);
+// 1/z for complex128: conj(z) / |z|^2 with one FP64 reciprocal where |z|^2 is
+// far from overflow and underflow (an FP64 division costs about 590 clocks
+// here, a reciprocal 410), else with z scaled by a power of two first.  The
+// second form is a call: inlined, it would be executed predicated off, and an
+// FP64 instruction that is predicated off still takes its time.
+__device__ __noinline__ inline double2 crecip_scaled(double2 z) {
+  const int ex = max((__double2hiint(z.x) >> 20) & 0x7ff, (__double2hiint(z.y) >> 20) & 0x7ff);
+  // 2^-(exponent of the larger part), in two factors so that neither overflows
+  const int h = (1023 - ex) / 2, k = 1023 - ex - h;
+  const double s1 = __hiloint2double((1023 + h) << 20, 0), s2 = __hiloint2double((1023 + k) << 20, 0);
+  const double x = z.x * s1 * s2, y = z.y * s1 * s2, inv = 1.0 / fma(x, x, y * y);
+  return make_double2(x * inv * s1 * s2, -y * inv * s1 * s2);
 }
+__device__ inline double2 crecip(double2 z) {
+  const int ex = max((__double2hiint(z.x) >> 20) & 0x7ff, (__double2hiint(z.y) >> 20) & 0x7ff);
+  if (ex <= 623 || ex >= 1423) return crecip_scaled(z);
+  const double inv = __drcp_rn(fma(z.x, z.x, z.y * z.y));
+  return make_double2(z.x * inv, -z.y * inv);
+}
+// 1/z with Smith's scaling (avoids overflow of |z|^2 for large entries)
 __device__ inline float2 crecip(float2 z) {
   if (fabsf(z.x) >= fabsf(z.y)) {
     float r = z.y / z.x, d = z.x + z.y * r;

@@ -1,36 +1,44 @@
 // SIMT complex GEMM update (FP64 pipe for complex128, FP32 pipe for
-// complex64).  64 x 64 output tile per CTA, K staged through shared memory
-// 16 at a time, 4 x 4 complex outputs per thread.
+// complex64).  16 RT x 16 RT output tile per CTA of 256 threads, K staged
+// through shared memory 16 at a time, RT x RT complex outputs per thread.
+//
+// complex128 is bound by the FP64 pipe (about 1.7 fused multiply-adds per
+// clock and SM) whatever the tile, so the tile is chosen for balance: a 64-wide
+// tile takes 142 us at K = 32, however few there are.  RT = 1 while 32-wide
+// tiles would give fewer than four per SM, else RT = 2.  The sum over K runs in
+// the same order for every RT: bit-identical results.  complex64 keeps RT = 4
+// (its FP32 pipe is bound by shared-memory reads per product).
 #include "gemm.cuh"
 #include "diag.cuh"
 
 namespace mgt {
 
-constexpr int kGT = 64, kGK = 16;
+constexpr int kGK = 16;
 
-template <typename T>
+template <typename T, int RT>
 __global__ void __launch_bounds__(256)
 cgemm_sub_kernel(int M, int N, int K, const cplx<T>* __restrict__ A, int64_t lda,
                  const cplx<T>* __restrict__ B, int64_t ldb, cplx<T>* __restrict__ C, int64_t ldc) {
   using V = cplx<T>;
-  __shared__ V As[kGK][kGT + 1];
-  __shared__ V Bs[kGK][kGT];
+  constexpr int GT = 16 * RT;
+  __shared__ V As[kGK][GT + 1];
+  __shared__ V Bs[kGK][GT];
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
-  const int row0 = blockIdx.y * kGT, col0 = blockIdx.x * kGT;
-  V acc[4][4];
+  const int row0 = blockIdx.y * GT, col0 = blockIdx.x * GT;
+  V acc[RT][RT];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < RT; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = czero<V>();
+    for (int j = 0; j < RT; ++j) acc[i][j] = czero<V>();
   for (int k0 = 0; k0 < K; k0 += kGK) {
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
+    for (int q = 0; q < RT; ++q) {
       int idx = tid + 256 * q;
       int r = idx >> 4, kk = idx & 15;
       V v = czero<V>();
       if (row0 + r < M && k0 + kk < K) v = A[(int64_t)(row0 + r) * lda + k0 + kk];
       As[kk][r] = v;
-      int kb = idx >> 6, cc = idx & 63;
+      int kb = idx / GT, cc = idx % GT;
       V u = czero<V>();
       if (k0 + kb < K && col0 + cc < N) u = B[(int64_t)(k0 + kb) * ldb + col0 + cc];
       Bs[kb][cc] = u;
@@ -38,24 +46,24 @@ cgemm_sub_kernel(int M, int N, int K, const cplx<T>* __restrict__ A, int64_t lda
     __syncthreads();
 #pragma unroll
     for (int kk = 0; kk < kGK; ++kk) {
-      V a[4], b[4];
+      V a[RT], b[RT];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) a[i] = As[kk][ty + 16 * i];
+      for (int i = 0; i < RT; ++i) a[i] = As[kk][ty + 16 * i];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) b[j] = Bs[kk][tx + 16 * j];
+      for (int j = 0; j < RT; ++j) b[j] = Bs[kk][tx + 16 * j];
 #pragma unroll
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < RT; ++i)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) cfma(acc[i][j], a[i], b[j]);
+        for (int j = 0; j < RT; ++j) cfma(acc[i][j], a[i], b[j]);
     }
     __syncthreads();
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
+  for (int i = 0; i < RT; ++i) {
     int r = row0 + ty + 16 * i;
     if (r >= M) continue;
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
+    for (int j = 0; j < RT; ++j) {
       int c = col0 + tx + 16 * j;
       if (c < N) {
         V* p = C + (int64_t)r * ldc + c;
@@ -65,15 +73,27 @@ cgemm_sub_kernel(int M, int N, int K, const cplx<T>* __restrict__ A, int64_t lda
   }
 }
 
+template <typename T, int RT>
+static int gemm_sub_rt(int M, int N, int K, const cplx<T>* A, int64_t lda, const cplx<T>* B, int64_t ldb,
+                       cplx<T>* C, int64_t ldc, cudaStream_t s) {
+  constexpr int GT = 16 * RT;
+  dim3 grid((N + GT - 1) / GT, (M + GT - 1) / GT);
+  if (grid.y > 65535) return MGT_ERR_UNSUPPORTED;
+  count_launch();
+  cgemm_sub_kernel<T, RT><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, C, ldc);
+  return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
+}
+
 template <typename T>
 int gemm_sub(int M, int N, int K, const cplx<T>* A, int64_t lda, const cplx<T>* B, int64_t ldb,
              cplx<T>* C, int64_t ldc, cudaStream_t s) {
   if (M <= 0 || N <= 0 || K <= 0) return MGT_OK;
-  dim3 grid((N + kGT - 1) / kGT, (M + kGT - 1) / kGT);
-  if (grid.y > 65535) return MGT_ERR_UNSUPPORTED;
-  count_launch();
-  cgemm_sub_kernel<T><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, C, ldc);
-  return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
+  if constexpr (sizeof(T) == 8) {
+    const int64_t tiles = (int64_t)((N + 31) / 32) * ((M + 31) / 32);
+    if (tiles < 4 * device_sm_count()) return gemm_sub_rt<T, 1>(M, N, K, A, lda, B, ldb, C, ldc, s);
+    if ((M + 31) / 32 <= 65535) return gemm_sub_rt<T, 2>(M, N, K, A, lda, B, ldb, C, ldc, s);
+  }
+  return gemm_sub_rt<T, 4>(M, N, K, A, lda, B, ldb, C, ldc, s);
 }
 
 template int gemm_sub<double>(int, int, int, const double2*, int64_t, const double2*, int64_t, double2*, int64_t, cudaStream_t);

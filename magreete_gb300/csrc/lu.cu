@@ -22,6 +22,8 @@
 #include "gemm.cuh"
 #include "gemm_tc.cuh"
 #include "diag.cuh"
+#include "zgemm_tc.cuh"
+#include "zpanel.cuh"
 
 namespace mgt {
 
@@ -30,6 +32,7 @@ constexpr int kPanelThreads = 256;
 constexpr int kPanelRowsTarget = 256;   // default rows per CTA the panel aims for
 constexpr size_t kPanelSmemBudget = 220 * 1024;
 constexpr int kNBmax = 64;
+constexpr int kZPanelRows = 32;   // rows per CTA the complex128 panel aims for (16 .. 48 within 2%)
 // one published record per (column parity, CTA): header + candidate row + diagonal row
 constexpr size_t kRecHeader = 64;
 constexpr size_t kRecBytes = (kRecHeader + 2 * kNBmax * sizeof(double2) + 127) & ~size_t(127);
@@ -51,6 +54,8 @@ struct LuWsLayout {
     total = uinv + 2 * (size_t)kNBmax * kNBmax * sizeof(float2);
   }
 };
+
+static_assert(zpanel_words(kMaxPanelBlocks) * 8 <= 2 * kMaxPanelBlocks * kRecBytes, "messages fit the records");
 
 struct PanelWs {
   int* status;
@@ -1211,14 +1216,16 @@ lu_block_right_kernel(cplx<T>* __restrict__ A, int64_t lda, int n, int J0, int w
   }
 }
 
-// perm = identity; the factorisation epoch moves on by one; the panel records'
-// flags are cleared (the complex64 panel's short column tags rely on it)
-__global__ void lu_start_kernel(int32_t* perm, int n, unsigned long long* epoch, unsigned char* records) {
+// perm = identity; the factorisation epoch moves on by one; `words` 64-bit words
+// at a distance of `stride` are cleared: the panel records' flags, or the
+// messages of the complex128 panel (the short column tags of both rely on it)
+__global__ void lu_start_kernel(int32_t* perm, int n, unsigned long long* epoch, unsigned char* records, int words,
+                                size_t stride) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) perm[i] = i;
   if (i == 0) *epoch += 1;
-  for (int r = i; r < 2 * kMaxPanelBlocks; r += gridDim.x * blockDim.x)
-    *reinterpret_cast<unsigned long long*>(records + (size_t)r * kRecBytes) = 0ull;
+  for (int r = i; r < words; r += gridDim.x * blockDim.x)
+    *reinterpret_cast<unsigned long long*>(records + (size_t)r * stride) = 0ull;
 }
 
 static int num_sms() { return device_sm_count(); }
@@ -1228,6 +1235,13 @@ static int num_sms() { return device_sm_count(); }
 struct TcLU {
   TcPlan plan;
   CUtensorMap cmap;   // the whole matrix being factored
+};
+// complex128: operand digits of the tensor-core products, inverse of a block's diagonal
+struct ZLU {
+  ZGemmPlan plan;
+  double2* inv;       // 64 x 64
+  int* kexp;          // per block: 64 row exponents of A12, 64 of U12
+  size_t kexp_bytes;
 };
 static int trailing_update(const TcLU* tc, int M, int N, int K, const double2* A, int64_t lda, const double2* B,
                            int64_t ldb, double2* C, int64_t ldc, int, int*, cudaStream_t s, int) {
@@ -1721,13 +1735,14 @@ static SideStream* side_stream() {
 
 template <typename T, int NB>
 static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* work, cudaStream_t s,
-                          const LuOpts& opt, const TcLU* tc = nullptr) {
+                          const LuOpts& opt, const TcLU* tc = nullptr, const ZLU* zlu = nullptr) {
   using V = cplx<T>;
   static OncePerDevice once;
   once([] {
     cudaFuncSetAttribute(lu_panel_kernel<T, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPanelSmemBudget);
-    cudaFuncSetAttribute(lu_swap_trsm_kernel<T, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)((2 * NB * kSwapCols + NB * NB) * sizeof(V)));
+    if constexpr (sizeof(T) == 4)
+      cudaFuncSetAttribute(lu_swap_trsm_kernel<T, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)((2 * NB * kSwapCols + NB * NB) * sizeof(V)));
     cudaFuncSetAttribute(lu_panel_reg_kernel<T, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)reg_panel_smem(NB, sizeof(V)));
     cudaFuncSetAttribute(lu_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmem);
@@ -1735,7 +1750,10 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
   });
   PanelWs ws = panel_ws(work);
   if (cudaMemsetAsync(work, 0, 32, s) != cudaSuccess) return MGT_ERR_CUDA;   // status, nslot
-  lu_start_kernel<<<(n + 255) / 256, 256, 0, s>>>(perm, n, ws.epoch, ws.records);
+  const bool zpanel = sizeof(T) == 8 && NB == kZNB && opt.panel_reg == 1;
+  lu_start_kernel<<<std::max((n + 255) / 256, zpanel ? 64 : 1), 256, 0, s>>>(
+      perm, n, ws.epoch, ws.records, zpanel ? (int)zpanel_words(kMaxPanelBlocks) : 2 * kMaxPanelBlocks,
+      zpanel ? 8 : kRecBytes);
   count_launch();
   const int sms = std::min(num_sms(), kMaxPanelBlocks);
   const size_t sm2 = (2 * NB * kSwapCols + NB * NB) * sizeof(V);
@@ -1767,6 +1785,17 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
       }
     }
     const int m = n - j0;
+    if constexpr (sizeof(T) == 8 && NB == kZNB) {
+      if (zpanel) {
+        const PanelWs pw = panel_ws(work, set);
+        const ZPanelWs zw{pw.status, pw.nslot, pw.slots, reinterpret_cast<unsigned long long*>(pw.records),
+                          kMaxPanelBlocks};
+        const int cap = opt.panel_max_ctas > 0 ? std::min(opt.panel_max_ctas, sms) : sms;
+        const int e = zpanel_factor(A + (int64_t)j0 * lda + j0, lda, m, w, j0, perm, zw, kZPanelRows, cap,
+                                    opt.cooperative != 0, opt.panel_cluster != 0, s);
+        if (e != MGT_ERR_UNSUPPORTED) return e;
+      }
+    }
     const int G = panel_ctas(m);
     int rpc = (m + G - 1) / G;
     size_t smem = (size_t)rpc * NB * sizeof(V);
@@ -1822,17 +1851,23 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
   // latter also get U12 = L11^-1 A12 on the panel's rows
   auto swap = [&](cudaStream_t st, int j0, int w, int set, int left_begin, int left_end, int right_begin,
                   int right_end, int do_trsm) {
-    const int nleft = left_end > left_begin ? (left_end - left_begin + kSwapCols - 1) / kSwapCols : 0;
-    const int nright = right_end > right_begin ? (right_end - right_begin + kSwapCols - 1) / kSwapCols : 0;
-    if (nleft + nright > 0) {
-      // tile pivoting: the tile kernel left L11^-1 of this panel in slot `set`
-      const V* Linv = nullptr;
-      if (opt.pivoting == MGT_PIVOT_TILE && do_trsm)
-        Linv = reinterpret_cast<const V*>((char*)work + LuWsLayout().inv) + (size_t)set * kNBmax * kNBmax;
-      lu_swap_trsm_kernel<T, NB><<<nleft + nright, 256, sm2, st>>>(A, lda, n, j0, w, left_begin, left_end,
-                                                                    right_begin, right_end, panel_ws(work, set),
-                                                                    do_trsm, Linv);
-      count_launch();
+    if constexpr (sizeof(T) == 8 && NB == kZNB) {
+      const PanelWs pw = panel_ws(work, set);
+      zswap_panel(A, lda, n, j0, w, ZSlots{pw.slots, pw.nslot}, left_begin, left_end, right_begin, right_end,
+                  do_trsm != 0, nullptr, 0, st);
+    } else {
+      const int nleft = left_end > left_begin ? (left_end - left_begin + kSwapCols - 1) / kSwapCols : 0;
+      const int nright = right_end > right_begin ? (right_end - right_begin + kSwapCols - 1) / kSwapCols : 0;
+      if (nleft + nright > 0) {
+        // tile pivoting: the tile kernel left L11^-1 of this panel in slot `set`
+        const V* Linv = nullptr;
+        if (opt.pivoting == MGT_PIVOT_TILE && do_trsm)
+          Linv = reinterpret_cast<const V*>((char*)work + LuWsLayout().inv) + (size_t)set * kNBmax * kNBmax;
+        lu_swap_trsm_kernel<T, NB><<<nleft + nright, 256, sm2, st>>>(A, lda, n, j0, w, left_begin, left_end,
+                                                                      right_begin, right_end, panel_ws(work, set),
+                                                                      do_trsm, Linv);
+        count_launch();
+      }
     }
   };
   // Tile pivoting moves rows only within their 64-row tile, and nothing reads
@@ -1879,6 +1914,45 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
   auto update = [&](int r0, int c0, int k0, int K, int rows, int cols, bool dominant) -> int {
     return update_on(s, r0, c0, k0, K, rows, cols, dominant, 0);
   };
+  if constexpr (sizeof(T) == 8 && NB == kZNB) {
+    // complex128 with tensor-core scratch: 64-wide blocks of two inner panels;
+    // the columns right of a block get U12 = L^-1 A12 and the trailing update
+    // as tensor-core products of FP64 accuracy (zgemm_tc.cu)
+    if (zlu) {
+      const PanelWs p0 = panel_ws(work, 0), p1 = panel_ws(work, 1);
+      const ZSlots s0{p0.slots, p0.nslot}, s1{p1.slots, p1.nslot};
+      if (cudaMemsetAsync(zlu->kexp, 0, zlu->kexp_bytes, s) != cudaSuccess) return MGT_ERR_CUDA;
+      for (int J0 = 0; J0 < n; J0 += kZK) {
+        const int W = std::min(kZK, n - J0), wa = std::min(NB, W), wb = W - wa, j1 = J0 + wa, P0 = J0 + W;
+        const int right = n - P0;
+        double2* inv = right > 0 ? zlu->inv : nullptr;
+        int* ke = zlu->kexp + 2 * J0;
+        int e = panel_only(J0, wa, 0);
+        if (e == MGT_OK && wb > 0) {
+          e = zswap_panel(A, lda, n, J0, wa, s0, 0, 0, j1, P0, true, inv, kZK, s);
+          if (e == MGT_OK) e = update(j1, j1, J0, wa, n - j1, wb, false);
+          if (e == MGT_OK) e = panel_only(j1, wb, 1);
+          if (e == MGT_OK) e = zswap_panel(A, lda, n, j1, wb, s1, J0, j1, 0, 0, false, nullptr, 0, s);
+        }
+        if (e == MGT_OK) e = zswap_block(A, lda, n, J0, wa, wb, s0, s1, inv, ke, s);
+        if (e == MGT_OK && right > 0) {
+          V* A12 = A + (int64_t)J0 * lda + P0;
+          V* A21 = A + (int64_t)P0 * lda + J0;
+          e = zgemm_digits(zlu->plan, inv, kZK, kZK, A12, lda, right, kZK, ke, s);
+          if (e == MGT_OK) e = zgemm_apply(zlu->plan, 0, kZK, 0, right, kZK, A12, lda, false, ke + kZK, ws.status, s);
+          if (e == MGT_OK) e = zgemm_digits(zlu->plan, A21, lda, right, A12, lda, right, kZK, ke + kZK, s);
+          dom_begin(s);
+          if (e == MGT_OK)
+            e = zgemm_apply(zlu->plan, 0, right, 0, right, kZK, A + (int64_t)P0 * lda + P0, lda, true, nullptr,
+                            ws.status, s);
+          dom_end(s, 8.0 * right * (double)right * kZK,
+                  sizeof(V) * (2.0 * right * (double)right + 2.0 * (double)right * kZK));
+        }
+        if (e != MGT_OK) return e;
+      }
+      return MGT_OK;
+    }
+  }
   if (tc == nullptr || opt.outer_block == NB) {
     for (int j0 = 0; j0 < n; j0 += NB) {
       const int w = std::min(NB, n - j0);
@@ -2211,10 +2285,22 @@ constexpr int64_t kTcMinN = 256;
 
 static size_t tc_region_offset() { return (LuWsLayout().total + 1023) & ~size_t(1023); }
 
+// Below this order the complex128 LU updates on the FP64 pipe.  At 768 the
+// tensor-core path is already faster; the line is not drawn lower because the
+// no-allocation entry point has no room for the digits, and up to this order
+// both entry points give the same bits.
+constexpr int64_t kZMinN = 768;
+// complex128 tensor-core region: the inverse of a block's diagonal, row exponents, the digits
+static size_t z_kexp_bytes(int64_t n) { return (size_t)((n + kZK - 1) / kZK) * 2 * kZK * sizeof(int); }
+static size_t z_region_bytes(int64_t n) {
+  return kZK * kZK * sizeof(double2) + z_kexp_bytes(n) + zgemm_bytes(n, n);
+}
+
 extern "C" int mgt_lu_workspace_bytes(int dtype, int64_t n, size_t* bytes) {
   if (!bytes || n <= 0 || (dtype != MGT_C128 && dtype != MGT_C64)) return MGT_ERR_ARG;
   *bytes = LuWsLayout().total;
   if (dtype == MGT_C64 && n >= kTcMinN) *bytes = tc_region_offset() + tc_scratch_bytes(n);
+  if (dtype == MGT_C128 && n >= kZMinN) *bytes = tc_region_offset() + z_region_bytes(n);
   return MGT_OK;
 }
 
@@ -2228,6 +2314,14 @@ extern "C" int mgt_lu_factor_ex(int dtype, void* A, int64_t n, int64_t lda, int3
   cudaStream_t s = (cudaStream_t)stream;
   if (dtype == MGT_C128) {
     if (opt.pivoting != MGT_PIVOT_PARTIAL) return MGT_ERR_UNSUPPORTED;
+    if (n >= kZMinN && work_bytes >= tc_region_offset() + z_region_bytes(n)) {
+      ZLU z;
+      z.inv = (double2*)((char*)work + tc_region_offset());
+      z.kexp = (int*)(z.inv + kZK * kZK);
+      z.kexp_bytes = z_kexp_bytes(n);
+      z.plan.init((char*)z.kexp + z.kexp_bytes, n, n);
+      return lu_factor_impl<double, 32>((double2*)A, (int)n, lda, perm, work, s, opt, nullptr, &z);
+    }
     return lu_factor_impl<double, 32>((double2*)A, (int)n, lda, perm, work, s, opt);
   }
   if (dtype == MGT_C64) {

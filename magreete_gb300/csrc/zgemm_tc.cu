@@ -1,0 +1,694 @@
+// complex128 products C (M x N) -= A (M x K) B (K x N), K <= 64, on the tensor
+// cores: the trailing update of the complex128 LU.
+//
+// Why: the FP64 pipe of this part does about 1.7 fused multiply-adds per clock
+// and SM (1.0-1.2 TFLOP/s in all), so a product of FP64 accuracy is made from
+// exact FP16 products instead -- the Ozaki scheme of residual_tc.cu (Ozaki,
+// Ogita, Oishi, Rump 2012; Mukunoki, Ozaki, Ogita, Imamura 2020):
+//  * rows of A (as the real rows re, im, re, im, ...) and columns of B are
+//    scaled by powers of two and written as 54-bit integers in seven balanced
+//    base-256 digits, exact in FP16.  The largest entry of a row or column keeps
+//    all its 53 bits.
+//  * digit pairs (s, t) of equal weight s + t = l accumulate in one TMEM
+//    accumulator per level l = 0 .. 7 (34 of the 49 pairs; the rest lie below
+//    2^-60 of the scales).  128 real K at a time every level sum is an integer
+//    below 2^24, exact in FP32.
+//  * the levels are folded into one 64-bit integer per output in units of 2^-54
+//    of the scales (levels 0 .. 5 exactly, 6 and 7 rounded to the unit), which
+//    is rounded once to a double and subtracted from C: errors at the level of
+//    one FP64 rounding of the product's scale, where a 128-term FP64 sum makes 128.
+//
+// zgemm_kernel: persistent, one CTA per SM walking tiles of 128 rows x 32
+// complex columns (8 levels x 64 real columns fill TMEM):
+//   warp 0     : TMEM allocation; bulk copies of B's digit blocks (56 KB per 32
+//                complex K, 2 stages) and A's digit slices (8 KB, 6-slice ring)
+//   warp 1     : MMA issuer: for digit s of A one MMA per 16-wide K step covers
+//                up to four levels (B's digit slices are stacked along N)
+//   warps 2-9  : epilogue: levels -> 64-bit integers -> C.  The integer is turned
+//                into a double by integer instructions: one FP64 instruction per
+//                output is left (an FP64 conversion costs as much as the subtraction)
+//   warps 10-15: converters: byte digits -> FP16 operand slices
+// The MMAs of the next tile run while the epilogue finishes the last one.
+// Every wait is bounded; on expiry MGT_ERR_TIMEOUT is recorded, the issued work
+// drained and TMEM freed.
+#include <cuda_fp16.h>
+
+#include <algorithm>
+
+#include "common.cuh"
+#include "diag.cuh"
+#include "tcgen05.cuh"
+#include "zgemm_tc.cuh"
+
+namespace mgt {
+namespace zg {
+
+constexpr int BM = 128;
+constexpr int BNC = 32;
+constexpr int BN = 2 * BNC;
+constexpr int KCC = 32;                 // complex K per chunk
+constexpr int NCH = kZK / KCC;          // chunk stride of the digit buffers
+constexpr int DIG = 7, LEV = 8;
+constexpr int ASLOTS = 4, DSLOTS = 6;
+constexpr uint32_t A_SLICE = BM * 128, D_SLICE = BM * 64, B_SLICE = BN * 128, B_BLOCK = DIG * B_SLICE;
+constexpr uint32_t TMEM_COLS = LEV * BN;
+constexpr int NEPI = 8, NCONV = 6, EPI0 = 2;
+constexpr int THREADS = (EPI0 + NEPI + NCONV) * 32;
+constexpr int EPI_COLS = BN / (NEPI / 4);
+constexpr long long BIAS = 0x0080808080808080LL;
+constexpr int kNonFinite = 0x40000000;
+constexpr int FIX = 54;
+static_assert(TMEM_COLS == 512, "all of TMEM");
+
+constexpr size_t smem_bytes() { return 1024 + ASLOTS * A_SLICE + DSLOTS * D_SLICE + 2 * B_BLOCK + 256; }
+
+constexpr int kZeroExp = -100000;   // exponent of an exact zero
+constexpr int kBadExp = 1000000;    // of an infinity or a NaN
+
+// Exponent field (at least 1) of v 2^off.
+__device__ __forceinline__ int expo(double v, int off) {
+  const int hi = __double2hiint(v), ex = (hi >> 20) & 0x7ff;
+  if (ex == 2047) return kBadExp;
+  if (((hi & 0x7fffffff) | __double2loint(v)) == 0) return kZeroExp;
+  return max(ex, 1) + off;
+}
+
+constexpr int kRowSpread = 4;
+// Power of two scaled out of row k of B (see digits_kernel); every lane of a warp calls it.
+__device__ __forceinline__ bool rows_differ(const int* kexp, int K, int lane) {
+  int lo = 1 << 20, hi = -1;
+  for (int k = lane; k < K; k += 32) {
+    const int e = kexp[k];
+    if (e > 0 && e < 2047) {
+      lo = min(lo, e);
+      hi = max(hi, e);
+    }
+  }
+  lo = __reduce_min_sync(0xffffffffu, lo);
+  hi = __reduce_max_sync(0xffffffffu, hi);
+  return hi - lo > kRowSpread;
+}
+__device__ __forceinline__ int row_scale(int e) { return (e <= 0 || e >= 2047) ? 0 : e - 1023; }
+
+// Larger exponent field of both parts; 0 for zeros, infinities and NaN.
+__device__ __forceinline__ int field(double2 v) {
+  const int x = (__double2hiint(v.x) >> 20) & 0x7ff, y = (__double2hiint(v.y) >> 20) & 0x7ff;
+  return max(x == 2047 ? 0 : x, y == 2047 ? 0 : y);
+}
+
+// v 2^(off + FIX - e) as an integer (round to nearest) for e = emax - 1022, emax >= expo(v, off):
+// |result| < 2^54
+__device__ __forceinline__ long long fixed54(double v, int off, int emax) {
+  const long long b = __double_as_longlong(v);
+  const int ex = (int)((b >> 52) & 0x7ff);
+  long long m = b & 0xFFFFFFFFFFFFFll;
+  if (ex) m |= 1ll << 52;
+  const int sh = min(max(ex, 1) + off - emax + 1, 1);
+  long long r;
+  if (sh >= 0) r = m << sh;
+  else if (sh > -54) r = (m + (1ll << (-sh - 1))) >> (-sh);
+  else r = 0;
+  return b < 0 ? -r : r;
+}
+
+__device__ __forceinline__ uint32_t pick4(long long a, long long b, long long c, long long d, int p) {
+  const uint32_t x = p < 4 ? (uint32_t)a : (uint32_t)((unsigned long long)a >> 32);
+  const uint32_t y = p < 4 ? (uint32_t)b : (uint32_t)((unsigned long long)b >> 32);
+  const uint32_t z = p < 4 ? (uint32_t)c : (uint32_t)((unsigned long long)c >> 32);
+  const uint32_t w = p < 4 ? (uint32_t)d : (uint32_t)((unsigned long long)d >> 32);
+  const int k = p & 3;
+  const uint32_t sel = (uint32_t)(k | ((4 + k) << 4));
+  return __byte_perm(__byte_perm(x, y, sel), __byte_perm(z, w, sel), 0x5410);
+}
+
+// four biased digit bytes -> four FP16 values byte - 128 (exact)
+__device__ __forceinline__ uint2 widen4(uint32_t x) {
+  const uint32_t h0 = __byte_perm(x, 0x64646464u, 0x4140), h1 = __byte_perm(x, 0x64646464u, 0x4342);
+  const __half2 c = __halves2half2(__ushort_as_half((unsigned short)0x6480), __ushort_as_half((unsigned short)0x6480));
+  const __half2 d0 = __hsub2(*reinterpret_cast<const __half2*>(&h0), c);
+  const __half2 d1 = __hsub2(*reinterpret_cast<const __half2*>(&h1), c);
+  return make_uint2(*reinterpret_cast<const uint32_t*>(&d0), *reinterpret_cast<const uint32_t*>(&d1));
+}
+
+// Operand digits, both operands in one launch: blocks [0, ablocks) take 32 rows
+// of A each, the others 32 columns of B.  A: byte slices (row tile, chunk,
+// digit) at half the width of the swizzled FP16 operand; B: the swizzled FP16
+// operand itself (block (column tile, chunk): rows s 64 + 2 j, + 1).  Zeros
+// beyond the operand.  K <= 64.  kexp (or null): the largest exponent field of
+// row k of B's whole row (0: zero row).  Where the rows' sizes differ by more
+// than 2^4, column k of A is scaled up and row k of B down by that power of
+// two, so that rows of B of very different size (a badly row-scaled matrix)
+// do not share one column scale; a well-scaled operand is left as it is.
+__global__ void __launch_bounds__(256)
+digits_kernel(const double2* __restrict__ A, int64_t lda, int M, int ablocks, const double2* __restrict__ B,
+              int64_t ldb, int N, int K, const int* __restrict__ kexp, unsigned char* __restrict__ adig,
+              int* __restrict__ aexp, unsigned char* __restrict__ bdig, int* __restrict__ bexp) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const bool rows = kexp && rows_differ(kexp, K, lane);
+  if ((int)blockIdx.x < ablocks) {
+    for (int q = 0; q < 4; ++q) {
+      const int row = blockIdx.x * 32 + warp * 4 + q;
+      double2 v[NCH];
+      int off[NCH], em = kZeroExp;
+#pragma unroll
+      for (int c = 0; c < NCH; ++c) {
+        const int k = c * KCC + lane;
+        off[c] = (rows && k < K) ? row_scale(kexp[k]) : 0;
+        v[c] = (row < M && k < K) ? A[(int64_t)row * lda + k] : make_double2(0.0, 0.0);
+        em = max(em, max(expo(v[c].x, off[c]), expo(v[c].y, off[c])));
+      }
+      em = __reduce_max_sync(0xffffffffu, em);
+      if (lane == 0 && row < M) aexp[row] = em == kBadExp ? kNonFinite : em - 1022;
+      const int rt = row / BM, rho = row % BM;
+      const uint32_t at = (uint32_t)rho * 64u + ((uint32_t)((lane >> 2) ^ (rho & 7)) << 3) + (uint32_t)(lane & 3) * 2u;
+#pragma unroll
+      for (int c = 0; c < NCH; ++c) {
+        const long long yr = fixed54(v[c].x, off[c], em) + BIAS, yi = fixed54(v[c].y, off[c], em) + BIAS;
+        unsigned char* blk = adig + ((size_t)rt * NCH + c) * DIG * D_SLICE + at;
+#pragma unroll
+        for (int s = 0; s < DIG; ++s) {
+          const int p = 8 * (DIG - 1 - s);
+          const unsigned d = (unsigned)((yr >> p) & 255) | ((unsigned)((yi >> p) & 255) << 8);
+          *reinterpret_cast<unsigned short*>(blk + s * D_SLICE) = (unsigned short)d;
+        }
+      }
+    }
+    return;
+  }
+  __shared__ int sm[8][32];
+  const int ct = blockIdx.x - ablocks, j = ct * BNC + lane;
+  double2 v[kZK / 8];
+  int off[kZK / 8], em = kZeroExp;
+#pragma unroll
+  for (int i = 0; i < kZK / 8; ++i) {
+    const int k = warp * (kZK / 8) + i;
+    off[i] = (rows && k < K) ? -row_scale(kexp[k]) : 0;
+    v[i] = (k < K && j < N) ? B[(int64_t)k * ldb + j] : make_double2(0.0, 0.0);
+    em = max(em, max(expo(v[i].x, off[i]), expo(v[i].y, off[i])));
+  }
+  sm[warp][lane] = em;
+  __syncthreads();
+#pragma unroll
+  for (int t = 0; t < 8; ++t) em = max(em, sm[t][lane]);
+  if (warp == 0 && j < N) bexp[j] = em == kBadExp ? kNonFinite : em - 1022;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int k0 = warp * 8 + 4 * h, c = k0 / KCC, kk = k0 % KCC;
+    long long yr[4], yi[4], yn[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int o = off[4 * h + i];
+      const long long xr = fixed54(v[4 * h + i].x, o, em), xi = fixed54(v[4 * h + i].y, o, em);
+      yr[i] = xr + BIAS;
+      yi[i] = xi + BIAS;
+      yn[i] = BIAS - xi;
+    }
+    unsigned char* blk = bdig + ((size_t)ct * NCH + c) * B_BLOCK;
+#pragma unroll
+    for (int s = 0; s < DIG; ++s) {
+      const int p = DIG - 1 - s;
+      const int rho = s * BN + 2 * lane;
+      const uint2 a0 = widen4(pick4(yr[0], yn[0], yr[1], yn[1], p)), a1 = widen4(pick4(yr[2], yn[2], yr[3], yn[3], p));
+      const uint2 b0 = widen4(pick4(yi[0], yr[0], yi[1], yr[1], p)), b1 = widen4(pick4(yi[2], yr[2], yi[3], yr[3], p));
+      const int ch = kk >> 2;   // 16-byte chunk: real K 2 kk .. 2 kk + 7
+      *reinterpret_cast<uint4*>(blk + (uint32_t)rho * 128u + ((uint32_t)(ch ^ (rho & 7)) << 4)) =
+          make_uint4(a0.x, a0.y, a1.x, a1.y);
+      *reinterpret_cast<uint4*>(blk + (uint32_t)(rho + 1) * 128u + ((uint32_t)(ch ^ ((rho + 1) & 7)) << 4)) =
+          make_uint4(b0.x, b0.y, b1.x, b1.y);
+    }
+  }
+}
+
+// acc 2^sc rounded to nearest even, without FP64 arithmetic on the normal path
+__device__ __forceinline__ double scaled_double(long long acc, int sc) {
+  if (acc == 0) return 0.0;
+  const unsigned long long u = acc < 0 ? 0ull - (unsigned long long)acc : (unsigned long long)acc;
+  const int lz = __clzll((long long)u);
+  const unsigned long long m = u << lz;
+  unsigned long long keep = m >> 11;
+  const unsigned rem = (unsigned)m & 0x7ffu;
+  keep += (rem > 0x400u || (rem == 0x400u && (keep & 1ull))) ? 1ull : 0ull;
+  const int be = 1023 + 63 - lz + sc;   // biased exponent
+  if (be < 1 || be > 2045) return ldexp((double)acc, sc);
+  const unsigned long long bits = ((unsigned long long)(be - 1) << 52) + keep;
+  return __longlong_as_double((long long)(bits | (acc < 0 ? 0x8000000000000000ull : 0ull)));
+}
+
+// one MMA group per (digit s of A, 16-wide K step): levels s .. min(6 + s, 7)
+__device__ __forceinline__ void issue_digit(uint32_t tmem, uint64_t ad, uint32_t bb, int s, bool first) {
+  using namespace tc;
+  const int nt_all = min(DIG, LEV - s);
+#pragma unroll
+  for (int ks = 0; ks < 4; ++ks) {
+    const bool fresh = first && ks == 0;
+    for (int t0 = 0; t0 < nt_all; t0 += 4) {
+      int nt = min(4, nt_all - t0);
+      const uint64_t bd = kmajor_sw128_desc(bb + (uint32_t)t0 * B_SLICE) + (uint64_t)(2 * ks);
+      if (fresh && s == 1 && t0 == 4) {
+        // level 7 starts here (levels 0 .. 6 started with s = 0)
+        mma_f16(tmem + (uint32_t)((s + 6) * BN), ad + (uint64_t)(2 * ks),
+                kmajor_sw128_desc(bb + 6u * B_SLICE) + (uint64_t)(2 * ks), idesc_f16_m128(BN), 0u);
+        nt = 2;
+      }
+      mma_f16(tmem + (uint32_t)((s + t0) * BN), ad + (uint64_t)(2 * ks), bd, idesc_f16_m128(nt * BN),
+              (fresh && s == 0) ? 0u : 1u);
+    }
+  }
+}
+
+__global__ void __launch_bounds__(THREADS, 1)
+zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aexp,
+             const unsigned char* __restrict__ bdig, const int* __restrict__ bexp, int M, int N, int nch, int ctiles,
+             int total_tiles, double2* C, int64_t ldc, int sub, int* __restrict__ rowmax, int* status) {
+  using namespace tc;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* aring = base;
+  unsigned char* bring = aring + ASLOTS * A_SLICE;
+  unsigned char* dring = bring + 2 * B_BLOCK;
+  uint64_t* full_a = reinterpret_cast<uint64_t*>(dring + DSLOTS * D_SLICE);
+  uint64_t* empty_a = full_a + ASLOTS;
+  uint64_t* full_d = empty_a + ASLOTS;
+  uint64_t* empty_d = full_d + DSLOTS;
+  uint64_t* full_b = empty_d + DSLOTS;
+  uint64_t* empty_b = full_b + 2;
+  uint64_t* tfull = empty_b + 2;
+  uint64_t* tempty = tfull + 1;
+  uint64_t* done = tempty + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
+  volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int first = blockIdx.x, stride = gridDim.x;
+  const int ntiles = total_tiles > first ? (total_tiles - first + stride - 1) / stride : 0;
+  const int nblk = ntiles * nch;   // B blocks (and DIG times as many A slices) of this CTA
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < ASLOTS; ++s) { mbar_init(&full_a[s], NCONV); mbar_init(&empty_a[s], 1); }
+    for (int s = 0; s < DSLOTS; ++s) { mbar_init(&full_d[s], 1); mbar_init(&empty_d[s], NCONV); }
+    for (int s = 0; s < 2; ++s) { mbar_init(&full_b[s], 1); mbar_init(&empty_b[s], 1); }
+    mbar_init(tfull, 1);
+    mbar_init(tempty, NEPI);
+    mbar_init(done, 1);
+    *abort = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                 "r"(TMEM_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot;
+
+  if (warp == 0 && lane == 0) {
+    // ---------------- producer: whichever copy has a free slot
+    const int nq = nblk * DIG;
+    int ib = 0, q = 0;
+    uint32_t idle = 0;
+    while ((ib < nblk || q < nq) && !*abort) {
+      bool progress = false;
+      if (ib < nblk && (ib < 2 || mbar_try_wait(&empty_b[ib & 1], ((ib >> 1) - 1) & 1))) {
+        const int t = first + (ib / nch) * stride, ct = t % ctiles;
+        mbar_expect_tx(&full_b[ib & 1], B_BLOCK);
+        bulk_load(bring + (ib & 1) * B_BLOCK, bdig + ((size_t)ct * NCH + ib % nch) * B_BLOCK, B_BLOCK, &full_b[ib & 1]);
+        ++ib;
+        progress = true;
+      }
+      if (q < nq && (q < DSLOTS || mbar_try_wait(&empty_d[q % DSLOTS], ((q / DSLOTS) - 1) & 1))) {
+        const int blk = q / DIG, t = first + (blk / nch) * stride, rt = t / ctiles;
+        mbar_expect_tx(&full_d[q % DSLOTS], D_SLICE);
+        bulk_load(dring + (q % DSLOTS) * D_SLICE,
+                  adig + (((size_t)rt * NCH + blk % nch) * DIG + q % DIG) * D_SLICE, D_SLICE, &full_d[q % DSLOTS]);
+        ++q;
+        progress = true;
+      }
+      if (progress) idle = 0;
+      else if (++idle >= kWaitLimit) { *abort = 1; break; }
+    }
+    // copies in flight land before the CTA may exit
+    for (int j = max(0, ib - 2); j < ib; ++j) mbar_wait_plain(&full_b[j & 1], (j >> 1) & 1);
+    for (int j = max(0, q - DSLOTS); j < q; ++j) mbar_wait_plain(&full_d[j % DSLOTS], (j / DSLOTS) & 1);
+  } else if (warp == 1 && lane == 0) {
+    // ---------------- MMA issuer: one readout (at most 128 real K) per tile
+    int q = 0, i = 0;
+    bool ok = true;
+    for (int lt = 0; lt < ntiles && ok; ++lt) {
+      if (lt > 0) {
+        if (!mbar_wait(tempty, (lt - 1) & 1, abort)) { ok = false; break; }
+        tc_fence_after();
+      }
+      for (int c = 0; c < nch && ok; ++c, ++i) {
+        const int st = i & 1;
+        if (!mbar_wait(&full_b[st], (i >> 1) & 1, abort)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t bb = smem_u32(bring + st * B_BLOCK);
+        for (int s = 0; s < DIG; ++s, ++q) {
+          const int slot = q % ASLOTS;
+          if (!mbar_wait(&full_a[slot], (q / ASLOTS) & 1, abort)) { ok = false; break; }
+          tc_fence_after();
+          issue_digit(tmem, kmajor_sw128_desc(smem_u32(aring + slot * A_SLICE)), bb, s, c == 0);
+          mma_commit(&empty_a[slot]);
+        }
+        if (ok) mma_commit(&empty_b[st]);
+      }
+      if (ok) mma_commit(tfull);
+    }
+    mma_commit(done);   // arrives once every MMA issued above has completed
+  } else if (warp >= EPI0 && warp < EPI0 + NEPI) {
+    // ---------------- epilogue: thread = (row, half of the real columns)
+    const int qd = warp & 3, part = (warp - EPI0) >> 2, r = qd * 32 + lane;
+    const uint32_t tbase = tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(part * EPI_COLS);
+    for (int lt = 0; lt < ntiles; ++lt) {
+      const int t = first + lt * stride, row = (t / ctiles) * BM + r;
+      const int col0 = (t % ctiles) * BNC + part * (EPI_COLS / 2);
+      double2* crow = C + (int64_t)row * ldc + col0;
+      const int ncol = row < M ? min(EPI_COLS / 2, N - col0) : 0;
+      if (sub && ncol > 0) {
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(crow));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(crow + (ncol - 1)));
+      }
+      if (!mbar_wait(tfull, lt & 1, abort)) break;
+      tc_fence_after();
+      long long acc[EPI_COLS];
+#pragma unroll
+      for (int p = 0; p < EPI_COLS / 4; ++p) {
+        uint32_t v[LEV][4];
+#pragma unroll
+        for (int l = 0; l < LEV; ++l) tmem_ld4(tbase + (uint32_t)(l * BN + p * 4), v[l]);
+        tmem_wait_ld();
+        if (p == EPI_COLS / 4 - 1) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(tempty)) : "memory");
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          // level l weighs 2^(42 - 8 l) units of 2^-54; |L_0| <= 2^19, |L_1| <= 2^21, |L_2| <= 2^22,
+          // |L_3| < 2^22.6: hi and mid are exact in 32 bits
+          const int hi = (__float2int_rz(__uint_as_float(v[0][j])) << 8) + __float2int_rz(__uint_as_float(v[1][j]));
+          const int mid = (__float2int_rz(__uint_as_float(v[2][j])) << 8) + __float2int_rz(__uint_as_float(v[3][j]));
+          const int l4 = __float2int_rz(__uint_as_float(v[4][j])), l5 = __float2int_rz(__uint_as_float(v[5][j]));
+          const int l67 = __float2int_rn(
+              0.015625f * fmaf(__uint_as_float(v[7][j]), 0.00390625f, __uint_as_float(v[6][j])));
+          acc[p * 4 + j] = ((long long)hi << 34) + ((long long)mid << 18) + ((long long)l4 << 10) +
+                           (long long)((l5 << 2) + l67);
+        }
+      }
+      if (ncol <= 0) continue;
+      const int ea = aexp[row];
+      int em = 0;
+#pragma unroll
+      for (int j = 0; j < EPI_COLS / 2; ++j) {
+        if (j < ncol) {
+          const int eb = bexp[col0 + j];
+          double2 o = sub ? crow[j] : make_double2(0.0, 0.0);
+          if (ea == kNonFinite || eb == kNonFinite) {
+            o.x = o.y = __longlong_as_double(0x7FF8000000000000LL);
+          } else {
+            const int sc = ea + eb - FIX;
+            const double x = scaled_double(acc[2 * j], sc), y = scaled_double(acc[2 * j + 1], sc);
+            if (sub) {
+              o.x -= x;
+              o.y -= y;
+            } else {
+              o.x = x;
+              o.y = y;
+            }
+          }
+          crow[j] = o;
+          em = max(em, field(o));
+        }
+      }
+      if (rowmax && em > 0) atomicMax(rowmax + row, em);
+    }
+  } else if (warp >= EPI0 + NEPI) {
+    // ---------------- converters: staged byte slice -> FP16 operand slice
+    const int ctid = threadIdx.x - (EPI0 + NEPI) * 32;
+    const int nq = nblk * DIG;
+    for (int q = 0; q < nq; ++q) {
+      const int ds = q % DSLOTS, as = q % ASLOTS;
+      if (!mbar_wait(&full_d[ds], (q / DSLOTS) & 1, abort)) break;
+      if (q >= ASLOTS && !mbar_wait(&empty_a[as], ((q / ASLOTS) - 1) & 1, abort)) break;
+      const unsigned char* src = dring + ds * D_SLICE;
+      unsigned char* dst = aring + as * A_SLICE;
+      for (int u = ctid; u < (int)(D_SLICE / 8); u += NCONV * 32) {
+        const uint32_t off = (uint32_t)u * 8u;
+        const uint2 v = *reinterpret_cast<const uint2*>(src + off);
+        const uint2 w0 = widen4(v.x), w1 = widen4(v.y);
+        *reinterpret_cast<uint4*>(dst + 2 * off) = make_uint4(w0.x, w0.y, w1.x, w1.y);
+      }
+      fence_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full_a[as])) : "memory");
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&empty_d[ds])) : "memory");
+      }
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (threadIdx.x == 0 && *abort) atomicExch(status, MGT_ERR_TIMEOUT);
+  if (warp == 0) {
+    if (lane == 0) mbar_wait_plain(done, 0);
+    __syncwarp();
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+  }
+}
+
+// ---------------------------------------------------------------- interchanges of the blocked LU
+
+constexpr int SB = 32;       // panel width
+constexpr int SLAB = 8;      // columns per CTA of zswap_kernel (one warp each in the solve)
+
+// Forward substitution with a unit lower 32 x 32 factor, one column per warp, lane = row.
+__device__ __forceinline__ double2 lower_solve32(const double2* L, int w, double2 x, int lane) {
+  for (int k = 0; k < w - 1; ++k) {
+    double2 xk;
+    xk.x = __shfl_sync(0xffffffffu, x.x, k);
+    xk.y = __shfl_sync(0xffffffffu, x.y, k);
+    if (lane > k) cfms(x, L[lane * (SB + 1) + k], xk);
+  }
+  return x;
+}
+
+// Blocks: 8-column slabs of [lb, le), then of [rb, re), then (inv) four blocks of L11^-1's columns.
+__global__ void __launch_bounds__(256)
+zswap_kernel(double2* __restrict__ A, int64_t lda, int n, int j0, int w, ZSlots sl, int lb, int le, int rb, int re,
+             int solve, double2* __restrict__ inv, int ldinv) {
+  __shared__ __align__(16) double2 buf[2 * SB][SLAB];
+  __shared__ __align__(16) double2 L[SB * (SB + 1)];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int nleft = le > lb ? (le - lb + SLAB - 1) / SLAB : 0, nright = re > rb ? (re - rb + SLAB - 1) / SLAB : 0;
+  const int b = blockIdx.x;
+  const bool is_inv = b >= nleft + nright, right = !is_inv && b >= nleft;
+  if (is_inv || (right && solve))
+    for (int i = tid; i < SB * SB; i += 256) {
+      const int r = i / SB, k = i % SB;
+      const bool ok = r < w && k < w;
+      cp_async_elem<16>(L + r * (SB + 1) + k, ok ? A + (int64_t)(j0 + r) * lda + j0 + k : A, ok);
+    }
+  if (is_inv) {
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    const int col = (b - nleft - nright) * 8 + warp;
+    const double2 x = lower_solve32(L, w, make_double2(lane == col ? 1.0 : 0.0, 0.0), lane);
+    inv[(int64_t)lane * ldinv + col] = x;
+    return;
+  }
+  const int c0 = right ? rb + (b - nleft) * SLAB : lb + b * SLAB;
+  const int ncols = min(SLAB, (right ? re : le) - c0);
+  const int m = n - j0, ns = min(*sl.nslot, 2 * SB);
+  const bool top_needed = right && solve;
+  for (int i = tid; i < ns * SLAB; i += 256) {
+    const int q = i / SLAB, cc = i % SLAB;
+    const int2 v = sl.slots[q];
+    const bool in = v.x >= 0 && v.x < m && v.y >= 0 && v.y < m;
+    if (cc < ncols && in && (v.x != v.y || (top_needed && v.x < w)))
+      cp_async_elem<16>(&buf[q][cc], A + (int64_t)(j0 + v.y) * lda + c0 + cc, true);
+  }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  if (top_needed && warp < ncols) {
+    // the first 32 slots are the panel's own rows, in order
+    double2 x = lane < w ? buf[lane][warp] : make_double2(0.0, 0.0);
+    x = lower_solve32(L, w, x, lane);
+    if (lane < w) buf[lane][warp] = x;
+  }
+  __syncthreads();
+  for (int i = tid; i < ns * SLAB; i += 256) {
+    const int q = i / SLAB, cc = i % SLAB;
+    const int2 v = sl.slots[q];
+    const bool in = v.x >= 0 && v.x < m && v.y >= 0 && v.y < m;
+    if (cc < ncols && in && (v.x != v.y || (top_needed && v.x < w))) A[(int64_t)(j0 + v.x) * lda + c0 + cc] = buf[q][cc];
+  }
+}
+
+// Both panels' interchanges on the columns left and right of a 64-wide block,
+// 32 columns per CTA, one panel after the other; eight more CTAs (Inv) finish
+// the block's inverse L^-1 = [[Ia, 0], [-Lb^-1 Lba Ia, Lb^-1]], a column per
+// warp.  kexp (64 zeros) receives the largest exponent fields of the block's
+// rows right of it.
+__global__ void __launch_bounds__(256)
+zswap_block_kernel(double2* __restrict__ A, int64_t lda, int n, int J0, int wa, int wb, ZSlots sa, ZSlots sb,
+                   int nleft, int nright, double2* __restrict__ Inv, int* __restrict__ kexp) {
+  // the moved rows (2 SB x 32), or the inverse's two 32 x 33 factors
+  __shared__ __align__(16) unsigned char raw[2 * SB * (SB + 1) * sizeof(double2)];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int b = blockIdx.x, j1 = J0 + wa, W = wa + wb;
+  if (b >= nleft + nright) {
+    // inverse CTAs: columns 0..31 are -Lb^-1 Lba Ia, columns 32..63 are Lb^-1
+    double2* Lb = reinterpret_cast<double2*>(raw);
+    double2* Lba = Lb + SB * (SB + 1);
+    const int c8 = b - nleft - nright;
+    for (int i = tid; i < SB * SB; i += 256) {
+      const int r = i / SB, k = i % SB;
+      const bool okb = r < wb && k < wb, oka = r < wb && k < wa;
+      cp_async_elem<16>(Lb + r * (SB + 1) + k, okb ? A + (int64_t)(j1 + r) * lda + j1 + k : A, okb);
+      cp_async_elem<16>(Lba + r * (SB + 1) + k, oka ? A + (int64_t)(j1 + r) * lda + J0 + k : A, oka);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    const int col = c8 * 8 + warp;
+    double2 x;
+    if (col < SB) {
+      const double2 ia = Inv[(int64_t)lane * kZK + col];   // Ia[lane][col]
+      x = make_double2(0.0, 0.0);
+      for (int k = col; k < SB; ++k) {
+        double2 v;
+        v.x = __shfl_sync(0xffffffffu, ia.x, k);
+        v.y = __shfl_sync(0xffffffffu, ia.y, k);
+        cfms(x, Lba[lane * (SB + 1) + k], v);
+      }
+    } else {
+      x = make_double2(lane == col - SB ? 1.0 : 0.0, 0.0);
+    }
+    x = lower_solve32(Lb, wb, x, lane);
+    Inv[(int64_t)(SB + lane) * kZK + col] = x;
+    if (col >= SB) Inv[(int64_t)lane * kZK + col] = make_double2(0.0, 0.0);
+    return;
+  }
+  double2* buf = reinterpret_cast<double2*>(raw);   // [2 SB][32]
+  const bool right = b >= nleft;
+  const int c0 = right ? J0 + W + (b - nleft) * 32 : b * 32;
+  const int ncols = min(32, (right ? n : J0) - c0);
+  for (int set = 0; set < (wb > 0 ? 2 : 1); ++set) {
+    const int jj = set ? j1 : J0, m = n - jj;
+    const int2* slots = set ? sb.slots : sa.slots;
+    const int ns = min(set ? *sb.nslot : *sa.nslot, 2 * SB);
+    for (int i = tid; i < ns * 32; i += 256) {
+      const int q = i >> 5, cc = i & 31;
+      const int2 v = slots[q];
+      const bool in = v.x >= 0 && v.x < m && v.y >= 0 && v.y < m && v.x != v.y;
+      if (cc < ncols && in) cp_async_elem<16>(buf + i, A + (int64_t)(jj + v.y) * lda + c0 + cc, true);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    for (int i = tid; i < ns * 32; i += 256) {
+      const int q = i >> 5, cc = i & 31;
+      const int2 v = slots[q];
+      const bool in = v.x >= 0 && v.x < m && v.y >= 0 && v.y < m && v.x != v.y;
+      if (cc < ncols && in) A[(int64_t)(jj + v.x) * lda + c0 + cc] = buf[i];
+    }
+    __syncthreads();
+  }
+  if (right && kexp)
+    for (int k = warp; k < W; k += 8) {
+      const double2 v = lane < ncols ? A[(int64_t)(J0 + k) * lda + c0 + lane] : make_double2(0.0, 0.0);
+      const int em = __reduce_max_sync(0xffffffffu, field(v));
+      if (lane == 0 && em > 0) atomicMax(kexp + k, em);
+    }
+}
+
+static size_t up(size_t v, size_t a) { return (v + a - 1) / a * a; }
+
+}  // namespace zg
+
+size_t zgemm_bytes(int64_t rows, int64_t cols) {
+  using namespace zg;
+  const size_t rt = (size_t)((rows + BM - 1) / BM), ct = (size_t)((cols + BNC - 1) / BNC);
+  return 1024 + up(rt * NCH * DIG * D_SLICE, 1024) + up(ct * NCH * B_BLOCK, 1024) + up(rt * BM * sizeof(int), 256) +
+         up(ct * BNC * sizeof(int), 256);
+}
+
+void ZGemmPlan::init(void* work, int64_t r, int64_t c) {
+  using namespace zg;
+  const size_t rt = (size_t)((r + BM - 1) / BM), ct = (size_t)((c + BNC - 1) / BNC);
+  char* b = (char*)up((size_t)work, 1024);
+  adig = (unsigned char*)b;
+  b += up(rt * NCH * DIG * D_SLICE, 1024);
+  bdig = (unsigned char*)b;
+  b += up(ct * NCH * B_BLOCK, 1024);
+  aexp = (int*)b;
+  b += up(rt * BM * sizeof(int), 256);
+  bexp = (int*)b;
+  rows = r;
+  cols = c;
+}
+
+int zgemm_digits(const ZGemmPlan& p, const double2* A, int64_t lda, int M, const double2* B, int64_t ldb, int N, int K,
+                 const int* kexp, cudaStream_t s) {
+  using namespace zg;
+  if (!A) M = 0;
+  if (!B) N = 0;
+  if (K <= 0 || K > kZK || M > p.rows || N > p.cols || M < 0 || N < 0) return MGT_ERR_ARG;
+  // whole 128-row tiles of A: rows beyond M are written as zeros
+  const int ab = (M + BM - 1) / BM * (BM / 32), bb = (N + BNC - 1) / BNC;
+  if (ab + bb == 0) return MGT_OK;
+  count_launch();
+  digits_kernel<<<ab + bb, 256, 0, s>>>(A, lda, M, ab, B, ldb, N, K, kexp, p.adig, p.aexp, p.bdig, p.bexp);
+  return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
+}
+
+int zgemm_apply(const ZGemmPlan& p, int arow, int M, int bcol, int N, int K, double2* C, int64_t ldc, bool sub,
+                int* rowmax, int* status, cudaStream_t s, int max_ctas) {
+  using namespace zg;
+  if (M <= 0 || N <= 0) return MGT_OK;
+  if (K <= 0 || K > kZK || arow % BM || bcol % BNC || arow < 0 || bcol < 0 || (int64_t)arow + M > p.rows ||
+      (int64_t)bcol + N > p.cols)
+    return MGT_ERR_ARG;
+  static OncePerDevice once;
+  once([] { cudaFuncSetAttribute(zgemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes()); });
+  const int rt = (M + BM - 1) / BM, ct = (N + BNC - 1) / BNC;
+  const int64_t total = (int64_t)rt * ct;
+  if (total > (1 << 30)) return MGT_ERR_UNSUPPORTED;
+  const int ctas = (int)std::min<int64_t>(total, max_ctas > 0 ? max_ctas : device_sm_count());
+  count_launch();
+  zgemm_kernel<<<ctas, THREADS, smem_bytes(), s>>>(p.adig + (size_t)(arow / BM) * NCH * DIG * D_SLICE, p.aexp + arow,
+                                                   p.bdig + (size_t)(bcol / BNC) * NCH * B_BLOCK, p.bexp + bcol, M, N,
+                                                   (K + KCC - 1) / KCC, ct, (int)total, C, ldc, sub ? 1 : 0, rowmax,
+                                                   status);
+  return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
+}
+
+int zswap_panel(double2* A, int64_t lda, int n, int j0, int w, const ZSlots& sl, int lb, int le, int rb, int re,
+                bool solve, double2* inv, int ldinv, cudaStream_t st) {
+  using namespace zg;
+  const int nl = le > lb ? (le - lb + SLAB - 1) / SLAB : 0, nr = re > rb ? (re - rb + SLAB - 1) / SLAB : 0;
+  const int blocks = nl + nr + (inv ? 4 : 0);
+  if (blocks == 0) return MGT_OK;
+  count_launch();
+  zswap_kernel<<<blocks, 256, 0, st>>>(A, lda, n, j0, w, sl, lb, le, rb, re, solve ? 1 : 0, inv, ldinv);
+  return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
+}
+
+int zswap_block(double2* A, int64_t lda, int n, int J0, int wa, int wb, const ZSlots& a, const ZSlots& b,
+                double2* Inv, int* kexp, cudaStream_t st) {
+  using namespace zg;
+  const int nleft = (J0 + 31) / 32, nright = (n - J0 - wa - wb + 31) / 32;
+  const int blocks = nleft + nright + (Inv ? 8 : 0);
+  if (blocks == 0) return MGT_OK;
+  count_launch();
+  zswap_block_kernel<<<blocks, 256, 0, st>>>(A, lda, n, J0, wa, wb, a, b, nleft, nright, Inv, kexp);
+  return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
+}
+
+}  // namespace mgt
