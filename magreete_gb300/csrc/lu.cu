@@ -2229,16 +2229,20 @@ static int lu_solve_impl(const cplx<T>* LU, int n, int64_t lda, const int32_t* p
                          int64_t ldb, cplx<T>* X, int64_t ldx, int nrhs, cudaStream_t s, void* work = nullptr) {
   using V = cplx<T>;
   if (work) {
-    // persistent flag-ordered triangular solves (one launch per triangle and 64 columns)
-    int* status = (int*)((char*)work + 128);
-    if (cudaMemsetAsync(status, 0, 2 * sizeof(int), s) != cudaSuccess) return MGT_ERR_CUDA;
-    dim3 pg((nrhs + 127) / 128, n);
     if (n > 65535) return MGT_ERR_UNSUPPORTED;
-    permute_rows_kernel<V><<<pg, 128, 0, s>>>(B, ldb, perm, X, ldx, n, nrhs);
+    permute_rows_kernel<V><<<dim3((nrhs + 127) / 128, n), 128, 0, s>>>(B, ldb, perm, X, ldx, n, nrhs);
     count_launch();
-    int e = tri_solve<T, false>(LU, lda, X, ldx, n, nrhs, work, status, s);
-    if (e == MGT_OK) e = tri_solve<T, true>(LU, lda, X, ldx, n, nrhs, work, status, s);
-    return e;
+    if constexpr (sizeof(T) == 8) {
+      // one tensor-core product per 64-row block
+      return zsolve(LU, lda, X, ldx, n, nrhs, work, s);
+    } else {
+      // persistent flag-ordered triangular solves (one launch per triangle and 64 columns)
+      int* status = (int*)((char*)work + 128);
+      if (cudaMemsetAsync(status, 0, 2 * sizeof(int), s) != cudaSuccess) return MGT_ERR_CUDA;
+      int e = tri_solve<T, false>(LU, lda, X, ldx, n, nrhs, work, status, s);
+      if (e == MGT_OK) e = tri_solve<T, true>(LU, lda, X, ldx, n, nrhs, work, status, s);
+      return e;
+    }
   }
   constexpr int BS = 64;
   static OncePerDevice once;
@@ -2343,9 +2347,13 @@ extern "C" int mgt_lu_factor(int dtype, void* A, int64_t n, int64_t lda, int32_t
   return mgt_lu_factor_ex(dtype, A, n, lda, perm, work, work_bytes, nullptr, stream);
 }
 
+static size_t lu_solve_bytes(int dtype, int64_t n, int64_t nrhs) {
+  return dtype == MGT_C128 ? zsolve_workspace_bytes(n, nrhs) : tri_solve_workspace_bytes(n, nrhs, sizeof(float2));
+}
+
 extern "C" int mgt_lu_solve_workspace_bytes(int dtype, int64_t n, int64_t nrhs, size_t* bytes) {
   if (!bytes || n <= 0 || nrhs <= 0 || (dtype != MGT_C128 && dtype != MGT_C64)) return MGT_ERR_ARG;
-  *bytes = tri_solve_workspace_bytes(n, nrhs, dtype == MGT_C128 ? sizeof(double2) : sizeof(float2));
+  *bytes = lu_solve_bytes(dtype, n, nrhs);
   return MGT_OK;
 }
 
@@ -2354,8 +2362,7 @@ extern "C" int mgt_lu_solve(int dtype, const void* LU, int64_t n, int64_t lda, c
                             size_t work_bytes, void* stream) {
   if (!LU || !perm || !B || !X || n <= 0 || nrhs <= 0 || lda < n || ldb < nrhs || ldx < nrhs) return MGT_ERR_ARG;
   if (B == X) return MGT_ERR_ARG;
-  if (work && work_bytes < tri_solve_workspace_bytes(n, nrhs, dtype == MGT_C128 ? sizeof(double2) : sizeof(float2)))
-    return MGT_ERR_WORKSPACE;
+  if (work && work_bytes < lu_solve_bytes(dtype, n, nrhs)) return MGT_ERR_WORKSPACE;
   cudaStream_t s = (cudaStream_t)stream;
   if (dtype == MGT_C128)
     return lu_solve_impl<double>((const double2*)LU, (int)n, lda, perm, (const double2*)B, ldb, (double2*)X, ldx,

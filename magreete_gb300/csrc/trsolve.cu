@@ -530,8 +530,6 @@ int lower_block_inverses(const cplx<T>* F, int64_t ldf, int n, cplx<T>* Inv, cud
 }
 template int lower_block_inverses<float>(const float2*, int64_t, int, float2*, cudaStream_t);
 
-template int tri_solve<double, false>(const double2*, int64_t, double2*, int64_t, int, int, void*, int*, cudaStream_t);
-template int tri_solve<double, true>(const double2*, int64_t, double2*, int64_t, int, int, void*, int*, cudaStream_t);
 template int tri_solve<float, false>(const float2*, int64_t, float2*, int64_t, int, int, void*, int*, cudaStream_t);
 template int tri_solve<float, true>(const float2*, int64_t, float2*, int64_t, int, int, void*, int*, cudaStream_t);
 

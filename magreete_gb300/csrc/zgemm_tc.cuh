@@ -43,4 +43,8 @@ int zswap_panel(double2* A, int64_t lda, int n, int j0, int w, const ZSlots& s, 
 int zswap_block(double2* A, int64_t lda, int n, int J0, int wa, int wb, const ZSlots& a, const ZSlots& b,
                 double2* Inv, int* kexp, cudaStream_t st);
 
+// ---- triangular solves X = U^-1 L^-1 X in place (zsolve.cu); the status word is the first int of work
+size_t zsolve_workspace_bytes(int64_t n, int64_t nrhs);
+int zsolve(const double2* F, int64_t ldf, double2* X, int64_t ldx, int n, int nrhs, void* work, cudaStream_t s);
+
 }  // namespace mgt

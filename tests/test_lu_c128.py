@@ -1,4 +1,5 @@
-"""The complex128 LU on the tensor cores (csrc/zpanel.cu, zgemm_tc.cu).
+"""The complex128 LU and its solves on the tensor cores (csrc/zpanel.cu,
+zgemm_tc.cu, zsolve.cu).
 
 The panel kernel (one row per four threads, messages in distributed shared
 memory or through L2) picks the pivots of the shared-memory panel and gives
@@ -89,6 +90,33 @@ def test_blocked_lu_is_a_factorisation(n, pad, scaling):
         D, ref = Lm @ U - PA, PA
     err = (torch.linalg.norm(D) / torch.linalg.norm(ref)).item()
     assert err <= 4 * n * EPS, err
+
+
+@pytest.mark.parametrize("n,R", [(1, 1), (63, 2), (64, 33), (65, 1), (129, 305), (767, 32), (1000, 64), (1153, 700)])
+def test_solves(n, R):
+    """Backward error of the solves around the 64-row block, with one column,
+    columns off the 32-column tile and more columns than twice the SMs."""
+    from magreete_gb300 import engine as E
+    A, B = _random(n, n, n + R), _random(n, R, 7 * n + R)
+    f = E.lu_factor(A.clone())
+    X = E.lu_solve(f, B)
+    be = torch.linalg.norm(A @ X - B) / (torch.linalg.norm(A) * torch.linalg.norm(X))
+    assert be.item() <= 4 * n * EPS, be.item()
+
+
+def test_solve_with_badly_scaled_rows():
+    """Right-hand sides and factors whose rows differ by up to 1e30: the solve of
+    a row-scaled system is that of the unscaled one."""
+    from magreete_gb300 import engine as E
+    n, R = 900, 5
+    A, B = _random(n, n, 1), _random(n, R, 2)
+    e = torch.randint(-50, 51, (n,), generator=torch.Generator().manual_seed(3)).cuda()
+    s = torch.pow(torch.tensor(2.0, dtype=torch.float64), e.to(torch.float64).cpu()).cuda()
+    f = E.lu_factor(A * s[:, None])
+    X = E.lu_solve(f, B * s[:, None])
+    r = torch.linalg.norm(A @ X - B) / (torch.linalg.norm(A) * torch.linalg.norm(X))
+    # the pivot order differs (the largest scaled row), the growth with it: n^2 covers both
+    assert r.item() <= n * n * EPS, r.item()
 
 
 @pytest.mark.parametrize("n", [100, 900])
