@@ -3,8 +3,7 @@
 // One thread per (row point, column point) pair writes that pair's d x d
 // block of complex entries; threads of a warp take consecutive column points,
 // so each of the d output rows a warp touches is one contiguous run of
-// 32*d*16 bytes.  The kernel is store-bandwidth bound for the 3D kinds and
-// FP64-pipe bound (Bessel J0/Y0/J1/Y1) for the 2D kinds.
+// 32*d*16 bytes.  Bound by the FP64 pipe (1.7 operations a clock and SM).
 // The Green's blocks themselves are in green.cuh.
 #include <atomic>
 
@@ -27,15 +26,18 @@ struct OutSpec {
 __device__ __forceinline__ void store_entry(const OutSpec& o, int64_t row, int64_t col, double2 v) {
   if (!o.p) return;
   if (o.dtype == MGT_C128) reinterpret_cast<double2*>(o.p)[row * o.ld + col] = v;
-  else if (o.dtype == MGT_C64) reinterpret_cast<float2*>(o.p)[row * o.ld + col] = make_float2((float)v.x, (float)v.y);
-  else reinterpret_cast<float4*>(o.p)[row * o.ld + col] = df_split(v);
+  else {
+    const float4 f = df_split(v);
+    if (o.dtype == MGT_C64) reinterpret_cast<float2*>(o.p)[row * o.ld + col] = make_float2(f.x, f.z);
+    else reinterpret_cast<float4*>(o.p)[row * o.ld + col] = f;
+  }
 }
 
 // System matrix: block (i, j) = -coef * G(r_i - r_j) for i != j,
 // (1 - shift) * I for i == j.
 template <int KIND>
 __global__ void __launch_bounds__(kAsmThreads)
-assemble_system_kernel(const double* __restrict__ pts, int n, double k0, double2 coef,
+assemble_system_kernel(const double* __restrict__ pts, int n, double k0, double ik0, double2 coef,
                        double2 diag, OutSpec o1, OutSpec o2) {
   constexpr int dim = Kind<KIND>::dim, d = Kind<KIND>::d;
   int j = blockIdx.x * kAsmThreads + threadIdx.x;
@@ -58,7 +60,7 @@ assemble_system_kernel(const double* __restrict__ pts, int n, double k0, double2
 #pragma unroll
       for (int c = 0; c < dim; ++c) r[c] = pts[(int64_t)i * dim + c] - sj[c];
       // distinct scatterers at the same position give the reference a NaN block
-      if (!green_block<KIND>(r, k0, false, 0.0, g)) {
+      if (!green_block<KIND>(r, k0, ik0, false, 0.0, g)) {
 #pragma unroll
         for (int q = 0; q < d * d; ++q)
           g[q] = make_double2(__longlong_as_double(0x7ff8000000000000ll), __longlong_as_double(0x7ff8000000000000ll));
@@ -90,10 +92,13 @@ assemble_system_kernel(const double* __restrict__ pts, int n, double k0, double2
 // of its components, so the mirrored values are bitwise those of the lower
 // triangle evaluated directly.
 constexpr int kSymTP = 16;
+// MIXED: o1 is double-float and o2 complex64 (the mixed method's pair).  Each
+// entry is then converted once, by the thread that evaluated it, instead of
+// once per copy and format.
 
-template <int KIND>
+template <int KIND, bool MIXED>
 __global__ void __launch_bounds__(kSymTP * kSymTP)
-assemble_system_sym_kernel(const double* __restrict__ pts, int n, double k0, double2 coef, double2 diag,
+assemble_system_sym_kernel(const double* __restrict__ pts, int n, double k0, double ik0, double2 coef, double2 diag,
                            OutSpec o1, OutSpec o2) {
   constexpr int dim = Kind<KIND>::dim, d = Kind<KIND>::d;
   constexpr int TP = kSymTP, W = TP * d;          // tile side in matrix rows / columns
@@ -114,7 +119,7 @@ assemble_system_sym_kernel(const double* __restrict__ pts, int n, double k0, dou
       double r[dim];
 #pragma unroll
       for (int c = 0; c < dim; ++c) r[c] = pts[(int64_t)i * dim + c] - pts[(int64_t)j * dim + c];
-      if (!green_block<KIND>(r, k0, false, 0.0, g)) {
+      if (!green_block<KIND>(r, k0, ik0, false, 0.0, g)) {
 #pragma unroll
         for (int e = 0; e < d * d; ++e)
           g[e] = make_double2(__longlong_as_double(0x7ff8000000000000ll), __longlong_as_double(0x7ff8000000000000ll));
@@ -131,17 +136,29 @@ assemble_system_sym_kernel(const double* __restrict__ pts, int n, double k0, dou
     for (int e = 0; e < d * d; ++e) g[e] = make_double2(0.0, 0.0);
   }
 #pragma unroll
-  for (int e = 0; e < d * d; ++e) S[(p * TP + q) * d * d + e] = g[e];
+  for (int e = 0; e < d * d; ++e) {
+    if constexpr (MIXED) reinterpret_cast<float4*>(asm_smem)[(p * TP + q) * d * d + e] = df_split(g[e]);
+    else S[(p * TP + q) * d * d + e] = g[e];
+  }
   __syncthreads();
+  auto put = [&](int64_t row, int64_t col, int at) {
+    if constexpr (MIXED) {
+      const float4 f = reinterpret_cast<const float4*>(asm_smem)[at];
+      reinterpret_cast<float4*>(o1.p)[row * o1.ld + col] = f;
+      reinterpret_cast<float2*>(o2.p)[row * o2.ld + col] = make_float2(f.x, f.z);
+    } else {
+      const double2 v = S[at];
+      store_entry(o1, row, col, v);
+      store_entry(o2, row, col, v);
+    }
+  };
   // tile (bi, bj): row i d + a, column j d + b
   for (int idx = tid; idx < W * W; idx += TP * TP) {
     const int rr = idx / W, cc = idx - rr * W;
     const int pp = rr / d, a = rr - pp * d, qq = cc / d, b = cc - qq * d;
     const int ii = bi * TP + pp, jj = bj * TP + qq;
     if (ii < n && jj < n) {
-      const double2 v = S[(pp * TP + qq) * d * d + a * d + b];
-      store_entry(o1, (int64_t)ii * d + a, (int64_t)jj * d + b, v);
-      store_entry(o2, (int64_t)ii * d + a, (int64_t)jj * d + b, v);
+      put((int64_t)ii * d + a, (int64_t)jj * d + b, (pp * TP + qq) * d * d + a * d + b);
     }
   }
   if (bi == bj) return;
@@ -151,9 +168,7 @@ assemble_system_sym_kernel(const double* __restrict__ pts, int n, double k0, dou
     const int qq = rr / d, b = rr - qq * d, pp = cc / d, a = cc - pp * d;
     const int ii = bi * TP + pp, jj = bj * TP + qq;
     if (ii < n && jj < n) {
-      const double2 v = S[(pp * TP + qq) * d * d + a * d + b];
-      store_entry(o1, (int64_t)jj * d + b, (int64_t)ii * d + a, v);
-      store_entry(o2, (int64_t)jj * d + b, (int64_t)ii * d + a, v);
+      put((int64_t)jj * d + b, (int64_t)ii * d + a, (pp * TP + qq) * d * d + a * d + b);
     }
   }
 }
@@ -163,7 +178,7 @@ assemble_system_sym_kernel(const double* __restrict__ pts, int n, double k0, dou
 template <int KIND, bool TRANSPOSE>
 __global__ void __launch_bounds__(kAsmThreads)
 assemble_propagator_kernel(const double* __restrict__ tgt, int nt, const double* __restrict__ src,
-                           int ns, double k0, double2 coef, bool regularize, double radius,
+                           int ns, double k0, double ik0, double2 coef, bool regularize, double radius,
                            int nan_policy, double2 fill, OutSpec out) {
   constexpr int dim = Kind<KIND>::dim, d = Kind<KIND>::d;
   int ncol = TRANSPOSE ? nt : ns, nrow = TRANSPOSE ? ns : nt;
@@ -185,7 +200,7 @@ assemble_propagator_kernel(const double* __restrict__ tgt, int nt, const double*
       r[c] = TRANSPOSE ? (cq[c] - rp) : (rp - cq[c]);  // always target - source
     }
     double2 g[d * d];
-    if (green_block<KIND>(r, k0, regularize, radius, g)) {
+    if (green_block<KIND>(r, k0, ik0, regularize, radius, g)) {
 #pragma unroll
       for (int e = 0; e < d * d; ++e) {
         double2 v = g[e];
@@ -213,18 +228,26 @@ static std::atomic<int> g_sym_assembly{1};   // assemble from half the Green's b
 template <int KIND>
 static cudaError_t launch_system(const double* pts, int n, double k0, double2 coef, double2 diag,
                                  OutSpec o1, OutSpec o2, cudaStream_t s) {
+  const cudaError_t pe = prepare_green<KIND>(s);
+  if (pe != cudaSuccess) return pe;
+  const double ik0 = 1.0 / k0;
   if (g_sym_assembly.load(std::memory_order_relaxed)) {
     constexpr int d = Kind<KIND>::d;
     const int nb = (n + kSymTP - 1) / kSymTP;
     if (nb <= 65535) {
       const size_t smem = (size_t)kSymTP * kSymTP * d * d * sizeof(double2);
-      assemble_system_sym_kernel<KIND><<<dim3(nb, nb), kSymTP * kSymTP, smem, s>>>(pts, n, k0, coef, diag, o1, o2);
+      if (o1.dtype == MGT_CDF && o2.p && o2.dtype == MGT_C64)
+        assemble_system_sym_kernel<KIND, true><<<dim3(nb, nb), kSymTP * kSymTP, smem, s>>>(pts, n, k0, ik0, coef, diag,
+                                                                                         o1, o2);
+      else
+        assemble_system_sym_kernel<KIND, false><<<dim3(nb, nb), kSymTP * kSymTP, smem, s>>>(pts, n, k0, ik0, coef,
+                                                                                          diag, o1, o2);
       count_launch();
       return cudaGetLastError();
     }
   }
   dim3 grid((n + kAsmThreads - 1) / kAsmThreads, (n + kAsmRows - 1) / kAsmRows);
-  assemble_system_kernel<KIND><<<grid, kAsmThreads, 0, s>>>(pts, n, k0, coef, diag, o1, o2);
+  assemble_system_kernel<KIND><<<grid, kAsmThreads, 0, s>>>(pts, n, k0, ik0, coef, diag, o1, o2);
   count_launch();
   return cudaGetLastError();
 }
@@ -239,13 +262,16 @@ template <int KIND>
 static cudaError_t launch_prop(const double* t, int nt, const double* src, int ns, double k0,
                                double2 coef, bool reg, double radius, int nanp, double2 fill,
                                int transpose, OutSpec out, cudaStream_t s) {
+  const cudaError_t pe = prepare_green<KIND>(s);
+  if (pe != cudaSuccess) return pe;
+  const double ik0 = 1.0 / k0;
   int ncol = transpose ? nt : ns, nrow = transpose ? ns : nt;
   dim3 grid((ncol + kAsmThreads - 1) / kAsmThreads, (nrow + kAsmRows - 1) / kAsmRows);
   count_launch();
   if (transpose)
-    assemble_propagator_kernel<KIND, true><<<grid, kAsmThreads, 0, s>>>(t, nt, src, ns, k0, coef, reg, radius, nanp, fill, out);
+    assemble_propagator_kernel<KIND, true><<<grid, kAsmThreads, 0, s>>>(t, nt, src, ns, k0, ik0, coef, reg, radius, nanp, fill, out);
   else
-    assemble_propagator_kernel<KIND, false><<<grid, kAsmThreads, 0, s>>>(t, nt, src, ns, k0, coef, reg, radius, nanp, fill, out);
+    assemble_propagator_kernel<KIND, false><<<grid, kAsmThreads, 0, s>>>(t, nt, src, ns, k0, ik0, coef, reg, radius, nanp, fill, out);
   return cudaGetLastError();
 }
 

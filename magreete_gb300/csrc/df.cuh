@@ -9,10 +9,32 @@
 
 namespace mgt {
 
+// v = hi + lo, hi the nearest float (ties away from zero), lo the rounded rest.
+// By integer instructions: a conversion between double and float takes the FP64
+// pipe's 19 clocks per warp and SM, the split three of them and a subtraction.
+__device__ __noinline__ inline float2 split_any(double v) {
+  const float h = (float)v;
+  return make_float2(h, (float)(v - (double)h));
+}
+__device__ __forceinline__ float2 split_double(double v) {
+  const unsigned hw = (unsigned)__double2hiint(v), lw = (unsigned)__double2loint(v);
+  const int e = (int)((hw >> 20) & 0x7ffu) - 1023;
+  if (((hw << 1) | lw) == 0u) return make_float2(0.f, 0.f);
+  if (e < -70 || e > 126) return split_any(v);   // infinities, NaN and where a part is not a normal float
+  // 53-bit significand: 24 bits (rounded) and a signed rest of 29
+  const unsigned top = ((hw & 0xFFFFFu) | 0x100000u) << 3 | lw >> 29, low = lw & 0x1FFFFFFFu;
+  const unsigned up = low >> 28;
+  const int rest = (int)low - (int)(up << 29);
+  const unsigned sign = hw & 0x80000000u;
+  const float h = __uint_as_float((((unsigned)(e + 126)) << 23) + top + up);
+  const float l = (float)rest * __uint_as_float((unsigned)(e - 52 + 127) << 23);
+  return make_float2(__uint_as_float(__float_as_uint(h) | sign), __uint_as_float(__float_as_uint(l) ^ sign));
+}
+
 // complex double-float: x = re_hi, y = re_lo, z = im_hi, w = im_lo
 __device__ __forceinline__ float4 df_split(double2 v) {
-  float rh = (float)v.x, ih = (float)v.y;
-  return make_float4(rh, (float)(v.x - (double)rh), ih, (float)(v.y - (double)ih));
+  const float2 r = split_double(v.x), i = split_double(v.y);
+  return make_float4(r.x, r.y, i.x, i.y);
 }
 __device__ __forceinline__ double2 df_join(float4 v) {
   return make_double2((double)v.x + (double)v.y, (double)v.z + (double)v.w);

@@ -51,7 +51,7 @@ template <> struct Acc<true> {
 template <int KIND, int RT, bool DF>
 __global__ void __launch_bounds__(256)
 propagate_partial_kernel(const double* __restrict__ tgt, int nt, const double* __restrict__ src, int ns, double k0,
-                         bool regularize, double radius, const double2* __restrict__ Ek, int64_t ld_ek, int ncols,
+                         double ik0, bool regularize, double radius, const double2* __restrict__ Ek, int64_t ld_ek, int ncols,
                          int src_per_split, double2* __restrict__ partial) {
   constexpr int d = Kind<KIND>::d, dim = Kind<KIND>::dim;
   constexpr int ROWS = kPT * d, KC = kPJ * d;
@@ -81,7 +81,7 @@ propagate_partial_kernel(const double* __restrict__ tgt, int nt, const double* _
         double r[dim];
 #pragma unroll
         for (int c = 0; c < dim; ++c) r[c] = tpos[tt][c] - src[(int64_t)j * dim + c];
-        if (!green_block<KIND>(r, k0, regularize, radius, g)) {
+        if (!green_block<KIND>(r, k0, ik0, regularize, radius, g)) {
           const double nan = __longlong_as_double(0x7ff8000000000000ll);
 #pragma unroll
           for (int e = 0; e < d * d; ++e) g[e] = make_double2(nan, nan);
@@ -167,8 +167,9 @@ static void launch_partial(dim3 grid, const double* t, int nt, const double* s, 
                            double radius, const double2* Ek, int64_t ld_ek, int ncols, int sps, double2* part,
                            cudaStream_t st) {
   count_launch();
-  propagate_partial_kernel<KIND, RT, DF><<<grid, 256, 0, st>>>(t, nt, s, ns, k0, reg, radius, Ek, ld_ek, ncols, sps,
-                                                              part);
+  prepare_green<KIND>(st);
+  propagate_partial_kernel<KIND, RT, DF><<<grid, 256, 0, st>>>(t, nt, s, ns, k0, 1.0 / k0, reg, radius, Ek, ld_ek,
+                                                              ncols, sps, part);
 }
 
 template <int KIND, bool DF>
