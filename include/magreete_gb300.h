@@ -274,12 +274,13 @@ int mgt_refine_norms(const void* M, int64_t ldm, int64_t n, const void* B, int64
 /*
  * Propagation to detectors:
  *   out[m*d + a, r] = coef * sum_{j,b} G_ab(t_m - s_j) Ek[j*d + b, r] + E0[m*d + a, r]
- * dtype MGT_C128 (the plain method): matrix-free, G is recomputed on the fly
- * in FP64 and contracted in FP64, never stored.  MGT_CDF (the mixed method):
- * the rows -coef G are evaluated in FP64, stored double-float in chunks of at
- * most 1 GiB of the workspace and contracted with Ek by the tensor-core
- * residual kernel (out = E0 - (-coef G) Ek; see mgt_residual), or in
- * double-float on the FP32 pipes where the tensor cores are unavailable.
+ * The rows -coef G are evaluated in FP64 in chunks of at most 1 GiB of the
+ * workspace and contracted with Ek on the tensor cores.  dtype MGT_C128 (the
+ * plain method): 64 columns of K at a time with FP64 accuracy, summed in FP64;
+ * small calls are matrix-free instead (G recomputed on the fly and contracted
+ * in FP64).  MGT_CDF (the mixed method): by the residual kernel (out = E0 -
+ * (-coef G) Ek; see mgt_residual), or in double-float on the FP32 pipes where
+ * the tensor cores are unavailable.
  * Ek, E0 and out are complex128 in both cases.  Replaces the dense
  * G0(points) + matmul of propagate() (Transmission2D.py:190, :701;
  * Transmission3D.py:163, :675) and propagate_ss().  Rows where the

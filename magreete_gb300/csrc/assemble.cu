@@ -37,7 +37,7 @@ __device__ __forceinline__ void store_entry(const OutSpec& o, int64_t row, int64
 // (1 - shift) * I for i == j.
 template <int KIND>
 __global__ void __launch_bounds__(kAsmThreads)
-assemble_system_kernel(const double* __restrict__ pts, int n, double k0, double ik0, double2 coef,
+assemble_system_kernel(const double* __restrict__ pts, int n, double k0, double2 coef,
                        double2 diag, OutSpec o1, OutSpec o2) {
   constexpr int dim = Kind<KIND>::dim, d = Kind<KIND>::d;
   int j = blockIdx.x * kAsmThreads + threadIdx.x;
@@ -60,7 +60,7 @@ assemble_system_kernel(const double* __restrict__ pts, int n, double k0, double 
 #pragma unroll
       for (int c = 0; c < dim; ++c) r[c] = pts[(int64_t)i * dim + c] - sj[c];
       // distinct scatterers at the same position give the reference a NaN block
-      if (!green_block<KIND>(r, k0, ik0, false, 0.0, g)) {
+      if (!green_block<KIND>(r, k0, false, 0.0, g)) {
 #pragma unroll
         for (int q = 0; q < d * d; ++q)
           g[q] = make_double2(__longlong_as_double(0x7ff8000000000000ll), __longlong_as_double(0x7ff8000000000000ll));
@@ -98,7 +98,7 @@ constexpr int kSymTP = 16;
 
 template <int KIND, bool MIXED>
 __global__ void __launch_bounds__(kSymTP * kSymTP)
-assemble_system_sym_kernel(const double* __restrict__ pts, int n, double k0, double ik0, double2 coef, double2 diag,
+assemble_system_sym_kernel(const double* __restrict__ pts, int n, double k0, double2 coef, double2 diag,
                            OutSpec o1, OutSpec o2) {
   constexpr int dim = Kind<KIND>::dim, d = Kind<KIND>::d;
   constexpr int TP = kSymTP, W = TP * d;          // tile side in matrix rows / columns
@@ -119,7 +119,7 @@ assemble_system_sym_kernel(const double* __restrict__ pts, int n, double k0, dou
       double r[dim];
 #pragma unroll
       for (int c = 0; c < dim; ++c) r[c] = pts[(int64_t)i * dim + c] - pts[(int64_t)j * dim + c];
-      if (!green_block<KIND>(r, k0, ik0, false, 0.0, g)) {
+      if (!green_block<KIND>(r, k0, false, 0.0, g)) {
 #pragma unroll
         for (int e = 0; e < d * d; ++e)
           g[e] = make_double2(__longlong_as_double(0x7ff8000000000000ll), __longlong_as_double(0x7ff8000000000000ll));
@@ -178,7 +178,7 @@ assemble_system_sym_kernel(const double* __restrict__ pts, int n, double k0, dou
 template <int KIND, bool TRANSPOSE>
 __global__ void __launch_bounds__(kAsmThreads)
 assemble_propagator_kernel(const double* __restrict__ tgt, int nt, const double* __restrict__ src,
-                           int ns, double k0, double ik0, double2 coef, bool regularize, double radius,
+                           int ns, double k0, double2 coef, bool regularize, double radius,
                            int nan_policy, double2 fill, OutSpec out) {
   constexpr int dim = Kind<KIND>::dim, d = Kind<KIND>::d;
   int ncol = TRANSPOSE ? nt : ns, nrow = TRANSPOSE ? ns : nt;
@@ -200,7 +200,7 @@ assemble_propagator_kernel(const double* __restrict__ tgt, int nt, const double*
       r[c] = TRANSPOSE ? (cq[c] - rp) : (rp - cq[c]);  // always target - source
     }
     double2 g[d * d];
-    if (green_block<KIND>(r, k0, ik0, regularize, radius, g)) {
+    if (green_block<KIND>(r, k0, regularize, radius, g)) {
 #pragma unroll
       for (int e = 0; e < d * d; ++e) {
         double2 v = g[e];
@@ -230,24 +230,23 @@ static cudaError_t launch_system(const double* pts, int n, double k0, double2 co
                                  OutSpec o1, OutSpec o2, cudaStream_t s) {
   const cudaError_t pe = prepare_green<KIND>(s);
   if (pe != cudaSuccess) return pe;
-  const double ik0 = 1.0 / k0;
   if (g_sym_assembly.load(std::memory_order_relaxed)) {
     constexpr int d = Kind<KIND>::d;
     const int nb = (n + kSymTP - 1) / kSymTP;
     if (nb <= 65535) {
       const size_t smem = (size_t)kSymTP * kSymTP * d * d * sizeof(double2);
       if (o1.dtype == MGT_CDF && o2.p && o2.dtype == MGT_C64)
-        assemble_system_sym_kernel<KIND, true><<<dim3(nb, nb), kSymTP * kSymTP, smem, s>>>(pts, n, k0, ik0, coef, diag,
+        assemble_system_sym_kernel<KIND, true><<<dim3(nb, nb), kSymTP * kSymTP, smem, s>>>(pts, n, k0, coef, diag,
                                                                                          o1, o2);
       else
-        assemble_system_sym_kernel<KIND, false><<<dim3(nb, nb), kSymTP * kSymTP, smem, s>>>(pts, n, k0, ik0, coef,
+        assemble_system_sym_kernel<KIND, false><<<dim3(nb, nb), kSymTP * kSymTP, smem, s>>>(pts, n, k0, coef,
                                                                                           diag, o1, o2);
       count_launch();
       return cudaGetLastError();
     }
   }
   dim3 grid((n + kAsmThreads - 1) / kAsmThreads, (n + kAsmRows - 1) / kAsmRows);
-  assemble_system_kernel<KIND><<<grid, kAsmThreads, 0, s>>>(pts, n, k0, ik0, coef, diag, o1, o2);
+  assemble_system_kernel<KIND><<<grid, kAsmThreads, 0, s>>>(pts, n, k0, coef, diag, o1, o2);
   count_launch();
   return cudaGetLastError();
 }
@@ -264,14 +263,13 @@ static cudaError_t launch_prop(const double* t, int nt, const double* src, int n
                                int transpose, OutSpec out, cudaStream_t s) {
   const cudaError_t pe = prepare_green<KIND>(s);
   if (pe != cudaSuccess) return pe;
-  const double ik0 = 1.0 / k0;
   int ncol = transpose ? nt : ns, nrow = transpose ? ns : nt;
   dim3 grid((ncol + kAsmThreads - 1) / kAsmThreads, (nrow + kAsmRows - 1) / kAsmRows);
   count_launch();
   if (transpose)
-    assemble_propagator_kernel<KIND, true><<<grid, kAsmThreads, 0, s>>>(t, nt, src, ns, k0, ik0, coef, reg, radius, nanp, fill, out);
+    assemble_propagator_kernel<KIND, true><<<grid, kAsmThreads, 0, s>>>(t, nt, src, ns, k0, coef, reg, radius, nanp, fill, out);
   else
-    assemble_propagator_kernel<KIND, false><<<grid, kAsmThreads, 0, s>>>(t, nt, src, ns, k0, ik0, coef, reg, radius, nanp, fill, out);
+    assemble_propagator_kernel<KIND, false><<<grid, kAsmThreads, 0, s>>>(t, nt, src, ns, k0, coef, reg, radius, nanp, fill, out);
   return cudaGetLastError();
 }
 

@@ -8,7 +8,7 @@
 //   3D sca (Transmission3D.py:573-601): e^{ikR}/(4 pi R)
 // with H_nu from hankel.cuh.  FP64 operations are what these cost (1.7 a clock
 // and SM), so each block is formed from its two scalar coefficients -- the
-// identity's and the projector's -- and one reciprocal, 1 / R.
+// identity's and the projector's.
 #pragma once
 #include "common.cuh"
 #include "hankel.cuh"
@@ -27,11 +27,11 @@ static inline cudaError_t prepare_green(cudaStream_t s) {
   return Kind<KIND>::dim == 2 ? hk::ensure_table(s) : cudaSuccess;
 }
 
-// d x d Green's block for separation r (row-major in g); ik0 = 1 / k0.
+// d x d Green's block for separation r (row-major in g).
 // Returns false where the reference's value is NaN: R == 0, or R (k*R for the
 // 2D TE kind) below `radius` when regularising.
 template <int KIND>
-__device__ __forceinline__ bool green_block(const double* r, double k0, double ik0, bool regularize,
+__device__ __forceinline__ bool green_block(const double* r, double k0, bool regularize,
                                             double radius, double2* g) {
   constexpr double kPi = 3.14159265358979323846;
   if constexpr (KIND == MGT_2D_VECTOR) {
@@ -40,7 +40,7 @@ __device__ __forceinline__ bool green_block(const double* r, double k0, double i
     double kR = k0 * R;
     if (regularize && kR < radius) kR = 0.0;
     if (R2 == 0.0 || kR == 0.0) return false;
-    const double iR = __drcp_rn(R), ikR = iR * ik0, q = iR * iR;
+    const double ikR = __drcp_rn(kR), q = __drcp_rn(R2);
     double2 h0, h1;
     hk::hankel01<true>(kR, h0, h1);
     h1.x *= ikR;
@@ -67,10 +67,10 @@ __device__ __forceinline__ bool green_block(const double* r, double k0, double i
     double R = sqrt(R2);
     if (regularize && R < radius) R = 0.0;
     if (R2 == 0.0 || R == 0.0) return false;
-    const double iR = __drcp_rn(R), kR = k0 * R, inv = iR * ik0, q = iR * iR;
+    const double kR = k0 * R, inv = __drcp_rn(kR), q = __drcp_rn(R2);
     double s, c;
     sincos(kR, &s, &c);
-    const double amp = iR * (1.0 / (4.0 * kPi));
+    const double amp = __drcp_rn(4.0 * kPi * R);
     const double er = c * amp, ei = s * amp;
     // f = 1/(ikR) + 1/(kR)^2 = inv^2 - i inv; identity 1 - f, projector -(1 - 3 f)
     const double fr = inv * inv, dr = 1.0 - fr, pr = fma(3.0, fr, -1.0), pi = -3.0 * inv;
@@ -91,7 +91,7 @@ __device__ __forceinline__ bool green_block(const double* r, double k0, double i
     if (R == 0.0) return false;
     double s, c;
     sincos(k0 * R, &s, &c);
-    const double amp = __drcp_rn(R) * (1.0 / (4.0 * kPi));
+    const double amp = __drcp_rn(4.0 * kPi * R);
     g[0] = make_double2(c * amp, s * amp);
     return true;
   }

@@ -4,16 +4,20 @@
 //
 // The reference builds the dense (d*M x d*N) G0(points) and multiplies
 // (propagate(): Transmission2D.py:190, :701; Transmission3D.py:163, :675).
-// Here each CTA owns 16 detectors and all (up to 64) right-hand-side
-// columns of one source range: it evaluates the 16 x 8 Green's blocks of a
-// source chunk in FP64 into shared memory, stages the matching Ek rows, and
-// contracts in FP64.  Source ranges are split across CTAs for parallelism; a
-// second kernel sums the partials in FP64 and applies coef and E0.  That is
-// the plain method.  The fast method (MGT_CDF) assembles the propagator rows
-// in FP64 once, stored double-float, and contracts them with the residual
-// kernel in double-float on the FP32 pipes: each Green's block is evaluated
-// once for all right-hand sides, and the FP64 evaluation no longer stalls the
-// contraction.
+// Three ways:
+//  * plain method, from kPropTcMinFma on: the rows -coef G are evaluated in FP64
+//    in chunks of at most 1 GiB and contracted with Ek by the FP64-accurate
+//    tensor-core products of zgemm_tc.cu, 64 columns of K each, summed in FP64.
+//    Scaling each row per 64 columns keeps the accuracy of an FP64 sum for rows
+//    with one source much nearer than the others.
+//  * plain method, small calls: matrix-free.  Each CTA owns 16 detectors and all
+//    (up to 64) right-hand-side columns of one source range: it evaluates the
+//    16 x 8 Green's blocks of a source chunk in FP64 into shared memory, stages
+//    the matching Ek rows, and contracts in FP64.  Source ranges are split across
+//    CTAs; a second kernel sums the partials in FP64 and applies coef and E0.
+//  * mixed method: the assembled rows in one digit-split product over all of K
+//    (residual_tc.cu, one scale per row); in double-float on the FP32 pipes where
+//    the tensor cores are unavailable.
 #include <algorithm>
 #include <mutex>
 #include <type_traits>
@@ -23,6 +27,7 @@
 #include "green.cuh"
 #include "diag.cuh"
 #include "residual_tc.cuh"
+#include "zgemm_tc.cuh"
 
 namespace mgt {
 
@@ -51,7 +56,7 @@ template <> struct Acc<true> {
 template <int KIND, int RT, bool DF>
 __global__ void __launch_bounds__(256)
 propagate_partial_kernel(const double* __restrict__ tgt, int nt, const double* __restrict__ src, int ns, double k0,
-                         double ik0, bool regularize, double radius, const double2* __restrict__ Ek, int64_t ld_ek, int ncols,
+                         bool regularize, double radius, const double2* __restrict__ Ek, int64_t ld_ek, int ncols,
                          int src_per_split, double2* __restrict__ partial) {
   constexpr int d = Kind<KIND>::d, dim = Kind<KIND>::dim;
   constexpr int ROWS = kPT * d, KC = kPJ * d;
@@ -81,7 +86,7 @@ propagate_partial_kernel(const double* __restrict__ tgt, int nt, const double* _
         double r[dim];
 #pragma unroll
         for (int c = 0; c < dim; ++c) r[c] = tpos[tt][c] - src[(int64_t)j * dim + c];
-        if (!green_block<KIND>(r, k0, ik0, regularize, radius, g)) {
+        if (!green_block<KIND>(r, k0, regularize, radius, g)) {
           const double nan = __longlong_as_double(0x7ff8000000000000ll);
 #pragma unroll
           for (int e = 0; e < d * d; ++e) g[e] = make_double2(nan, nan);
@@ -168,7 +173,7 @@ static void launch_partial(dim3 grid, const double* t, int nt, const double* s, 
                            cudaStream_t st) {
   count_launch();
   prepare_green<KIND>(st);
-  propagate_partial_kernel<KIND, RT, DF><<<grid, 256, 0, st>>>(t, nt, s, ns, k0, 1.0 / k0, reg, radius, Ek, ld_ek,
+  propagate_partial_kernel<KIND, RT, DF><<<grid, 256, 0, st>>>(t, nt, s, ns, k0, reg, radius, Ek, ld_ek,
                                                               ncols, sps, part);
 }
 
@@ -229,6 +234,25 @@ static size_t prop_df_bytes(int64_t nt, int64_t ns, int64_t nrhs, int d) {
 static bool prop_tc_ok(int64_t nt, int64_t ns, int64_t nrhs, int d) {
   return residual_tc_supported(prop_chunk_targets(nt, ns, d) * d, (int64_t)d * ns, nrhs);
 }
+// Plain method: FP64 multiply-adds of the matrix-free kernel (its column tiles are 16, 32 or 64 wide) above
+// which the assembled way is faster.  The FP64 pipes do 254 a clock; the assembled way takes two launches per
+// 64 columns of K, about 20 us.
+constexpr double kPropTcMinFma = 6e7;
+static bool prop_z_pays(int64_t nt, int64_t ns, int64_t nrhs, int d) {
+  return 4.0 * d * d * (double)nt * (double)ns * (double)((nrhs + 15) / 16 * 16) >= kPropTcMinFma &&
+         (int64_t)d * nt <= (1 << 28) && nrhs <= (1 << 16);
+}
+// targets per chunk: rows, their digits and the partial products within about 1 GiB each
+static int64_t prop_z_targets(int64_t nt, int64_t ns, int64_t nrhs, int d) {
+  const int64_t slabs = (d * ns + kZK - 1) / kZK;
+  const int64_t per = std::max((int64_t)d * d * ns * 16, (int64_t)d * slabs * nrhs * 16);
+  return std::max<int64_t>(1, std::min<int64_t>(nt, (int64_t)kPropChunkBytes / per));
+}
+static size_t prop_z_bytes(int64_t nt, int64_t ns, int64_t nrhs, int d) {
+  if (!prop_z_pays(nt, ns, nrhs, d)) return 0;
+  const int64_t ct = prop_z_targets(nt, ns, nrhs, d);
+  return (size_t)ct * d * d * ns * sizeof(double2) + zgemm_wide_bytes(ct * d, nrhs, (int64_t)d * ns) + 1024;
+}
 static size_t prop_tc_bytes(int64_t nt, int64_t ns, int64_t nrhs, int d) {
   if (!prop_tc_ok(nt, ns, nrhs, d)) return 0;
   return prop_chunk_bytes(nt, ns, d) +
@@ -258,7 +282,8 @@ extern "C" int mgt_propagate_workspace_bytes(int kind, int64_t n_targets, int64_
   // the larger of the two methods' needs: FP64 partial sums, or the
   // double-float copy of Ek plus one chunk of assembled propagator rows
   *bytes = std::max({(size_t)nsplit * n_targets * d * std::min<int64_t>(nrhs, kPCols) * sizeof(double2),
-                     prop_df_bytes(n_targets, n_sources, nrhs, d), prop_tc_bytes(n_targets, n_sources, nrhs, d)});
+                     prop_df_bytes(n_targets, n_sources, nrhs, d), prop_tc_bytes(n_targets, n_sources, nrhs, d),
+                     prop_z_bytes(n_targets, n_sources, nrhs, d)});
   return MGT_OK;
 }
 
@@ -278,12 +303,30 @@ extern "C" int mgt_propagate(int kind, int dtype, const double* targets, int64_t
   if (work_bytes < need) return MGT_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
   const int nt = (int)n_targets, ns = (int)n_sources;
+  if (dtype == MGT_C128 && prop_z_pays(nt, ns, nrhs, d)) {
+    const int64_t ct = prop_z_targets(nt, ns, nrhs, d);
+    double2* Gc = (double2*)work;
+    void* zw = (char*)work + (size_t)ct * d * d * ns * sizeof(double2);
+    const double2 mcoef = make_double2(-coef_re, -coef_im);
+    const int kd = d * ns;
+    int e = MGT_OK;
+    for (int64_t t0 = 0; t0 < nt && e == MGT_OK; t0 += ct) {
+      const int tc = (int)std::min<int64_t>(ct, nt - t0);
+      e = assemble_propagator_into(kind, targets + t0 * dim, tc, sources, ns, k0, mcoef, regularize != 0, radius,
+                                   MGT_NAN_KEEP, make_double2(0.0, 0.0), 0, Gc, kd, MGT_C128, st);
+      if (e == MGT_OK)
+        e = zgemm_wide(Gc, kd, tc * d, (const double2*)Ek, ld_ek, (int)nrhs, kd,
+                       E0 ? (const double2*)E0 + t0 * d * ld_e0 : nullptr, ld_e0, (double2*)out + t0 * d * ld_out,
+                       ld_out, zw, st);
+    }
+    return e;
+  }
   if (dtype == MGT_CDF && prop_tc_ok(nt, ns, nrhs, d)) {
-    // propagator rows (-coef G, double-float) contracted on the tensor cores:
+    // propagator rows (-coef G, complex128) contracted on the tensor cores:
     // out = E0 - (-coef G) Ek; rows with NaN blocks (a detector on a scatterer)
     // come out NaN for the host's fix-up
     const int64_t ct = prop_chunk_targets(nt, ns, d);
-    float4* Gc = (float4*)work;
+    double2* Gc = (double2*)work;
     char* tw = (char*)work + ((prop_chunk_bytes(nt, ns, d) + 1023) & ~size_t(1023));
     const size_t tw_bytes = work_bytes - (size_t)(tw - (char*)work);
     const double2 mcoef = make_double2(-coef_re, -coef_im);
@@ -292,7 +335,7 @@ extern "C" int mgt_propagate(int kind, int dtype, const double* targets, int64_t
     for (int64_t t0 = 0; t0 < nt && e == MGT_OK; t0 += ct) {
       const int tc = (int)std::min<int64_t>(ct, nt - t0);
       e = assemble_propagator_into(kind, targets + t0 * dim, tc, sources, ns, k0, mcoef, regularize != 0, radius,
-                                   MGT_NAN_KEEP, nanfill, 0, Gc, (int64_t)d * ns, MGT_CDF, st);
+                                   MGT_NAN_KEEP, nanfill, 0, Gc, (int64_t)d * ns, MGT_C128, st);
       if (e != MGT_OK) break;
       const double2* b = E0 ? (const double2*)E0 + t0 * d * ld_e0 : nullptr;
       e = residual_tc(Gc, (int64_t)d * ns, tc * d, d * ns, (const double2*)Ek, ld_ek, (int)nrhs, b, ld_e0,

@@ -139,10 +139,48 @@ __device__ __forceinline__ uint2 widen4(uint32_t x) {
   return make_uint2(*reinterpret_cast<const uint32_t*>(&d0), *reinterpret_cast<const uint32_t*>(&d1));
 }
 
-// row exponent of a row holding a NaN or an infinity: its outputs are NaN
-constexpr int kRowNonFinite = 0x40000000;
+// exponent of a row of M, or a column of X, holding a NaN or an infinity: its outputs are NaN
+constexpr int kNonFinite = 0x40000000;
 
-__device__ __forceinline__ int clamp_exp(int e) { return (e < -300 || e > 300) ? 0 : e; }
+__device__ __forceinline__ int clamp_exp(int e) { return (e < -1200 || e > 1200) ? 0 : e; }
+
+// (re, im) of an entry as integers round(v 2^(FIX - e)), 2^e above the row's largest part
+__device__ __forceinline__ void entry_fixed(float4 v, int e, long long& re, long long& im) {
+  re = fixed_point(v.x, FIX - e) + fixed_low(v.y, FIX - e);
+  im = fixed_point(v.z, FIX - e) + fixed_low(v.w, FIX - e);
+}
+__device__ __forceinline__ long long fixed_double(double v, int e) {
+  const long long b = __double_as_longlong(v);
+  const int ex = (int)((b >> 52) & 0x7ff);
+  long long m = b & 0xFFFFFFFFFFFFFll;
+  if (ex) m |= 1ll << 52;
+  const int sh = min(max(ex, 1) - 1075 + FIX - e, 1);
+  const long long r = sh >= 0 ? m << sh : sh > -54 ? (m + (1ll << (-sh - 1))) >> (-sh) : 0ll;
+  return b < 0 ? -r : r;
+}
+__device__ __forceinline__ void entry_fixed(double2 v, int e, long long& re, long long& im) {
+  re = fixed_double(v.x, e);
+  im = fixed_double(v.y, e);
+}
+// size of an entry as an ordered integer: the bits of its larger high part, or exponent field
+__device__ __forceinline__ uint32_t entry_size(float4 v) {
+  return max(__float_as_uint(fabsf(v.x)), __float_as_uint(fabsf(v.z)));
+}
+__device__ __forceinline__ uint32_t entry_size(double2 v) {
+  return (uint32_t)max((__double2hiint(v.x) >> 20) & 0x7ff, (__double2hiint(v.y) >> 20) & 0x7ff);
+}
+// e with 2^e above every entry of at most that size
+__device__ __forceinline__ int size_exponent(uint32_t m, float4) {
+  int e = 0;
+  if (m >= 0x7F800000u) return kNonFinite;
+  if (m != 0u) frexpf(__uint_as_float(m), &e);
+  return e;
+}
+__device__ __forceinline__ int size_exponent(uint32_t m, double2) {
+  return m == 2047u ? kNonFinite : (int)max(m, 1u) - 1022;
+}
+__device__ __forceinline__ float4 zero_of(float4) { return make_float4(0.f, 0.f, 0.f, 0.f); }
+__device__ __forceinline__ double2 zero_of(double2) { return make_double2(0.0, 0.0); }
 
 // Byte offset of real K index kr (even) of row rho in a 128-row tile whose rows
 // are 128-byte lines (64 fp16), 8-row groups 1024 B apart, 16-byte chunks
@@ -314,17 +352,24 @@ residual_tc_kernel(const unsigned char* __restrict__ D, int rows, const int* __r
     }
     const int row = row0 + r;
     if (row < rows) {
-      const bool good = ok && !*abort && row_exp[row] != kRowNonFinite;
+      const bool good = ok && !*abort && row_exp[row] != kNonFinite;
       const int ea = rexp[r];
 #pragma unroll
       for (int jc = 0; jc < EPI_COLS / 2; ++jc) {
         const int col = ct * BNC + part * (EPI_COLS / 2) + jc;
         if (col < ncols) {
           double2 val;
-          if (good) {
-            // 2^sc, sc in [-648, 552]: a normal double
-            const double sc = __longlong_as_double((long long)(ea + clamp_exp(col_exp[col]) - 48 + 1023) << 52);
-            val = make_double2((double)acc[2 * jc] * sc, (double)acc[2 * jc + 1] * sc);
+          if (good && col_exp[col] != kNonFinite) {
+            const int e = ea + clamp_exp(col_exp[col]) - 48;
+            val = make_double2((double)acc[2 * jc], (double)acc[2 * jc + 1]);
+            if (e > -900 && e < 900) {
+              const double sc = __longlong_as_double((long long)(e + 1023) << 52);
+              val.x *= sc;
+              val.y *= sc;
+            } else {
+              val.x = ldexp(val.x, e);
+              val.y = ldexp(val.y, e);
+            }
           } else {
             val = make_double2(__longlong_as_double(0x7FF8000000000000LL),
                                __longlong_as_double(0x7FF8000000000000LL));
@@ -376,21 +421,17 @@ residual_tc_kernel(const unsigned char* __restrict__ D, int rows, const int* __r
   }
 }
 
-// e_i of each row: 2^e_i bounds the row's largest |re|, |im| (hi parts); one
-// warp per row.  Rows with a NaN or an infinity get kRowNonFinite.
-__global__ void rowexp_kernel(const float4* __restrict__ M, int64_t ldm, int rows, int kdim, int* __restrict__ out) {
+// e_i of each row: 2^e_i bounds the row's largest |re|, |im|; one warp per
+// row.  Rows with a NaN or an infinity get kNonFinite.  V: float4 (double-float)
+// or double2 (complex128).
+template <typename V>
+__global__ void rowexp_kernel(const V* __restrict__ M, int64_t ldm, int rows, int kdim, int* __restrict__ out) {
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= rows) return;
   uint32_t m = 0;
-  for (int k = lane; k < kdim; k += 32) {
-    const float4 v = __ldg(&M[(int64_t)row * ldm + k]);
-    m = max(m, max(__float_as_uint(fabsf(v.x)), __float_as_uint(fabsf(v.z))));
-  }
+  for (int k = lane; k < kdim; k += 32) m = max(m, entry_size(__ldg(&M[(int64_t)row * ldm + k])));
   m = __reduce_max_sync(0xffffffffu, m);
-  int e = 0;
-  if (m >= 0x7F800000u) e = kRowNonFinite;
-  else if (m != 0u) frexpf(__uint_as_float(m), &e);
-  if (lane == 0) out[row] = e;
+  if (lane == 0) out[row] = size_exponent(m, V());
 }
 
 // Byte p (0 = lowest) of each of four 64-bit words, packed low to high.
@@ -408,8 +449,9 @@ __device__ __forceinline__ uint32_t pick_bytes(const long long* y, int p) {
 // (rho, kr) of a slice at rho * 64 + (((kr >> 3) ^ (rho & 7)) << 3) + (kr & 7):
 // the swizzled fp16 operand layout at half width.  Zeros beyond rows and kdim.
 // Thread = (row, 8 real K = 4 complex entries), four per thread.
+template <typename V>
 __global__ void __launch_bounds__(256)
-digitize_kernel(const float4* __restrict__ M, int64_t ldm, int rows, int kdim, const int* __restrict__ row_exp,
+digitize_kernel(const V* __restrict__ M, int64_t ldm, int rows, int kdim, const int* __restrict__ row_exp,
                 unsigned char* __restrict__ D, int nch) {
   const int c = blockIdx.x, rt = blockIdx.y;
   unsigned char* blk = D + ((size_t)rt * nch + c) * DIG * D_SLICE;
@@ -417,14 +459,15 @@ digitize_kernel(const float4* __restrict__ M, int64_t ldm, int rows, int kdim, c
   for (int t = threadIdx.x; t < BM * 8; t += 256) {
     const int rho = t >> 3, grp = t & 7, row = rt * BM + rho;
     const bool rin = row < rows;
-    const int sh = FIX - (rin ? clamp_exp(row_exp[row]) : 0);
+    const int ex = rin ? clamp_exp(row_exp[row]) : 0;
     long long y[8];
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const int kc = c * KCC + grp * 4 + e;
-      const float4 v = (rin && kc < kdim) ? __ldg(&M[(int64_t)row * ldm + kc]) : make_float4(0.f, 0.f, 0.f, 0.f);
-      y[2 * e] = fixed_point(v.x, sh) + fixed_low(v.y, sh) + BIAS;
-      y[2 * e + 1] = fixed_point(v.z, sh) + fixed_low(v.w, sh) + BIAS;
+      const V v = (rin && kc < kdim) ? __ldg(&M[(int64_t)row * ldm + kc]) : zero_of(V());
+      entry_fixed(v, ex, y[2 * e], y[2 * e + 1]);
+      y[2 * e] += BIAS;
+      y[2 * e + 1] += BIAS;
     }
     const uint32_t off = (uint32_t)rho * 64u + ((uint32_t)(grp ^ (rho & 7)) << 3);
 #pragma unroll
@@ -440,22 +483,24 @@ digitize_kernel(const float4* __restrict__ M, int64_t ldm, int rows, int kdim, c
 // (the output starts at a large negative value).
 __global__ void colexp_kernel(const double2* __restrict__ X, int64_t ldx, int kdim, int ncols, int* __restrict__ out) {
   const int j = blockIdx.x * 32 + (threadIdx.x & 31), ty = threadIdx.x >> 5;
-  __shared__ double red[8][32];
-  double m = 0.0;
+  __shared__ uint32_t red[8][32];
+  uint32_t m = 0;      // largest exponent field (no FP64 comparisons: their pipe is slow)
+  bool any = false;
   if (j < ncols)
     for (int k = blockIdx.y * 8 + ty; k < kdim; k += gridDim.y * 8) {
       const double2 x = X[(int64_t)k * ldx + j];
-      m = fmax(m, fmax(fabs(x.x), fabs(x.y)));
+      any |= ((__double_as_longlong(x.x) | __double_as_longlong(x.y)) << 1) != 0;
+      m = max(m, entry_size(x));
     }
-  red[ty][threadIdx.x & 31] = m;
+  red[ty][threadIdx.x & 31] = m | (any ? 0x8000u : 0u);
   __syncthreads();
   if (ty == 0 && j < ncols) {
-    for (int t = 1; t < 8; ++t) m = fmax(m, red[t][threadIdx.x & 31]);
-    if (m > 0.0) {
-      int e = 0;
-      frexp(m, &e);
-      atomicMax(&out[j], e);
+    uint32_t a = any ? 0x8000u : 0u;
+    for (int t = 1; t < 8; ++t) {
+      m = max(m, red[t][threadIdx.x & 31] & 0x7fffu);
+      a |= red[t][threadIdx.x & 31] & 0x8000u;
     }
+    if (a) atomicMax(&out[j], size_exponent(m, double2()));
   }
 }
 
@@ -475,7 +520,7 @@ __global__ void bdigits_kernel(const double2* __restrict__ X, int64_t ldx, int k
     e = clamp_exp(col_exp[j]);
     if (k < kdim) x = X[(int64_t)k * ldx + j];
   }
-  const long long xr = __double2ll_rn(ldexp(x.x, FIX - e)), xi = __double2ll_rn(ldexp(x.y, FIX - e));
+  const long long xr = fixed_double(x.x, e), xi = fixed_double(x.y, e);
   const long long yr = xr + BIAS, yi = xi + BIAS, yn = BIAS - xi;
   const int ctile = j / BNC, jj = j % BNC, c = k / KCC, kk = k % KCC;
   unsigned char* blk = out + ((size_t)ctile * nch + c) * B_BLOCK;
@@ -574,17 +619,20 @@ size_t residual_tc_workspace_bytes(int64_t rows, int64_t kdim, int64_t ncols) {
          residual_tc_apply_bytes(rows, kdim, ncols);
 }
 
-int residual_tc_prepare(const float4* M, int64_t ldm, int rows, int kdim, int* rowexp, unsigned char* digits,
+template <typename V>
+int residual_tc_prepare(const V* M, int64_t ldm, int rows, int kdim, int* rowexp, unsigned char* digits,
                         cudaStream_t s) {
   using namespace rtc;
   if (!residual_tc_supported(rows, kdim, 1)) return MGT_ERR_UNSUPPORTED;
   if (!M || !rowexp || !digits || ((uintptr_t)digits & 15)) return MGT_ERR_ARG;
   const int nch = (kdim + KCC - 1) / KCC;
   count_launch(2);
-  rowexp_kernel<<<(rows + 7) / 8, 256, 0, s>>>(M, ldm, rows, kdim, rowexp);
-  digitize_kernel<<<dim3(nch, (rows + BM - 1) / BM), 256, 0, s>>>(M, ldm, rows, kdim, rowexp, digits, nch);
+  rowexp_kernel<V><<<(rows + 7) / 8, 256, 0, s>>>(M, ldm, rows, kdim, rowexp);
+  digitize_kernel<V><<<dim3(nch, (rows + BM - 1) / BM), 256, 0, s>>>(M, ldm, rows, kdim, rowexp, digits, nch);
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }
+template int residual_tc_prepare(const float4*, int64_t, int, int, int*, unsigned char*, cudaStream_t);
+template int residual_tc_prepare(const double2*, int64_t, int, int, int*, unsigned char*, cudaStream_t);
 
 int residual_tc_apply(const unsigned char* digits, const int* rowexp, int rows, int kdim, const double2* X,
                       int64_t ldx, int ncols, const double2* B, int64_t ldb, double2* R, int64_t ldr, void* work,
@@ -630,7 +678,8 @@ size_t residual_tc_split(void* work, int64_t rows, int64_t kdim, int** rowexp, u
   return a_off;
 }
 
-int residual_tc(const float4* M, int64_t ldm, int rows, int kdim, const double2* X, int64_t ldx, int ncols,
+template <typename V>
+int residual_tc(const V* M, int64_t ldm, int rows, int kdim, const double2* X, int64_t ldx, int ncols,
                 const double2* B, int64_t ldb, double2* R, int64_t ldr, void* work, size_t work_bytes,
                 cudaStream_t s) {
   if (!residual_tc_supported(rows, kdim, ncols)) return MGT_ERR_UNSUPPORTED;
@@ -643,6 +692,10 @@ int residual_tc(const float4* M, int64_t ldm, int rows, int kdim, const double2*
   if (e != MGT_OK) return e;
   return residual_tc_apply(digits, rowexp, rows, kdim, X, ldx, ncols, B, ldb, R, ldr, aw, work_bytes - a_off, s);
 }
+template int residual_tc(const float4*, int64_t, int, int, const double2*, int64_t, int, const double2*, int64_t, double2*,
+                         int64_t, void*, size_t, cudaStream_t);
+template int residual_tc(const double2*, int64_t, int, int, const double2*, int64_t, int, const double2*, int64_t,
+                         double2*, int64_t, void*, size_t, cudaStream_t);
 
 
 }  // namespace mgt

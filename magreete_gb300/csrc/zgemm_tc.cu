@@ -130,6 +130,13 @@ __device__ __forceinline__ uint2 widen4(uint32_t x) {
   return make_uint2(*reinterpret_cast<const uint32_t*>(&d0), *reinterpret_cast<const uint32_t*>(&d1));
 }
 
+// Distances between the slabs of a product over more than 64 columns of K: digit
+// bytes, exponents, and elements of the output.
+struct Slabs {
+  size_t adig = 0, bdig = 0, aexp = 0, bexp = 0, c = 0;
+  int tiles = 1 << 30;   // tiles per slab
+};
+
 // Operand digits, both operands in one launch: blocks [0, ablocks) take 32 rows
 // of A each, the others 32 columns of B.  A: byte slices (row tile, chunk,
 // digit) at half the width of the swizzled FP16 operand; B: the swizzled FP16
@@ -142,8 +149,16 @@ __device__ __forceinline__ uint2 widen4(uint32_t x) {
 __global__ void __launch_bounds__(256)
 digits_kernel(const double2* __restrict__ A, int64_t lda, int M, int ablocks, const double2* __restrict__ B,
               int64_t ldb, int N, int K, const int* __restrict__ kexp, unsigned char* __restrict__ adig,
-              int* __restrict__ aexp, unsigned char* __restrict__ bdig, int* __restrict__ bexp) {
+              int* __restrict__ aexp, unsigned char* __restrict__ bdig, int* __restrict__ bexp, Slabs sl) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // slab blockIdx.y: columns 64 y .. of A, rows 64 y .. of B, its own digits and scales
+  A += (int64_t)blockIdx.y * kZK;
+  B += (int64_t)blockIdx.y * kZK * ldb;
+  adig += blockIdx.y * sl.adig;
+  aexp += blockIdx.y * sl.aexp;
+  bdig += blockIdx.y * sl.bdig;
+  bexp += blockIdx.y * sl.bexp;
+  K = min(kZK, K - (int)blockIdx.y * kZK);
   const bool rows = kexp && rows_differ(kexp, K, lane);
   if ((int)blockIdx.x < ablocks) {
     for (int q = 0; q < 4; ++q) {
@@ -259,7 +274,7 @@ __device__ __forceinline__ void issue_digit(uint32_t tmem, uint64_t ad, uint32_t
 __global__ void __launch_bounds__(THREADS, 1)
 zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aexp,
              const unsigned char* __restrict__ bdig, const int* __restrict__ bexp, int M, int N, int nch, int ctiles,
-             int total_tiles, double2* C, int64_t ldc, int sub, int* __restrict__ rowmax, int* status) {
+             int total_tiles, double2* C, int64_t ldc, int sub, int* __restrict__ rowmax, int* status, Slabs sl) {
   using namespace tc;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -312,17 +327,19 @@ zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aex
     while ((ib < nblk || q < nq) && !*abort) {
       bool progress = false;
       if (ib < nblk && (ib < 2 || mbar_try_wait(&empty_b[ib & 1], ((ib >> 1) - 1) & 1))) {
-        const int t = first + (ib / nch) * stride, ct = t % ctiles;
+        const int tt = first + (ib / nch) * stride, slab = tt / sl.tiles, ct = (tt - slab * sl.tiles) % ctiles;
         mbar_expect_tx(&full_b[ib & 1], B_BLOCK);
-        bulk_load(bring + (ib & 1) * B_BLOCK, bdig + ((size_t)ct * NCH + ib % nch) * B_BLOCK, B_BLOCK, &full_b[ib & 1]);
+        bulk_load(bring + (ib & 1) * B_BLOCK, bdig + slab * sl.bdig + ((size_t)ct * NCH + ib % nch) * B_BLOCK, B_BLOCK,
+                  &full_b[ib & 1]);
         ++ib;
         progress = true;
       }
       if (q < nq && (q < DSLOTS || mbar_try_wait(&empty_d[q % DSLOTS], ((q / DSLOTS) - 1) & 1))) {
-        const int blk = q / DIG, t = first + (blk / nch) * stride, rt = t / ctiles;
+        const int blk = q / DIG, tt = first + (blk / nch) * stride, slab = tt / sl.tiles;
+        const int rt = (tt - slab * sl.tiles) / ctiles;
         mbar_expect_tx(&full_d[q % DSLOTS], D_SLICE);
         bulk_load(dring + (q % DSLOTS) * D_SLICE,
-                  adig + (((size_t)rt * NCH + blk % nch) * DIG + q % DIG) * D_SLICE, D_SLICE, &full_d[q % DSLOTS]);
+                  adig + slab * sl.adig + (((size_t)rt * NCH + blk % nch) * DIG + q % DIG) * D_SLICE, D_SLICE, &full_d[q % DSLOTS]);
         ++q;
         progress = true;
       }
@@ -363,9 +380,9 @@ zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aex
     const int qd = warp & 3, part = (warp - EPI0) >> 2, r = qd * 32 + lane;
     const uint32_t tbase = tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(part * EPI_COLS);
     for (int lt = 0; lt < ntiles; ++lt) {
-      const int t = first + lt * stride, row = (t / ctiles) * BM + r;
-      const int col0 = (t % ctiles) * BNC + part * (EPI_COLS / 2);
-      double2* crow = C + (int64_t)row * ldc + col0;
+      const int tt = first + lt * stride, slab = tt / sl.tiles, t = tt - slab * sl.tiles;
+      const int row = (t / ctiles) * BM + r, col0 = (t % ctiles) * BNC + part * (EPI_COLS / 2);
+      double2* crow = C + slab * sl.c + (int64_t)row * ldc + col0;
       const int ncol = row < M ? min(EPI_COLS / 2, N - col0) : 0;
       if (sub && ncol > 0) {
         asm volatile("prefetch.global.L2 [%0];" ::"l"(crow));
@@ -399,12 +416,13 @@ zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aex
         }
       }
       if (ncol <= 0) continue;
-      const int ea = aexp[row];
+      const int ea = aexp[slab * sl.aexp + row];
+      const int* be = bexp + slab * sl.bexp + col0;
       int em = 0;
 #pragma unroll
       for (int j = 0; j < EPI_COLS / 2; ++j) {
         if (j < ncol) {
-          const int eb = bexp[col0 + j];
+          const int eb = be[j];
           double2 o = sub ? crow[j] : make_double2(0.0, 0.0);
           if (ea == kNonFinite || eb == kNonFinite) {
             o.x = o.y = __longlong_as_double(0x7FF8000000000000LL);
@@ -612,6 +630,13 @@ static size_t up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 
 }  // namespace zg
 
+static void set_attributes() {
+  static OncePerDevice once;
+  once([] {
+    cudaFuncSetAttribute(zg::zgemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)zg::smem_bytes());
+  });
+}
+
 size_t zgemm_bytes(int64_t rows, int64_t cols) {
   using namespace zg;
   const size_t rt = (size_t)((rows + BM - 1) / BM), ct = (size_t)((cols + BNC - 1) / BNC);
@@ -644,7 +669,8 @@ int zgemm_digits(const ZGemmPlan& p, const double2* A, int64_t lda, int M, const
   const int ab = (M + BM - 1) / BM * (BM / 32), bb = (N + BNC - 1) / BNC;
   if (ab + bb == 0) return MGT_OK;
   count_launch();
-  digits_kernel<<<ab + bb, 256, 0, s>>>(A, lda, M, ab, B, ldb, N, K, kexp, p.adig, p.aexp, p.bdig, p.bexp);
+  digits_kernel<<<ab + bb, 256, 0, s>>>(A, lda, M, ab, B, ldb, N, K, kexp, p.adig, p.aexp, p.bdig, p.bexp,
+                                      Slabs());
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }
 
@@ -655,8 +681,7 @@ int zgemm_apply(const ZGemmPlan& p, int arow, int M, int bcol, int N, int K, dou
   if (K <= 0 || K > kZK || arow % BM || bcol % BNC || arow < 0 || bcol < 0 || (int64_t)arow + M > p.rows ||
       (int64_t)bcol + N > p.cols)
     return MGT_ERR_ARG;
-  static OncePerDevice once;
-  once([] { cudaFuncSetAttribute(zgemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes()); });
+  set_attributes();
   const int rt = (M + BM - 1) / BM, ct = (N + BNC - 1) / BNC;
   const int64_t total = (int64_t)rt * ct;
   if (total > (1 << 30)) return MGT_ERR_UNSUPPORTED;
@@ -665,7 +690,74 @@ int zgemm_apply(const ZGemmPlan& p, int arow, int M, int bcol, int N, int K, dou
   zgemm_kernel<<<ctas, THREADS, smem_bytes(), s>>>(p.adig + (size_t)(arow / BM) * NCH * DIG * D_SLICE, p.aexp + arow,
                                                    p.bdig + (size_t)(bcol / BNC) * NCH * B_BLOCK, p.bexp + bcol, M, N,
                                                    (K + KCC - 1) / KCC, ct, (int)total, C, ldc, sub ? 1 : 0, rowmax,
-                                                   status);
+                                                   status, Slabs());
+  return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
+}
+
+// ---- products over any K: slabs of 64 columns, partial products summed in FP64
+
+namespace zg {
+
+// out = E0 - sum over slabs of part
+__global__ void slab_sum_kernel(const double2* __restrict__ part, int slabs, int M, int N,
+                                const double2* __restrict__ E0, int64_t ld0, double2* __restrict__ out, int64_t ldo) {
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= (int64_t)M * N) return;
+  const int64_t r = i / N, c = i - r * N;
+  double2 s = make_double2(0.0, 0.0);
+  for (int q = 0; q < slabs; ++q) s = cadd(s, part[(int64_t)q * M * N + i]);
+  const double2 e = E0 ? E0[r * ld0 + c] : make_double2(0.0, 0.0);
+  out[r * ldo + c] = csub(e, s);
+}
+
+struct Wide {
+  int slabs;
+  size_t rt, ct, adig, bdig, aexp, bexp, part, total;
+  Wide(int64_t M, int64_t N, int64_t K) {
+    slabs = (int)((K + kZK - 1) / kZK);
+    rt = (size_t)((M + BM - 1) / BM);
+    ct = (size_t)((N + BNC - 1) / BNC);
+    adig = 1024;
+    bdig = adig + up(slabs * rt * NCH * DIG * D_SLICE, 1024);
+    aexp = bdig + up(slabs * ct * NCH * B_BLOCK, 1024);
+    bexp = aexp + up(slabs * rt * BM * sizeof(int), 256);
+    part = bexp + up(slabs * ct * BNC * sizeof(int), 256);
+    total = part + (size_t)slabs * M * N * sizeof(double2) + 1024;
+  }
+};
+
+}  // namespace zg
+
+size_t zgemm_wide_bytes(int64_t M, int64_t N, int64_t K) { return zg::Wide(M, N, K).total; }
+
+int zgemm_wide(const double2* A, int64_t lda, int M, const double2* B, int64_t ldb, int N, int K, const double2* E0,
+               int64_t ld0, double2* out, int64_t ldo, void* work, cudaStream_t s) {
+  using namespace zg;
+  const Wide w(M, N, K);
+  char* b = (char*)up((size_t)work, 1024);
+  unsigned char* adig = (unsigned char*)b + w.adig;
+  unsigned char* bdig = (unsigned char*)b + w.bdig;
+  int* aexp = (int*)(b + w.aexp);
+  int* bexp = (int*)(b + w.bexp);
+  double2* part = (double2*)(b + w.part);
+  const int64_t total = (int64_t)w.rt * w.ct * w.slabs;
+  if (w.slabs > 65535 || total > (1 << 30)) return MGT_ERR_UNSUPPORTED;
+  Slabs sl;
+  sl.adig = w.rt * NCH * DIG * D_SLICE;
+  sl.bdig = w.ct * NCH * B_BLOCK;
+  sl.aexp = w.rt * BM;
+  sl.bexp = w.ct * BNC;
+  sl.c = (size_t)M * N;
+  sl.tiles = (int)(w.rt * w.ct);
+  set_attributes();
+  if (cudaMemsetAsync(b, 0, 256, s) != cudaSuccess) return MGT_ERR_CUDA;   // status
+  const int ab = (int)w.rt * (BM / 32);
+  count_launch(3);
+  digits_kernel<<<dim3(ab + (unsigned)w.ct, w.slabs), 256, 0, s>>>(A, lda, M, ab, B, ldb, N, K, nullptr, adig, aexp,
+                                                                  bdig, bexp, sl);
+  zgemm_kernel<<<(int)std::min<int64_t>(total, device_sm_count()), THREADS, smem_bytes(), s>>>(
+      adig, aexp, bdig, bexp, M, N, NCH, (int)w.ct, (int)total, part, N, 0, nullptr, (int*)b, sl);
+  slab_sum_kernel<<<(unsigned)(((int64_t)M * N + 255) / 256), 256, 0, s>>>(part, w.slabs, M, N, E0, ld0, out, ldo);
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }
 

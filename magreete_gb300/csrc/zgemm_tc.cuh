@@ -28,6 +28,13 @@ int zgemm_digits(const ZGemmPlan& p, const double2* A, int64_t lda, int M, const
 int zgemm_apply(const ZGemmPlan& p, int arow, int M, int bcol, int N, int K, double2* C, int64_t ldc, bool sub,
                 int* rowmax, int* status, cudaStream_t s, int max_ctas = 0);
 
+// out (M x N) = E0 - A B for any K (E0 may be null: zero), in a workspace of zgemm_wide_bytes: every 64
+// columns of K have their own scales, their products are summed in FP64.  The status word is the first int
+// of the workspace's first 1024-byte boundary.
+size_t zgemm_wide_bytes(int64_t M, int64_t N, int64_t K);
+int zgemm_wide(const double2* A, int64_t lda, int M, const double2* B, int64_t ldb, int N, int K, const double2* E0,
+               int64_t ld0, double2* out, int64_t ldo, void* work, cudaStream_t s);
+
 // ---- blocked complex128 LU: interchanges and block inverses
 struct ZSlots {
   const int2* slots;   // (position, source) pairs relative to the panel's first row
