@@ -1306,16 +1306,19 @@ static int resolve_lu_options(const mgt_lu_options* o, LuOpts* r) {
 // swaps a few rows in a thousand there); the growth that remains is what
 // iterative refinement absorbs.
 constexpr int kTileLD = 65;   // padded row stride of the tile in shared memory
-// dynamic shared memory of lu_tile_kernel: the tile by row and by position,
-// two inversion scratch blocks, the staged candidate rows
-constexpr int kCandLD = 128;  // a staged candidate row: columns 4 (j + k) + g < 128
-constexpr size_t kTileSmem = (2 * 64 * kTileLD + 2 * 32 * 33 + 2 * 8 * kCandLD) * sizeof(float2);
+// dynamic shared memory of lu_tile_kernel: the tile by row (then U^-1), by position, L^-1, block scratch
+constexpr size_t kTileSmem = (3 * 64 * kTileLD + 6 * 256) * sizeof(float2);
 
-// 1/z for the tile's pivots: Smith's scaling with two correctly rounded
-// reciprocals instead of three divisions (each result within a few ulp of
-// the quotient; the LU is only FP32-accurate and the mixed method's
-// refinement certifies the solution)
+// 1/z for the tile's pivots: conj(z) / |z|^2 with one correctly rounded
+// reciprocal where |z|^2 stays a normal number, else Smith's scaling with two
+// (each result within a few ulp of the quotient; the LU is only FP32-accurate
+// and the mixed method's refinement certifies the solution)
 __device__ __forceinline__ float2 crecip_tile(float2 z) {
+  const float m = fmaxf(fabsf(z.x), fabsf(z.y));
+  if (m > 1e-15f && m < 1e15f) {
+    const float inv = __frcp_rn(fmaf(z.x, z.x, z.y * z.y));
+    return make_float2(z.x * inv, -z.y * inv);
+  }
   if (fabsf(z.x) >= fabsf(z.y)) {
     const float r = z.y * __frcp_rn(z.x), inv = __frcp_rn(fmaf(z.y, r, z.x));
     return make_float2(inv, -r * inv);
@@ -1324,203 +1327,266 @@ __device__ __forceinline__ float2 crecip_tile(float2 z) {
   return make_float2(r * inv, -inv);
 }
 
-// One level of the recursion, blocks of h = 2^LH rows: the (up to 8) items of
-// a thread are interleaved inside the k loop, so their dependent chains of
-// multiply-adds overlap (item = (block q, row i, column j), upper items first)
-template <int LH>
-__device__ __forceinline__ void tile_inv_level(float2* T, float2* S1, float2* S2, int tid) {
-  constexpr int h = 1 << LH, per = h * h, tot = 32 * h, M = (2 * tot + 255) / 256;
-  int qi[M], ii[M], jj[M];
-  bool val[M], up[M];
-  float2 acc[M];
-#pragma unroll
-  for (int m = 0; m < M; ++m) {
-    const int e = tid + 256 * m;
-    val[m] = e < 2 * tot;
-    up[m] = e < tot;
-    const int f = up[m] ? e : e - tot;
-    qi[m] = f >> (2 * LH);
-    ii[m] = (f >> LH) & (h - 1);
-    jj[m] = f & (h - 1);
-  }
-  // step 1: S1 = A^-1 B (upper), S2 = B A^-1 (lower; A^-1 unit lower, diagonal 1)
-#pragma unroll
-  for (int m = 0; m < M; ++m) {
-    const int b = 2 * h * qi[m];
-    acc[m] = (val[m] && !up[m]) ? T[(b + h + ii[m]) * kTileLD + b + jj[m]] : make_float2(0.f, 0.f);
-  }
-#pragma unroll 4
-  for (int k = 0; k < h; ++k) {
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-      const int b = 2 * h * qi[m];
-      if (val[m] && up[m] && k >= ii[m])
-        cfma(acc[m], T[(b + ii[m]) * kTileLD + b + k], T[(b + k) * kTileLD + b + h + jj[m]]);
-      if (val[m] && !up[m] && k > jj[m])
-        cfma(acc[m], T[(b + h + ii[m]) * kTileLD + b + k], T[(b + k) * kTileLD + b + jj[m]]);
-    }
-  }
-#pragma unroll
-  for (int m = 0; m < M; ++m)
-    if (val[m]) (up[m] ? S1 : S2)[qi[m] * per + ii[m] * h + jj[m]] = acc[m];
-  __syncthreads();
-  // step 2: B <- -(S1 C^-1) (upper), B <- -(C^-1 S2) (lower)
-#pragma unroll
-  for (int m = 0; m < M; ++m)
-    acc[m] = (val[m] && !up[m]) ? S2[qi[m] * per + ii[m] * h + jj[m]] : make_float2(0.f, 0.f);
-#pragma unroll 4
-  for (int k = 0; k < h; ++k) {
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-      const int b = 2 * h * qi[m];
-      if (val[m] && up[m] && k <= jj[m])
-        cfma(acc[m], S1[qi[m] * per + ii[m] * h + k], T[(b + h + k) * kTileLD + b + h + jj[m]]);
-      if (val[m] && !up[m] && k < ii[m])
-        cfma(acc[m], T[(b + h + ii[m]) * kTileLD + b + h + k], S2[qi[m] * per + k * h + jj[m]]);
-    }
-  }
-#pragma unroll
-  for (int m = 0; m < M; ++m) {
-    if (!val[m]) continue;
-    const int b = 2 * h * qi[m];
-    const float2 v = make_float2(-acc[m].x, -acc[m].y);
-    if (up[m]) T[(b + ii[m]) * kTileLD + b + h + jj[m]] = v;
-    else T[(b + h + ii[m]) * kTileLD + b + jj[m]] = v;
-  }
-  __syncthreads();
+constexpr int kTileThreads = 512;
+constexpr int kTileBar = 32 + 14 * 32;   // threads of the tile's named barriers: warp 0 and 14 update warps
+
+__device__ __forceinline__ void bar_sync_n(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kTileBar) : "memory"); }
+__device__ __forceinline__ void bar_arrive_n(int id) {
+  asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kTileBar) : "memory");
 }
 
-// In-place inverses of the upper triangle U (diagonal included) and of the
-// unit lower triangle L (strict lower part) of the 64 x 64 tile T, by block
-// recursion: for a block [[A, B], [0, C]] of U, the off-diagonal block of the
-// inverse is -(A^-1 B) C^-1; for [[A, 0], [B, C]] of L it is -C^-1 (B A^-1).
-// Level h combines 32 / h pairs of inverted h x h blocks; 256 threads.
-// A zero diagonal entry of U inverts to zero (the factorisation has already
-// recorded it as a zero pivot).
-__device__ void tile_triangular_inverses(float2* T, float2* S1, float2* S2, int tid) {
-  for (int i = tid; i < 64; i += 256) {
-    const float2 u = T[i * kTileLD + i];
-    T[i * kTileLD + i] = (u.x != 0.f || u.y != 0.f) ? crecip_tile(u) : make_float2(0.f, 0.f);
+// UI = U^-1 (upper, diagonal reciprocals given) and LI = L^-1 (unit lower) of
+// the 64 x 64 tile F by 16 x 16 blocks: the eight diagonal blocks by
+// substitution, one per warp, then the block diagonals outwards:
+// UI_ij = -UI_ii sum_k U_ik UI_kj by threads 0 .. 255 and likewise L by the
+// others.  S: 6 x 256 scratch.  Only the triangles' blocks are written.
+__device__ __forceinline__ void tile_inverses(const float2* F, float2* UI, float2* LI, float2* S, const float2* dinv,
+                                              int tid) {
+  const int warp = tid >> 5, lane = tid & 31;
+  if (warp < 8 && lane < 16) {
+    const int b = (warp & 3) * 16, c = lane;
+    float2 x[16];
+    if (warp < 4) {
+#pragma unroll
+      for (int i = 15; i >= 0; --i) {
+        float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int k = i + 1; k < 16; ++k) cfms(s, F[(b + i) * kTileLD + b + k], x[k]);
+        const float2 d = dinv[b + i];
+        x[i] = i == c ? d : i < c ? cmul(s, d) : make_float2(0.f, 0.f);
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) UI[(b + i) * kTileLD + b + c] = x[i];
+    } else {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        float2 s = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < i; ++k) cfms(s, F[(b + i) * kTileLD + b + k], x[k]);
+        x[i] = i == c ? make_float2(1.f, 0.f) : i > c ? s : make_float2(0.f, 0.f);
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) LI[(b + i) * kTileLD + b + c] = x[i];
+    }
   }
   __syncthreads();
-  tile_inv_level<0>(T, S1, S2, tid);
-  tile_inv_level<1>(T, S1, S2, tid);
-  tile_inv_level<2>(T, S1, S2, tid);
-  tile_inv_level<3>(T, S1, S2, tid);
-  tile_inv_level<4>(T, S1, S2, tid);
-  tile_inv_level<5>(T, S1, S2, tid);
+  const bool upper = tid < 256;
+  const int t = tid & 255, r = t >> 4, c = t & 15;   // this thread's entry of every block
+  float2* I = upper ? UI : LI;
+  float2* Sq = S + (upper ? 0 : 3 * 256);
+#pragma unroll 1
+  for (int d = 1; d < 4; ++d) {
+    const int np = 4 - d;
+#pragma unroll 1
+    for (int q = 0; q < np; ++q) {
+      // U: row block i, column block i + 16 d; L: the mirror image
+      const int i = 16 * q, j = 16 * (q + d);
+      const float2* f = upper ? F + (i + r) * kTileLD + i + 16 : F + (j + r) * kTileLD + i;
+      const float2* x = upper ? I + (i + 16) * kTileLD + j + c : I + i * kTileLD + i + c;
+      float2 s0 = make_float2(0.f, 0.f), s1 = s0;
+#pragma unroll 8
+      for (int k = 0; k < 16 * d; k += 2) {
+        cfms(s0, f[k], x[k * kTileLD]);
+        cfms(s1, f[k + 1], x[(k + 1) * kTileLD]);
+      }
+      Sq[q * 256 + t] = cadd(s0, s1);
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int q = 0; q < np; ++q) {
+      const int i = 16 * q, j = 16 * (q + d);
+      const float2* f = upper ? I + (i + r) * kTileLD + i : I + (j + r) * kTileLD + j;
+      const float2* x = Sq + q * 256 + c;
+      float2 s0 = make_float2(0.f, 0.f), s1 = s0;
+#pragma unroll
+      for (int k = 0; k < 16; k += 2) {
+        cfma(s0, f[k], x[k * 16]);
+        cfma(s1, f[k + 1], x[(k + 1) * 16]);
+      }
+      (upper ? I[(i + r) * kTileLD + j + c] : I[(j + r) * kTileLD + i + c]) = cadd(s0, s1);
+    }
+    __syncthreads();
+  }
 }
 
-// One CTA of 256 threads; thread (r, g) = (tid / 4, tid % 4) holds the
-// columns g, g + 4, ... of tile row r in registers, a[k] = column 4 (j + k) + g
-// after j shifts (every fourth column), so register indices stay compile-time
-// constants and no loop has a data-dependent bound.  Per column c, with one
-// block barrier: the holders of column c bid |re| + |im| (lowest tile row on
-// ties); each warp's best row stages itself in cand[warp] before the barrier;
-// after it every thread reads the eight bids, the winner retires (its staged
-// row is row c of U), and the other rows compute their multiplier and update.
-// Rows never move between threads: the row chosen at column c goes to
-// position c, which gives the interchange slots directly.  Then all warps
-// invert U11 and L11 in place, for the rows below (L21 = A21 U11^-1) and the
-// columns to the right (U12 = L11^-1 A12).
-__global__ void __launch_bounds__(256, 1)
+// One CTA: the w x w tile's LU with partial pivoting among its rows, then
+// U11^-1 and L11^-1, for the rows below (L21 = A21 U11^-1) and the columns to
+// the right (U12 = L11^-1 A12).  Bound by the chain of 64 pivots, so that
+// chain is one warp's: warp 0, lane = tile rows lane and lane + 32, factors
+// four columns at a time in registers (per column two warp reductions pick the
+// pivot, shuffles broadcast its row, every lane computes its reciprocal) and
+// brings the next four up to date itself, while warps 1 .. 14 apply the four
+// pivots to the columns beyond (8 columns x half of the rows per warp).  Two
+// pairs of named barriers, by parity, hand the work over: (1, 3) four columns
+// are factored, (2, 4) the columns beyond are updated.
+// Rows never move: s_piv[c] is the tile row chosen at column c, s_state its
+// inverse (64: not chosen yet); rows of U go to F by position.
+// Measured: a version with one block barrier per column 57 us; 775 clocks a
+// column when warp 0 took 16 columns at a time.
+__global__ void __launch_bounds__(kTileThreads, 1)
 lu_tile_kernel(float2* __restrict__ A, int64_t lda, int w, int j0, int32_t* __restrict__ perm, PanelWs ws,
                float2* __restrict__ Uinv, float2* __restrict__ Linv) {
   // A: the tile's top-left element (row j0, column j0); w <= 64
   extern __shared__ __align__(16) unsigned char tile_smem[];
-  float2* T = reinterpret_cast<float2*>(tile_smem);    // [64][kTileLD]: the tile, then the multipliers by tile row
+  float2* T = reinterpret_cast<float2*>(tile_smem);    // [64][kTileLD]: the tile by tile row; then U^-1
   float2* F = T + 64 * kTileLD;                         // [64][kTileLD], row q = position q
-  float2* S1 = F + 64 * kTileLD;
-  float2* S2 = S1 + 32 * 33;
-  float2* cand = S2 + 32 * 33;                          // [2][8][kCandLD]: each warp's best row, by column parity
-  __shared__ uint32_t s_key[2][8];
-  __shared__ int s_row[2][8];
-  __shared__ float2 s_inv[2][8];                       // 1 / each warp's candidate pivot
+  float2* LI = F + 64 * kTileLD;                        // [64][kTileLD]: L^-1
+  float2* S = LI + 64 * kTileLD;                        // 6 x 256
   __shared__ int s_piv[64];
+  __shared__ volatile int s_state[64];
+  __shared__ float2 s_dinv[64];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int r = tid >> 2, g = tid & 3;
-  for (int idx = tid; idx < 64 * 64; idx += 256) {
+  for (int idx = tid; idx < 64 * 64; idx += kTileThreads) {
     const int i = idx >> 6, k = idx & 63;
     const bool in = i < w && k < w;
     cp_async_elem<8>(T + i * kTileLD + k, in ? A + (int64_t)i * lda + k : A, in);
   }
   cp_async_commit();
-  if (tid < 64) s_piv[tid] = tid;
+  if (tid < 64) {
+    s_piv[tid] = tid;
+    s_state[tid] = tid < w ? 64 : -1;
+    s_dinv[tid] = make_float2(1.f, 0.f);
+  }
   cp_async_wait<0>();
   __syncthreads();
-  float2 a[16];
+  const int steps = (w + 3) / 4;
+  if (warp == 0) {
+    bool act0 = lane < w, act1 = lane + 32 < w;
+    float2 a0[4], a1[4];
 #pragma unroll
-  for (int k = 0; k < 16; ++k) a[k] = T[r * kTileLD + 4 * k + g];
-  bool active = r < w;
-  for (int j = 0; j < 16 && 4 * j < w; ++j) {
-    // not unrolled: u only selects threads, and one copy of the column body
-    // keeps the loop within the instruction cache
-#pragma unroll 1
-    for (int u = 0; u < 4; ++u) {
-      const int c = 4 * j + u;
-      if (c >= w) break;
-      const int buf = c & 1;
-      float2* cb = cand + buf * 8 * kCandLD;
-      // bid: key 0 = no bid; +1 keeps the rows of a zero column valid bidders
-      const uint32_t key = (active && g == u) ? __float_as_uint(fabsf(a[0].x) + fabsf(a[0].y)) + 1u : 0u;
-      const uint32_t mx = __reduce_max_sync(0xffffffffu, key);
-      const uint32_t ml = __reduce_min_sync(0xffffffffu, (key == mx && mx != 0u) ? (uint32_t)lane : 32u);
-      if (mx != 0u && (lane >> 2) == (int)(ml >> 2)) {
-#pragma unroll
-        for (int k = 0; k < 16; ++k) cb[warp * kCandLD + 4 * (j + k) + g] = a[k];
-        // the candidate's reciprocal before the barrier, off the chain after it
-        if (g == u) {
-          const bool z = a[0].x == 0.f && a[0].y == 0.f;
-          s_inv[buf][warp] = z ? make_float2(0.f, 0.f) : crecip_tile(a[0]);
-        }
-      }
-      if (lane == 0) {
-        s_key[buf][warp] = mx;
-        s_row[buf][warp] = warp * 8 + (int)(ml >> 2);
-      }
-      __syncthreads();
-      // the winning warp: largest bid, lowest warp (lowest rows) on ties; lanes
-      // 0..7 read one bid each and two warp reductions decide
-      const uint32_t kq = lane < 8 ? s_key[buf][lane] : 0u;
-      const uint32_t kmax = __reduce_max_sync(0xffffffffu, kq);
-      const int best = (int)__reduce_min_sync(0xffffffffu, (lane < 8 && kq == kmax) ? (uint32_t)lane : 8u);
-      const int p = s_row[buf][best];
-      const float2* prow = cb + best * kCandLD;
-      const float2 pinv = s_inv[buf][best];
-      if (r == p) {
-        if (g == 0) {
-          s_piv[c] = r;
-          const float2 piv = prow[c];
-          if (piv.x == 0.f && piv.y == 0.f && ws.status[1] == 0) ws.status[1] = j0 + c + 1;
-        }
-        active = false;
-      }
-      float2 l = g == u ? cmul(a[0], pinv) : make_float2(0.f, 0.f);
-      l.x = __shfl_sync(0xffffffffu, l.x, (lane & ~3) | u);
-      l.y = __shfl_sync(0xffffffffu, l.y, (lane & ~3) | u);
-      if (active) {
-        if (g == u) T[r * kTileLD + c] = l;
-#pragma unroll
-        for (int k = 0; k < 16; ++k) cfms(a[k], l, prow[4 * (j + k) + g]);
-      }
-      // row c of U (read from the staged row until the next column's barrier)
-      if (tid < 64 && tid >= c) F[c * kTileLD + tid] = prow[tid];
+    for (int k = 0; k < 4; ++k) {
+      a0[k] = T[lane * kTileLD + k];
+      a1[k] = T[(lane + 32) * kTileLD + k];
     }
+    for (int s = 0; s < steps; ++s) {
+      const int c0 = 4 * s;
+      int p[4] = {0, 0, 0, 0};
 #pragma unroll
-    for (int k = 0; k < 15; ++k) a[k] = a[k + 1];
+      for (int u = 0; u < 4; ++u) {
+        if (c0 + u < w) {
+          // key 0 = no bid; +1 keeps the rows of a zero column valid bidders
+          const uint32_t k0 = act0 ? __float_as_uint(fabsf(a0[u].x) + fabsf(a0[u].y)) + 1u : 0u;
+          const uint32_t k1 = act1 ? __float_as_uint(fabsf(a1[u].x) + fabsf(a1[u].y)) + 1u : 0u;
+          const uint32_t mx = __reduce_max_sync(0xffffffffu, max(k0, k1));
+          p[u] = (int)__reduce_min_sync(0xffffffffu,
+                                        k0 == mx ? (uint32_t)lane : k1 == mx ? (uint32_t)lane + 32u : 64u);
+          const int src = p[u] & 31;
+          const bool hi = p[u] >= 32;
+          float2 prow[4];
+#pragma unroll
+          for (int k = u; k < 4; ++k) {
+            prow[k].x = __shfl_sync(0xffffffffu, hi ? a1[k].x : a0[k].x, src);
+            prow[k].y = __shfl_sync(0xffffffffu, hi ? a1[k].y : a0[k].y, src);
+          }
+          const bool zero = prow[u].x == 0.f && prow[u].y == 0.f;
+          const float2 inv = zero ? make_float2(0.f, 0.f) : crecip_tile(prow[u]);
+          if (lane == src) (hi ? act1 : act0) = false;
+          if (act0) {
+            a0[u] = cmul(a0[u], inv);
+#pragma unroll
+            for (int k = u + 1; k < 4; ++k) cfms(a0[k], a0[u], prow[k]);
+          }
+          if (act1) {
+            a1[u] = cmul(a1[u], inv);
+#pragma unroll
+            for (int k = u + 1; k < 4; ++k) cfms(a1[k], a1[u], prow[k]);
+          }
+          if (lane == 0) {
+            s_piv[c0 + u] = p[u];
+            s_state[p[u]] = c0 + u;
+            s_dinv[c0 + u] = inv;
+            if (zero && ws.status[1] == 0) ws.status[1] = j0 + c0 + u + 1;
+          }
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        T[lane * kTileLD + c0 + u] = a0[u];
+        T[(lane + 32) * kTileLD + c0 + u] = a1[u];
+      }
+      __syncwarp();
+      bar_arrive_n(1 + 2 * (s & 1));
+      if (s + 1 < steps) {
+        // the next four columns (up to date but for these four pivots once the update warps are)
+        if (s > 0) bar_sync_n(2 + 2 * ((s - 1) & 1));
+        float2 n0[4], n1[4], uu[4][4];
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          n0[v] = T[lane * kTileLD + c0 + 4 + v];
+          n1[v] = T[(lane + 32) * kTileLD + c0 + 4 + v];
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float2* row = T + p[k] * kTileLD + c0;
+#pragma unroll
+          for (int v = 0; v < 4; ++v) uu[k][v] = row[4 + v];
+#pragma unroll
+          for (int i = 0; i < k; ++i) {
+            const float2 l = row[i];
+#pragma unroll
+            for (int v = 0; v < 4; ++v) cfms(uu[k][v], l, uu[i][v]);
+          }
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+#pragma unroll
+          for (int v = 0; v < 4; ++v) {
+            if (lane == 4 * k + v) F[(c0 + k) * kTileLD + c0 + 4 + v] = uu[k][v];
+            cfms(n0[v], a0[k], uu[k][v]);
+            cfms(n1[v], a1[k], uu[k][v]);
+          }
+#pragma unroll
+        for (int v = 0; v < 4; ++v) {
+          a0[v] = n0[v];
+          a1[v] = n1[v];
+        }
+      }
+    }
+    // the barriers of the last two updates are completed too
+    for (int s = max(0, steps - 2); s < steps; ++s) bar_sync_n(2 + 2 * (s & 1));
+  } else if (warp < 15) {
+    const int ww = warp - 1, half = ww / 7, rg = lane >> 3;
+    for (int s = 0; s < steps; ++s) {
+      const int c0 = 4 * s, j = c0 + 8 + (ww % 7) * 8 + (lane & 7);
+      bar_sync_n(1 + 2 * (s & 1));
+      if (j < w) {
+        float2 u[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const float2* row = T + s_piv[c0 + k] * kTileLD;
+          u[k] = row[j];
+#pragma unroll
+          for (int i = 0; i < k; ++i) cfms(u[k], row[c0 + i], u[i]);
+        }
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if (half == 0 && rg == k) F[(c0 + k) * kTileLD + j] = u[k];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int r = rg + 4 * half + 8 * i;
+          if (s_state[r] > c0 + 3) {
+            float2* row = T + r * kTileLD;
+            float2 x = row[j];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) cfms(x, row[c0 + k], u[k]);
+            row[j] = x;
+          }
+        }
+      }
+      bar_arrive_n(2 + 2 * (s & 1));
+    }
   }
   __syncthreads();
-  // the multipliers in position order (position q holds tile row s_piv[q]);
-  // identity beyond w (the last panel)
-  for (int idx = tid; idx < 64 * 64; idx += 256) {
+  // the factors in position order (position q holds tile row s_piv[q]; U right of
+  // q's four columns is there); identity beyond w (the last panel)
+  for (int idx = tid; idx < 64 * 64; idx += kTileThreads) {
     const int q = idx >> 6, k = idx & 63;
-    if (q >= w) F[q * kTileLD + k] = make_float2(q == k ? 1.f : 0.f, 0.f);
-    else if (k < q) F[q * kTileLD + k] = T[s_piv[q] * kTileLD + k];
-  }
-  __syncthreads();
-  for (int idx = tid; idx < 64 * 64; idx += 256) {
-    const int q = idx >> 6, k = idx & 63;
-    if (q < w && k < w) A[(int64_t)q * lda + k] = F[q * kTileLD + k];
+    float2 v;
+    if (q >= w) v = make_float2(q == k ? 1.f : 0.f, 0.f);
+    else if (k < (q & ~3) + 4) v = T[s_piv[q] * kTileLD + k];
+    else v = k < w ? F[q * kTileLD + k] : make_float2(0.f, 0.f);
+    F[q * kTileLD + k] = v;
+    if (q < w && k < w) A[(int64_t)q * lda + k] = v;
   }
   if (warp == 0) {
     for (int q = lane; q < kNBmax; q += 32) ws.slots[q] = make_int2(q, q < w ? s_piv[q] : q);
@@ -1539,13 +1605,12 @@ lu_tile_kernel(float2* __restrict__ A, int64_t lda, int w, int j0, int32_t* __re
     }
   }
   __syncthreads();
-  tile_triangular_inverses(F, S1, S2, tid);
-  for (int idx = tid; idx < 64 * 64; idx += 256) {
+  tile_inverses(F, T, LI, S, s_dinv, tid);
+  for (int idx = tid; idx < 64 * 64; idx += kTileThreads) {
     const int i = idx >> 6, k = idx & 63;
-    const float2 v = F[i * kTileLD + k];
     const bool inw = i < w && k < w;
-    Uinv[idx] = (inw && k >= i) ? v : make_float2(0.f, 0.f);
-    Linv[idx] = (inw && k < i) ? v : make_float2(i == k ? 1.f : 0.f, 0.f);
+    Uinv[idx] = (inw && k >= i) ? T[i * kTileLD + k] : make_float2(0.f, 0.f);
+    Linv[idx] = (inw && k < i) ? LI[i * kTileLD + k] : make_float2(i == k ? 1.f : 0.f, 0.f);
   }
 }
 
@@ -1773,7 +1838,7 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
         float2* Ui = reinterpret_cast<float2*>((char*)work + Lw.uinv);
         // L11^-1 where the fused right-column pass reads the block's diagonal inverses
         float2* Li = reinterpret_cast<float2*>((char*)work + Lw.inv) + (size_t)set * kNBmax * kNBmax;
-        lu_tile_kernel<<<1, 256, kTileSmem, s>>>(A + (int64_t)j0 * lda + j0, lda, w, j0, perm, panel_ws(work, set),
+        lu_tile_kernel<<<1, kTileThreads, kTileSmem, s>>>(A + (int64_t)j0 * lda + j0, lda, w, j0, perm, panel_ws(work, set),
                                                   Ui, Li);
         count_launch();
         const int below = n - j0 - w;
