@@ -254,6 +254,18 @@ int mgt_solve_refined(const void* M, int64_t ldm, const void* LU, int64_t ldlu,
                       void* stream);
 
 /*
+ * mgt_solve_refined from digits prepared in another workspace (the one given
+ * to mgt_refine_prepare, for any nrhs): everything else is in `work`, of
+ * mgt_refine_scratch_bytes(n, nrhs) bytes, so that right-hand sides wider than
+ * the prepared workspace was sized for are solved in one block.  `prepared`
+ * is only read.
+ */
+int mgt_refine_scratch_bytes(int64_t n, int64_t nrhs, size_t* bytes);
+int mgt_solve_prepared(const void* prepared, const void* LU, int64_t ldlu, const int32_t* perm, int64_t n,
+                       const void* B, int64_t ldb, void* X, int64_t ldx, int64_t nrhs, double tol, int max_iter,
+                       void* work, size_t work_bytes, int* iters, double* rel_res, void* stream);
+
+/*
  * The refinement of mgt_solve_refined as stream-ordered steps that never
  * synchronise with the host, so a whole refined solve can be captured into a
  * CUDA graph (the batched sweep does).  Same workspace as mgt_solve_refined.

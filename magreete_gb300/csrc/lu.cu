@@ -2286,12 +2286,13 @@ __global__ void permute_rows_kernel(const V* __restrict__ B, int64_t ldb, const 
 
 template <typename T, bool UPPER>
 int tri_solve(const cplx<T>* F, int64_t ldf, cplx<T>* X, int64_t ldx, int n, int nrhs, void* work, int* status,
-              cudaStream_t s);
+              bool inverses_ready, cudaStream_t s);
 size_t tri_solve_workspace_bytes(int64_t n, int64_t nrhs, size_t elem);
 
 template <typename T>
 static int lu_solve_impl(const cplx<T>* LU, int n, int64_t lda, const int32_t* perm, const cplx<T>* B,
-                         int64_t ldb, cplx<T>* X, int64_t ldx, int nrhs, cudaStream_t s, void* work = nullptr) {
+                         int64_t ldb, cplx<T>* X, int64_t ldx, int nrhs, cudaStream_t s, void* work = nullptr,
+                         bool inverses_ready = false) {
   using V = cplx<T>;
   if (work) {
     if (n > 65535) return MGT_ERR_UNSUPPORTED;
@@ -2304,8 +2305,8 @@ static int lu_solve_impl(const cplx<T>* LU, int n, int64_t lda, const int32_t* p
       // persistent flag-ordered triangular solves (one launch per triangle and 64 columns)
       int* status = (int*)((char*)work + 128);
       if (cudaMemsetAsync(status, 0, 2 * sizeof(int), s) != cudaSuccess) return MGT_ERR_CUDA;
-      int e = tri_solve<T, false>(LU, lda, X, ldx, n, nrhs, work, status, s);
-      if (e == MGT_OK) e = tri_solve<T, true>(LU, lda, X, ldx, n, nrhs, work, status, s);
+      int e = tri_solve<T, false>(LU, lda, X, ldx, n, nrhs, work, status, inverses_ready, s);
+      if (e == MGT_OK) e = tri_solve<T, true>(LU, lda, X, ldx, n, nrhs, work, status, inverses_ready, s);
       return e;
     }
   }
@@ -2343,6 +2344,13 @@ static int lu_solve_impl(const cplx<T>* LU, int n, int64_t lda, const int32_t* p
     }
   }
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
+}
+
+// complex64 solve of the refinement; inverses_ready: this workspace served a solve with the same factors
+// and number of columns before
+int lu_solve_c64(const float2* LU, int n, int64_t lda, const int32_t* perm, const float2* B, float2* X, int nrhs,
+                 void* work, bool inverses_ready, cudaStream_t s) {
+  return lu_solve_impl<float>(LU, n, lda, perm, B, nrhs, X, nrhs, nrhs, s, work, inverses_ready);
 }
 
 }  // namespace mgt

@@ -294,7 +294,9 @@ struct RefineWs {
   void* tcw;      // (tensor-core residual) one application's workspace
   size_t tcw_bytes;
   size_t total;
-  RefineWs(void* base, int64_t n, int64_t r) {
+  // prepared: a workspace of mgt_refine_prepare that holds M's row exponents and
+  // digits; the rest is laid out in base without them
+  RefineWs(void* base, int64_t n, int64_t r, const void* prepared = nullptr) {
     char* b = (char*)base;
     size_t off = 0;
     auto take = [&](size_t bytes) { char* p = b ? b + off : nullptr; off += (bytes + 255) & ~size_t(255); return p; };
@@ -304,10 +306,15 @@ struct RefineWs {
     if (tc) {
       // M's row exponents and digits first: their place does not depend on
       // nrhs, so a workspace prepared once serves solves of fewer columns
+      if (prepared) b = (char*)prepared;
       rowexp = (int*)take(n * sizeof(int));
       off = (off + 1023) & ~size_t(1023);
       digits = (unsigned char*)take(residual_tc_digits_bytes(n, n));
       off = (off + 1023) & ~size_t(1023);
+      if (prepared) {
+        b = (char*)base;
+        off = 0;
+      }
     }
     Rr = (double2*)take(n * r * sizeof(double2));
     R32 = (float2*)take(n * r * sizeof(float2));
@@ -352,9 +359,10 @@ struct RefineWs {
 
 using namespace mgt;
 
-extern "C" int mgt_lu_solve(int dtype, const void* LU, int64_t n, int64_t lda, const int32_t* perm,
-                            const void* B, int64_t ldb, void* X, int64_t ldx, int64_t nrhs, void* work,
-                            size_t work_bytes, void* stream);
+namespace mgt {
+int lu_solve_c64(const float2* LU, int n, int64_t lda, const int32_t* perm, const float2* B, float2* X, int nrhs,
+                 void* work, bool inverses_ready, cudaStream_t s);
+}
 
 extern "C" int mgt_residual_workspace_bytes(int64_t n, int64_t nrhs, size_t* bytes) {
   if (!bytes || n <= 0 || nrhs <= 0) return MGT_ERR_ARG;
@@ -418,14 +426,14 @@ extern "C" int mgt_refine_workspace_bytes(int64_t n, int64_t nrhs, size_t* bytes
   return MGT_OK;
 }
 
-extern "C" int mgt_solve_refined(const void* M, int64_t ldm, const void* LU, int64_t ldlu, const int32_t* perm,
-                                 int64_t n, const void* B, int64_t ldb, void* X, int64_t ldx, int64_t nrhs,
-                                 double tol, int max_iter, void* work, size_t work_bytes, int* iters,
-                                 double* rel_res, void* stream) {
+static int solve_refined(const void* M, int64_t ldm, const void* prepared, const void* LU, int64_t ldlu,
+                         const int32_t* perm, int64_t n, const void* B, int64_t ldb, void* X, int64_t ldx,
+                         int64_t nrhs, double tol, int max_iter, void* work, size_t work_bytes, int* iters,
+                         double* rel_res, void* stream) {
   if (!LU || !perm || !B || !X || !work || n <= 0 || nrhs <= 0 || (M && ldm < n) || ldlu < n || ldb < nrhs ||
       ldx < nrhs || max_iter < 0)
     return MGT_ERR_ARG;
-  RefineWs w(work, n, nrhs);
+  RefineWs w(work, n, nrhs, prepared);
   if (!M && !w.tc) return MGT_ERR_ARG;   // prepared digits exist only for the tensor-core residual
   if (work_bytes < w.total) return MGT_ERR_WORKSPACE;
   cudaStream_t s = (cudaStream_t)stream;
@@ -441,8 +449,7 @@ extern "C" int mgt_solve_refined(const void* M, int64_t ldm, const void* LU, int
   // x0 = LU^-1 b in complex64
   count_launch();
   c128_to_c64_kernel<<<eg, 256, 0, s>>>(Bd, ldb, w.R32, nr, nn, nr);
-  const size_t tri_bytes = tri_solve_workspace_bytes(n, nrhs, sizeof(float2));
-  int e = mgt_lu_solve(MGT_C64, LU, n, ldlu, perm, w.R32, nr, w.D32, nr, nrhs, w.tri, tri_bytes, stream);
+  int e = lu_solve_c64((const float2*)LU, nn, ldlu, perm, w.R32, w.D32, nr, w.tri, false, s);
   if (e != MGT_OK) return e;
   count_launch();
   c64_into_c128_kernel<<<eg, 256, 0, s>>>(w.D32, nr, Xd, ldx, nn, nr, 1);
@@ -467,7 +474,7 @@ extern "C" int mgt_solve_refined(const void* M, int64_t ldm, const void* LU, int
     prev = rel;
     count_launch();
     c128_to_c64_kernel<<<eg, 256, 0, s>>>(w.Rr, nr, w.R32, nr, nn, nr);
-    e = mgt_lu_solve(MGT_C64, LU, n, ldlu, perm, w.R32, nr, w.D32, nr, nrhs, w.tri, tri_bytes, stream);
+    e = lu_solve_c64((const float2*)LU, nn, ldlu, perm, w.R32, w.D32, nr, w.tri, true, s);
     if (e != MGT_OK) return e;
     count_launch();
     c64_into_c128_kernel<<<eg, 256, 0, s>>>(w.D32, nr, Xd, ldx, nn, nr, 0);
@@ -476,6 +483,30 @@ extern "C" int mgt_solve_refined(const void* M, int64_t ldm, const void* LU, int
   if (rel_res) *rel_res = rel;
   if (cudaGetLastError() != cudaSuccess) return MGT_ERR_CUDA;
   return (rel <= tol && rel == rel) ? MGT_OK : MGT_ERR_NOT_CONVERGED;
+}
+
+extern "C" int mgt_solve_refined(const void* M, int64_t ldm, const void* LU, int64_t ldlu, const int32_t* perm,
+                                 int64_t n, const void* B, int64_t ldb, void* X, int64_t ldx, int64_t nrhs,
+                                 double tol, int max_iter, void* work, size_t work_bytes, int* iters,
+                                 double* rel_res, void* stream) {
+  return solve_refined(M, ldm, nullptr, LU, ldlu, perm, n, B, ldb, X, ldx, nrhs, tol, max_iter, work, work_bytes,
+                       iters, rel_res, stream);
+}
+
+extern "C" int mgt_refine_scratch_bytes(int64_t n, int64_t nrhs, size_t* bytes) {
+  if (!bytes || n <= 0 || nrhs <= 0) return MGT_ERR_ARG;
+  if (!residual_tc_supported(n, n, nrhs)) return MGT_ERR_UNSUPPORTED;
+  *bytes = RefineWs(nullptr, n, nrhs, bytes).total;   // any non-null `prepared`: the layout without digits
+  return MGT_OK;
+}
+
+extern "C" int mgt_solve_prepared(const void* prepared, const void* LU, int64_t ldlu, const int32_t* perm, int64_t n,
+                                  const void* B, int64_t ldb, void* X, int64_t ldx, int64_t nrhs, double tol,
+                                  int max_iter, void* work, size_t work_bytes, int* iters, double* rel_res,
+                                  void* stream) {
+  if (!prepared) return MGT_ERR_ARG;
+  return solve_refined(nullptr, 0, prepared, LU, ldlu, perm, n, B, ldb, X, ldx, nrhs, tol, max_iter, work, work_bytes,
+                       iters, rel_res, stream);
 }
 
 // ---------------------------------------------------------------- DOS dots
@@ -533,8 +564,7 @@ extern "C" int mgt_refine_start(const void* LU, int64_t ldlu, const int32_t* per
   const unsigned eg = (unsigned)((n * nrhs + 255) / 256);
   count_launch();
   c128_to_c64_kernel<<<eg, 256, 0, s>>>((const double2*)B, ldb, w.R32, nr, nn, nr);
-  int e = mgt_lu_solve(MGT_C64, LU, n, ldlu, perm, w.R32, nr, w.D32, nr, nrhs, w.tri,
-                       tri_solve_workspace_bytes(n, nrhs, sizeof(float2)), stream);
+  int e = lu_solve_c64((const float2*)LU, nn, ldlu, perm, w.R32, w.D32, nr, w.tri, false, s);
   if (e != MGT_OK) return e;
   count_launch();
   c64_into_c128_kernel<<<eg, 256, 0, s>>>(w.D32, nr, (double2*)X, ldx, nn, nr, 1);
@@ -557,8 +587,7 @@ extern "C" int mgt_refine_correct(const void* M, int64_t ldm, const void* LU, in
   if (e != MGT_OK) return e;
   count_launch();
   c128_to_c64_kernel<<<eg, 256, 0, s>>>(w.Rr, nr, w.R32, nr, nn, nr);
-  e = mgt_lu_solve(MGT_C64, LU, n, ldlu, perm, w.R32, nr, w.D32, nr, nrhs, w.tri,
-                   tri_solve_workspace_bytes(n, nrhs, sizeof(float2)), stream);
+  e = lu_solve_c64((const float2*)LU, nn, ldlu, perm, w.R32, w.D32, nr, w.tri, false, s);
   if (e != MGT_OK) return e;
   count_launch();
   c64_into_c128_kernel<<<eg, 256, 0, s>>>(w.D32, nr, (double2*)X, ldx, nn, nr, 0);

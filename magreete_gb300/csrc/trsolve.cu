@@ -444,9 +444,11 @@ static int resident_ctas(const void* kern, size_t smem) {
 }
 
 // In-place X = T^-1 X (T = unit lower or upper part of F), nrhs columns.
+// inverses_ready: an earlier call with this workspace, n, nrhs and F made the
+// inverted diagonal blocks and chain factors.
 template <typename T, bool UPPER>
 int tri_solve(const cplx<T>* F, int64_t ldf, cplx<T>* X, int64_t ldx, int n, int nrhs, void* work, int* status,
-              cudaStream_t s) {
+              bool inverses_ready, cudaStream_t s) {
   using V = cplx<T>;
   const size_t smem_inv = (size_t)(kTB * (kTB + 1) + kTB * kInvLd) * sizeof(V);
   const size_t smem = (size_t)(tri_nbuf<T>() * kTB * (kTB + 1) + kTB * kTG) * sizeof(V);
@@ -487,9 +489,11 @@ int tri_solve(const cplx<T>* F, int64_t ldf, cplx<T>* X, int64_t ldx, int n, int
   V* inv = (V*)((char*)work + L.inv) + (UPPER ? (size_t)nb * kTB * kTB : 0);
   V* wch = (V*)((char*)work + L.wch) + (UPPER ? (size_t)nb * kTB * kTB : 0);
   V* part = (V*)((char*)work + L.part);
-  count_launch(2);
-  diag_inverse_kernel<T, UPPER><<<nb, 256, smem_inv, s>>>(F, ldf, n, inv);
-  chain_factor_kernel<T, UPPER><<<nb, 256, smem_cf, s>>>(F, ldf, n, inv, wch);
+  if (!inverses_ready) {
+    count_launch(2);
+    diag_inverse_kernel<T, UPPER><<<nb, 256, smem_inv, s>>>(F, ldf, n, inv);
+    chain_factor_kernel<T, UPPER><<<nb, 256, smem_cf, s>>>(F, ldf, n, inv, wch);
+  }
   unsigned* epoch = counter + 1;   // completion mark, set by tri_start_kernel
   const int nflags = nb * ng * parts;
   const int64_t items = (int64_t)nb * ng * parts;
@@ -530,7 +534,9 @@ int lower_block_inverses(const cplx<T>* F, int64_t ldf, int n, cplx<T>* Inv, cud
 }
 template int lower_block_inverses<float>(const float2*, int64_t, int, float2*, cudaStream_t);
 
-template int tri_solve<float, false>(const float2*, int64_t, float2*, int64_t, int, int, void*, int*, cudaStream_t);
-template int tri_solve<float, true>(const float2*, int64_t, float2*, int64_t, int, int, void*, int*, cudaStream_t);
+template int tri_solve<float, false>(const float2*, int64_t, float2*, int64_t, int, int, void*, int*, bool,
+                                     cudaStream_t);
+template int tri_solve<float, true>(const float2*, int64_t, float2*, int64_t, int, int, void*, int*, bool,
+                                     cudaStream_t);
 
 }  // namespace mgt

@@ -227,7 +227,7 @@ class RefineContext:
 def solve_refined(M, f, B, tol=DEFAULT_TOL, max_iter=DEFAULT_MAX_ITER, require=True):
     """Refined solve of M X = B (B complex128 n x R) with complex64 factors f.
     M: the double-float matrix, or a RefineContext (right-hand sides wider
-    than it was prepared for are solved in blocks of columns).  Returns
+    than it was prepared for are solved in blocks of up to WIDE_NRHS columns).  Returns
     (X, iterations, rel_residual)."""
     if isinstance(M, RefineContext):
         if M.work is None:
@@ -253,28 +253,44 @@ def solve_refined(M, f, B, tol=DEFAULT_TOL, max_iter=DEFAULT_MAX_ITER, require=T
     return X, it.value, rr.value
 
 
+# Columns refined together when there are more than the context's workspace
+# holds: the triangular solves' chain and the residual's pass over M are shared
+# (n = 3750: 4.2 ms for 64 columns, 30 ms for 1024).
+WIDE_NRHS = 1024
+
+
 def _solve_prepared(ctx, f, B, tol, max_iter, require):
     lib = L.load()
     n = f.n
     B = B.contiguous()
     R = B.shape[1]
     X = torch.empty_like(B)
+    width, work = ctx.max_nrhs, ctx.work
+    if R > width:
+        # blocks of equal width, in a workspace of their own
+        width = max(width, -(-R // -(-R // WIDE_NRHS)))
+        nbytes = ctypes.c_size_t()
+        L.check(lib.mgt_refine_scratch_bytes(n, width, ctypes.byref(nbytes)), "mgt_refine_scratch_bytes")
+        work = workspace(nbytes.value, B.device)
     its, sq = [], 0.0
-    for c0 in range(0, R, ctx.max_nrhs):
-        Bc = B[:, c0:c0 + ctx.max_nrhs].contiguous()
-        Xc = torch.empty_like(Bc)
+    for c0 in range(0, R, width):
+        Bc = B if width >= R else B[:, c0:c0 + width].contiguous()
+        Xc = X if width >= R else torch.empty_like(Bc)
         rc = Bc.shape[1]
         it = ctypes.c_int(0)
         rr = ctypes.c_double(0.0)
-        st = lib.mgt_solve_refined(None, n, _ptr(f.lu), f.lu.stride(0), _ptr(f.perm), n, _ptr(Bc), rc, _ptr(Xc), rc,
-                                   rc, float(tol), int(max_iter), _ptr(ctx.work), ctx.work.numel(), ctypes.byref(it),
-                                   ctypes.byref(rr), _stream())
+        args = (_ptr(f.lu), f.lu.stride(0), _ptr(f.perm), n, _ptr(Bc), rc, _ptr(Xc), rc, rc, float(tol), int(max_iter),
+                _ptr(work), work.numel(), ctypes.byref(it), ctypes.byref(rr), _stream())
+        if work is ctx.work:
+            st = lib.mgt_solve_refined(None, n, *args)
+        else:
+            st = lib.mgt_solve_prepared(_ptr(ctx.work), *args)
         if not (st == L.MGT_ERR_NOT_CONVERGED and not require):
             L.check(st, f"mgt_solve_refined (iterations {it.value}, relative residual {rr.value:.3e})")
-        X[:, c0:c0 + rc] = Xc
         its.append(it.value)
         if rc == R:
             return X, it.value, rr.value
+        X[:, c0:c0 + rc] = Xc
         sq += (rr.value * torch.linalg.norm(Bc).item()) ** 2
     nb = torch.linalg.norm(B).item()
     return X, max(its), (sq ** 0.5 / nb if nb > 0 else sq ** 0.5)
