@@ -509,6 +509,10 @@ int tc_make_cmap(CUtensorMap* map, float2* C, int64_t rows, int64_t cols, int64_
              : MGT_ERR_CUDA;
 }
 
+TcSplitOut tc_split_out(const TcPlan& p) {
+  return TcSplitOut{(__half*)p.Ahi, (__half*)p.Alo, (__half*)p.Bhi, (__half*)p.Blo, p.invA, p.invB, tc::KR};
+}
+
 static int tc_num_sms() { return device_sm_count(); }
 
 static void tc_init_attrs() {

@@ -1,6 +1,7 @@
 // tcgen05 (TF32x3) complex trailing update for the complex64 LU.
 #pragma once
 #include <cuda.h>
+#include <cuda_fp16.h>
 
 #include "common.cuh"
 
@@ -42,6 +43,80 @@ int gemm_sub_tc(const TcPlan& plan, const CUtensorMap& cmap, int M, int N, int K
 // the tcgen05 kernel, which reads only the split buffers and the C block.
 int tc_split_a(const TcPlan& plan, int M, int K, const float2* A, int64_t lda, cudaStream_t s);
 int tc_split_b(const TcPlan& plan, int N, int K, const float2* B, int64_t ldb, cudaStream_t s);
+// The F16x2 splits of K = 128 operands, for kernels that have the operands at hand:
+// the plan's buffers (row stride `stride` halves) and inverse scales.
+struct TcSplitOut {
+  __half *ahi, *alo, *bhi, *blo;
+  float *inva, *invb;
+  int stride;
+};
+TcSplitOut tc_split_out(const TcPlan& plan);
+
+// power-of-two exponent e with max 2^-e in [0.5, 1) (0 for zero or non-finite maxima); bits of max given
+__device__ __forceinline__ int tc_scale_exp(unsigned mx) {
+  int e = 0;
+  if (mx != 0u && mx < 0x7F800000u) {
+    frexpf(__uint_as_float(mx), &e);
+    e = max(-120, min(120, e));
+  }
+  return e;
+}
+__device__ __forceinline__ void tc_split2(float x, __half& h, __half& l) {
+  h = __float2half_rn(x);
+  l = __float2half_rn(x - __half2float(h));
+}
+// row i of A: 128 complex values at a, by one warp
+__device__ __forceinline__ void tc_split_row(const TcSplitOut& o, const float2* a, int i, int lane) {
+  float2 v[4];
+  unsigned mx = 0;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    v[j] = a[lane + 32 * j];
+    mx = max(mx, max(__float_as_uint(fabsf(v[j].x)), __float_as_uint(fabsf(v[j].y))));
+  }
+  const int e = tc_scale_exp(__reduce_max_sync(0xffffffffu, mx));
+  const float sc = ldexpf(1.f, -e);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    __half2 h, l;
+    tc_split2(v[j].x * sc, h.x, l.x);
+    tc_split2(v[j].y * sc, h.y, l.y);
+    const int64_t at = (int64_t)i * o.stride + 2 * (lane + 32 * j);
+    *reinterpret_cast<__half2*>(o.ahi + at) = h;
+    *reinterpret_cast<__half2*>(o.alo + at) = l;
+  }
+  if (lane == 0) o.inva[i] = ldexpf(1.f, e);
+}
+// columns col0, col0 + 1, ... of B, 128 complex values each at U[k * ld + c]: QN consecutive threads per column
+template <int QN>
+__device__ __forceinline__ void tc_split_cols(const TcSplitOut& o, const float2* U, int ld, int col0, int tid) {
+  const int c = tid / QN, q = tid % QN;
+  unsigned mx = 0;
+#pragma unroll 8
+  for (int k = q; k < 128; k += QN) {
+    const float2 u = U[k * ld + c];
+    mx = max(mx, max(__float_as_uint(fabsf(u.x)), __float_as_uint(fabsf(u.y))));
+  }
+#pragma unroll
+  for (int off = QN / 2; off; off >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+  const int e = tc_scale_exp(mx);
+  const float sc = ldexpf(1.f, -e);
+  const int64_t row = (int64_t)2 * (col0 + c) * o.stride;
+#pragma unroll 4
+  for (int k = q; k < 128; k += QN) {
+    const float2 u = U[k * ld + c];
+    __half rh, rl, ih, il;
+    tc_split2(u.x * sc, rh, rl);
+    tc_split2(u.y * sc, ih, il);
+    // row 2j: Br, -Bi; row 2j + 1: Bi, Br
+    *reinterpret_cast<__half2*>(o.bhi + row + 2 * k) = __halves2half2(rh, __hneg(ih));
+    *reinterpret_cast<__half2*>(o.blo + row + 2 * k) = __halves2half2(rl, __hneg(il));
+    *reinterpret_cast<__half2*>(o.bhi + row + o.stride + 2 * k) = __halves2half2(ih, rh);
+    *reinterpret_cast<__half2*>(o.blo + row + o.stride + 2 * k) = __halves2half2(il, rl);
+  }
+  if (q == 0) o.invb[col0 + c] = ldexpf(1.f, e);
+}
+
 // bcol: the first column of B (within the split) this launch uses.
 int tc_gemm(const TcPlan& plan, const CUtensorMap& cmap, int M, int N, int K, int cx0, int cy0, int* status,
             cudaStream_t s, int max_ctas = 0, int bcol = 0);

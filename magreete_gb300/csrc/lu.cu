@@ -1706,12 +1706,31 @@ lu_tile_left_perm_kernel(float2* __restrict__ A, int64_t lda, int n, const int32
 
 // Rows below the tile: A21 <- A21 U11^-1 (w columns), 32 rows per CTA; the
 // operands are staged with asynchronous copies (all in flight at once).
+// With Lba, one more CTA applies the tile's interchanges (slots) to its rows of
+// the 64 columns at Lba (the block's first panel).
 __global__ void __launch_bounds__(256)
-lu_l21_kernel(float2* __restrict__ A, int64_t lda, int rows, int w, const float2* __restrict__ Uinv) {
+lu_l21_kernel(float2* __restrict__ A, int64_t lda, int rows, int w, const float2* __restrict__ Uinv,
+              float2* __restrict__ Lba, const int2* __restrict__ slots) {
   // A: first row below the tile, first column of the panel
   __shared__ __align__(16) float2 Ui[64 * 64];
   __shared__ __align__(16) float2 Ar[32 * 64];
   const int tid = threadIdx.x, r0 = blockIdx.x * 32;
+  if (r0 >= rows) {
+    for (int idx = tid; idx < 64 * 64; idx += 256) {
+      const int q = idx >> 6, k = idx & 63;
+      const int src = slots[q].y;
+      const bool in = q < w && src >= 0 && src < w;
+      cp_async_elem<8>(Ui + idx, in ? Lba + (int64_t)src * lda + k : Lba, in);
+    }
+    cp_async_commit();
+    cp_async_wait<0>();
+    __syncthreads();
+    for (int idx = tid; idx < 64 * 64; idx += 256) {
+      const int q = idx >> 6, k = idx & 63;
+      if (q < w && slots[q].y != q) Lba[(int64_t)q * lda + k] = Ui[idx];
+    }
+    return;
+  }
   for (int idx = tid; idx < 64 * 32; idx += 256) cp_async_elem<16>(Ui + 2 * idx, Uinv + 2 * idx, true);
   for (int idx = tid; idx < 32 * 64; idx += 256) {
     const int r = idx >> 6, k = idx & 63;
@@ -1737,6 +1756,120 @@ lu_l21_kernel(float2* __restrict__ A, int64_t lda, int rows, int w, const float2
       if (k < w) A[(int64_t)(r0 + r) * lda + k] = acc[q];
     }
   }
+}
+
+// U12 of the block's second panel: the first tile's interchanges and
+// U12 = L11^-1 A12 on wb columns, four columns per CTA, thread = (row, column).
+__global__ void __launch_bounds__(256)
+lu_tile_u12_kernel(float2* __restrict__ A, int64_t lda, int w, int wb, const int2* __restrict__ slots,
+                   const float2* __restrict__ Linv) {
+  // A: first row of the tile, first column of the second panel
+  __shared__ __align__(16) float2 L[64 * 66];
+  __shared__ float2 X[64][4];
+  const int tid = threadIdx.x, r = tid >> 2, c = tid & 3, col = blockIdx.x * 4 + c;
+  const bool in = r < w && col < wb;
+  cp_async_elem<8>(&X[r][c], in ? A + (int64_t)slots[r].y * lda + col : A, in);
+  for (int idx = tid; idx < 64 * 32; idx += 256)
+    cp_async_elem<16>(L + (idx >> 5) * 66 + 2 * (idx & 31), Linv + 2 * idx, true);
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  float2 a0 = make_float2(0.f, 0.f), a1 = a0;
+  const int end = (tid >> 5) * 8 + 8;   // L11^-1 is lower triangular: the warp's rows end here
+#pragma unroll 4
+  for (int k = 0; k < end; k += 2) {
+    const float4 l = *reinterpret_cast<const float4*>(L + r * 66 + k);
+    cfma(a0, make_float2(l.x, l.y), X[k][c]);
+    cfma(a1, make_float2(l.z, l.w), X[k + 1][c]);
+  }
+  if (in) A[(int64_t)r * lda + col] = cadd(a0, a1);
+}
+
+// Columns right of a 128-wide block, tile pivoting: both tiles' interchanges
+// (rows move only within their tile), U_A = L_AA^-1 X_A, X_B -= L_BA U_A,
+// U_B = L_BB^-1 X_B for CW columns per CTA, every operand loaded at once.
+// With SPLIT the same launch makes the trailing update's F16x2 operands: a
+// column CTA scales and splits its columns of U (zeros up to the update's last
+// 128-column tile), and CTAs from cblocks on split the rows of L21, one per
+// warp -- two launches and a pass over U and L21 less per block.
+template <int CW>
+constexpr size_t tile_right_smem() {
+  return (size_t)(3 * 64 * 65 + 128 * (CW + 1)) * sizeof(float2);
+}
+template <int CW, bool SPLIT>
+__global__ void __launch_bounds__(256)
+lu_tile_right_kernel(float2* __restrict__ A, int64_t lda, int n, int J0, const int2* __restrict__ slotsA,
+                     const int2* __restrict__ slotsB, const float2* __restrict__ Inv, int cblocks, TcSplitOut out) {
+  constexpr int W = 128, LDT = CW + 1, NC = CW / 8, QN = 256 / CW;   // QN threads per column in the split
+  extern __shared__ __align__(16) unsigned char tr_smem[];
+  float2* LA = reinterpret_cast<float2*>(tr_smem);   // [64][65]: L_AA^-1, L_BA, L_BB^-1
+  float2* LBA = LA + 64 * 65;
+  float2* LB = LBA + 64 * 65;
+  float2* Tb = LB + 64 * 65;                          // [128][LDT]
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, P0 = J0 + W;
+  if (SPLIT && (int)blockIdx.x >= cblocks) {
+    const int i = ((int)blockIdx.x - cblocks) * 8 + warp;
+    if (i < n - P0) tc_split_row(out, A + (int64_t)(P0 + i) * lda + J0, i, lane);
+    return;
+  }
+  const int col0 = P0 + blockIdx.x * CW, ncols = min(CW, n - col0);   // ncols <= 0: padding, zeros only
+  for (int idx = tid; idx < W * CW; idx += 256) {
+    const int r = idx / CW, c = idx % CW;
+    const int src = r < 64 ? slotsA[r].y : 64 + slotsB[r - 64].y;
+    const bool ok = c < ncols;
+    cp_async_elem<8>(Tb + r * LDT + c, ok ? A + (int64_t)(J0 + src) * lda + col0 + c : A, ok);
+  }
+  if (ncols > 0)
+    for (int idx = tid; idx < 64 * 64; idx += 256) {
+      const int r = idx >> 6, k = idx & 63, at = r * 65 + k;
+      cp_async_elem<8>(LA + at, Inv + idx, true);
+      cp_async_elem<8>(LBA + at, A + (int64_t)(J0 + 64 + r) * lda + J0 + k, true);
+      cp_async_elem<8>(LB + at, Inv + 64 * 64 + idx, true);
+    }
+  cp_async_commit();
+  cp_async_wait<0>();
+  __syncthreads();
+  if (ncols > 0) {
+    // thread: rows 2 tr, 2 tr + 1 of 64, columns tc + 8 j
+    const int tr = tid >> 3, tc = tid & 7;
+    auto apply = [&](const float2* L, const float2* X, float2* Y, bool sub, int end) {
+      float2 acc[2][NC];
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < NC; ++j) acc[i][j] = sub ? Y[(2 * tr + i) * LDT + tc + 8 * j] : make_float2(0.f, 0.f);
+#pragma unroll 4
+      for (int k = 0; k < end; ++k) {
+        const float2 l0 = L[(2 * tr) * 65 + k], l1 = L[(2 * tr + 1) * 65 + k];
+#pragma unroll
+        for (int j = 0; j < NC; ++j) {
+          const float2 x = X[k * LDT + tc + 8 * j];
+          if (sub) {
+            cfms(acc[0][j], l0, x);
+            cfms(acc[1][j], l1, x);
+          } else {
+            cfma(acc[0][j], l0, x);
+            cfma(acc[1][j], l1, x);
+          }
+        }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < NC; ++j) Y[(2 * tr + i) * LDT + tc + 8 * j] = acc[i][j];
+      __syncthreads();
+    };
+    const int tri = 8 * warp + 8;   // rows of the warp end here: the inverses are lower triangular
+    apply(LA, Tb, Tb, false, tri);
+    apply(LBA, Tb, Tb + 64 * LDT, true, 64);
+    apply(LB, Tb + 64 * LDT, Tb + 64 * LDT, false, tri);
+    for (int idx = tid; idx < W * CW; idx += 256) {
+      const int r = idx / CW, c = idx % CW;
+      if (c < ncols) A[(int64_t)(J0 + r) * lda + col0 + c] = Tb[r * LDT + c];
+    }
+  }
+  if constexpr (SPLIT) tc_split_cols<QN>(out, Tb, LDT, blockIdx.x * CW, tid);
 }
 
 // Largest cluster of register panel CTAs the device schedules (16, 8 or 0).
@@ -1831,7 +1964,8 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
     return std::min(G, gmax > 0 ? std::min(gmax, sms) : sms);
   };
   // factor columns [j0, j0+w) over rows [j0, n); the interchanges go to slot set `set`
-  auto panel_only = [&](int j0, int w, int set, bool with_l21 = true) -> int {
+  // (lba: also their effect on the columns [j0 - 64, j0) of a block's first panel, tile pivoting)
+  auto panel_only = [&](int j0, int w, int set, bool with_l21 = true, bool lba = false) -> int {
     if constexpr (sizeof(T) == 4) {
       if (opt.pivoting == MGT_PIVOT_TILE) {
         LuWsLayout Lw;
@@ -1842,8 +1976,10 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
                                                   Ui, Li);
         count_launch();
         const int below = n - j0 - w;
-        if (below > 0 && with_l21) {
-          lu_l21_kernel<<<(below + 31) / 32, 256, 0, s>>>(A + (int64_t)(j0 + w) * lda + j0, lda, below, w, Ui);
+        if ((below > 0 && with_l21) || lba) {
+          lu_l21_kernel<<<(below + 31) / 32 + (lba ? 1 : 0), 256, 0, s>>>(
+              A + (int64_t)(j0 + w) * lda + j0, lda, below, w, Ui, lba ? A + (int64_t)j0 * lda + j0 - NB : nullptr,
+              panel_ws(work, set).slots);
           count_launch();
         }
         return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
@@ -2033,9 +2169,15 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
   const size_t sm3 = (NB * kSwapCols + NB * (NB + 1) + NB * kSwapCols) * sizeof(V);
   once2([sm3] {
     cudaFuncSetAttribute(lu_preupdate_trsm_kernel<T, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm3);
-    if constexpr (sizeof(T) == 4)
+    if constexpr (sizeof(T) == 4) {
       cudaFuncSetAttribute(lu_block_right_kernel<T, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)block_right_smem<NB>(sizeof(V)));
+      const int t16 = (int)tile_right_smem<16>(), t32 = (int)tile_right_smem<32>();
+      cudaFuncSetAttribute(lu_tile_right_kernel<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, t16);
+      cudaFuncSetAttribute(lu_tile_right_kernel<16, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, t16);
+      cudaFuncSetAttribute(lu_tile_right_kernel<32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, t32);
+      cudaFuncSetAttribute(lu_tile_right_kernel<32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, t32);
+    }
   });
   // Lookahead (cooperative panels, not under stream capture): the trailing
   // update of block J0 first brings the next block's columns up to date, then
@@ -2062,8 +2204,17 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
     if (e != MGT_OK) return e;
     // (tile pivoting) columns left of J0 wait for the final pass; the
     // second panel's rows of the first panel's columns (L_BA, read by the
-    // right-column pass) are swapped here
-    swap(s, J0, wa, 0, defer_left ? J0 : 0, J0, j1, std::min(far, J0 + W), 1);
+    // right-column pass) are swapped with the second panel
+    if (fuse) {
+      if constexpr (sizeof(T) == 4) {
+        lu_tile_u12_kernel<<<(wb + 3) / 4, 256, 0, s>>>(
+            A + (int64_t)J0 * lda + j1, lda, wa, wb, panel_ws(work, 0).slots,
+            reinterpret_cast<const float2*>((char*)work + LuWsLayout().inv));
+        count_launch();
+      }
+    } else {
+      swap(s, J0, wa, 0, defer_left ? J0 : 0, J0, j1, std::min(far, J0 + W), 1);
+    }
     if (wb > 0) {
       if (fuse) {
         if constexpr (sizeof(T) == 4) {
@@ -2076,19 +2227,41 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
       } else {
         e = update(j1, j1, J0, wa, n - j1, wb, false);
       }
-      if (e == MGT_OK) e = panel_only(j1, wb, 1);
+      if (e == MGT_OK) e = panel_only(j1, wb, 1, true, fuse);
       if (e != MGT_OK) return e;
-      swap(s, j1, wb, 1, defer_left ? J0 : 0, j1, 0, 0, 0);
+      if (!fuse) swap(s, j1, wb, 1, 0, j1, 0, 0, 0);
     }
     return MGT_OK;
   };
   // the far-right columns [J0 + W, n) of the block at J0: both panels'
   // interchanges, the first panel's solve, the second panel's pre-update + solve
-  auto block_right = [&](int J0) {
+  // split: the pass also leaves the update's operands in the plan's buffers
+  // (tile pivoting, F16x2); returns whether it did
+  auto block_right = [&](int J0, bool split) -> bool {
     const int W = std::min(2 * NB, n - J0), wa = std::min(NB, W), wb = W - wa, j1 = J0 + wa;
     const int right = n - J0 - W;
-    if (right <= 0) return;
+    if (right <= 0) return false;
     if constexpr (sizeof(T) == 4) {
+      if (defer_left && W == 2 * NB && opt.fused_right) {
+        split = split && tc->plan.mode == MGT_TC_F16X2;
+        const int2 *sa = panel_ws(work, 0).slots, *sb = panel_ws(work, 1).slots;
+        const float2* Inv = reinterpret_cast<const float2*>((char*)work + LuWsLayout().inv);
+        // 16 columns per CTA while that still leaves CTAs for every SM to spare
+        const bool narrow = right <= 32 * sms;
+        const int cw = narrow ? 16 : 32, cols = split ? (right + 127) / 128 * 128 : right, cb = (cols + cw - 1) / cw;
+        const int blocks = cb + (split ? (right + 7) / 8 : 0);
+        const TcSplitOut o = tc_split_out(tc->plan);
+        count_launch();
+        if (narrow && split)
+          lu_tile_right_kernel<16, true><<<blocks, 256, tile_right_smem<16>(), s>>>(A, lda, n, J0, sa, sb, Inv, cb, o);
+        else if (narrow)
+          lu_tile_right_kernel<16, false><<<blocks, 256, tile_right_smem<16>(), s>>>(A, lda, n, J0, sa, sb, Inv, cb, o);
+        else if (split)
+          lu_tile_right_kernel<32, true><<<blocks, 256, tile_right_smem<32>(), s>>>(A, lda, n, J0, sa, sb, Inv, cb, o);
+        else
+          lu_tile_right_kernel<32, false><<<blocks, 256, tile_right_smem<32>(), s>>>(A, lda, n, J0, sa, sb, Inv, cb, o);
+        return split;
+      }
       if (wb > 0 && opt.fused_right) {
         V* Inv = reinterpret_cast<V*>((char*)work + LuWsLayout().inv);
         // tile pivoting: the tile kernels left both diagonal blocks' inverses there
@@ -2096,7 +2269,7 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
         lu_block_right_kernel<T, NB><<<(right + kSwapCols - 1) / kSwapCols, 256, block_right_smem<NB>(sizeof(V)), s>>>(
             A, lda, n, J0, wa, wb, J0 + W, panel_ws(work, 0), panel_ws(work, 1), Inv);
         count_launch();
-        return;
+        return false;
       }
     }
     swap(s, J0, wa, 0, 0, 0, J0 + W, n, 1);
@@ -2106,15 +2279,17 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
                                                                                            wb, J0 + W);
       count_launch();
     }
+    return false;
   };
-  auto lookahead_update = [&](int J0, int W, int P0, int WN, int rest, cudaStream_t s2) -> int {
+  // ready: the pending block's right-column pass made the operand splits
+  auto lookahead_update = [&](int J0, int W, int P0, int WN, int rest, bool ready, cudaStream_t s2) -> int {
     if constexpr (sizeof(T) == 4) {
       const int M = n - P0;
       const float2* L21 = reinterpret_cast<const float2*>(A + (int64_t)P0 * lda + J0);
       const float2* U12 = reinterpret_cast<const float2*>(A + (int64_t)J0 * lda + P0);
       dom_begin(s);
-      int e = tc_split_a(tc->plan, M, W, L21, lda, s);
-      if (e == MGT_OK) e = tc_split_b(tc->plan, WN, W, U12, lda, s);
+      int e = ready ? MGT_OK : tc_split_a(tc->plan, M, W, L21, lda, s);
+      if (e == MGT_OK && !ready) e = tc_split_b(tc->plan, WN, W, U12, lda, s);
       if (e == MGT_OK) e = tc_gemm(tc->plan, tc->cmap, M, WN, W, 2 * P0, P0, ws.status, s);
       dom_end(s, 8.0 * M * (double)WN * W, sizeof(V) * (2.0 * M * (double)WN + (double)M * W + (double)W * WN));
       if (e != MGT_OK) return e;
@@ -2123,7 +2298,8 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
       // the rest's B split on the side stream too (this stream touches no
       // split buffer before the join)
       dom_begin(s2);
-      e = tc_split_b(tc->plan, rest, W, U12 + WN, lda, s2);
+      const int b0 = ready ? WN : 0;   // first column of the rest in the split
+      if (!ready) e = tc_split_b(tc->plan, rest, W, U12 + WN, lda, s2);
       // the first columns beside the next block's panels, on the SMs they
       // leave free; the rest, by when the panels should be done, on every SM
       // (a persistent launch keeps the SMs it started on)
@@ -2133,9 +2309,10 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
       const double head = t_pan * 3e14 * (sms - reserve) / sms / (8.0 * M * (double)W);
       const int c1 = (int)std::min<double>(rest, (std::floor(head / (2 * NB)) + 1) * (2 * NB));
       if (e == MGT_OK)
-        e = tc_gemm(tc->plan, tc->cmap, M, c1, W, 2 * (P0 + WN), P0, ws.status, s2, std::max(1, sms - reserve));
+        e = tc_gemm(tc->plan, tc->cmap, M, c1, W, 2 * (P0 + WN), P0, ws.status, s2, std::max(1, sms - reserve),
+                    b0);
       if (e == MGT_OK && c1 < rest)
-        e = tc_gemm(tc->plan, tc->cmap, M, rest - c1, W, 2 * (P0 + WN + c1), P0, ws.status, s2, 0, c1);
+        e = tc_gemm(tc->plan, tc->cmap, M, rest - c1, W, 2 * (P0 + WN + c1), P0, ws.status, s2, 0, b0 + c1);
       dom_end(s2, 8.0 * M * (double)rest * W, sizeof(V) * (2.0 * M * (double)rest + (double)W * rest));
       // once forked, the join is recorded whatever happened
       const bool joined = cudaEventRecord(side->join, s2) == cudaSuccess;
@@ -2153,14 +2330,14 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
   // product with K = 256 (half the C traffic per flop of two K = 128
   // updates).  Tile pivoting moves Y's rows only within Y's tiles, every one
   // of which already carries X's update.
-  auto pair_update = [&](int X0, int Y0, int WY) -> int {
+  auto pair_update = [&](int X0, int Y0, int WY, bool ready) -> int {
     if constexpr (sizeof(T) == 4) {
       const int KX = Y0 - X0, M = n - Y0, far0 = Y0 + WY, nfar = n - far0;
       const float2* L21 = reinterpret_cast<const float2*>(A + (int64_t)Y0 * lda + X0);
       const float2* U12 = reinterpret_cast<const float2*>(A + (int64_t)X0 * lda + Y0);
       dom_begin(s);
-      int e = tc_split_a(tc->plan, M, KX, L21, lda, s);
-      if (e == MGT_OK) e = tc_split_b(tc->plan, WY + nfar, KX, U12, lda, s);
+      int e = ready ? MGT_OK : tc_split_a(tc->plan, M, KX, L21, lda, s);
+      if (e == MGT_OK && !ready) e = tc_split_b(tc->plan, WY + nfar, KX, U12, lda, s);
       if (e == MGT_OK) e = tc_gemm(tc->plan, tc->cmap, M, WY, KX, 2 * Y0, Y0, ws.status, s);
       // Y's rows are the first WY rows of the split L21
       if (e == MGT_OK && nfar > 0)
@@ -2177,7 +2354,7 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
   const bool pairs = sizeof(T) == 4 && opt.pivoting == MGT_PIVOT_TILE && opt.wide_min > 0;
   int e = block_panels(0, n);
   if (e != MGT_OK) return e;
-  block_right(0);
+  bool ready = block_right(0, true);   // the pending update's operand splits are made
   // the factored columns [K0, K0 + KW) (one block, or a pair) whose update of
   // the trailing matrix is pending
   int K0 = 0, KW = std::min(2 * NB, n);
@@ -2191,28 +2368,37 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
     const bool overlap = side != nullptr && rest > 0 &&
                          (opt.pivoting == MGT_PIVOT_TILE || sms - panel_ctas(n - P0) >= 16);
     if (!overlap) {
-      e = update(P0, P0, K0, KW, n - P0, n - P0, true);
+      if (ready) {
+        if constexpr (sizeof(T) == 4) {
+          const int M = n - P0;
+          dom_begin(s);
+          e = tc_gemm(tc->plan, tc->cmap, M, M, KW, 2 * P0, P0, ws.status, s);
+          dom_end(s, 8.0 * M * (double)M * KW, sizeof(V) * (2.0 * M * (double)M + 2.0 * (double)M * KW));
+        }
+      } else {
+        e = update(P0, P0, K0, KW, n - P0, n - P0, true);
+      }
       if (e == MGT_OK) e = block_panels(P0, n);
       if (e != MGT_OK) return e;
     } else {
       // A[P0:, P0:] -= L21 U12 of the pending columns: the operand splits (the
       // rows of L21 are permuted by the next panels' interchanges) and the
       // next block's columns here; the rest of the update on the side stream
-      e = lookahead_update(K0, KW, P0, WN, rest, side->s);
+      e = lookahead_update(K0, KW, P0, WN, rest, ready, side->s);
       if (e == MGT_OK) e = block_panels(P0, P0 + WN);
       // always join: nothing of the side stream may outlive this call
       if (cudaStreamWaitEvent(s, side->join, 0) != cudaSuccess && e == MGT_OK) e = MGT_ERR_CUDA;
       if (e != MGT_OK) return e;
     }
-    block_right(P0);
+    ready = block_right(P0, true);
     K0 = P0;
     KW = WN;
     const int Y0 = P0 + WN, WY = std::min(2 * NB, n - Y0);
     if (pairs && WN == 2 * NB && WY == 2 * NB && n - P0 >= opt.wide_min) {
-      e = pair_update(P0, Y0, WY);
+      e = pair_update(P0, Y0, WY, ready);
       if (e == MGT_OK) e = block_panels(Y0, n);
       if (e != MGT_OK) return e;
-      block_right(Y0);
+      ready = block_right(Y0, false);   // the pair's K = 256 product has scales of its own
       KW = WN + WY;
     }
   }
