@@ -113,13 +113,14 @@ int mgt_lu_factor(int dtype, void* A, int64_t n, int64_t lda, int32_t* perm,
  *             of the column, lowest row on ties; the reference's pivot
  *             sequence).  MGT_PIVOT_TILE (complex64 only): each 64-column
  *             panel chooses its pivots among the 64 rows of its diagonal
- *             tile; the rows below are solved against the tile's U
- *             (L21 = A21 U11^-1), so no panel needs any exchange between
- *             CTAs.  P A = L U still holds; the growth of the factors is not
- *             bounded like partial pivoting's, so it is meant for the mixed
- *             method, whose refinement certifies the solution (callers fall
- *             back to partial pivoting when it does not converge).  An exact
- *             zero tile pivot sets info as a zero pivot does.
+ *             tile (largest |re|+|im| to 17 bits); the rows below are solved
+ *             against the tile's U (L21 = A21 U11^-1), so no panel needs any
+ *             exchange between CTAs.  P A = L U still holds; the growth of the
+ *             factors is not bounded like partial pivoting's, so it is meant
+ *             for the mixed method, whose refinement certifies the solution
+ *             (callers fall back to partial pivoting when it does not
+ *             converge).  An exact zero tile pivot sets info as a zero pivot
+ *             does.
  *   panel_rows, panel_max_ctas, cooperative, lookahead, outer_block: as the
  *             MGT_TUNE_* keys of the same names (cooperative / lookahead: -1 =
  *             process value; outer_block 64 or 128)

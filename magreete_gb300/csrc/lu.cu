@@ -1305,7 +1305,7 @@ static int resolve_lu_options(const mgt_lu_options* o, LuOpts* r) {
 // matrices of this engine rarely need a pivot from outside the tile (LAPACK
 // swaps a few rows in a thousand there); the growth that remains is what
 // iterative refinement absorbs.
-constexpr int kTileLD = 65;   // padded row stride of the tile in shared memory
+constexpr int kTileLD = 66;   // padded row stride of the tile in shared memory (even: pairs of entries load at once)
 // dynamic shared memory of lu_tile_kernel: the tile by row (then U^-1), by position, L^-1, block scratch
 constexpr size_t kTileSmem = (3 * 64 * kTileLD + 6 * 256) * sizeof(float2);
 
@@ -1327,8 +1327,19 @@ __device__ __forceinline__ float2 crecip_tile(float2 z) {
   return make_float2(r * inv, -inv);
 }
 
+// the same for |z|^2 in the normal range (the caller checks): an approximate
+// reciprocal (2 ulp) with one Newton step, 80 clocks less than a correctly
+// rounded one on the chain of pivots
+__device__ __forceinline__ float2 crecip_fast(float2 z) {
+  const float d = fmaf(z.x, z.x, z.y * z.y);
+  float r = __fdividef(1.f, d);
+  r = fmaf(r, fmaf(-d, r, 1.f), r);
+  return make_float2(z.x * r, -z.y * r);
+}
+
 constexpr int kTileThreads = 512;
-constexpr int kTileBar = 32 + 14 * 32;   // threads of the tile's named barriers: warp 0 and 14 update warps
+constexpr int kTileWorkers = 12;                     // update warps: those that do not share warp 0's scheduler
+constexpr int kTileBar = 32 + kTileWorkers * 32;     // threads of the tile's named barriers
 
 __device__ __forceinline__ void bar_sync_n(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kTileBar) : "memory"); }
 __device__ __forceinline__ void bar_arrive_n(int id) {
@@ -1344,30 +1355,25 @@ __device__ __forceinline__ void tile_inverses(const float2* F, float2* UI, float
                                               int tid) {
   const int warp = tid >> 5, lane = tid & 31;
   if (warp < 8 && lane < 16) {
-    const int b = (warp & 3) * 16, c = lane;
+    // Columns of the inverse, one per lane, right-looking.  L's blocks read from
+    // the last row and column backwards are upper triangular with a unit
+    // diagonal: one piece of code for both.
+    const int b = (warp & 3) * 16;
+    const bool up = warp < 4;
+    const float2* f = up ? F + b * kTileLD + b : F + (b + 15) * kTileLD + b + 15;
+    const int rs = up ? kTileLD : -kTileLD, cs = up ? 1 : -1;
     float2 x[16];
-    if (warp < 4) {
 #pragma unroll
-      for (int i = 15; i >= 0; --i) {
-        float2 s = make_float2(0.f, 0.f);
+    for (int i = 0; i < 16; ++i) x[i] = make_float2(i == lane ? 1.f : 0.f, 0.f);
 #pragma unroll
-        for (int k = i + 1; k < 16; ++k) cfms(s, F[(b + i) * kTileLD + b + k], x[k]);
-        const float2 d = dinv[b + i];
-        x[i] = i == c ? d : i < c ? cmul(s, d) : make_float2(0.f, 0.f);
-      }
+    for (int i = 15; i >= 0; --i) {
+      if (up) x[i] = cmul(x[i], dinv[b + i]);
 #pragma unroll
-      for (int i = 0; i < 16; ++i) UI[(b + i) * kTileLD + b + c] = x[i];
-    } else {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        float2 s = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int k = 0; k < i; ++k) cfms(s, F[(b + i) * kTileLD + b + k], x[k]);
-        x[i] = i == c ? make_float2(1.f, 0.f) : i > c ? s : make_float2(0.f, 0.f);
-      }
-#pragma unroll
-      for (int i = 0; i < 16; ++i) LI[(b + i) * kTileLD + b + c] = x[i];
+      for (int k = 0; k < i; ++k) cfms(x[k], f[k * rs + i * cs], x[i]);
     }
+    float2* out = up ? UI + b * kTileLD + b + lane : LI + (b + 15) * kTileLD + b + 15 - lane;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) out[i * rs] = x[i];
   }
   __syncthreads();
   const bool upper = tid < 256;
@@ -1386,8 +1392,9 @@ __device__ __forceinline__ void tile_inverses(const float2* F, float2* UI, float
       float2 s0 = make_float2(0.f, 0.f), s1 = s0;
 #pragma unroll 8
       for (int k = 0; k < 16 * d; k += 2) {
-        cfms(s0, f[k], x[k * kTileLD]);
-        cfms(s1, f[k + 1], x[(k + 1) * kTileLD]);
+        const float4 v = *reinterpret_cast<const float4*>(f + k);
+        cfms(s0, make_float2(v.x, v.y), x[k * kTileLD]);
+        cfms(s1, make_float2(v.z, v.w), x[(k + 1) * kTileLD]);
       }
       Sq[q * 256 + t] = cadd(s0, s1);
     }
@@ -1400,8 +1407,9 @@ __device__ __forceinline__ void tile_inverses(const float2* F, float2* UI, float
       float2 s0 = make_float2(0.f, 0.f), s1 = s0;
 #pragma unroll
       for (int k = 0; k < 16; k += 2) {
-        cfma(s0, f[k], x[k * 16]);
-        cfma(s1, f[k + 1], x[(k + 1) * 16]);
+        const float4 v = *reinterpret_cast<const float4*>(f + k);
+        cfma(s0, make_float2(v.x, v.y), x[k * 16]);
+        cfma(s1, make_float2(v.z, v.w), x[(k + 1) * 16]);
       }
       (upper ? I[(i + r) * kTileLD + j + c] : I[(j + r) * kTileLD + i + c]) = cadd(s0, s1);
     }
@@ -1413,16 +1421,18 @@ __device__ __forceinline__ void tile_inverses(const float2* F, float2* UI, float
 // U11^-1 and L11^-1, for the rows below (L21 = A21 U11^-1) and the columns to
 // the right (U12 = L11^-1 A12).  Bound by the chain of 64 pivots, so that
 // chain is one warp's: warp 0, lane = tile rows lane and lane + 32, factors
-// four columns at a time in registers (per column two warp reductions pick the
-// pivot, shuffles broadcast its row, every lane computes its reciprocal) and
-// brings the next four up to date itself, while warps 1 .. 14 apply the four
-// pivots to the columns beyond (8 columns x half of the rows per warp).  Two
-// pairs of named barriers, by parity, hand the work over: (1, 3) four columns
-// are factored, (2, 4) the columns beyond are updated.
+// four columns at a time in registers (per column one warp reduction picks the
+// pivot, shuffles broadcast its row and reciprocal) and brings the next four up
+// to date itself, while twelve warps on the other schedulers apply the four
+// pivots to the columns beyond.  Two pairs of named barriers, by parity, hand
+// the work over: (1, 3) four columns are factored, (2, 4) the columns beyond
+// are updated.
 // Rows never move: s_piv[c] is the tile row chosen at column c, s_state its
 // inverse (64: not chosen yet); rows of U go to F by position.
-// Measured: a version with one block barrier per column 57 us; 775 clocks a
-// column when warp 0 took 16 columns at a time.
+// Measured at w = 64: 31 us (59 K clocks: the pivot chain 25 K, warp 0's next
+// four columns 8 K, the inverses 17 K); with the largest value and its row found
+// by two reductions and update warps on warp 0's scheduler too 38 us; with one
+// block barrier per column 57 us.
 __global__ void __launch_bounds__(kTileThreads, 1)
 lu_tile_kernel(float2* __restrict__ A, int64_t lda, int w, int j0, int32_t* __restrict__ perm, PanelWs ws,
                float2* __restrict__ Uinv, float2* __restrict__ Linv) {
@@ -1464,32 +1474,41 @@ lu_tile_kernel(float2* __restrict__ A, int64_t lda, int w, int j0, int32_t* __re
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         if (c0 + u < w) {
-          // key 0 = no bid; +1 keeps the rows of a zero column valid bidders
-          const uint32_t k0 = act0 ? __float_as_uint(fabsf(a0[u].x) + fabsf(a0[u].y)) + 1u : 0u;
-          const uint32_t k1 = act1 ? __float_as_uint(fabsf(a1[u].x) + fabsf(a1[u].y)) + 1u : 0u;
+          // One reduction picks the pivot: the leading 26 bits of |re| + |im| over
+          // the row (lowest on ties); 0 = no bid, + 1 keeps the rows of a zero
+          // column valid bidders.  Every lane makes its own candidates'
+          // reciprocals meanwhile.
+          const uint32_t k0 =
+              act0 ? (((__float_as_uint(fabsf(a0[u].x) + fabsf(a0[u].y)) >> 6) + 1u) << 6) | (63u - (uint32_t)lane) : 0u;
+          const uint32_t k1 =
+              act1 ? (((__float_as_uint(fabsf(a1[u].x) + fabsf(a1[u].y)) >> 6) + 1u) << 6) | (31u - (uint32_t)lane) : 0u;
           const uint32_t mx = __reduce_max_sync(0xffffffffu, max(k0, k1));
-          p[u] = (int)__reduce_min_sync(0xffffffffu,
-                                        k0 == mx ? (uint32_t)lane : k1 == mx ? (uint32_t)lane + 32u : 64u);
+          const float2 r0 = crecip_fast(a0[u]), r1 = crecip_fast(a1[u]);
+          p[u] = 63 - (int)(mx & 63u);
           const int src = p[u] & 31;
           const bool hi = p[u] >= 32;
-          float2 prow[4];
+          float2 prow[4], inv;
+          inv.x = __shfl_sync(0xffffffffu, hi ? r1.x : r0.x, src);
+          inv.y = __shfl_sync(0xffffffffu, hi ? r1.y : r0.y, src);
 #pragma unroll
           for (int k = u; k < 4; ++k) {
             prow[k].x = __shfl_sync(0xffffffffu, hi ? a1[k].x : a0[k].x, src);
             prow[k].y = __shfl_sync(0xffffffffu, hi ? a1[k].y : a0[k].y, src);
           }
-          const bool zero = prow[u].x == 0.f && prow[u].y == 0.f;
-          const float2 inv = zero ? make_float2(0.f, 0.f) : crecip_tile(prow[u]);
-          if (lane == src) (hi ? act1 : act0) = false;
-          if (act0) {
-            a0[u] = cmul(a0[u], inv);
+          const float m = fmaxf(fabsf(prow[u].x), fabsf(prow[u].y));
+          const bool zero = m == 0.f;
+          if (!(m > 1e-15f && m < 1e15f)) inv = zero ? make_float2(0.f, 0.f) : crecip_tile(prow[u]);
+          act0 = act0 && p[u] != lane;
+          act1 = act1 && p[u] != lane + 32;
+          // retired rows take a zero multiplier (no branches on the chain)
+          const float2 l0 = act0 ? cmul(a0[u], inv) : make_float2(0.f, 0.f);
+          const float2 l1 = act1 ? cmul(a1[u], inv) : make_float2(0.f, 0.f);
+          if (act0) a0[u] = l0;
+          if (act1) a1[u] = l1;
 #pragma unroll
-            for (int k = u + 1; k < 4; ++k) cfms(a0[k], a0[u], prow[k]);
-          }
-          if (act1) {
-            a1[u] = cmul(a1[u], inv);
-#pragma unroll
-            for (int k = u + 1; k < 4; ++k) cfms(a1[k], a1[u], prow[k]);
+          for (int k = u + 1; k < 4; ++k) {
+            cfms(a0[k], l0, prow[k]);
+            cfms(a1[k], l1, prow[k]);
           }
           if (lane == 0) {
             s_piv[c0 + u] = p[u];
@@ -1500,9 +1519,10 @@ lu_tile_kernel(float2* __restrict__ A, int64_t lda, int w, int j0, int32_t* __re
         }
       }
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        T[lane * kTileLD + c0 + u] = a0[u];
-        T[(lane + 32) * kTileLD + c0 + u] = a1[u];
+      for (int u = 0; u < 4; u += 2) {
+        *reinterpret_cast<float4*>(T + lane * kTileLD + c0 + u) = make_float4(a0[u].x, a0[u].y, a0[u + 1].x, a0[u + 1].y);
+        *reinterpret_cast<float4*>(T + (lane + 32) * kTileLD + c0 + u) =
+            make_float4(a1[u].x, a1[u].y, a1[u + 1].x, a1[u + 1].y);
       }
       __syncwarp();
       bar_arrive_n(1 + 2 * (s & 1));
@@ -1544,12 +1564,15 @@ lu_tile_kernel(float2* __restrict__ A, int64_t lda, int w, int j0, int32_t* __re
     }
     // the barriers of the last two updates are completed too
     for (int s = max(0, steps - 2); s < steps; ++s) bar_sync_n(2 + 2 * (s & 1));
-  } else if (warp < 15) {
-    const int ww = warp - 1, half = ww / 7, rg = lane >> 3;
+  } else if (warp & 3) {
+    const int ww = 3 * (warp >> 2) + (warp & 3) - 1, rg = lane >> 3;
     for (int s = 0; s < steps; ++s) {
-      const int c0 = 4 * s, j = c0 + 8 + (ww % 7) * 8 + (lane & 7);
+      const int c0 = 4 * s;
       bar_sync_n(1 + 2 * (s & 1));
-      if (j < w) {
+      // a task: eight columns x every second group of four rows
+      for (int t = ww; t < 14; t += kTileWorkers) {
+        const int half = t & 1, j = c0 + 8 + (t >> 1) * 8 + (lane & 7);
+        if (j >= w) continue;
         float2 u[4];
 #pragma unroll
         for (int k = 0; k < 4; ++k) {
