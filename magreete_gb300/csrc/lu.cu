@@ -21,6 +21,7 @@
 #include "common.cuh"
 #include "gemm.cuh"
 #include "gemm_tc.cuh"
+#include "tile_inverse.cuh"
 #include "diag.cuh"
 #include "zgemm_tc.cuh"
 #include "zpanel.cuh"
@@ -1056,8 +1057,7 @@ lu_preupdate_trsm_kernel(cplx<T>* __restrict__ A, int64_t lda, int n, int J0, in
   }
 }
 
-template <typename T>
-int lower_block_inverses(const cplx<T>* F, int64_t ldf, int n, cplx<T>* Inv, cudaStream_t s);
+int lower_block_inverses(const float2* F, int64_t ldf, int n, float2* Inv, cudaStream_t s);
 
 // dynamic shared memory of lu_block_right_kernel: block rows, moved rows, one operator
 template <int NB>
@@ -1305,7 +1305,6 @@ static int resolve_lu_options(const mgt_lu_options* o, LuOpts* r) {
 // matrices of this engine rarely need a pivot from outside the tile (LAPACK
 // swaps a few rows in a thousand there); the growth that remains is what
 // iterative refinement absorbs.
-constexpr int kTileLD = 66;   // padded row stride of the tile in shared memory (even: pairs of entries load at once)
 // dynamic shared memory of lu_tile_kernel: the tile by row (then U^-1), by position, L^-1, block scratch
 constexpr size_t kTileSmem = (3 * 64 * kTileLD + 6 * 256) * sizeof(float2);
 
@@ -1337,84 +1336,12 @@ __device__ __forceinline__ float2 crecip_fast(float2 z) {
   return make_float2(z.x * r, -z.y * r);
 }
 
-constexpr int kTileThreads = 512;
 constexpr int kTileWorkers = 12;                     // update warps: those that do not share warp 0's scheduler
 constexpr int kTileBar = 32 + kTileWorkers * 32;     // threads of the tile's named barriers
 
 __device__ __forceinline__ void bar_sync_n(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kTileBar) : "memory"); }
 __device__ __forceinline__ void bar_arrive_n(int id) {
   asm volatile("bar.arrive %0, %1;" ::"r"(id), "n"(kTileBar) : "memory");
-}
-
-// UI = U^-1 (upper, diagonal reciprocals given) and LI = L^-1 (unit lower) of
-// the 64 x 64 tile F by 16 x 16 blocks: the eight diagonal blocks by
-// substitution, one per warp, then the block diagonals outwards:
-// UI_ij = -UI_ii sum_k U_ik UI_kj by threads 0 .. 255 and likewise L by the
-// others.  S: 6 x 256 scratch.  Only the triangles' blocks are written.
-__device__ __forceinline__ void tile_inverses(const float2* F, float2* UI, float2* LI, float2* S, const float2* dinv,
-                                              int tid) {
-  const int warp = tid >> 5, lane = tid & 31;
-  if (warp < 8 && lane < 16) {
-    // Columns of the inverse, one per lane, right-looking.  L's blocks read from
-    // the last row and column backwards are upper triangular with a unit
-    // diagonal: one piece of code for both.
-    const int b = (warp & 3) * 16;
-    const bool up = warp < 4;
-    const float2* f = up ? F + b * kTileLD + b : F + (b + 15) * kTileLD + b + 15;
-    const int rs = up ? kTileLD : -kTileLD, cs = up ? 1 : -1;
-    float2 x[16];
-#pragma unroll
-    for (int i = 0; i < 16; ++i) x[i] = make_float2(i == lane ? 1.f : 0.f, 0.f);
-#pragma unroll
-    for (int i = 15; i >= 0; --i) {
-      if (up) x[i] = cmul(x[i], dinv[b + i]);
-#pragma unroll
-      for (int k = 0; k < i; ++k) cfms(x[k], f[k * rs + i * cs], x[i]);
-    }
-    float2* out = up ? UI + b * kTileLD + b + lane : LI + (b + 15) * kTileLD + b + 15 - lane;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) out[i * rs] = x[i];
-  }
-  __syncthreads();
-  const bool upper = tid < 256;
-  const int t = tid & 255, r = t >> 4, c = t & 15;   // this thread's entry of every block
-  float2* I = upper ? UI : LI;
-  float2* Sq = S + (upper ? 0 : 3 * 256);
-#pragma unroll 1
-  for (int d = 1; d < 4; ++d) {
-    const int np = 4 - d;
-#pragma unroll 1
-    for (int q = 0; q < np; ++q) {
-      // U: row block i, column block i + 16 d; L: the mirror image
-      const int i = 16 * q, j = 16 * (q + d);
-      const float2* f = upper ? F + (i + r) * kTileLD + i + 16 : F + (j + r) * kTileLD + i;
-      const float2* x = upper ? I + (i + 16) * kTileLD + j + c : I + i * kTileLD + i + c;
-      float2 s0 = make_float2(0.f, 0.f), s1 = s0;
-#pragma unroll 8
-      for (int k = 0; k < 16 * d; k += 2) {
-        const float4 v = *reinterpret_cast<const float4*>(f + k);
-        cfms(s0, make_float2(v.x, v.y), x[k * kTileLD]);
-        cfms(s1, make_float2(v.z, v.w), x[(k + 1) * kTileLD]);
-      }
-      Sq[q * 256 + t] = cadd(s0, s1);
-    }
-    __syncthreads();
-#pragma unroll 1
-    for (int q = 0; q < np; ++q) {
-      const int i = 16 * q, j = 16 * (q + d);
-      const float2* f = upper ? I + (i + r) * kTileLD + i : I + (j + r) * kTileLD + j;
-      const float2* x = Sq + q * 256 + c;
-      float2 s0 = make_float2(0.f, 0.f), s1 = s0;
-#pragma unroll
-      for (int k = 0; k < 16; k += 2) {
-        const float4 v = *reinterpret_cast<const float4*>(f + k);
-        cfma(s0, make_float2(v.x, v.y), x[k * 16]);
-        cfma(s1, make_float2(v.z, v.w), x[(k + 1) * 16]);
-      }
-      (upper ? I[(i + r) * kTileLD + j + c] : I[(j + r) * kTileLD + i + c]) = cadd(s0, s1);
-    }
-    __syncthreads();
-  }
 }
 
 // One CTA: the w x w tile's LU with partial pivoting among its rows, then
@@ -2288,7 +2215,7 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
       if (wb > 0 && opt.fused_right) {
         V* Inv = reinterpret_cast<V*>((char*)work + LuWsLayout().inv);
         // tile pivoting: the tile kernels left both diagonal blocks' inverses there
-        if (opt.pivoting != MGT_PIVOT_TILE) lower_block_inverses<T>(A + (int64_t)J0 * lda + J0, lda, W, Inv, s);
+        if (opt.pivoting != MGT_PIVOT_TILE) lower_block_inverses(A + (int64_t)J0 * lda + J0, lda, W, Inv, s);
         lu_block_right_kernel<T, NB><<<(right + kSwapCols - 1) / kSwapCols, 256, block_right_smem<NB>(sizeof(V)), s>>>(
             A, lda, n, J0, wa, wb, J0 + W, panel_ws(work, 0), panel_ws(work, 1), Inv);
         count_launch();
@@ -2493,10 +2420,9 @@ __global__ void permute_rows_kernel(const V* __restrict__ B, int64_t ldb, const 
   if (i < n && c < nrhs) X[(int64_t)i * ldx + c] = B[(int64_t)perm[i] * ldb + c];
 }
 
-template <typename T, bool UPPER>
-int tri_solve(const cplx<T>* F, int64_t ldf, cplx<T>* X, int64_t ldx, int n, int nrhs, void* work, int* status,
-              bool inverses_ready, cudaStream_t s);
-size_t tri_solve_workspace_bytes(int64_t n, int64_t nrhs, size_t elem);
+int tri_solve(const float2* F, int64_t ldf, float2* X, int64_t ldx, int n, int nrhs, void* work, bool inverses_ready,
+              cudaStream_t s);
+size_t tri_solve_workspace_bytes(int64_t n);
 
 template <typename T>
 static int lu_solve_impl(const cplx<T>* LU, int n, int64_t lda, const int32_t* perm, const cplx<T>* B,
@@ -2511,12 +2437,8 @@ static int lu_solve_impl(const cplx<T>* LU, int n, int64_t lda, const int32_t* p
       // one tensor-core product per 64-row block
       return zsolve(LU, lda, X, ldx, n, nrhs, work, s);
     } else {
-      // persistent flag-ordered triangular solves (one launch per triangle and 64 columns)
-      int* status = (int*)((char*)work + 128);
-      if (cudaMemsetAsync(status, 0, 2 * sizeof(int), s) != cudaSuccess) return MGT_ERR_CUDA;
-      int e = tri_solve<T, false>(LU, lda, X, ldx, n, nrhs, work, status, inverses_ready, s);
-      if (e == MGT_OK) e = tri_solve<T, true>(LU, lda, X, ldx, n, nrhs, work, status, inverses_ready, s);
-      return e;
+      // one launch per 256-row block and triangle
+      return tri_solve(LU, lda, X, ldx, n, nrhs, work, inverses_ready, s);
     }
   }
   constexpr int BS = 64;
@@ -2630,7 +2552,7 @@ extern "C" int mgt_lu_factor(int dtype, void* A, int64_t n, int64_t lda, int32_t
 }
 
 static size_t lu_solve_bytes(int dtype, int64_t n, int64_t nrhs) {
-  return dtype == MGT_C128 ? zsolve_workspace_bytes(n, nrhs) : tri_solve_workspace_bytes(n, nrhs, sizeof(float2));
+  return dtype == MGT_C128 ? zsolve_workspace_bytes(n, nrhs) : tri_solve_workspace_bytes(n);
 }
 
 extern "C" int mgt_lu_solve_workspace_bytes(int dtype, int64_t n, int64_t nrhs, size_t* bytes) {

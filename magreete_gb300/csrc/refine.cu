@@ -274,7 +274,7 @@ static int residual_impl(const float4* M, int64_t ldm, const double2* X, int64_t
   return residual_rect(M, ldm, Xs, nrhs, B, ldb, R, ldr, n, n, nrhs, s, part, part_elems);
 }
 
-size_t tri_solve_workspace_bytes(int64_t n, int64_t nrhs, size_t elem);
+size_t tri_solve_workspace_bytes(int64_t n);
 
 // refinement workspace layout: the residual runs on the tensor cores
 // (residual_tc.cu) where the device and shape allow, in double-float on the
@@ -286,7 +286,7 @@ struct RefineWs {
   float2* R32;    // n x nrhs complex64 residual / right-hand side
   float2* D32;    // n x nrhs complex64 correction
   double* norms;  // [0] = ||B||^2, [1] = ||R||^2
-  void* tri;      // triangular-solve flags
+  void* tri;      // triangular solves: inverted diagonal blocks
   double2* part;  // (double-float residual) split-K partial sums
   int64_t part_elems;
   int* rowexp;    // (tensor-core residual) row exponents of M
@@ -320,7 +320,7 @@ struct RefineWs {
     R32 = (float2*)take(n * r * sizeof(float2));
     D32 = (float2*)take(n * r * sizeof(float2));
     norms = (double*)take(2 * sizeof(double));
-    tri = take(tri_solve_workspace_bytes(n, r, sizeof(float2)));
+    tri = take(tri_solve_workspace_bytes(n));
     Xs = nullptr;
     part = nullptr;
     part_elems = 0;

@@ -1,542 +1,871 @@
-// K3: multi-RHS triangular solves with the LU factors, one persistent launch
-// per triangle (the ?getrs half of torch.linalg.solve in solve(),
-// Transmission2D.py:230 / Transmission3D.py:205).
+// K3: complex64 multi-RHS triangular solves with the LU factors (the ?getrs
+// half of torch.linalg.solve in solve(), Transmission2D.py:230 /
+// Transmission3D.py:205).
 //
-// Block rows of 64.  CTAs claim block rows in dependency order from an
-// atomic counter (first row first for L, last row first for U).  A CTA
-// accumulates B_i - sum_j T_ij X_j over the blocks j its row depends on,
-// waiting (bounded) on each X_j's ready flag as it goes, then solves the
-// 64 x 64 diagonal block in shared memory, writes X_i and releases its flag.
-// Rows that depend on many blocks do their updates while earlier rows are
-// still being solved, so the solve costs about one block step per block row
-// instead of four kernel launches per block row.  No CTA waits on a row that
-// was not claimed earlier by a running CTA, so progress is guaranteed.
+// Block rows of 256, right-looking, one launch per block row: launch i
+// subtracts T_ki X_i from every block row k that depends on it, and the
+// cluster that holds the next block row goes on to X_k = T_kk^-1 B_k.  The
+// inverses of the 256 x 256 diagonal blocks are made first: 64 x 64 blocks by
+// substitution, doubled twice.
+//
+// What bounds a solve of few columns is the chain from block row to block row
+// (n / 256 per triangle), then the factor's bytes; so a launch is one
+// eight-CTA cluster per block row and 32 columns -- two halves of 128 rows,
+// the K = 256 split over four CTAs, their sums exchanged through distributed
+// shared memory -- and starts while its predecessor runs (programmatic
+// dependent launch): barriers, tensor memory, the factor's block and its
+// conversion are done before it waits for X_i.
+//
+// Products on the tensor cores: both operands scaled by a power of two (each
+// row of the factor's tile, each right-hand side) and split into two fp16
+// parts, x = h + 2^-11 l, each rounded to nearest, so that h and l keep the
+// full 22 bits down to 2^-28 of the largest value; the four part products
+// accumulate in FP32 by weight (h h | h l + l h | l l).
+//
+// Measured, LU solve of 64 columns with the inverses made (ms): n = 2000 0.26,
+// 6000 0.90, 12000 2.14; work items of 64-row blocks claimed by persistent CTAs,
+// products on the FP32 pipe: 0.54, 1.66, 3.93.  A step takes 11 us on the chain
+// (two products, each with its exchange of partial sums); from n = 6000 on the
+// block rows beyond take as long or longer (12000: 20 us).
+#include <cuda_fp16.h>
+
 #include <algorithm>
 #include <mutex>
 
 #include "common.cuh"
 #include "diag.cuh"
+#include "tcgen05.cuh"
+#include "tile_inverse.cuh"
 
 namespace mgt {
 
-constexpr int kTB = 64;      // block rows
-constexpr int kTG = 16;      // right-hand-side columns per chain (independent column groups), narrow
-constexpr int kTGWide = 64;  // wide chains: complex64, large n (more work per loaded block, fewer chains)
-constexpr int kWideMinN = 20000;
+constexpr int kTB = 64;       // order of the blocks inverted by substitution
+constexpr int kTD = 256;      // block rows of the solve
+constexpr int kTC = 32;       // right-hand sides per cluster
+constexpr int kTK = 64;       // complex K per CTA
+constexpr int kTThreads = 256;
 
-// register tile of one thread in a 64 x TG block: TR rows x 4 columns
-template <int TG> struct TriTile;
-template <> struct TriTile<16> { static constexpr int TR = 1, TC = 4, TPR = 4; };    // 64 x 4 threads
-template <> struct TriTile<64> { static constexpr int TR = 4, TC = 4, TPR = 16; };   // 16 x 16 threads
-
-__device__ __forceinline__ void st_release_u32(unsigned* p, unsigned v) {
-  asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned* p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-// Factor blocks staged per CTA: two (the next block loads during the current
-// product) for complex64, one for complex128 (shared memory).
-template <typename T> constexpr int tri_nbuf() { return sizeof(T) == 4 ? 2 : 1; }
-
-// Row stride of the right-hand sides in diag_inverse_kernel: the four lanes
+// Row stride of the right-hand sides in lower_inverse_kernel: the four lanes
 // of a column group read rows r..r+3, and a stride of 72 complex64 (an odd
 // multiple of 64 bytes) puts those rows on different banks (with 64 they
 // shared one: 4-way conflicts on every access).
 constexpr int kInvLd = kTB + 8;
+constexpr size_t kInvSmem = (size_t)(kTB * (kTB + 1) + kTB * kInvLd) * sizeof(float2);
 
-// Inverse of every 64 x 64 diagonal block of the unit lower (or upper) factor:
-// one CTA per block, identity right-hand sides, substitution in shared memory.
-// Warp w owns columns 8w..8w+7 of the inverse, which is lower (upper)
-// triangular: the steps above (below) those columns multiply exact zeros and
-// are skipped.
-template <typename T, bool UPPER>
+// Inverses of the 64 x 64 diagonal blocks of a unit lower factor: one CTA per
+// block, identity right-hand sides, substitution in shared memory.  Warp w owns
+// columns 8w..8w+7 of the inverse, which is lower triangular: the steps above
+// those columns multiply exact zeros and are skipped.
 __global__ void __launch_bounds__(256)
-diag_inverse_kernel(const cplx<T>* __restrict__ F, int64_t ldf, int n, cplx<T>* __restrict__ Inv) {
-  using V = cplx<T>;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  V* Ts = reinterpret_cast<V*>(smem_raw);          // [kTB][kTB + 1]
-  V* Xs = Ts + kTB * (kTB + 1);                      // [kTB][kInvLd]
-  __shared__ V dinv[kTB];
-  const int tid = threadIdx.x, i = blockIdx.x;
-  const int r0 = i * kTB, rb = min(kTB, n - r0);
+lower_inverse_kernel(const float2* __restrict__ F, int64_t ldf, int n, float2* __restrict__ Inv) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  float2* Ts = reinterpret_cast<float2*>(smem_raw);   // [kTB][kTB + 1]
+  float2* Xs = Ts + kTB * (kTB + 1);                    // [kTB][kInvLd]
+  const int tid = threadIdx.x, r0 = blockIdx.x * kTB, rb = min(kTB, n - r0);
   for (int idx = tid; idx < kTB * kTB; idx += 256) {
     int r = idx >> 6, c = idx & 63;
     const bool ok = r < rb && c < rb;
-    cp_async_elem<(int)sizeof(V)>(Ts + r * (kTB + 1) + c, ok ? F + (int64_t)(r0 + r) * ldf + r0 + c : F, ok);
-    V e = czero<V>();
-    if (r == c) e.x = 1;
-    Xs[r * kInvLd + c] = e;
+    cp_async_elem<8>(Ts + r * (kTB + 1) + c, ok ? F + (int64_t)(r0 + r) * ldf + r0 + c : F, ok);
+    Xs[r * kInvLd + c] = make_float2(r == c ? 1.f : 0.f, 0.f);
   }
   cp_async_commit();
   cp_async_wait<0>();
-  __syncthreads();
-  if (UPPER)
-    for (int r = tid; r < kTB; r += 256) dinv[r] = r < rb ? crecip(Ts[r * (kTB + 1) + r]) : czero<V>();
   __syncthreads();
   const int warp = tid >> 5, lane = tid & 31;
   const int col = warp * 8 + (lane >> 2), t4 = lane & 3;   // 4 lanes per column, 64 columns
-  if (!UPPER) {
-    for (int kk = warp * 8; kk < rb - 1; ++kk) {
-      __syncwarp();
-      const V xk = Xs[kk * kInvLd + col];
-      for (int r = kk + 1 + t4; r < rb; r += 4) cfms(Xs[r * kInvLd + col], Ts[r * (kTB + 1) + kk], xk);
-    }
-  } else {
-    for (int kk = min(rb - 1, warp * 8 + 7); kk >= 0; --kk) {
-      __syncwarp();
-      if (t4 == 0) Xs[kk * kInvLd + col] = cmul(Xs[kk * kInvLd + col], dinv[kk]);
-      __syncwarp();
-      const V xk = Xs[kk * kInvLd + col];
-      for (int r = t4; r < kk; r += 4) cfms(Xs[r * kInvLd + col], Ts[r * (kTB + 1) + kk], xk);
-    }
+  for (int kk = warp * 8; kk < rb - 1; ++kk) {
+    __syncwarp();
+    const float2 xk = Xs[kk * kInvLd + col];
+    for (int r = kk + 1 + t4; r < rb; r += 4) cfms(Xs[r * kInvLd + col], Ts[r * (kTB + 1) + kk], xk);
   }
   __syncthreads();
-  V* out = Inv + (int64_t)i * kTB * kTB;
+  float2* out = Inv + (int64_t)blockIdx.x * kTB * kTB;
   for (int idx = tid; idx < kTB * kTB; idx += 256) out[idx] = Xs[(idx >> 6) * kInvLd + (idx & 63)];
 }
 
-// W_i = Inv_i F_(i, j): the inverted diagonal block times the factor block of
-// the last dependency j of block row i (j = i - 1 for L, i + 1 for U), so
-// that the solve can form Inv_i (B_i - all other products) before block j
-// is done and needs only X_i = Z - W_i X_j after it.  One CTA per block row,
-// thread = (4 rows, 4 columns) of W_i.
-template <typename T, bool UPPER>
-__global__ void __launch_bounds__(256)
-chain_factor_kernel(const cplx<T>* __restrict__ F, int64_t ldf, int n, const cplx<T>* __restrict__ Inv,
-                    cplx<T>* __restrict__ W) {
-  using V = cplx<T>;
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  V* Is = reinterpret_cast<V*>(smem_raw);   // [kTB][kTB + 1]
-  V* Fs = Is + kTB * (kTB + 1);              // [kTB][kTB + 1]
-  const int tid = threadIdx.x, i = blockIdx.x, nb = gridDim.x;
-  const int j = UPPER ? i + 1 : i - 1;
-  if (j < 0 || j >= nb) return;
-  const int r0 = i * kTB, rb = min(kTB, n - r0), c0 = j * kTB, cb = min(kTB, n - c0);
-  const V* inv = Inv + (int64_t)i * kTB * kTB;
-  for (int idx = tid; idx < kTB * kTB; idx += 256) {
+// The 64 x 64 diagonal blocks of the block rows' inverses, L's and U's, and
+// zeros in the 64-column blocks beside each that lie outside the triangle; the
+// sums of |entries| of the 256 x 256 diagonal blocks' rows.
+constexpr size_t kInv64Smem = (3 * 64 * kTileLD + 6 * 256) * sizeof(float2);
+__global__ void __launch_bounds__(kTileThreads)
+tri_inverse64_kernel(const float2* __restrict__ F, int64_t ldf, int n, int nb, float2* __restrict__ Inv,
+                     float* __restrict__ rowsum, float* __restrict__ cond) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  float2* Ts = reinterpret_cast<float2*>(smem_raw);   // [64][kTileLD]: the factors' block
+  float2* UI = Ts + 64 * kTileLD;
+  float2* LI = UI + 64 * kTileLD;
+  float2* S = LI + 64 * kTileLD;                        // 6 x 256
+  __shared__ float2 dinv[64];
+  const int tid = threadIdx.x, q = blockIdx.x & 3, b = blockIdx.x >> 2;
+  const int r0 = b * kTD + q * kTB, rb = max(0, min(kTB, n - r0));
+  float2* lrows = Inv + (int64_t)b * kTD * kTD + q * kTB * kTD;
+  float2* urows = lrows + (int64_t)nb * kTD * kTD;
+  for (int idx = tid; idx < kTB * kTB; idx += kTileThreads) {
     const int r = idx >> 6, c = idx & 63;
-    cp_async_elem<(int)sizeof(V)>(Is + r * (kTB + 1) + c, inv + idx, true);
-    const bool ok = r < rb && c < cb;
-    cp_async_elem<(int)sizeof(V)>(Fs + r * (kTB + 1) + c, ok ? F + (int64_t)(r0 + r) * ldf + c0 + c : F, ok);
+    Ts[r * kTileLD + c] = r < rb && c < rb ? F[(int64_t)(r0 + r) * ldf + r0 + c] : make_float2(r == c ? 1.f : 0.f, 0.f);
   }
-  cp_async_commit();
-  cp_async_wait<0>();
+  for (int r = tid >> 5; r < kTB; r += kTileThreads / 32) {
+    for (int c = (q + 1) * kTB + (tid & 31); c < kTD; c += 32) lrows[r * kTD + c] = make_float2(0.f, 0.f);
+    for (int c = tid & 31; c < q * kTB; c += 32) urows[r * kTD + c] = make_float2(0.f, 0.f);
+    float sl = 0.f, su = 0.f;
+#pragma unroll
+    for (int j = 0; j < kTD / 32; ++j) {
+      const int c = (tid & 31) + 32 * j, rr = q * kTB + r;
+      if (r < rb && b * kTD + c < n) {
+        const float2 v = F[(int64_t)(r0 + r) * ldf + b * kTD + c];
+        (c < rr ? sl : su) += fabsf(v.x) + fabsf(v.y);
+      }
+    }
+    for (int o = 16; o; o >>= 1) {
+      sl += __shfl_xor_sync(0xffffffffu, sl, o);
+      su += __shfl_xor_sync(0xffffffffu, su, o);
+    }
+    if ((tid & 31) == 0) {
+      rowsum[b * kTD + q * kTB + r] = sl + 1.f;
+      rowsum[(nb + b) * kTD + q * kTB + r] = su;
+    }
+  }
+  if (tid < 2 && q == 0) cond[tid * nb + b] = 0.f;
   __syncthreads();
-  const int tr = tid >> 4, tc = tid & 15;   // rows 4 tr .., columns tc + 16 q
-  V acc[4][4];
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) acc[a][q] = czero<V>();
-  for (int k = 0; k < kTB; ++k) {
-    V f[4];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) f[q] = Fs[k * (kTB + 1) + tc + 16 * q];
-#pragma unroll
-    for (int a = 0; a < 4; ++a) {
-      const V x = Is[(4 * tr + a) * (kTB + 1) + k];
-#pragma unroll
-      for (int q = 0; q < 4; ++q) cfma(acc[a][q], x, f[q]);
-    }
-  }
-  V* out = W + (int64_t)i * kTB * kTB;
-#pragma unroll
-  for (int a = 0; a < 4; ++a)
-#pragma unroll
-    for (int q = 0; q < 4; ++q) out[(4 * tr + a) * kTB + tc + 16 * q] = acc[a][q];
-}
-
-// acc (64 x TG, a TR x TC tile per thread: rows TR tr + i, columns tc + TPR j)
-// -= A (64 x 64, smem, padded) * Y (64 x TG, smem)
-template <int TG, typename V>
-__device__ __forceinline__ void block_gemm_sub(V (&acc)[TriTile<TG>::TR][TriTile<TG>::TC], const V* As, const V* Ys,
-                                               int tr, int tc) {
-  constexpr int TR = TriTile<TG>::TR, TC = TriTile<TG>::TC, TPR = TriTile<TG>::TPR;
-#pragma unroll 4
-  for (int kk = 0; kk < kTB; ++kk) {
-    V a[TR], y[TC];
-#pragma unroll
-    for (int i = 0; i < TR; ++i) a[i] = As[(TR * tr + i) * (kTB + 1) + kk];
-#pragma unroll
-    for (int j = 0; j < TC; ++j) y[j] = Ys[kk * TG + tc + TPR * j];
-#pragma unroll
-    for (int i = 0; i < TR; ++i)
-#pragma unroll
-      for (int j = 0; j < TC; ++j) cfms(acc[i][j], a[i], y[j]);
+  if (tid < kTB) dinv[tid] = crecip(Ts[tid * kTileLD + tid]);
+  __syncthreads();
+  tile_inverses(Ts, UI, LI, S, dinv, tid);
+  for (int idx = tid; idx < kTB * kTB; idx += kTileThreads) {
+    const int r = idx >> 6, c = idx & 63;
+    urows[r * kTD + q * kTB + c] = c >= r ? UI[r * kTileLD + c] : make_float2(0.f, 0.f);
+    lrows[r * kTD + q * kTB + c] = c < r ? LI[r * kTileLD + c] : make_float2(r == c ? 1.f : 0.f, 0.f);
   }
 }
 
-// Stage st of work item (block row i, ndep dependencies) into buf: for
-// st < ndep - 1 the factor block of dependency st (it does not depend on the
-// flag), then the inverted diagonal block (full 64 x 64; the only stage when
-// ndep = 0), then W_i = Inv_i F_(i, last dependency).
-template <bool UPPER, typename V>
-__device__ __forceinline__ void tri_stage(V* buf, int st, int ndep, const V* __restrict__ F, int64_t ldf,
-                                          const V* __restrict__ Inv, const V* __restrict__ W, int i, int nb, int n,
-                                          int r0, int rb, int tid) {
-  if (ndep > 0 && st == ndep) {
-    const V* w = W + (int64_t)i * kTB * kTB;
-    for (int idx = tid; idx < kTB * kTB; idx += 256)
-      cp_async_elem<(int)sizeof(V)>(buf + (idx >> 6) * (kTB + 1) + (idx & 63), w + idx, true);
-  } else if (st < ndep - 1) {
-    const int j = UPPER ? nb - 1 - st : st;
-    const int c0 = j * kTB, cb = min(kTB, n - c0);
-    for (int idx = tid; idx < kTB * kTB; idx += 256) {
-      const int r = idx >> 6, c = idx & 63;
-      const bool ok = r < rb && c < cb;
-      cp_async_elem<(int)sizeof(V)>(buf + r * (kTB + 1) + c, ok ? F + (int64_t)(r0 + r) * ldf + c0 + c : F, ok);
+// acc (H x 16, this thread's rows rg + 32 a, columns 2 cg, 2 cg + 1) += A (H x H, row stride lda,
+// rows < rn and columns < cn) * Bs (H x 16 in shared memory), K chunks of 32 from kb to ke.
+// TRI 1 (2): A is lower (upper) triangular.  The next chunk loads during the products.
+template <int H, int TRI>
+__device__ __forceinline__ void strip_mm(float2 (&acc)[H / 32][2], const float2* __restrict__ A, int64_t lda, int rn,
+                                         int cn, const float2* Bs, float2* As, int kb, int ke, int tid) {
+  const int rg = tid >> 3, cg = tid & 7;
+  auto load = [&](int kc) {
+    float2* d = As + (kc & 1) * (H * 33);
+    for (int idx = tid; idx < H * 32; idx += 256) {
+      const int r = idx >> 5, c = 32 * kc + (idx & 31);
+      const bool ok = r < rn && c < cn;
+      cp_async_elem<8>(d + r * 33 + (idx & 31), ok ? A + (int64_t)r * lda + c : A, ok);
     }
-  } else {
-    const V* inv = Inv + (int64_t)i * kTB * kTB;
-    for (int idx = tid; idx < kTB * kTB; idx += 256)
-      cp_async_elem<(int)sizeof(V)>(buf + (idx >> 6) * (kTB + 1) + (idx & 63), inv + idx, true);
-  }
-  cp_async_commit();
-}
-
-// Persistent solve of one triangle.  Work items (block row, column group) are
-// claimed in dependency order; groups are independent chains.  An item's
-// stages are the factor blocks it depends on, then its inverted diagonal
-// block; each is copied asynchronously, and with two buffers the next stage
-// loads while the current block product runs.
-// Split sums: each (block row, group) is `parts` items, claimed helpers
-// first.  Helper p >= 1 sums the products of dependencies
-// [last - (p+1) dper, last - p dper) into its slot of `part` and releases its
-// flag in `hflags`; the main item (p = 0) sums the dper dependencies before
-// the last, adds the helpers' slots, then solves as above.  A row's long sum
-// of block products is thus spread over `parts` CTAs.  Every item waits only
-// on items claimed before it, so progress is guaranteed as before.
-template <typename T, bool UPPER, int TG>
-__global__ void __launch_bounds__(256)
-tri_solve_kernel(const cplx<T>* __restrict__ F, int64_t ldf, const cplx<T>* __restrict__ Inv,
-                 const cplx<T>* __restrict__ W, cplx<T>* __restrict__ X, int64_t ldx, int n, int ncols,
-                 unsigned* counter, unsigned* flags, const unsigned* epoch_ptr, int* status, int parts, int dper,
-                 cplx<T>* __restrict__ part, unsigned* hflags) {
-  // flag value of this solve: bumped on the device before the launch, so a
-  // replay from a CUDA graph never sees the previous run's flags as ready
-  const unsigned epoch = *(volatile const unsigned*)epoch_ptr;
-  using V = cplx<T>;
-  constexpr int TR = TriTile<TG>::TR, TC = TriTile<TG>::TC, TPR = TriTile<TG>::TPR;
-  constexpr int NBUF = tri_nbuf<T>();
-  constexpr int kAs = kTB * (kTB + 1);               // one padded 64 x 64 block
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  V* Asb = reinterpret_cast<V*>(smem_raw);          // NBUF x [kTB][kTB + 1]
-  V* Ys = Asb + NBUF * kAs;                          // [kTB][TG]
-  __shared__ unsigned s_item;
-  __shared__ int s_fail;
-  const int tid = threadIdx.x, tr = tid / TPR, tc = tid % TPR;
-  const int nb = (n + kTB - 1) / kTB, ng = (ncols + TG - 1) / TG;
-  const unsigned items = (unsigned)nb * ng * parts;
-  while (true) {
-    if (tid == 0) { s_item = atomicAdd(counter, 1u); s_fail = 0; }
-    __syncthreads();
-    const unsigned k = s_item;
-    if (k >= items) break;
-    const unsigned rg = k / parts;
-    const int p = parts - 1 - (int)(k % parts);   // helpers (p >= 1, farthest first), then the main item
-    const int kr = (int)(rg / ng), g = (int)(rg % ng);
-    const int i = UPPER ? nb - 1 - kr : kr;
-    const int r0 = i * kTB, rb = min(kTB, n - r0), cg = g * TG;
-    unsigned* gflags = flags + (size_t)g * nb;
-    // dependencies in completion order: ascending for L, descending for U.
-    // All but the last are applied as they complete; then Z = Inv_i acc is
-    // formed before the last one is done, and after it X_i = Z - W_i X_last:
-    // one product on the chain from block to block instead of two.
-    const int ndep = UPPER ? nb - 1 - i : i;
-    // dependencies [dlo(q), dhi(q)) of part q (the last one, ndep - 1, is the main item's)
-    auto dlo = [&](int q) { return max(0, ndep - 1 - (q + 1) * dper); };
-    auto dhi = [&](int q) { return max(0, ndep - 1 - q * dper); };
-    const size_t slot = ((size_t)i * ng + g) * (parts - 1);   // + q - 1 for helper q
-    auto stage = [&](V* buf, int st) { tri_stage<UPPER>(buf, st, ndep, F, ldf, Inv, W, i, nb, n, r0, rb, tid); };
-    auto bufof = [&](int st) { return Asb + (NBUF == 2 ? (st & 1) * kAs : 0); };
-    // wait for dependency d's completion flag and stage its rows of X in Ys
-    auto take_dep = [&](int d) -> bool {
-      const int j = UPPER ? nb - 1 - d : d;
-      const int c0 = j * kTB, cb = min(kTB, n - c0);
-      if (tid == 0) {
-        unsigned it = 0;
-        while (ld_acquire_u32(gflags + j) != epoch) {
-          if (++it > kSpinLimit) { s_fail = 1; atomicExch(status, MGT_ERR_TIMEOUT); break; }
-          if (it > 64) __nanosleep(32);
-        }
-      }
-      __syncthreads();
-      if (s_fail) return false;
-      for (int idx = tid; idx < kTB * TG; idx += 256) {
-        int r = idx / TG, c = idx % TG;
-        Ys[idx] = (r < cb && cg + c < ncols) ? ldcg(X + (int64_t)(c0 + r) * ldx + cg + c) : czero<V>();
-      }
-      __syncthreads();
-      return true;
-    };
-    V acc[TR][TC];
-    if (p > 0) {
-      // helper: -(sum of its dependencies' products) into its slot
-      const int lo = dlo(p), hi = dhi(p);
-      if (lo >= hi) {
-        __syncthreads();   // every thread has read s_item before it is claimed again
-        continue;
-      }
+    cp_async_commit();
+  };
+  __syncthreads();
+  load(kb);
 #pragma unroll
-      for (int a = 0; a < TR; ++a)
-#pragma unroll
-        for (int b = 0; b < TC; ++b) acc[a][b] = czero<V>();
-      stage(bufof(lo), lo);
-      for (int d = lo; d < hi; ++d) {
-        const bool next = d + 1 < hi;
-        if (NBUF == 2 && next) stage(bufof(d + 1), d + 1);
-        if (NBUF == 2 && next) cp_async_wait<1>(); else cp_async_wait<0>();
-        if (!take_dep(d)) {
-          cp_async_wait<0>();
-          return;
-        }
-        block_gemm_sub<TG>(acc, bufof(d), Ys, tr, tc);
-        __syncthreads();
-        if (NBUF == 1 && next) stage(bufof(d + 1), d + 1);
-      }
-      V* out = part + (slot + p - 1) * (size_t)(kTB * TG);
-#pragma unroll
-      for (int a = 0; a < TR; ++a)
-#pragma unroll
-        for (int b = 0; b < TC; ++b) out[(TR * tr + a) * TG + tc + TPR * b] = acc[a][b];
-      __threadfence();
-      __syncthreads();
-      if (tid == 0) st_release_u32(hflags + slot + p - 1, epoch);
-      continue;
-    }
-#pragma unroll
-    for (int a = 0; a < TR; ++a)
-#pragma unroll
-      for (int b = 0; b < TC; ++b) {
-        const int r = TR * tr + a, c = cg + tc + TPR * b;
-        acc[a][b] = (r < rb && c < ncols) ? X[(int64_t)(r0 + r) * ldx + c] : czero<V>();
-      }
-    const int d0 = dlo(0);
-    stage(bufof(d0), d0);
-    for (int d = d0; d < ndep - 1; ++d) {
-      if (NBUF == 2) stage(bufof(d + 1), d + 1);
-      if (NBUF == 2) cp_async_wait<1>(); else cp_async_wait<0>();
-      if (!take_dep(d)) {
-        cp_async_wait<0>();
-        return;
-      }
-      block_gemm_sub<TG>(acc, bufof(d), Ys, tr, tc);
-      __syncthreads();
-      if (NBUF == 1) stage(bufof(d + 1), d + 1);
-    }
-    // the helpers' sums (helpers beyond the first empty one are empty too)
-    for (int q = 1; q < parts && dlo(q) < dhi(q); ++q) {
-      if (tid == 0) {
-        unsigned it = 0;
-        while (ld_acquire_u32(hflags + slot + q - 1) != epoch) {
-          if (++it > kSpinLimit) { s_fail = 1; atomicExch(status, MGT_ERR_TIMEOUT); break; }
-          if (it > 64) __nanosleep(32);
-        }
-      }
-      __syncthreads();
-      if (s_fail) {
-        cp_async_wait<0>();
-        return;
-      }
-      const V* in = part + (slot + q - 1) * (size_t)(kTB * TG);
-#pragma unroll
-      for (int a = 0; a < TR; ++a)
-#pragma unroll
-        for (int b = 0; b < TC; ++b) {
-          const V v = ldcg(in + (TR * tr + a) * TG + tc + TPR * b);
-          acc[a][b].x += v.x;
-          acc[a][b].y += v.y;
-        }
-    }
-    // Z = Inv_i * acc (Inv_i is stage max(ndep - 1, 0)); W_i loads meanwhile
-    const int sinv = ndep > 0 ? ndep - 1 : 0;
-    if (NBUF == 2 && ndep > 0) {
-      stage(bufof(ndep), ndep);
+  for (int kc = 0; kc < H / 32; ++kc) {
+    if (kc < kb || kc >= ke) continue;
+    if (kc + 1 < ke) {
+      load(kc + 1);
       cp_async_wait<1>();
     } else {
       cp_async_wait<0>();
     }
-#pragma unroll
-    for (int a = 0; a < TR; ++a)
-#pragma unroll
-      for (int b = 0; b < TC; ++b) Ys[(TR * tr + a) * TG + tc + TPR * b] = acc[a][b];
     __syncthreads();
-    V out[TR][TC];
+    const float2* d = As + (kc & 1) * (H * 33);
+#pragma unroll 8
+    for (int k = 0; k < 32; ++k) {
+      const float4 b = *reinterpret_cast<const float4*>(Bs + (32 * kc + k) * 16 + 2 * cg);
 #pragma unroll
-    for (int a = 0; a < TR; ++a)
-#pragma unroll
-      for (int b = 0; b < TC; ++b) out[a][b] = czero<V>();
-    block_gemm_sub<TG>(out, bufof(sinv), Ys, tr, tc);   // out = -Z
-#pragma unroll
-    for (int a = 0; a < TR; ++a)
-#pragma unroll
-      for (int b = 0; b < TC; ++b) {
-        out[a][b].x = -out[a][b].x;
-        out[a][b].y = -out[a][b].y;
+      for (int a = TRI == 1 ? kc : 0; a < (TRI == 2 ? kc + 1 : H / 32); ++a) {
+        const float2 x = d[(rg + 32 * a) * 33 + k];
+        cfma(acc[a][0], x, make_float2(b.x, b.y));
+        cfma(acc[a][1], x, make_float2(b.z, b.w));
       }
+    }
     __syncthreads();
-    if (ndep > 0) {
-      if (NBUF == 1) stage(bufof(ndep), ndep);
-      cp_async_wait<0>();
-      if (!take_dep(ndep - 1)) return;
-      block_gemm_sub<TG>(out, bufof(ndep), Ys, tr, tc);   // X_i = Z - W_i X_last
+  }
+}
+
+// One doubling of the inverses, H x H blocks to 2H x 2H: for L = [A 0; C B],
+// -B^-1 (C A^-1); for U = [A C; 0 B], -A^-1 (C B^-1); 16 columns per CTA.
+// Grid: x = (block row, pair, strip), y = L / U.
+template <int H> constexpr size_t tri_double_smem() { return (size_t)H * (2 * 16 + 2 * 33) * sizeof(float2); }
+template <int H>
+__global__ void __launch_bounds__(256)
+tri_double_kernel(const float2* __restrict__ F, int64_t ldf, int n, int nb, float2* __restrict__ Inv) {
+  constexpr int PAIRS = kTD / (2 * H), STRIPS = H / 16, KC = H / 32;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  float2* Bs = reinterpret_cast<float2*>(smem_raw);   // [H][16]
+  float2* Ss = Bs + H * 16;                             // [H][16]
+  float2* As = Ss + H * 16;                             // 2 x [H][33]
+  const int tid = threadIdx.x;
+  const int strip = blockIdx.x % STRIPS, pair = (blockIdx.x / STRIPS) % PAIRS, b = blockIdx.x / (STRIPS * PAIRS);
+  const bool upper = blockIdx.y != 0;
+  const int o = pair * 2 * H, c0 = strip * 16;   // the pair's offset within the block row
+  float2* I = Inv + ((int64_t)(upper ? nb : 0) + b) * kTD * kTD;
+  // the right factor's diagonal block (A for L, B for U), the left one's, C
+  const int ro = o + (upper ? H : 0), lo = o + (upper ? 0 : H);
+  const int crow = b * kTD + lo, ccol = b * kTD + ro;
+  for (int idx = tid; idx < H * 16; idx += 256) {
+    const int r = idx >> 4, c = idx & 15;
+    Bs[idx] = I[(int64_t)(ro + r) * kTD + ro + c0 + c];
+  }
+  const int rg = tid >> 3, cg = tid & 7;
+  float2 acc[KC][2];
+#pragma unroll
+  for (int a = 0; a < KC; ++a) acc[a][0] = acc[a][1] = make_float2(0.f, 0.f);
+  const int rn = max(0, min(H, n - crow)), cn = max(0, min(H, n - ccol));
+  // columns c0 .. + 15 of a triangular inverse: rows from c0 on (L), to c0 + 15 (U)
+  strip_mm<H, 0>(acc, rn > 0 && cn > 0 ? F + (int64_t)crow * ldf + ccol : F, ldf, rn, cn, Bs, As, upper ? 0 : c0 >> 5,
+                 upper ? (c0 >> 5) + 1 : KC, tid);
+#pragma unroll
+  for (int a = 0; a < KC; ++a) {
+    *reinterpret_cast<float4*>(Ss + (rg + 32 * a) * 16 + 2 * cg) =
+        make_float4(acc[a][0].x, acc[a][0].y, acc[a][1].x, acc[a][1].y);
+    acc[a][0] = acc[a][1] = make_float2(0.f, 0.f);
+  }
+  const float2* D = I + (int64_t)lo * kTD + lo;
+  if (upper) strip_mm<H, 2>(acc, D, kTD, H, H, Ss, As, 0, KC, tid);
+  else strip_mm<H, 1>(acc, D, kTD, H, H, Ss, As, 0, KC, tid);
+#pragma unroll
+  for (int a = 0; a < KC; ++a)
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      I[(int64_t)(lo + rg + 32 * a) * kTD + ro + c0 + 2 * cg + j] = make_float2(-acc[a][j].x, -acc[a][j].y);
+}
+
+// Skeel's condition number || |R| |T| e || of each diagonal block T with its
+// inverse R, as the bits of a float (a NaN is the largest); grid x = (block row,
+// quarter of its rows), y = L / U.
+__global__ void __launch_bounds__(512)
+tri_cond_kernel(int nb, const float2* __restrict__ Inv, const float* __restrict__ rowsum, unsigned* __restrict__ cond) {
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, b = blockIdx.x >> 2;
+  const int64_t block = (blockIdx.y ? nb : 0) + b;
+  const float2* I = Inv + block * kTD * kTD;
+  float t[kTD / 32];
+#pragma unroll
+  for (int j = 0; j < kTD / 32; ++j) t[j] = rowsum[block * kTD + lane + 32 * j];
+  unsigned mx = 0;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int r = (blockIdx.x & 3) * 64 + 16 * i + warp;
+    float s = 0.f;
+#pragma unroll
+    for (int j = 0; j < kTD / 32; ++j) {
+      const float2 v = I[r * kTD + lane + 32 * j];
+      s = fmaf(fabsf(v.x) + fabsf(v.y), t[j], s);
+    }
+    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    mx = max(mx, __float_as_uint(s) & 0x7FFFFFFFu);
+  }
+  if (lane == 0) atomicMax(cond + block, mx);
+}
+
+// (hi, lo) += a b: the product and the sum exactly, their errors into lo
+__device__ __forceinline__ void df_fma(float& hi, float& lo, float a, float b) {
+  const float p = a * b, e = fmaf(a, b, -p);
+  const float s = hi + p, z = s - hi;
+  lo += e + ((hi - (s - z)) + (p - z));
+  hi = s;
+}
+
+// One Newton step R + R (I - T R) for the inverses R of ill-conditioned
+// diagonal blocks, the residual in double-float.  Without it a solve with
+// random factors (condition numbers of 5000 to 8000) has 2.5 times the residual
+// that substitution in 64-row blocks leaves, with it a third; blocks of system
+// matrices (10 to 400) solve to a half to a seventh of it as they are.
+// 16 columns of a block per CTA; grid x = (block row, strip), y = L / U.
+constexpr float kTCond = 500.f;
+constexpr size_t kTNewtonSmem = (size_t)kTD * (16 + 16 + 17) * sizeof(float2);
+__global__ void __launch_bounds__(512)
+tri_newton_kernel(const float2* __restrict__ F, int64_t ldf, int n, int nb, const float2* __restrict__ Inv,
+                  const float* __restrict__ cond, float2* __restrict__ Out) {
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  float2* Bs = reinterpret_cast<float2*>(smem_raw);   // [256][16]
+  float2* Es = Bs + kTD * 16;                           // [256][16]
+  float2* As = Es + kTD * 16;                           // [256][17]
+  const int tid = threadIdx.x, b = blockIdx.x >> 4, c0 = (blockIdx.x & 15) * 16, d0 = b * kTD;
+  const bool upper = blockIdx.y != 0;
+  const int64_t block = (upper ? nb : 0) + b;
+  const float2* I = Inv + block * kTD * kTD;
+  float2* O = Out + block * kTD * kTD;
+  if (cond[block] <= kTCond) return;   // (a NaN goes on)
+  for (int idx = tid; idx < kTD * 16; idx += 512) Bs[idx] = I[(int64_t)(idx >> 4) * kTD + c0 + (idx & 15)];
+  const int rg = tid >> 3, cg = tid & 7;   // rows rg + 64 a, columns 2 cg, 2 cg + 1
+  float2 hi[4][2], lo[4][2];
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) hi[a][j] = lo[a][j] = make_float2(0.f, 0.f);
+  // rows of a column of R: from its own on (L), up to its own (U)
+  const int kb = upper ? 0 : c0, ke = upper ? c0 + 16 : kTD;
+  for (int k0 = kb; k0 < ke; k0 += 16) {
+    __syncthreads();
+    for (int idx = tid; idx < kTD * 16; idx += 512) {
+      const int r = idx >> 4, c = k0 + (idx & 15);
+      float2 v = make_float2(r == c && (!upper || d0 + r >= n) ? 1.f : 0.f, 0.f);
+      if (d0 + r < n && d0 + c < n && (upper ? c >= r : c < r)) v = F[(int64_t)(d0 + r) * ldf + d0 + c];
+      As[r * 17 + (idx & 15)] = v;
+    }
+    __syncthreads();
+#pragma unroll 1
+    for (int k = 0; k < 16; ++k) {
+      const float4 x = *reinterpret_cast<const float4*>(Bs + (k0 + k) * 16 + 2 * cg);
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        const float2 t = As[(rg + 64 * a) * 17 + k];
+        df_fma(hi[a][0].x, lo[a][0].x, t.x, x.x);
+        df_fma(hi[a][0].x, lo[a][0].x, -t.y, x.y);
+        df_fma(hi[a][0].y, lo[a][0].y, t.x, x.y);
+        df_fma(hi[a][0].y, lo[a][0].y, t.y, x.x);
+        df_fma(hi[a][1].x, lo[a][1].x, t.x, x.z);
+        df_fma(hi[a][1].x, lo[a][1].x, -t.y, x.w);
+        df_fma(hi[a][1].y, lo[a][1].y, t.x, x.w);
+        df_fma(hi[a][1].y, lo[a][1].y, t.y, x.z);
+      }
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int r = rg + 64 * a, c = 2 * cg + j;
+      Es[r * 16 + c] = make_float2(((r == c0 + c ? 1.f : 0.f) - hi[a][j].x) - lo[a][j].x, -hi[a][j].y - lo[a][j].y);
+      hi[a][j] = make_float2(0.f, 0.f);
+    }
+  for (int k0 = kb; k0 < ke; k0 += 16) {
+    __syncthreads();
+    for (int idx = tid; idx < kTD * 16; idx += 512)
+      As[(idx >> 4) * 17 + (idx & 15)] = I[(int64_t)(idx >> 4) * kTD + k0 + (idx & 15)];
+    __syncthreads();
+#pragma unroll 4
+    for (int k = 0; k < 16; ++k) {
+      const float4 x = *reinterpret_cast<const float4*>(Es + (k0 + k) * 16 + 2 * cg);
+#pragma unroll
+      for (int a = 0; a < 4; ++a) {
+        const float2 t = As[(rg + 64 * a) * 17 + k];
+        cfma(hi[a][0], t, make_float2(x.x, x.y));
+        cfma(hi[a][1], t, make_float2(x.z, x.w));
+      }
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int r = rg + 64 * a, c = 2 * cg + j;
+      O[(int64_t)r * kTD + c0 + c] = cadd(Bs[r * 16 + c], hi[a][j]);
+    }
+}
+
+// ---------------------------------------------------------------- one block row
+
+// Shared memory of tri_step_kernel: A operand [part][K slice][128 rows x 128 B],
+// B operand [K slice][64 rows of h, 64 of l][128 B] (the same bytes hold the
+// partial sums, 128 x 64 floats, once the products are done), the cluster's new
+// block row (this CTA's 32 rows x 32 columns).
+constexpr uint32_t kTSlice = 128 * 128;
+constexpr size_t kTSmem = 1024 + 4 * kTSlice + 2 * kTSlice + kTC * kTC * sizeof(float2);
+
+__device__ __forceinline__ uint32_t tri_mapa(uint32_t a, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ float4 tri_ld4(uint32_t a) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(a)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ float2 tri_ld2(uint32_t a) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ void tri_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// byte offset of half `kr` (even) of row `row` in rows of 128 bytes, 16-byte chunks
+// XOR-swizzled by the row (the K-major 128-byte-swizzle operand layout)
+__device__ __forceinline__ uint32_t tri_swz(int row, int kr) {
+  return (uint32_t)row * 128u + (uint32_t)((((kr >> 3) ^ (row & 7)) << 4) + (kr & 7) * 2);
+}
+// exponent e, |e| <= 126, with |x| 2^-e < 4 for every |x| up to the one with bits mx, which
+// stays at 2^-1 or above where it is normal (0 for zero and non-finite maxima)
+__device__ __forceinline__ int tri_exp(unsigned mx) {
+  return mx == 0u || mx >= 0x7F800000u ? 0 : min(max((int)(mx >> 23), 1) - 126, 126);
+}
+__device__ __forceinline__ float tri_pow2(int e) { return __int_as_float((127 + e) << 23); }   // |e| <= 126
+// (x, y) times sc as h + 2^-11 l, two fp16 pairs: the difference is exact
+__device__ __forceinline__ void tri_split(float2 v, float sc, uint32_t& h, uint32_t& l) {
+  const float x = v.x * sc, y = v.y * sc;
+  const __half2 hh = __floats2half2_rn(x, y);
+  const float2 f = __half22float2(hh);
+  const __half2 ll = __floats2half2_rn((x - f.x) * 2048.f, (y - f.y) * 2048.f);
+  h = *reinterpret_cast<const uint32_t*>(&hh);
+  l = *reinterpret_cast<const uint32_t*>(&ll);
+}
+
+// Rows warp, warp + 8, .. of a 128 x 64 tile, columns lane and lane + 32: into registers
+__device__ __forceinline__ void tri_load_tile(float2 (&v)[16][2], const float2* __restrict__ A, int64_t lda, int rn,
+                                              int cn, int warp, int lane) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int r = warp + 8 * i;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int c = lane + 32 * j;
+      v[i][j] = r < rn && c < cn ? A[(int64_t)r * lda + c] : make_float2(0.f, 0.f);
+    }
+  }
+}
+// and from there to the A operand, each row with its own exponent
+__device__ __forceinline__ void tri_store_tile(const float2 (&v)[16][2], unsigned char* abuf, int* rexp, int warp,
+                                               int lane) {
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const int r = warp + 8 * i;
+    unsigned mx = 0;
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+      mx = max(mx, max(__float_as_uint(fabsf(v[i][j].x)), __float_as_uint(fabsf(v[i][j].y))));
+    const int e = tri_exp(__reduce_max_sync(0xffffffffu, mx));
+    if (lane == 0) rexp[r] = e;
+    const float sc = tri_pow2(-e);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const uint32_t at = (uint32_t)j * kTSlice + tri_swz(r, 2 * lane);
+      tri_split(v[i][j], sc, *reinterpret_cast<uint32_t*>(abuf + at),
+                *reinterpret_cast<uint32_t*>(abuf + 2 * kTSlice + at));
+    }
+  }
+}
+
+// The B operand from 64 x 32 values, this thread's rows 8 warp .. + 7 of column
+// lane: rows 2c and 2c + 1 of B'^T hold (re, -im) and (im, re) of column c.
+__device__ __forceinline__ void tri_store_rhs(const float2 (&x)[8], unsigned char* bbuf, unsigned* cmax, int* cexp,
+                                              int warp, int lane) {
+  unsigned mx = 0;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) mx = max(mx, max(__float_as_uint(fabsf(x[i].x)), __float_as_uint(fabsf(x[i].y))));
+  cmax[warp * 32 + lane] = mx;
+  __syncthreads();
+#pragma unroll
+  for (int w = 0; w < 8; ++w) mx = max(mx, cmax[w * 32 + lane]);
+  const int e = tri_exp(mx);
+  if (warp == 0) cexp[lane] = e;
+  const float sc = tri_pow2(-e);
+  const int slice = warp >> 2, k0 = 16 * (warp & 3);   // 8 complex k: halves k0 .. k0 + 15 of the slice
+  unsigned char* base = bbuf + slice * kTSlice;
+#pragma unroll
+  for (int g = 0; g < 2; ++g) {
+    uint32_t h0[4], h1[4], l0[4], l1[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      uint32_t h, l;
+      tri_split(x[4 * g + i], sc, h, l);
+      h0[i] = h ^ 0x80000000u;                      // re, -im
+      h1[i] = __byte_perm(h, 0, 0x1032);            // im, re
+      l0[i] = l ^ 0x80000000u;
+      l1[i] = __byte_perm(l, 0, 0x1032);
+    }
+    const int kr = k0 + 8 * g;
+    *reinterpret_cast<uint4*>(base + tri_swz(2 * lane, kr)) = make_uint4(h0[0], h0[1], h0[2], h0[3]);
+    *reinterpret_cast<uint4*>(base + tri_swz(2 * lane + 1, kr)) = make_uint4(h1[0], h1[1], h1[2], h1[3]);
+    *reinterpret_cast<uint4*>(base + tri_swz(64 + 2 * lane, kr)) = make_uint4(l0[0], l0[1], l0[2], l0[3]);
+    *reinterpret_cast<uint4*>(base + tri_swz(64 + 2 * lane + 1, kr)) = make_uint4(l1[0], l1[1], l1[2], l1[3]);
+  }
+}
+
+// 128 x 64 real outputs over 128 real K: h parts of A into columns 0 .. 127 (h h | h l), l parts into
+// 64 .. 191 (l h | l l); one thread
+__device__ __forceinline__ void tri_issue(uint32_t tmem, const unsigned char* abuf, const unsigned char* bbuf) {
+  using namespace tc;
+#pragma unroll
+  for (int s = 0; s < 2; ++s) {
+    const uint64_t ah = kmajor_sw128_desc(smem_u32(abuf + s * kTSlice));
+    const uint64_t al = kmajor_sw128_desc(smem_u32(abuf + (2 + s) * kTSlice));
+    const uint64_t b = kmajor_sw128_desc(smem_u32(bbuf + s * kTSlice));
+    const uint64_t bl = kmajor_sw128_desc(smem_u32(bbuf + s * kTSlice + 64 * 128));
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {
+      const bool first = s == 0 && ks == 0;
+      const uint64_t o = (uint64_t)(2 * ks);
+      mma_f16(tmem, ah + o, b + o, idesc_f16_m128(128), first ? 0u : 1u);
+      if (first) {
+        mma_f16(tmem + 64, al + o, b + o, idesc_f16_m128(64), 1u);
+        mma_f16(tmem + 128, al + o, bl + o, idesc_f16_m128(64), 0u);
+      } else {
+        mma_f16(tmem + 64, al + o, b + o, idesc_f16_m128(128), 1u);
+      }
+    }
+  }
+}
+
+// acc (row 32 (warp & 3) + lane, real columns 32 (warp >> 2) .. + 31) += the products in tensor memory
+__device__ __forceinline__ void tri_read(float (&acc)[32], uint32_t tmem, const int* rexp, const int* cexp, int warp,
+                                         int lane) {
+  using namespace tc;
+  const int half = warp >> 2;
+  const uint32_t t = tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(32 * half);
+  const int er = rexp[32 * (warp & 3) + lane];
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    uint32_t hh[8], hl[8], ll[8];
+    tmem_ld8(t + 8 * p, hh);
+    tmem_ld8(t + 64 + 8 * p, hl);
+    tmem_ld8(t + 128 + 8 * p, ll);
+    tmem_wait_ld();
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float s0 = tri_pow2(er), s1 = tri_pow2(cexp[16 * half + 4 * p + c]);
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int j = 2 * c + q;
+        const float lo = fmaf(__uint_as_float(ll[j]), 0x1p-11f, __uint_as_float(hl[j]));
+        acc[8 * p + j] += fmaf(lo, 0x1p-11f, __uint_as_float(hh[j])) * s0 * s1;
+      }
+    }
+  }
+}
+// acc into P (128 rows of 16 float4, chunk c of row r at c ^ (r & 15))
+__device__ __forceinline__ void tri_partials(const float (&acc)[32], float4* P, int warp, int lane) {
+  const int row = 32 * (warp & 3) + lane;
+#pragma unroll
+  for (int p = 0; p < 8; ++p)
+    P[row * 16 + ((8 * (warp >> 2) + p) ^ (row & 15))] =
+        make_float4(acc[4 * p], acc[4 * p + 1], acc[4 * p + 2], acc[4 * p + 3]);
+}
+
+// This CTA's 32 rows of the cluster half's sum: row 32 kq + tid / 8, complex columns 4 (tid & 7) .. + 3
+__device__ __forceinline__ void tri_gather(float2 (&s)[4], uint32_t paddr, int half, int kq, int tid) {
+  const int row = 32 * kq + (tid >> 3), c4 = 2 * (tid & 7);
+#pragma unroll
+  for (int j = 0; j < 4; ++j) s[j] = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const uint32_t base = tri_mapa(paddr, (uint32_t)(4 * half + q)) + (uint32_t)row * 256u;
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float4 v = tri_ld4(base + (uint32_t)(((c4 + j) ^ (row & 15)) * 16));
+      s[2 * j].x += v.x;
+      s[2 * j].y += v.y;
+      s[2 * j + 1].x += v.z;
+      s[2 * j + 1].y += v.w;
+    }
+  }
+}
+
+// The inverses as A operands: tile (triangle, block row, half, K quarter) in the
+// layout of abuf, and its 128 row exponents.
+__global__ void __launch_bounds__(kTThreads)
+tri_operand_kernel(const float2* __restrict__ Inv, const float2* __restrict__ refined, const float* __restrict__ cond,
+                   unsigned char* __restrict__ ops, int* __restrict__ exps) {
+  const int64_t tile = blockIdx.x, b = tile >> 3;
+  const int half = (int)(tile >> 2) & 1, kq = (int)tile & 3, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  float2 v[16][2];
+  tri_load_tile(v, (cond[b] <= kTCond ? Inv : refined) + b * kTD * kTD + (int64_t)half * 128 * kTD + kq * kTK, kTD, 128, kTK, warp, lane);
+  tri_store_tile(v, ops + tile * (4 * kTSlice), exps + tile * 128, warp, lane);
+}
+
+// One step of the solve in place on X.  src: the block row solved last (< 0:
+// none, the first step).  The first cluster of grid x updates the next block
+// row (src + 1 for L, src - 1 for U) with it and solves that.  The block rows
+// beyond are updated by a cluster each (SPLIT), or by one CTA per 128 rows
+// that takes the four quarters of K in turn.
+template <bool UPPER, bool SPLIT>
+__global__ void __launch_bounds__(kTThreads, 2)
+tri_step_kernel(const float2* __restrict__ F, int64_t ldf, const unsigned char* __restrict__ ops,
+                const int* __restrict__ exps, float2* X, int64_t ldx, int n, int ncols, int src, int first,
+                int* status) {
+  using namespace tc;
+  extern __shared__ __align__(1024) unsigned char smem_raw[];
+  unsigned char* abuf = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
+  unsigned char* bbuf = abuf + 4 * kTSlice;
+  float2* fresh = reinterpret_cast<float2*>(bbuf + 2 * kTSlice);   // 32 rows x 32 columns
+  __shared__ int rexp[128], cexp[kTC];
+  __shared__ unsigned cmax[8 * 32];
+  __shared__ uint64_t bar, bar_inv;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int abort_flag;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int rank = (int)(blockIdx.x & 7), cl = (int)(blockIdx.x >> 3), cg = blockIdx.y * kTC;
+  const bool alone = !SPLIT && cl > 0;   // no exchange with the cluster
+  const int next = src < 0 ? first : UPPER ? src - 1 : src + 1;
+  int half, kq, row0;
+  if (alone) {
+    half = 0;
+    kq = 0;
+    row0 = ((cl - 1) * 8 + rank) * 128 + (UPPER ? 0 : (next + 1) * kTD);
+    if (row0 >= (UPPER ? next * kTD : n)) return;
+  } else {
+    half = rank >> 2;
+    kq = rank & 3;
+    row0 = (UPPER ? next - cl : next + cl) * kTD + half * 128;
+  }
+  if (tid == 0) {
+    mbar_init(&bar, 1);
+    mbar_init(&bar_inv, 1);
+    abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)), "r"(256)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  const int64_t tile = (int64_t)next * 8 + rank;   // of the inverse, for the first cluster
+  float2 v[16][2];
+  // the factor's (first) tile: nothing that a step writes
+  if (src >= 0) {
+    const int c0 = src * kTD + kq * kTK;
+    tri_load_tile(v, F + (int64_t)row0 * ldf + c0, ldf, n - row0, n - c0, warp, lane);
+    // the other three quarters on their way to L2: 12 lines of 128 bytes a row
+    if (alone)
+      for (int idx = tid; idx < 128 * 12; idx += kTThreads) {
+        const int r = idx / 12, c = c0 + kTK + 16 * (idx % 12);
+        if (row0 + r < n && c < n) asm volatile("prefetch.global.L2 [%0];" ::"l"(F + (int64_t)(row0 + r) * ldf + c));
+      }
+    tri_store_tile(v, abuf, rexp, warp, lane);
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_slot;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+
+  // this CTA's share of a cluster's block row: 4 columns of one row per thread
+  const int orow = row0 + 32 * kq + (tid >> 3), ocol = cg + 4 * (tid & 7);
+  float2 b[4];
+  if (!alone) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      b[j] = orow < n && ocol + j < ncols ? ldcg(X + (int64_t)orow * ldx + ocol + j) : make_float2(0.f, 0.f);
+  }
+  const uint32_t paddr = smem_u32(bbuf);
+  float4* P = reinterpret_cast<float4*>(bbuf);
+  uint32_t phase = 0;
+  float2 x[8];
+  float acc[32];
+#pragma unroll
+  for (int j = 0; j < 32; ++j) acc[j] = 0.f;
+  // acc += (the tile in abuf) x (the right-hand sides in x)
+  auto product = [&](bool inverse) {
+    tri_store_rhs(x, bbuf, cmax, cexp, warp, lane);
+    fence_async_smem();
+    tc_fence_before();
+    __syncthreads();
+    if (tid == 0) {
+      if (inverse && !mbar_wait_plain(&bar_inv, 0)) abort_flag = 1;
+      tc_fence_after();
+      tri_issue(tmem, abuf, bbuf);
+      mma_commit(&bar);
+    }
+    if (!mbar_wait_plain(&bar, phase)) abort_flag = 1;
+    phase ^= 1;
+    tc_fence_after();
+  };
+  auto load_inverse = [&]() {
+    if (tid == 0) {
+      mbar_expect_tx(&bar_inv, 4 * kTSlice);
+      bulk_load(abuf, ops + tile * (4 * kTSlice), 4 * kTSlice, &bar_inv);
+    }
+  };
+  if (src >= 0) {
+#pragma unroll 1
+    for (int q = kq;; ++q) {
+      const int k0 = src * kTD + q * kTK;
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const int k = k0 + 8 * warp + i;
+        x[i] = k < n && cg + lane < ncols ? ldcg(X + (int64_t)k * ldx + cg + lane) : make_float2(0.f, 0.f);
+      }
+      product(false);
+      if (!alone && cl == 0) load_inverse();   // the tile's products are done
+      tri_read(acc, tmem, rexp, cexp, warp, lane);
+      tc_fence_before();
+      if (!alone || q == 3) break;
+      __syncthreads();   // the exponents and tensor memory are read
+      tri_load_tile(v, F + (int64_t)row0 * ldf + k0 + kTK, ldf, n - row0, n - k0 - kTK, warp, lane);
+      tri_store_tile(v, abuf, rexp, warp, lane);
+    }
+    if (alone) {
+      // rows of this thread, 16 columns each: through shared memory to whole rows
+      __syncthreads();
+      tri_partials(acc, P, warp, lane);
+      __syncthreads();
+      const bool in = cg + lane < ncols;
+#pragma unroll 1
+      for (int h = 0; h < 2; ++h) {
+        float2* at = X + (int64_t)(row0 + 64 * h + warp) * ldx + cg + lane;   // rows 8 apart
+        float2 o[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+          if (in && row0 + 64 * h + warp + 8 * i < n) o[i] = ldcg(at + 8 * i * ldx);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int r = 64 * h + warp + 8 * i;
+          const float2 p = reinterpret_cast<const float2*>(P + r * 16 + ((lane >> 1) ^ (r & 15)))[lane & 1];
+          if (in && row0 + r < n) at[8 * i * ldx] = make_float2(o[i].x - p.x, o[i].y - p.y);
+        }
+      }
+    } else {
+      __syncthreads();
+      tri_partials(acc, P, warp, lane);
+      tri_cluster_sync();
+      float2 s[4];
+      tri_gather(s, paddr, half, kq, tid);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        b[j].x -= s[j].x;
+        b[j].y -= s[j].y;
+      }
+    }
+  } else {
+    load_inverse();
+  }
+  if (!alone) {
+    if (cl == 0) {
+      // X = T^-1 B of this block row
+#pragma unroll
+      for (int j = 0; j < 4; j += 2)
+        *reinterpret_cast<float4*>(fresh + (tid >> 3) * kTC + 4 * (tid & 7) + j) =
+            make_float4(b[j].x, b[j].y, b[j + 1].x, b[j + 1].y);
+      if (tid < 128) rexp[tid] = exps[tile * 128 + tid];
+      tri_cluster_sync();   // the block row is complete, and the partial sums are read
+      // rows 64 kq .. + 63 of the block row: 32 with each of two CTAs
+      const uint32_t from = tri_mapa(smem_u32(fresh), (uint32_t)(2 * kq + (warp >> 2))) +
+                            (uint32_t)((8 * (warp & 3) * kTC + lane) * 8);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) x[i] = tri_ld2(from + (uint32_t)(i * kTC * 8));
+      product(true);
+#pragma unroll
+      for (int j = 0; j < 32; ++j) acc[j] = 0.f;
+      tri_read(acc, tmem, rexp, cexp, warp, lane);
+      tc_fence_before();
+      __syncthreads();
+      tri_partials(acc, P, warp, lane);
+      tri_cluster_sync();
+      tri_gather(b, paddr, half, kq, tid);
     }
 #pragma unroll
-    for (int a = 0; a < TR; ++a)
-#pragma unroll
-      for (int b = 0; b < TC; ++b) {
-        const int r = TR * tr + a, c = cg + tc + TPR * b;
-        if (r < rb && c < ncols) X[(int64_t)(r0 + r) * ldx + c] = out[a][b];
-      }
-    __threadfence();
+    for (int j = 0; j < 4; ++j)
+      if (orow < n && ocol + j < ncols) X[(int64_t)orow * ldx + ocol + j] = b[j];
+    tri_cluster_sync();   // no CTA leaves while its partial sums are being read
+  } else {
     __syncthreads();
-    if (tid == 0) st_release_u32(gflags + i, epoch);
+  }
+  if (tid == 0 && *(volatile int*)&abort_flag) atomicExch(status, MGT_ERR_TIMEOUT);
+  if (warp == 0) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256) : "memory");
   }
 }
 
-// counter = 0 for the work-item claims; every completion flag of this solve
-// cleared and the completion mark set to 1.  The workspace is allocated by the
-// caller and may hold anything (a freed permutation holds every small
-// integer), so nothing of the protocol may depend on its previous contents.
-__global__ void tri_start_kernel(unsigned* counter, unsigned* mark, unsigned* flags, int nflags) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) {
-    *counter = 0;
-    *mark = 1;
-  }
-  for (int f = i; f < nflags; f += gridDim.x * blockDim.x) flags[f] = 0;
-}
-
-// Items per (block row, column group): the main item and its helpers, for a
-// solve of nb block rows (the last rows' sums then take about nb / parts
-// block products in a row instead of nb)
-static int tri_parts(int64_t nb) { return nb >= 64 ? 4 : 1; }
-
-// Workspace of one triangular solve: counter, completion mark and status
-// (256 B); completion flags (groups x blocks) followed by the helpers' flags
-// (groups x blocks x (parts - 1)); inverted diagonal blocks (L and U); chain
-// factors W (L and U); the helpers' partial sums (64 x group width each).
-// Sized for the narrow groups (the most flags); a solve in wide groups fits.
+// Workspace of a solve: the status words (at byte 128); the inverted diagonal
+// blocks of L and of U; those of ill-conditioned blocks after the Newton step;
+// the operands and their row exponents; the blocks' row sums and condition
+// numbers.
 struct TriWs {
-  size_t flags = 256, inv, wch, part, total;
-  TriWs(int64_t n, int64_t nrhs, size_t elem) {
-    const int64_t nb = (n + kTB - 1) / kTB, ng = (nrhs + kTG - 1) / kTG, P = tri_parts(nb);
-    inv = flags + (((size_t)(nb * ng * P) * sizeof(unsigned) + 255) & ~size_t(255));
-    wch = inv + 2 * (size_t)nb * kTB * kTB * elem;
-    part = wch + 2 * (size_t)nb * kTB * kTB * elem;
-    const int64_t cols = (nrhs + kTGWide - 1) / kTGWide * kTGWide;   // >= groups x group width
-    total = part + (size_t)(nb * (P - 1)) * kTB * cols * elem;
+  size_t inv = 256, refined, ops, exps, rowsum, cond, total;
+  explicit TriWs(int64_t n) {
+    const size_t blocks = 2 * (size_t)((n + kTD - 1) / kTD);
+    refined = inv + blocks * kTD * kTD * sizeof(float2);
+    ops = refined + blocks * kTD * kTD * sizeof(float2);
+    exps = ops + blocks * 8 * 4 * kTSlice;
+    rowsum = exps + blocks * 8 * 128 * sizeof(int);
+    cond = rowsum + blocks * kTD * sizeof(float);
+    total = cond + blocks * sizeof(float);
   }
 };
 
-size_t tri_solve_workspace_bytes(int64_t n, int64_t nrhs, size_t elem) { return TriWs(n, nrhs, elem).total; }
+size_t tri_solve_workspace_bytes(int64_t n) { return TriWs(n).total; }
 
-static int resident_ctas(const void* kern, size_t smem) {
-  int dev = 0, sms = 1, per = 1;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kern, 256, smem);
-  return std::max(1, sms * std::max(1, per));
+template <bool UPPER>
+static int tri_steps(const float2* F, int64_t ldf, const unsigned char* ops, const int* exps, float2* X, int64_t ldx,
+                     int n, int nrhs, int* status, cudaStream_t s) {
+  const int nb = (n + kTD - 1) / kTD, ng = (nrhs + kTC - 1) / kTC, sms = device_sm_count();
+  for (int i = 0; i < nb; ++i) {
+    // step i solves block row i (from the end for U) after updating it and all that follow
+    const int first = UPPER ? nb - 1 : 0, src = i == 0 ? -1 : UPPER ? nb - i : i - 1;
+    const int rest = i == 0 ? 0 : nb - 1 - i;   // block rows beyond
+    // K over the CTAs of a cluster while every CTA of the launch is resident at
+    // once (two per SM); beyond, one CTA takes all of K: a quarter of the sums
+    // to exchange none, at 38 K clocks for 128 rows against 4 x 25 K
+    const bool split = (int64_t)8 * (1 + rest) * ng <= 2 * sms;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(8 * (1 + (split ? rest : (2 * rest + 7) / 8)), ng);
+    cfg.blockDim = dim3(kTThreads);
+    cfg.dynamicSmemBytes = kTSmem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[2];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim = {8, 1, 1};
+    // a step may start early when the launch before it is a step of this solve: the
+    // factor and the inverses, which it reads before it waits, are complete
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = UPPER || i > 0 ? 2 : 1;
+    count_launch();
+    if (cudaLaunchKernelEx(&cfg, split ? tri_step_kernel<UPPER, true> : tri_step_kernel<UPPER, false>, F, ldf, ops, exps,
+                           X, ldx, n, nrhs, src, first, status) != cudaSuccess)
+      return MGT_ERR_CUDA;
+  }
+  return MGT_OK;
 }
 
-// In-place X = T^-1 X (T = unit lower or upper part of F), nrhs columns.
-// inverses_ready: an earlier call with this workspace, n, nrhs and F made the
-// inverted diagonal blocks and chain factors.
-template <typename T, bool UPPER>
-int tri_solve(const cplx<T>* F, int64_t ldf, cplx<T>* X, int64_t ldx, int n, int nrhs, void* work, int* status,
-              bool inverses_ready, cudaStream_t s) {
-  using V = cplx<T>;
-  const size_t smem_inv = (size_t)(kTB * (kTB + 1) + kTB * kInvLd) * sizeof(V);
-  const size_t smem = (size_t)(tri_nbuf<T>() * kTB * (kTB + 1) + kTB * kTG) * sizeof(V);
-  const size_t smem_w = (size_t)(tri_nbuf<T>() * kTB * (kTB + 1) + kTB * kTGWide) * sizeof(V);
-  const size_t smem_cf = (size_t)(2 * kTB * (kTB + 1)) * sizeof(V);
-  // resident-CTA caps per device (set with the device's function attributes)
-  static int max_ctas_dev[kMaxDevices], max_ctas_w_dev[kMaxDevices];
+// In-place X = U^-1 L^-1 X with the factors in F (unit lower and upper), nrhs
+// columns.  inverses_ready: an earlier call with this workspace, n and F made
+// the inverted diagonal blocks.
+int tri_solve(const float2* F, int64_t ldf, float2* X, int64_t ldx, int n, int nrhs, void* work, bool inverses_ready,
+              cudaStream_t s) {
   static OncePerDevice once;
-  const int dev = current_device();
-  once([smem, smem_w, smem_inv, smem_cf, dev] {
-    int& max_ctas = max_ctas_dev[dev];
-    int& max_ctas_w = max_ctas_w_dev[dev];
-    cudaFuncSetAttribute(diag_inverse_kernel<T, UPPER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_inv);
-    cudaFuncSetAttribute(chain_factor_kernel<T, UPPER>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_cf);
-    cudaFuncSetAttribute(tri_solve_kernel<T, UPPER, kTG>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    // at most two CTAs per SM: the block row on the dependency chain shares its
-    // SM with fewer off-chain products (n = 12000, 64 RHS: 5.15 -> 4.80 ms per
-    // complex64 LU solve against the three that fit)
-    max_ctas = std::min(resident_ctas((const void*)tri_solve_kernel<T, UPPER, kTG>, smem), 2 * device_sm_count());
-    if constexpr (sizeof(T) == 4) {
-      cudaFuncSetAttribute(tri_solve_kernel<T, UPPER, kTGWide>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem_w);
-      max_ctas_w = std::min(resident_ctas((const void*)tri_solve_kernel<T, UPPER, kTGWide>, smem_w),
-                            2 * device_sm_count());
-    }
+  once([] {
+    cudaFuncSetAttribute(tri_inverse64_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInv64Smem);
+    cudaFuncSetAttribute(tri_double_kernel<64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tri_double_smem<64>());
+    cudaFuncSetAttribute(tri_double_kernel<128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)tri_double_smem<128>());
+    cudaFuncSetAttribute(tri_newton_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTNewtonSmem);
+    cudaFuncSetAttribute(tri_step_kernel<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTSmem);
+    cudaFuncSetAttribute(tri_step_kernel<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTSmem);
+    cudaFuncSetAttribute(tri_step_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTSmem);
+    cudaFuncSetAttribute(tri_step_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTSmem);
   });
-  // wide column groups where block rows alone give enough parallelism
-  const bool wide = sizeof(T) == 4 && n >= kWideMinN;
-  const int tg = wide ? kTGWide : kTG;
-  const int nb = (n + kTB - 1) / kTB, ng = (nrhs + tg - 1) / tg;
-  const int parts = tri_parts(nb);
-  const int dper = parts > 1 ? (nb - 1 + parts - 1) / parts : std::max(1, nb);   // parts x dper >= nb - 1
-  const TriWs L(n, nrhs, sizeof(V));
-  unsigned* counter = (unsigned*)work;
-  unsigned* flags = (unsigned*)((char*)work + L.flags);
-  unsigned* hflags = flags + (size_t)nb * ng;
-  // inverted diagonal blocks (L, then U), then the chain factors W (L, then U)
-  V* inv = (V*)((char*)work + L.inv) + (UPPER ? (size_t)nb * kTB * kTB : 0);
-  V* wch = (V*)((char*)work + L.wch) + (UPPER ? (size_t)nb * kTB * kTB : 0);
-  V* part = (V*)((char*)work + L.part);
+  int* status = (int*)((char*)work + 128);
+  if (cudaMemsetAsync(status, 0, 2 * sizeof(int), s) != cudaSuccess) return MGT_ERR_CUDA;
+  const int nb = (n + kTD - 1) / kTD;
+  const TriWs L(n);
+  float2* inv = (float2*)((char*)work + L.inv);
+  float2* refined = (float2*)((char*)work + L.refined);
+  unsigned char* ops = (unsigned char*)work + L.ops;
+  float* rowsum = (float*)((char*)work + L.rowsum);
+  float* cond = (float*)((char*)work + L.cond);
+  int* exps = (int*)((char*)work + L.exps);
   if (!inverses_ready) {
-    count_launch(2);
-    diag_inverse_kernel<T, UPPER><<<nb, 256, smem_inv, s>>>(F, ldf, n, inv);
-    chain_factor_kernel<T, UPPER><<<nb, 256, smem_cf, s>>>(F, ldf, n, inv, wch);
+    count_launch(6);
+    tri_inverse64_kernel<<<nb * (kTD / kTB), kTileThreads, kInv64Smem, s>>>(F, ldf, n, nb, inv, rowsum, cond);
+    tri_double_kernel<64><<<dim3(nb * 8, 2), 256, tri_double_smem<64>(), s>>>(F, ldf, n, nb, inv);
+    tri_double_kernel<128><<<dim3(nb * 8, 2), 256, tri_double_smem<128>(), s>>>(F, ldf, n, nb, inv);
+    tri_cond_kernel<<<dim3(nb * 4, 2), 512, 0, s>>>(nb, inv, rowsum, (unsigned*)cond);
+    tri_newton_kernel<<<dim3(nb * 16, 2), 512, kTNewtonSmem, s>>>(F, ldf, n, nb, inv, cond, refined);
+    tri_operand_kernel<<<nb * 16, kTThreads, 0, s>>>(inv, refined, cond, ops, exps);
   }
-  unsigned* epoch = counter + 1;   // completion mark, set by tri_start_kernel
-  const int nflags = nb * ng * parts;
-  const int64_t items = (int64_t)nb * ng * parts;
-  count_launch();
-  tri_start_kernel<<<std::max(1, std::min(nflags, 1 << 16) / 256 + 1), 256, 0, s>>>(counter, epoch, flags, nflags);
-  count_launch();
-  if constexpr (sizeof(T) == 4) {
-    if (wide) {
-      const int grid = (int)std::min<int64_t>(items, std::max(1, max_ctas_w_dev[dev]));
-      tri_solve_kernel<T, UPPER, kTGWide><<<grid, 256, smem_w, s>>>(F, ldf, inv, wch, X, ldx, n, nrhs, counter,
-                                                                     flags, epoch, status, parts, dper, part,
-                                                                     hflags);
-      return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
-    }
-  }
-  {
-    const int grid = (int)std::min<int64_t>(items, std::max(1, max_ctas_dev[dev]));
-    tri_solve_kernel<T, UPPER, kTG><<<grid, 256, smem, s>>>(F, ldf, inv, wch, X, ldx, n, nrhs, counter, flags,
-                                                             epoch, status, parts, dper, part, hflags);
-  }
+  int e = tri_steps<false>(F, ldf, ops, exps, X, ldx, n, nrhs, status, s);
+  if (e == MGT_OK)
+    e = tri_steps<true>(F, ldf, ops + (size_t)nb * 8 * 4 * kTSlice, exps + (size_t)nb * 8 * 128, X, ldx, n, nrhs,
+                        status, s);
+  if (e != MGT_OK) return e;
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }
 
 // Inverses of the 64 x 64 diagonal blocks of a unit lower factor of order n
 // (rows / columns at F), written to Inv[block][64][64]; the LU uses it for the
 // two inner panels of a 128-wide block.
-template <typename T>
-int lower_block_inverses(const cplx<T>* F, int64_t ldf, int n, cplx<T>* Inv, cudaStream_t s) {
-  using V = cplx<T>;
-  const size_t smem_inv = (size_t)(kTB * (kTB + 1) + kTB * kInvLd) * sizeof(V);
+int lower_block_inverses(const float2* F, int64_t ldf, int n, float2* Inv, cudaStream_t s) {
   static OncePerDevice once;
-  once([smem_inv] {
-    cudaFuncSetAttribute(diag_inverse_kernel<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_inv);
-  });
+  once([] { cudaFuncSetAttribute(lower_inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kInvSmem); });
   count_launch();
-  diag_inverse_kernel<T, false><<<(n + kTB - 1) / kTB, 256, smem_inv, s>>>(F, ldf, n, Inv);
+  lower_inverse_kernel<<<(n + kTB - 1) / kTB, 256, kInvSmem, s>>>(F, ldf, n, Inv);
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }
-template int lower_block_inverses<float>(const float2*, int64_t, int, float2*, cudaStream_t);
-
-template int tri_solve<float, false>(const float2*, int64_t, float2*, int64_t, int, int, void*, int*, bool,
-                                     cudaStream_t);
-template int tri_solve<float, true>(const float2*, int64_t, float2*, int64_t, int, int, void*, int*, bool,
-                                     cudaStream_t);
 
 }  // namespace mgt
