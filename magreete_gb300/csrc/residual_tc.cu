@@ -23,13 +23,14 @@
 //    at most 2^14.  Counting digits from the top (s = 6 - p), the pairs
 //    (s, t) with s + t = l share the weight 256^-l and accumulate in one
 //    TMEM accumulator per level l = 0 .. 6; pairs with s + t > 6 lie below
-//    2^-55 of the row and column scales and are not formed.  A level
-//    receives at most 7 pairs x 128 products (6 * 2^21 < 2^24 with the
-//    smaller top digits) before it is read out, so its FP32 sum is an exact
-//    integer.
-//  * Every 128 real K the level sums are read out of TMEM and folded into
+//    2^-55 of the row and column scales and are not formed.  A level sums
+//    256 products of each of its pairs before it is read out; levels 0 .. 4
+//    then stay within 2^24 (the top digits are smaller), exact integers in
+//    FP32, and 5 and 6 would round only beyond 2^24, by units that weigh
+//    2^-4 and 2^-12.
+//  * Every 256 real K the level sums are read out of TMEM and folded into
 //    one 64-bit integer per output in units of 2^-48 of the row and column
-//    scales: levels 0 .. 4 exactly, 5 and 6 rounded to within 0.53 unit.  A
+//    scales: levels 0 .. 4 exactly, 5 and 6 rounded to within a unit.  A
 //    64-bit accumulator per output sums them exactly (at most 2^15 real K per
 //    CTA keeps it below 2^63); the result is scaled back once at the end.
 // Accuracy (a numpy emulation of exactly this scheme on 2D / 3D systems of
@@ -46,16 +47,26 @@
 // x (a range of K in chunks), 512 threads:
 //   warp 0      : TMEM allocation (7 levels x 64 columns); bulk copies: per chunk the right-hand sides' digit block
 //                 (bdigits_kernel, 56 KB, 2 stages) and the seven 8 KB digit
-//                 slices of M (6-slice ring), whichever has a free slot
-//   warp 1      : MMA issuer.  Per chunk and digit s of A', one MMA per
+//                 slices of M (10-slice ring), whichever has a free slot
+//   warp 1      : MMA issuer, A' from TMEM.  Per chunk and digit s of A', one MMA per
 //                 16-wide K step covers the levels s .. 6 at once: the seven
 //                 digit slices of B' are stacked along N, so the levels
 //                 s + t, t = 0 .. 6 - s, are adjacent TMEM columns (N <= 256
 //                 per MMA: 10 MMAs per K step instead of 28)
 //   warps 2-9   : epilogue: thread = (row, half of the 64 real columns);
 //                 level sums -> 64-bit accumulators in registers
-//   warps 10-15 : converters: a staged byte slice -> the fp16 operand slice
-//                 (one byte permute and one fp16 subtract per digit pair)
+//   warps 10-13 : converters: a staged byte slice -> the fp16 operand slice in
+//                 TMEM (32 columns, two slices; thread = row; one byte permute
+//                 and one fp16 subtract per digit pair)
+// Measured, n = 12000 and 64 right-hand sides, one residual: 2.4 ms with A' in
+// shared memory and descriptors made as the MMAs were issued (issue bound, 184
+// clocks an MMA), 1.4 ms now; n = 3750, 900: 3.46 -> 2.2 ms.
+// Bound by the tensor pipe (3584 clocks a chunk; the digits are exact in fp16
+// alone) and, next, by shared memory: with A' there too, written once and read
+// ten times per K step, 670 KB a chunk went through it, 5200 clocks at 128 bytes
+// a clock; with A' in TMEM 360 KB.  Slices in the order 0, 6, 1, 5, ..: a
+// conversion overlaps the products of the slice before, and a slice's products
+// shrink with s.
 // Every wait is bounded; a CTA whose wait runs out writes NaN outputs, sets
 // MGT_ERR_TIMEOUT in the status word, drains what it issued and returns.
 #include <cuda_fp16.h>
@@ -76,26 +87,32 @@ constexpr int BNC = 32;                 // complex right-hand sides per tile
 constexpr int BN = 2 * BNC;             // real columns per tile (TMEM columns per level)
 constexpr int KCC = 32;                 // complex K per chunk (64 real: one 128-byte fp16 row)
 constexpr int DIG = 7;                  // digits per operand
-constexpr int ASLOTS = 4;               // fp16 operand-slice ring
-constexpr int DSLOTS = 6;               // byte-slice staging ring
-constexpr uint32_t A_SLICE = BM * 128;              // 16 KB: one fp16 digit slice of A'
-constexpr uint32_t D_SLICE = BM * 64;               // 8 KB: the same slice, one byte per digit
+constexpr int ASLOTS = 2;               // fp16 operand slices in TMEM
+constexpr int DSLOTS = 10;              // byte-slice staging ring
+constexpr uint32_t A_COLS = 32;                     // TMEM columns of one fp16 digit slice of A' (64 real K)
+constexpr uint32_t D_SLICE = BM * 64;               // 8 KB: a digit slice of A', one byte per digit
 constexpr uint32_t B_SLICE = BN * 128;              // 8 KB
 constexpr uint32_t B_BLOCK = DIG * B_SLICE;         // 56 KB: one chunk of B', all digit slices
 constexpr uint32_t TMEM_COLS = 512;
-constexpr int NEPI = 8, NCONV = 6;
+constexpr int NEPI = 8, NCONV = 4;
 constexpr int EPI0 = 2;                             // first epilogue warp
-// 16 warps: four per SM sub-partition leave 128 registers per thread
 constexpr int THREADS = (EPI0 + NEPI + NCONV) * 32;
 constexpr int EPI_COLS = BN / (NEPI / 4);           // real columns per epilogue thread
 // at most 512 chunks (32768 real K) per CTA: |sum| <= 2^15 * 2^48 = 2^63
 // units of 2^-48, less the rounding of levels 5 and 6
 constexpr int MAX_SPLIT_CHUNKS = 512;
+constexpr int READ_CHUNKS = 4;          // chunks between readouts of the levels
 constexpr long long BIAS = 0x0080808080808080LL;    // 128 in each of the seven digit positions
 constexpr int FIX = 54;                             // |X| < 2^FIX
 
+// polls (of some 50 clocks) without progress after which the producer gives up
+constexpr uint32_t kProducerLimit = 1u << 27;
+
+// the digit slice of A' taken j-th in a chunk: 0, 6, 1, 5, 2, 4, 3
+__host__ __device__ constexpr int slice_at(int j) { return j & 1 ? DIG - 1 - (j >> 1) : j >> 1; }
+
 constexpr size_t smem_bytes() {
-  return 1024 + ASLOTS * A_SLICE + DSLOTS * D_SLICE + 2 * B_BLOCK + BM * sizeof(int) + 256;
+  return 1024 + DSLOTS * D_SLICE + 2 * B_BLOCK + BM * sizeof(int) + 256;
 }
 
 // round(f * 2^sh) as a 64-bit integer (|f| * 2^sh < 2^54 by the row scale);
@@ -197,8 +214,7 @@ residual_tc_kernel(const unsigned char* __restrict__ D, int rows, const int* __r
   using namespace tc;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  unsigned char* aring = base;
-  unsigned char* bring = aring + ASLOTS * A_SLICE;
+  unsigned char* bring = base;
   unsigned char* dring = bring + 2 * B_BLOCK;
   int* rexp = reinterpret_cast<int*>(dring + DSLOTS * D_SLICE);
   uint64_t* full_a = reinterpret_cast<uint64_t*>(rexp + BM);
@@ -217,7 +233,7 @@ residual_tc_kernel(const unsigned char* __restrict__ D, int rows, const int* __r
   const int ct = blockIdx.x, rt = blockIdx.y, sp = blockIdx.z, row0 = rt * BM;
   const int c_begin = sp * chunks_per_split;
   const int nchunk = max(0, min(nch_total, c_begin + chunks_per_split) - c_begin);
-  const int nread = (nchunk + 1) >> 1;
+  const int nread = (nchunk + READ_CHUNKS - 1) / READ_CHUNKS;
 
   if (threadIdx.x < BM) rexp[threadIdx.x] = (row0 + (int)threadIdx.x < rows) ? clamp_exp(row_exp[row0 + threadIdx.x]) : 0;
   if (threadIdx.x == 0) {
@@ -252,21 +268,22 @@ residual_tc_kernel(const unsigned char* __restrict__ D, int rows, const int* __r
     uint32_t idle = 0;
     while ((ib < nchunk || q < nq) && !*abort) {
       bool progress = false;
-      if (ib < nchunk && (ib < 2 || mbar_try_wait(&empty_b[ib & 1], ((ib >> 1) - 1) & 1))) {
+      if (ib < nchunk && (ib < 2 || mbar_test(&empty_b[ib & 1], ((ib >> 1) - 1) & 1))) {
         mbar_expect_tx(&full_b[ib & 1], B_BLOCK);
         bulk_load(bring + (ib & 1) * B_BLOCK, bdig + ((size_t)ct * nch_total + c_begin + ib) * B_BLOCK, B_BLOCK,
                   &full_b[ib & 1]);
         ++ib;
         progress = true;
       }
-      if (q < nq && (q < DSLOTS || mbar_try_wait(&empty_d[q % DSLOTS], ((q / DSLOTS) - 1) & 1))) {
+      if (q < nq && (q < DSLOTS || mbar_test(&empty_d[q % DSLOTS], ((q / DSLOTS) - 1) & 1))) {
         mbar_expect_tx(&full_d[q % DSLOTS], D_SLICE);
-        bulk_load(dring + (q % DSLOTS) * D_SLICE, dsrc + (size_t)q * D_SLICE, D_SLICE, &full_d[q % DSLOTS]);
+        bulk_load(dring + (q % DSLOTS) * D_SLICE, dsrc + (size_t)(q / DIG * DIG + slice_at(q % DIG)) * D_SLICE, D_SLICE,
+                  &full_d[q % DSLOTS]);
         ++q;
         progress = true;
       }
       if (progress) idle = 0;
-      else if (++idle >= kWaitLimit) { *abort = 1; break; }
+      else if (++idle >= kProducerLimit) { *abort = 1; break; }
     }
     // copies in flight land before the CTA may exit
     for (int j = max(0, ib - 2); j < ib; ++j) mbar_wait_plain(&full_b[j & 1], (j >> 1) & 1);
@@ -275,36 +292,40 @@ residual_tc_kernel(const unsigned char* __restrict__ D, int rows, const int* __r
     // ---------------- MMA issuer
     int q = 0;
     bool ok = true;
+    const uint32_t atm = tmem + (uint32_t)(DIG * BN);
     for (int i = 0; i < nchunk && ok; ++i) {
-      const bool first = (i & 1) == 0;
-      if (first && i >= 2) {
-        if (!mbar_wait(tempty, ((i >> 1) - 1) & 1, abort)) { ok = false; break; }
+      const bool first = i % READ_CHUNKS == 0;
+      if (first && i > 0) {
+        if (!mbar_wait(tempty, (i / READ_CHUNKS - 1) & 1, abort)) { ok = false; break; }
         tc_fence_after();
       }
       const int st = i & 1;
       if (!mbar_wait(&full_b[st], (i >> 1) & 1, abort)) { ok = false; break; }
       tc_fence_after();
-      const uint32_t bb = smem_u32(bring + st * B_BLOCK);
-      for (int s = 0; s < DIG; ++s, ++q) {
-        const int slot = q % ASLOTS;
-        if (!mbar_wait(&full_a[slot], (q / ASLOTS) & 1, abort)) { ok = false; break; }
-        tc_fence_after();
-        const uint64_t ad = kmajor_sw128_desc(smem_u32(aring + slot * A_SLICE));
+      const uint64_t bb = kmajor_sw128_desc(smem_u32(bring + st * B_BLOCK));
 #pragma unroll
-        for (int ks = 0; ks < 4; ++ks) {
-          const uint32_t acc = (first && s == 0 && ks == 0) ? 0u : 1u;
-          for (int t0 = 0; t0 < DIG - s; t0 += 4) {
-            const int nt = min(4, DIG - s - t0);
-            const uint64_t bd = kmajor_sw128_desc(bb + (uint32_t)t0 * B_SLICE);
-            mma_f16(tmem + (uint32_t)((s + t0) * BN), ad + (uint64_t)(2 * ks), bd + (uint64_t)(2 * ks),
-                    idesc_f16_m128(nt * BN), acc);
-          }
+      for (int j = 0; j < DIG; ++j, ++q) {
+        if (!ok) continue;
+        const int s = slice_at(j), slot = q & 1;
+        if (!mbar_wait(&full_a[slot], (q / ASLOTS) & 1, abort)) { ok = false; continue; }
+        tc_fence_after();
+        const uint32_t ad = atm + (uint32_t)slot * A_COLS;
+        // the K steps innermost: 3600 clocks a chunk, against 4500 with the two
+        // ranges of levels innermost (the accumulator changes less often)
+#pragma unroll
+        for (int t0 = 0; t0 < DIG - s; t0 += 4) {
+          const int nt = DIG - s - t0 < 4 ? DIG - s - t0 : 4;
+#pragma unroll
+          for (int ks = 0; ks < 4; ++ks)
+            mma_f16_ta(tmem + (uint32_t)((s + t0) * BN), ad + (uint32_t)(8 * ks),
+                       bb + (uint64_t)(t0 * (B_SLICE >> 4) + 2 * ks), idesc_f16_m128(nt * BN),
+                       first && j == 0 && ks == 0 ? 0u : 1u);
         }
         mma_commit(&empty_a[slot]);
       }
       if (!ok) break;
       mma_commit(&empty_b[st]);
-      if (!first || i == nchunk - 1) mma_commit(tfull);
+      if (i % READ_CHUNKS == READ_CHUNKS - 1 || i == nchunk - 1) mma_commit(tfull);
     }
     mma_commit(done);   // arrives once every MMA issued above has completed
   } else if (warp >= EPI0 && warp < EPI0 + NEPI) {
@@ -336,17 +357,17 @@ residual_tc_kernel(const unsigned char* __restrict__ D, int rows, const int* __r
         }
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
-          // level l weighs 2^(36 - 8 l) units of 2^-48.  With |L_0| <= 2^19,
-          // |L_1| <= 2^21, |L_2| <= 2^22, |L_3| < 2^22.6, |L_4| <= 2^23 (top
-          // digits at most 64): hi = L_0 2^8 + L_1 and mid = L_2 2^8 + L_3 are
-          // exact in 32 bits; levels 5 and 6 round to the nearest unit through
-          // one FMA ((L_5 + L_6 / 256) / 16, its own rounding below 1/32 unit)
+          // level l weighs 2^(36 - 8 l) units of 2^-48.  With |L_0| <= 2^20,
+          // |L_1| <= 2^22 (top digits at most 64), L_0 2^8 + L_1 is exact in 32
+          // bits; levels 5 and 6 round to the nearest unit through one FMA
+          // ((L_5 + L_6 / 256) / 16, its own rounding below 1/16 unit)
           const int hi = (__float2int_rz(__uint_as_float(v[0][j])) << 8) + __float2int_rz(__uint_as_float(v[1][j]));
-          const int mid = (__float2int_rz(__uint_as_float(v[2][j])) << 8) + __float2int_rz(__uint_as_float(v[3][j]));
           const int l4 = __float2int_rz(__uint_as_float(v[4][j]));
           const int l56 = __float2int_rn(
               0.0625f * fmaf(__uint_as_float(v[6][j]), 0.00390625f, __uint_as_float(v[5][j])));
-          acc[p * 4 + j] += ((long long)hi << 28) + ((long long)mid << 12) + (long long)((l4 << 4) + l56);
+          acc[p * 4 + j] += (long long)hi * (1 << 28) + (long long)__float2int_rz(__uint_as_float(v[2][j])) * (1 << 20) +
+                            (long long)__float2int_rz(__uint_as_float(v[3][j])) * (1 << 12) +
+                            (long long)((l4 << 4) + l56);
         }
       }
     }
@@ -384,29 +405,52 @@ residual_tc_kernel(const unsigned char* __restrict__ D, int rows, const int* __r
       }
     }
   } else if (warp >= EPI0 + NEPI) {
-    // ---------------- converters: staged byte slice -> fp16 operand slice
-    const int ctid = threadIdx.x - (EPI0 + NEPI) * 32;
+    // ---------------- converters: staged byte slice -> fp16 operand slice; thread = row
+    const int qd = warp & 3, row = qd * 32 + lane;
+    const uint32_t abase = tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(DIG * BN);
     const int nq = nchunk * DIG;
-    for (int q = 0; q < nq; ++q) {
-      const int ds = q % DSLOTS, as = q % ASLOTS;
-      if (!mbar_wait(&full_d[ds], (q / DSLOTS) & 1, abort)) break;
-      if (q >= ASLOTS && !mbar_wait(&empty_a[as], ((q / ASLOTS) - 1) & 1, abort)) break;
-      const unsigned char* src = dring + ds * D_SLICE;
-      unsigned char* dst = aring + as * A_SLICE;
-      // thread: 8 digit bytes -> 16 contiguous operand bytes (both accesses
-      // contiguous across the warp)
-      for (int u = ctid; u < (int)(D_SLICE / 8); u += NCONV * 32) {
-        const uint32_t off = (uint32_t)u * 8u;
-        const uint2 v = *reinterpret_cast<const uint2*>(src + off);
-        const uint2 w0 = widen4(v.x), w1 = widen4(v.y);
-        *reinterpret_cast<uint4*>(dst + 2 * off) = make_uint4(w0.x, w0.y, w1.x, w1.y);
+    // the row's 64 digits, 16 bytes at a time: halves of two of the operand's swizzled 16-byte chunks
+    uint4 raw[4];
+    auto fetch = [&](int q) -> bool {
+      const int ds = q % DSLOTS;
+      if (!mbar_wait(&full_d[ds], (q / DSLOTS) & 1, abort)) return false;
+      const unsigned char* src = dring + ds * D_SLICE + row * 64;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) raw[c] = *reinterpret_cast<const uint4*>(src + ((c ^ ((row >> 1) & 3)) << 4));
+      return true;
+    };
+    bool ok = nq > 0 && fetch(0);
+    for (int q = 0; ok && q < nq; ++q) {
+      uint32_t w[32];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        const bool odd = row & 1;   // the swizzle swaps the two halves of odd rows
+        const uint2 w0 = widen4(odd ? raw[c].z : raw[c].x), w1 = widen4(odd ? raw[c].w : raw[c].y);
+        const uint2 w2 = widen4(odd ? raw[c].x : raw[c].z), w3 = widen4(odd ? raw[c].y : raw[c].w);
+        w[8 * c] = w0.x;
+        w[8 * c + 1] = w0.y;
+        w[8 * c + 2] = w1.x;
+        w[8 * c + 3] = w1.y;
+        w[8 * c + 4] = w2.x;
+        w[8 * c + 5] = w2.y;
+        w[8 * c + 6] = w3.x;
+        w[8 * c + 7] = w3.y;
       }
-      fence_async_smem();
       __syncwarp();
-      if (lane == 0) {
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full_a[as])) : "memory");
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&empty_d[ds])) : "memory");
+      if (lane == 0)
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&empty_d[q % DSLOTS])) : "memory");
+      if (q + 1 < nq) ok = fetch(q + 1);   // on its way while this slice waits for its place
+      const int as = q % ASLOTS;
+      if (q >= ASLOTS) {
+        if (!mbar_wait(&empty_a[as], ((q / ASLOTS) - 1) & 1, abort)) break;
+        tc_fence_after();
       }
+      tmem_st16(abase + (uint32_t)as * A_COLS, w);
+      tmem_st16(abase + (uint32_t)as * A_COLS + 16, w + 16);
+      tmem_wait_st();
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full_a[as])) : "memory");
     }
   }
   tc_fence_before();

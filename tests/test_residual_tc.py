@@ -144,3 +144,43 @@ def test_refinement_from_prepared_digits():
     X2, it2, rr2 = E.solve_refined(narrow, f, B)
     assert rr2 <= 1e-10
     assert (torch.linalg.norm(X2 - X_ref) / torch.linalg.norm(X_ref)).item() < 1e-9
+
+
+@pytest.mark.parametrize("n", [33, 128, 129, 640, 673, 705, 737, 4100])
+def test_tc_residual_extreme_digits(n):
+    """Every digit at its largest size and every product positive (imaginary
+    part): the level sums reach their bounds (levels 5 and 6 beyond 2^24) before
+    each readout, for 1 to 4 chunks in the last one.  The reference is the sum
+    the scheme forms, in integers: digit pairs (s, t), s + t <= 6 from the top.
+    Bound: four units of 2^-48 a readout of 256 real K (one each for rounding
+    levels 5 and 6, two for their sums beyond 2^24), readouts of up to 32 K
+    ranges counted, and the rounding of the result to FP64 beside it."""
+    from magreete_gb300 import engine as E
+
+    def digits(x):   # balanced base 256, top first
+        d = []
+        for _ in range(6):
+            r = (x + 128) % 256 - 128
+            d.append(r)
+            x = (x - r) // 256
+        return ([x] + d[::-1])
+
+    def formed(x, y):   # x y in units of 2^-108, without the pairs below level 6
+        a, b = digits(x), digits(y)
+        return sum(a[s] * b[t] * 256 ** (12 - s - t) for s in range(7) for t in range(7 - s))
+
+    V = 63 * 256 ** 6 + sum(128 * 256 ** p for p in range(6))
+    v = -float(V) * 2.0 ** -54
+    assert int(v * 2.0 ** 54) == -V
+    hi = np.float32(v)
+    lo = np.float32(v - float(hi))
+    assert float(hi) + float(lo) == v
+    Mdf = torch.tensor([hi, lo, hi, lo], dtype=torch.float32).repeat(n, n, 1).contiguous().cuda()
+    X = torch.full((n, 3), complex(v, v), dtype=torch.complex128, device="cuda")
+    B = torch.zeros(n, 3, dtype=torch.complex128, device="cuda")
+    got = E.residual(Mdf, X, B)
+    re = -float(n * (formed(-V, -V) + formed(-V, V))) * 2.0 ** -108
+    im = -float(2 * n * formed(-V, -V)) * 2.0 ** -108
+    bound = 4 * (n / 128 + 32) * 2.0 ** -48 + n * 2.0 ** -51
+    assert (got.real - re).abs().max().item() <= bound
+    assert (got.imag - im).abs().max().item() <= bound
