@@ -121,6 +121,11 @@ int mgt_lu_factor(int dtype, void* A, int64_t n, int64_t lda, int32_t* perm,
  *             (callers fall back to partial pivoting when it does not
  *             converge).  An exact zero tile pivot sets info as a zero pivot
  *             does.
+ *   symmetric: nonzero: the caller vouches that A = A^T (the system matrices
+ *             of this library are complex symmetric).  Tile pivoting on the
+ *             tensor cores then updates only the tiles on and above the
+ *             diagonal while the trailing matrix is large, and takes each
+ *             block's column from its row; other paths ignore it.
  *   panel_rows, panel_max_ctas, cooperative, lookahead, outer_block: as the
  *             MGT_TUNE_* keys of the same names (cooperative / lookahead: -1 =
  *             process value; outer_block 64 or 128)
@@ -128,13 +133,14 @@ int mgt_lu_factor(int dtype, void* A, int64_t n, int64_t lda, int32_t* perm,
 #define MGT_PIVOT_PARTIAL 0
 #define MGT_PIVOT_TILE 1
 typedef struct mgt_lu_options {
-  int32_t size;            /* sizeof(mgt_lu_options) */
+  int32_t size;            /* sizeof(mgt_lu_options), or that without `symmetric` */
   int32_t pivoting;
   int32_t panel_rows;
   int32_t panel_max_ctas;
   int32_t cooperative;
   int32_t lookahead;
   int32_t outer_block;
+  int32_t symmetric;       /* read when size covers it; 0 otherwise */
 } mgt_lu_options;
 int mgt_lu_factor_ex(int dtype, void* A, int64_t n, int64_t lda, int32_t* perm, void* work, size_t work_bytes,
                      const mgt_lu_options* options, void* stream);

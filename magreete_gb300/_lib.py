@@ -41,11 +41,12 @@ class LuOptions(ctypes.Structure):
     fields take the process-wide tuning values)."""
     _fields_ = [("size", ctypes.c_int32), ("pivoting", ctypes.c_int32), ("panel_rows", ctypes.c_int32),
                 ("panel_max_ctas", ctypes.c_int32), ("cooperative", ctypes.c_int32), ("lookahead", ctypes.c_int32),
-                ("outer_block", ctypes.c_int32)]
+                ("outer_block", ctypes.c_int32), ("symmetric", ctypes.c_int32)]
 
-    def __init__(self, pivoting=0, panel_rows=0, panel_max_ctas=0, cooperative=-1, lookahead=-1, outer_block=0):
+    def __init__(self, pivoting=0, panel_rows=0, panel_max_ctas=0, cooperative=-1, lookahead=-1, outer_block=0,
+                 symmetric=0):
         super().__init__(ctypes.sizeof(LuOptions), pivoting, panel_rows, panel_max_ctas, cooperative, lookahead,
-                         outer_block)
+                         outer_block, symmetric)
 
 
 _vp = ctypes.c_void_p

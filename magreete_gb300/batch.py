@@ -151,7 +151,7 @@ class BatchedSweep:
         # launched without the cooperative attribute (capturable), no lookahead (capture)
         self.lu_options = L.LuOptions(pivoting=E.PIVOTING[pivoting], panel_rows=int(panel_rows),
                                       panel_max_ctas=max(1, sms // self.branches), cooperative=0, lookahead=0,
-                                      outer_block=int(outer_block))
+                                      outer_block=int(outer_block), symmetric=1)
         # largest first, so that the long solves start early in every branch
         order = sorted(range(len(problems)), key=lambda i: -problems[i].n)
         self.order = order

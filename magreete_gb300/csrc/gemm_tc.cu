@@ -101,6 +101,18 @@ __device__ __forceinline__ void mma_split(uint32_t d_tmem, uint64_t a, uint64_t 
         : "memory");
   }
 }
+// (row, column) of tile t in row-major order of all tiles, or of those on and above the diagonal
+__device__ __forceinline__ int2 tile_at(int t, int tiles_n, int upper) {
+  if (!upper) return make_int2(t / tiles_n, t % tiles_n);
+  // row i starts at i tiles_n - i (i - 1) / 2
+  const float b = (float)tiles_n + 0.5f;
+  int i = (int)(b - sqrtf(fmaxf(b * b - 2.f * (float)t, 0.f)));
+  i = max(0, min(i, tiles_n - 1));
+  while (i > 0 && i * tiles_n - i * (i - 1) / 2 > t) --i;
+  while ((i + 1) * tiles_n - (i + 1) * i / 2 <= t) ++i;
+  return make_int2(i, i + t - (i * tiles_n - i * (i - 1) / 2));
+}
+
 // Persistent kernel: each CTA walks tiles blockIdx.x, +gridDim.x, ...; TMEM
 // holds two accumulators so the epilogue of tile t overlaps the MMAs of
 // tile t+1.  C is never loaded into the SM: the epilogue stages -acc in a
@@ -109,13 +121,15 @@ __device__ __forceinline__ void mma_split(uint32_t d_tmem, uint64_t a, uint64_t 
 // read it.
 // invA / invB (F16 mode): inverse row scales of A and inverse complex-column
 // scales of B.  The update reads the B split from row boff (twice its first
-// complex column) on, so that one split serves several launches.
+// complex column) and the A split from row aoff on, so that one split serves
+// several launches.  The launch takes tiles tbegin .. tend of the row-major
+// order of all of them, or (upper; C square) of those on and above the diagonal.
 template <bool F16, int STAGES, int CSLOTS>
 __global__ void __launch_bounds__(THREADS, 1)
 cgemm_split3_kernel(const __grid_constant__ CUtensorMap mapAhi, const __grid_constant__ CUtensorMap mapAlo,
                     const __grid_constant__ CUtensorMap mapBhi, const __grid_constant__ CUtensorMap mapBlo,
-                    const __grid_constant__ CUtensorMap mapC, int cx0, int cy0, int boff, int tiles_n,
-                    int total_tiles, int kblocks, const float* __restrict__ invA, const float* __restrict__ invB,
+                    const __grid_constant__ CUtensorMap mapC, int cx0, int cy0, int aoff, int boff, int tiles_n,
+                    int upper, int tbegin, int total_tiles, int kblocks, const float* __restrict__ invA, const float* __restrict__ invB,
                     int* status) {
   constexpr int BK = Mode<F16>::BK;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -150,13 +164,14 @@ cgemm_split3_kernel(const __grid_constant__ CUtensorMap mapAhi, const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const int first = blockIdx.x, stride = gridDim.x;
+  const int first = tbegin + blockIdx.x, stride = gridDim.x;
 
   if (warp == 0 && lane == 0) {
     // ---------------- TMA producer: A/B K blocks into the stage ring
     int it = 0;
     for (int t = first; t < total_tiles && !*abort; t += stride) {
-      const int m0 = (t / tiles_n) * BM, n0 = (t % tiles_n) * BN;
+      const int2 mn = tile_at(t, tiles_n, upper);
+      const int m0 = aoff + mn.x * BM, n0 = mn.y * BN;
       for (int kb = 0; kb < kblocks; ++kb, ++it) {
         const int s = it % STAGES;
         if (it >= STAGES && !mbar_wait(&empty[s], ((it / STAGES) - 1) & 1, abort)) break;
@@ -205,12 +220,12 @@ cgemm_split3_kernel(const __grid_constant__ CUtensorMap mapAhi, const __grid_con
     // loaded into the SM; a slot is handed back once its reduce has read it
     const int ntiles = total_tiles > first ? (total_tiles - first + stride - 1) / stride : 0;
     const int G = ntiles * CHUNKS;
+    int2 mn = make_int2(0, 0);
     for (int g = 0; g < G; ++g) {
       const int slot = g % CSLOTS;
       if (!mbar_wait(&cdone[slot], (g / CSLOTS) & 1, abort)) break;
-      const int t = first + (g / CHUNKS) * stride;
-      tma_reduce_add_2d(&mapC, cring + slot * CHUNK_BYTES, cx0 + (t % tiles_n) * BN + (g % CHUNKS) * 32,
-                        cy0 + (t / tiles_n) * BM);
+      if (g % CHUNKS == 0) mn = tile_at(first + (g / CHUNKS) * stride, tiles_n, upper);
+      tma_reduce_add_2d(&mapC, cring + slot * CHUNK_BYTES, cx0 + mn.y * BN + (g % CHUNKS) * 32, cy0 + mn.x * BM);
       bulk_commit();
       // every reduce but the newest has read its slot
       if (g >= 1) {
@@ -230,8 +245,8 @@ cgemm_split3_kernel(const __grid_constant__ CUtensorMap mapAhi, const __grid_con
       if (!mbar_wait(&tfull[acc], (lt >> 1) & 1, abort)) break;
       tc_fence_after();
       bool ok = true;
-      const int tile = first + lt * stride;
-      const int tm0 = (tile / tiles_n) * BM, tn0 = (tile % tiles_n) * BN;
+      const int2 mn = tile_at(first + lt * stride, tiles_n, upper);
+      const int tm0 = aoff + mn.x * BM, tn0 = mn.y * BN;
       const float rs = F16 ? -__ldg(invA + tm0 + r) : -1.f;
       for (int c = 0; c < CHUNKS; ++c) {
         const int g = lt * CHUNKS + c, slot = g % CSLOTS;
@@ -561,26 +576,44 @@ int tc_split_b(const TcPlan& plan, int N, int K, const float2* B, int64_t ldb, c
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }
 
-int tc_gemm(const TcPlan& plan, const CUtensorMap& cmap, int M, int N, int K, int cx0, int cy0, int* status,
-            cudaStream_t s, int max_ctas, int bcol) {
-  if (M <= 0 || N <= 0 || K <= 0) return MGT_OK;
-  if (K > tc::KMAX || M > plan.nmax || bcol < 0 || (int64_t)bcol + N > plan.nmax) return MGT_ERR_UNSUPPORTED;
+static int tc_launch(const TcPlan& plan, const CUtensorMap& cmap, int K, int cx0, int cy0, int aoff, int bcol,
+                     int tiles_n, bool upper, int tbegin, int tend, int* status, cudaStream_t s, int max_ctas) {
+  if (tend <= tbegin) return MGT_OK;
   tc_init_attrs();
   const int kblocks = tc_kcols(plan, K) / (plan.mode == MGT_TC_F16X2 ? tc::Mode<true>::BK : tc::Mode<false>::BK);
-  const int tiles_n = (2 * N + tc::BN - 1) / tc::BN, tiles_m = (M + tc::BM - 1) / tc::BM;
-  const int total = tiles_n * tiles_m;
-  int ctas = std::min(total, max_ctas > 0 ? max_ctas : tc_num_sms());
+  const int ctas = std::min(tend - tbegin, max_ctas > 0 ? max_ctas : tc_num_sms());
   count_launch();
 #define MGT_TC_LAUNCH(F16, ST, CS)                                                                              \
   tc::cgemm_split3_kernel<F16, ST, CS><<<ctas, tc::THREADS, tc::smem_bytes<ST, CS>(), s>>>(                    \
-      plan.mAhi, plan.mAlo, plan.mBhi, plan.mBlo, cmap, cx0, cy0, 2 * bcol, tiles_n, total, kblocks, plan.invA,    \
-      plan.invB, status)
+      plan.mAhi, plan.mAlo, plan.mBhi, plan.mBlo, cmap, cx0, cy0, aoff, 2 * bcol, tiles_n, upper ? 1 : 0, tbegin,  \
+      tend, kblocks, plan.invA, plan.invB, status)
   if (plan.mode == MGT_TC_F16X2)
     MGT_TC_LAUNCH(true, 2, 2);
   else
     MGT_TC_LAUNCH(false, 2, 2);
 #undef MGT_TC_LAUNCH
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
+}
+
+int tc_gemm(const TcPlan& plan, const CUtensorMap& cmap, int M, int N, int K, int cx0, int cy0, int* status,
+            cudaStream_t s, int max_ctas, int bcol) {
+  if (M <= 0 || N <= 0 || K <= 0) return MGT_OK;
+  if (K > tc::KMAX || M > plan.nmax || bcol < 0 || (int64_t)bcol + N > plan.nmax) return MGT_ERR_UNSUPPORTED;
+  const int tiles_n = (2 * N + tc::BN - 1) / tc::BN, tiles_m = (M + tc::BM - 1) / tc::BM;
+  return tc_launch(plan, cmap, K, cx0, cy0, 0, bcol, tiles_n, false, 0, tiles_n * tiles_m, status, s, max_ctas);
+}
+
+int tc_upper_tiles(int M) {
+  const int t = (M + tc::BM - 1) / tc::BM;
+  return t * (t + 1) / 2;
+}
+
+int tc_gemm_upper(const TcPlan& plan, const CUtensorMap& cmap, int M, int K, int c0, int off, int tbegin, int tend,
+                  int* status, cudaStream_t s, int max_ctas) {
+  if (M <= 0 || K <= 0) return MGT_OK;
+  if (K > tc::KMAX || off < 0 || (int64_t)off + M > plan.nmax) return MGT_ERR_UNSUPPORTED;
+  return tc_launch(plan, cmap, K, 2 * c0, c0, off, off, (M + tc::BM - 1) / tc::BM, true, tbegin,
+                   std::min(tend, tc_upper_tiles(M)), status, s, max_ctas);
 }
 
 int gemm_sub_tc(const TcPlan& plan, const CUtensorMap& cmap, int M, int N, int K, const float2* A, int64_t lda,

@@ -121,4 +121,12 @@ __device__ __forceinline__ void tc_split_cols(const TcSplitOut& o, const float2*
 int tc_gemm(const TcPlan& plan, const CUtensorMap& cmap, int M, int N, int K, int cx0, int cy0, int* status,
             cudaStream_t s, int max_ctas = 0, int bcol = 0);
 
+// The 128 x 128 tiles on and above the diagonal of the M x M block of C at row
+// and column c0 (it ends at the matrix's last row and column); the operands
+// from row / column off of the splits on.  Tiles tbegin .. tend (of
+// tc_upper_tiles(M), row by row).
+int tc_upper_tiles(int M);
+int tc_gemm_upper(const TcPlan& plan, const CUtensorMap& cmap, int M, int K, int c0, int off, int tbegin, int tend,
+                  int* status, cudaStream_t s, int max_ctas = 0);
+
 }  // namespace mgt

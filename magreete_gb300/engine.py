@@ -355,17 +355,20 @@ def solve_system(kind, points, k0, coef, shift, E0, precision="fp64", tol=DEFAUL
         # the digits replace the double-float copy before the LU needs its memory
         ctx = RefineContext(Mdf, E0.shape[1])
         del Mdf
-        f, X, it, rr = mixed_factor_solve(ctx, M32, E0, _fresh(kind, points, k0, coef, shift), tol, max_iter)
+        f, X, it, rr = mixed_factor_solve(ctx, M32, E0, _fresh(kind, points, k0, coef, shift), tol, max_iter,
+                                           symmetric=True)
         if stats is not None:
             stats.update(method="mixed", iterations=it, rel_residual=rr, pivoting=f.pivoting)
         return X
     raise ValueError(f"unknown precision {precision!r} (expected 'fp64' or 'mixed')")
 
 
-def mixed_factor(M32, fresh_m32):
+def mixed_factor(M32, fresh_m32, symmetric=False):
     """complex64 LU of M32 with tile pivoting; with partial pivoting of a fresh
-    copy (fresh_m32() returns one) when a tile pivot is exactly zero."""
-    f = lu_factor(M32, check_singular=False, pivoting="tile")
+    copy (fresh_m32() returns one) when a tile pivot is exactly zero.
+    symmetric: M32 equals its transpose, as every assembled system matrix does."""
+    f = lu_factor(M32, check_singular=False,
+                  options=L.LuOptions(pivoting=L.MGT_PIVOT_TILE, symmetric=1 if symmetric else 0))
     err, info = lu_info(f)
     if err != 0:
         raise L.MagreeteError(err, "mgt_lu_factor_ex (device)")
@@ -374,13 +377,13 @@ def mixed_factor(M32, fresh_m32):
     return lu_factor(fresh_m32(), pivoting="partial")
 
 
-def mixed_factor_solve(Mdf, M32, B, fresh_m32, tol=DEFAULT_TOL, max_iter=DEFAULT_MAX_ITER):
+def mixed_factor_solve(Mdf, M32, B, fresh_m32, tol=DEFAULT_TOL, max_iter=DEFAULT_MAX_ITER, symmetric=False):
     """Factor M32 (tile pivoting first) and refine M X = B against the
     double-float Mdf (or a RefineContext made from it); if the refinement
     does not reach tol on tile-pivoted factors, factor a fresh copy with
     partial pivoting and refine again.  Returns (factors, X, iterations,
     relative residual)."""
-    f = mixed_factor(M32, fresh_m32)
+    f = mixed_factor(M32, fresh_m32, symmetric)
     X, it, rr = solve_refined(Mdf, f, B, tol, max_iter, require=f.pivoting == "partial")
     if rr <= tol:
         return f, X, it, rr
@@ -410,7 +413,7 @@ class SystemFactorization:
             self.Mdf = self.ctx.Mdf
             del Mdf
             self._fresh = _fresh(kind, points, k0, coef, shift)
-            self.f = mixed_factor(M32, self._fresh)
+            self.f = mixed_factor(M32, self._fresh, symmetric=True)
         else:
             raise ValueError(f"unknown precision {precision!r}")
         self.last_iterations = 0
