@@ -34,6 +34,7 @@
 #include <cuda_fp16.h>
 
 #include <algorithm>
+#include <climits>
 
 #include "common.cuh"
 #include "diag.cuh"
@@ -49,7 +50,7 @@ constexpr int BN = 2 * BNC;
 constexpr int KCC = 32;                 // complex K per chunk
 constexpr int NCH = kZK / KCC;          // chunk stride of the digit buffers
 constexpr int DIG = 7, LEV = 8;
-constexpr int ASLOTS = 4, DSLOTS = 6;
+constexpr int ASLOTS = 4, DSLOTS = 4;
 constexpr uint32_t A_SLICE = BM * 128, D_SLICE = BM * 64, B_SLICE = BN * 128, B_BLOCK = DIG * B_SLICE;
 constexpr uint32_t TMEM_COLS = LEV * BN;
 constexpr int NEPI = 8, NCONV = 6, EPI0 = 2;
@@ -60,7 +61,13 @@ constexpr int kNonFinite = 0x40000000;
 constexpr int FIX = 54;
 static_assert(TMEM_COLS == 512, "all of TMEM");
 
-constexpr size_t smem_bytes() { return 1024 + ASLOTS * A_SLICE + DSLOTS * D_SLICE + 2 * B_BLOCK + 256; }
+constexpr uint32_t STAGE = 32 * 4 * 16;   // a warp's group of four columns on its way to whole row segments
+constexpr size_t smem_bytes() {
+  return 1024 + ASLOTS * A_SLICE + DSLOTS * D_SLICE + 2 * B_BLOCK + NEPI * STAGE + 256;
+}
+
+// polls (of some 50 clocks) without progress after which the producer gives up
+constexpr uint32_t kProducerLimit = 1u << 27;
 
 constexpr int kZeroExp = -100000;   // exponent of an exact zero
 constexpr int kBadExp = 1000000;    // of an infinity or a NaN
@@ -248,25 +255,44 @@ __device__ __forceinline__ double scaled_double(long long acc, int sc) {
   const unsigned long long bits = ((unsigned long long)(be - 1) << 52) + keep;
   return __longlong_as_double((long long)(bits | (acc < 0 ? 0x8000000000000000ull : 0ull)));
 }
+// The same for |sc| <= 900, without branches: be0 = 1023 + 62 + sc.
+__device__ __forceinline__ double scaled_plain(long long acc, int be0) {
+  const unsigned long long u = acc < 0 ? 0ull - (unsigned long long)acc : (unsigned long long)acc;
+  const int lz = __clzll((long long)u);
+  const unsigned long long m = u << (lz & 63);
+  unsigned long long keep = m >> 11;
+  keep += ((unsigned)m & 0x7ffu) + ((unsigned)keep & 1u) > 0x400u ? 1ull : 0ull;
+  const unsigned hi = (unsigned)(keep >> 32) + ((unsigned)(be0 - lz) << 20) + ((unsigned)(acc >> 32) & 0x80000000u);
+  return u ? __hiloint2double((int)hi, (int)(unsigned)keep) : 0.0;
+}
 
-// one MMA group per (digit s of A, 16-wide K step): levels s .. min(6 + s, 7)
-__device__ __forceinline__ void issue_digit(uint32_t tmem, uint64_t ad, uint32_t bb, int s, bool first) {
+// a level sum, an integer of at most 2^22
+__device__ __forceinline__ int level_int(uint32_t bits) {
+  return __float_as_int(__uint_as_float(bits) + 12582912.f) - 0x4B400000;
+}
+
+// Digit slice s of A (descriptor ad) against B's slices (descriptor bb of the
+// first): up to four levels per MMA, the K steps innermost.  s is a constant
+// where this is inlined, so that an MMA costs its issuing thread no arithmetic
+// but on the descriptors' low words (184 clocks each with the descriptors made
+// on the way; 90 of tensor work).
+__device__ __forceinline__ void issue_digit(uint32_t tmem, uint64_t ad, uint64_t bb, const int s, bool first) {
   using namespace tc;
-  const int nt_all = min(DIG, LEV - s);
+  const int nt_all = DIG < LEV - s ? DIG : LEV - s;
 #pragma unroll
-  for (int ks = 0; ks < 4; ++ks) {
-    const bool fresh = first && ks == 0;
-    for (int t0 = 0; t0 < nt_all; t0 += 4) {
-      int nt = min(4, nt_all - t0);
-      const uint64_t bd = kmajor_sw128_desc(bb + (uint32_t)t0 * B_SLICE) + (uint64_t)(2 * ks);
-      if (fresh && s == 1 && t0 == 4) {
+  for (int t0 = 0; t0 < nt_all; t0 += 4) {
+    const int nt = nt_all - t0 < 4 ? nt_all - t0 : 4;
+#pragma unroll
+    for (int ks = 0; ks < 4; ++ks) {
+      const uint64_t a = ad + (uint64_t)(2 * ks), b = bb + (uint64_t)(t0 * (B_SLICE >> 4) + 2 * ks);
+      const uint32_t d = tmem + (uint32_t)((s + t0) * BN);
+      if (s == 1 && t0 == 4 && ks == 0) {
         // level 7 starts here (levels 0 .. 6 started with s = 0)
-        mma_f16(tmem + (uint32_t)((s + 6) * BN), ad + (uint64_t)(2 * ks),
-                kmajor_sw128_desc(bb + 6u * B_SLICE) + (uint64_t)(2 * ks), idesc_f16_m128(BN), 0u);
-        nt = 2;
+        mma_f16(d, a, b, idesc_f16_m128(2 * BN), 1u);
+        mma_f16(d + 2 * BN, a, b + (uint64_t)(2 * (B_SLICE >> 4)), idesc_f16_m128(BN), first ? 0u : 1u);
+      } else {
+        mma_f16(d, a, b, idesc_f16_m128(nt * BN), s == 0 && ks == 0 && first ? 0u : 1u);
       }
-      mma_f16(tmem + (uint32_t)((s + t0) * BN), ad + (uint64_t)(2 * ks), bd, idesc_f16_m128(nt * BN),
-              (fresh && s == 0) ? 0u : 1u);
     }
   }
 }
@@ -281,7 +307,8 @@ zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aex
   unsigned char* aring = base;
   unsigned char* bring = aring + ASLOTS * A_SLICE;
   unsigned char* dring = bring + 2 * B_BLOCK;
-  uint64_t* full_a = reinterpret_cast<uint64_t*>(dring + DSLOTS * D_SLICE);
+  unsigned char* cstage = dring + DSLOTS * D_SLICE;
+  uint64_t* full_a = reinterpret_cast<uint64_t*>(cstage + NEPI * STAGE);
   uint64_t* empty_a = full_a + ASLOTS;
   uint64_t* full_d = empty_a + ASLOTS;
   uint64_t* empty_d = full_d + DSLOTS;
@@ -326,7 +353,7 @@ zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aex
     uint32_t idle = 0;
     while ((ib < nblk || q < nq) && !*abort) {
       bool progress = false;
-      if (ib < nblk && (ib < 2 || mbar_try_wait(&empty_b[ib & 1], ((ib >> 1) - 1) & 1))) {
+      if (ib < nblk && (ib < 2 || mbar_test(&empty_b[ib & 1], ((ib >> 1) - 1) & 1))) {
         const int tt = first + (ib / nch) * stride, slab = tt / sl.tiles, ct = (tt - slab * sl.tiles) % ctiles;
         mbar_expect_tx(&full_b[ib & 1], B_BLOCK);
         bulk_load(bring + (ib & 1) * B_BLOCK, bdig + slab * sl.bdig + ((size_t)ct * NCH + ib % nch) * B_BLOCK, B_BLOCK,
@@ -334,7 +361,7 @@ zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aex
         ++ib;
         progress = true;
       }
-      if (q < nq && (q < DSLOTS || mbar_try_wait(&empty_d[q % DSLOTS], ((q / DSLOTS) - 1) & 1))) {
+      if (q < nq && (q < DSLOTS || mbar_test(&empty_d[q % DSLOTS], ((q / DSLOTS) - 1) & 1))) {
         const int blk = q / DIG, tt = first + (blk / nch) * stride, slab = tt / sl.tiles;
         const int rt = (tt - slab * sl.tiles) / ctiles;
         mbar_expect_tx(&full_d[q % DSLOTS], D_SLICE);
@@ -344,7 +371,7 @@ zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aex
         progress = true;
       }
       if (progress) idle = 0;
-      else if (++idle >= kWaitLimit) { *abort = 1; break; }
+      else if (++idle >= kProducerLimit) { *abort = 1; break; }
     }
     // copies in flight land before the CTA may exit
     for (int j = max(0, ib - 2); j < ib; ++j) mbar_wait_plain(&full_b[j & 1], (j >> 1) & 1);
@@ -353,6 +380,7 @@ zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aex
     // ---------------- MMA issuer: one readout (at most 128 real K) per tile
     int q = 0, i = 0;
     bool ok = true;
+    const uint64_t a0 = kmajor_sw128_desc(smem_u32(aring));
     for (int lt = 0; lt < ntiles && ok; ++lt) {
       if (lt > 0) {
         if (!mbar_wait(tempty, (lt - 1) & 1, abort)) { ok = false; break; }
@@ -362,12 +390,15 @@ zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aex
         const int st = i & 1;
         if (!mbar_wait(&full_b[st], (i >> 1) & 1, abort)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t bb = smem_u32(bring + st * B_BLOCK);
+        const uint64_t bb = kmajor_sw128_desc(smem_u32(bring + st * B_BLOCK));
+#pragma unroll
         for (int s = 0; s < DIG; ++s, ++q) {
+          if (!ok) continue;
           const int slot = q % ASLOTS;
-          if (!mbar_wait(&full_a[slot], (q / ASLOTS) & 1, abort)) { ok = false; break; }
+          if (!mbar_wait(&full_a[slot], (q / ASLOTS) & 1, abort)) { ok = false; continue; }
           tc_fence_after();
-          issue_digit(tmem, kmajor_sw128_desc(smem_u32(aring + slot * A_SLICE)), bb, s, c == 0);
+          const uint64_t ad = a0 + (uint64_t)(slot * (A_SLICE >> 4));
+          issue_digit(tmem, ad, bb, s, c == 0);
           mma_commit(&empty_a[slot]);
         }
         if (ok) mma_commit(&empty_b[st]);
@@ -405,9 +436,10 @@ zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aex
 #pragma unroll
         for (int j = 0; j < 4; ++j) {
           // level l weighs 2^(42 - 8 l) units of 2^-54; |L_0| <= 2^19, |L_1| <= 2^21, |L_2| <= 2^22,
-          // |L_3| < 2^22.6: hi and mid are exact in 32 bits
-          const int hi = (__float2int_rz(__uint_as_float(v[0][j])) << 8) + __float2int_rz(__uint_as_float(v[1][j]));
-          const int mid = (__float2int_rz(__uint_as_float(v[2][j])) << 8) + __float2int_rz(__uint_as_float(v[3][j]));
+          // |L_3| < 2^22.6: hi and mid are exact in 32 bits.  The conversions run at 16 lanes a clock
+          // (4 K clocks a tile); up to 2^22 the sum with 1.5 2^23 has the integer in its low bits
+          const int hi = (level_int(v[0][j]) << 8) + level_int(v[1][j]);
+          const int mid = (level_int(v[2][j]) << 8) + __float2int_rz(__uint_as_float(v[3][j]));
           const int l4 = __float2int_rz(__uint_as_float(v[4][j])), l5 = __float2int_rz(__uint_as_float(v[5][j]));
           const int l67 = __float2int_rn(
               0.015625f * fmaf(__uint_as_float(v[7][j]), 0.00390625f, __uint_as_float(v[6][j])));
@@ -415,30 +447,75 @@ zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aex
                            (long long)((l5 << 2) + l67);
         }
       }
-      if (ncol <= 0) continue;
-      const int ea = aexp[slab * sl.aexp + row];
-      const int* be = bexp + slab * sl.bexp + col0;
+      const int ea = row < M ? aexp[slab * sl.aexp + row] : 0;
+      const int ebl = lane < EPI_COLS / 2 && col0 + lane < N ? bexp[slab * sl.bexp + col0 + lane] : 0;
+      // Where the whole warp has full rows, finite operands and results far from
+      // overflow and underflow: no branch from entry to entry, and C in groups of
+      // four columns that pass through shared memory, so that an access covers 64
+      // bytes of 8 rows instead of 16 of 32 (entry by entry, 32 lines an access
+      // and each load behind the store before it, a tile took 22 K clocks).
+      constexpr int NC = EPI_COLS / 2, G = 4;
       int em = 0;
+      const int ebmax = __reduce_max_sync(0xffffffffu, lane < NC ? ebl : INT_MIN);
+      const int ebmin = __reduce_min_sync(0xffffffffu, lane < NC ? ebl : INT_MAX);
+      const bool plain = ncol == NC && ea != kNonFinite && ebmax < 1 << 20 && abs(ea + ebmax - FIX) <= 900 &&
+                         abs(ea + ebmin - FIX) <= 900;
+      if (__all_sync(0xffffffffu, plain)) {
+        unsigned char* stage = cstage + (warp - EPI0) * STAGE;
+        // this lane's place in the group: rows 8 i + lane / 4, column lane % 4
+        const int r4 = lane >> 2, c4 = lane & 3;
+        double2* cq = C + slab * sl.c + (int64_t)(row - lane + r4) * ldc + col0 + c4;
+        int emr[4];
 #pragma unroll
-      for (int j = 0; j < EPI_COLS / 2; ++j) {
-        if (j < ncol) {
-          const int eb = be[j];
-          double2 o = sub ? crow[j] : make_double2(0.0, 0.0);
-          if (ea == kNonFinite || eb == kNonFinite) {
-            o.x = o.y = __longlong_as_double(0x7FF8000000000000LL);
-          } else {
-            const int sc = ea + eb - FIX;
-            const double x = scaled_double(acc[2 * j], sc), y = scaled_double(acc[2 * j + 1], sc);
-            if (sub) {
-              o.x -= x;
-              o.y -= y;
-            } else {
-              o.x = x;
-              o.y = y;
-            }
+        for (int i = 0; i < 4; ++i) emr[i] = 0;
+#pragma unroll
+        for (int g = 0; g < NC / G; ++g) {
+          double2 o[4];
+          if (sub) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) o[i] = cq[8 * i * ldc + G * g];
           }
-          crow[j] = o;
-          em = max(em, field(o));
+#pragma unroll
+          for (int j = 0; j < G; ++j) {
+            const int be0 = ea + __shfl_sync(0xffffffffu, ebl, G * g + j) + (1023 + 62 - FIX);
+            *reinterpret_cast<double2*>(stage + lane * 64 + ((j ^ ((lane >> 1) & 3)) << 4)) =
+                make_double2(scaled_plain(acc[2 * (G * g + j)], be0), scaled_plain(acc[2 * (G * g + j) + 1], be0));
+          }
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int rr = 8 * i + r4;
+            double2 v = *reinterpret_cast<const double2*>(stage + rr * 64 + ((c4 ^ ((rr >> 1) & 3)) << 4));
+            if (sub) v = make_double2(o[i].x - v.x, o[i].y - v.y);
+            cq[8 * i * ldc + G * g] = v;
+            if (rowmax) emr[i] = max(emr[i], field(v));
+          }
+          __syncwarp();
+        }
+        if (rowmax) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            emr[i] = max(emr[i], __shfl_xor_sync(0xffffffffu, emr[i], 1));
+            emr[i] = max(emr[i], __shfl_xor_sync(0xffffffffu, emr[i], 2));
+            if (c4 == 0 && emr[i] > 0) atomicMax(rowmax + row - lane + 8 * i + r4, emr[i]);
+          }
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < NC; ++j) {
+          const int eb = __shfl_sync(0xffffffffu, ebl, j);
+          if (j < ncol) {
+            double2 v = sub ? crow[j] : make_double2(0.0, 0.0);
+            if (ea == kNonFinite || eb == kNonFinite) {
+              v.x = v.y = __longlong_as_double(0x7FF8000000000000LL);
+            } else {
+              const int sc = ea + eb - FIX;
+              const double x = scaled_double(acc[2 * j], sc), y = scaled_double(acc[2 * j + 1], sc);
+              v = sub ? make_double2(v.x - x, v.y - y) : make_double2(x, y);
+            }
+            crow[j] = v;
+            em = max(em, field(v));
+          }
         }
       }
       if (rowmax && em > 0) atomicMax(rowmax + row, em);
