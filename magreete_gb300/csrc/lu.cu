@@ -1359,10 +1359,11 @@ __device__ __forceinline__ void bar_arrive_n(int id) {
 // are updated.
 // Rows never move: s_piv[c] is the tile row chosen at column c, s_state its
 // inverse (64: not chosen yet); rows of U go to F by position.
-// Measured at w = 64: 31 us (59 K clocks: the pivot chain 25 K, warp 0's next
-// four columns 8 K, the inverses 17 K); with the largest value and its row found
-// by two reductions and update warps on warp 0's scheduler too 38 us; with one
-// block barrier per column 57 us.
+// Measured at w = 64: 28 us (53.5 K clocks: the pivot chain 25 K, warp 0's next
+// four columns 8 K, the inverses 11 K -- 17 K with one entry a thread in their
+// products); with the largest value and its row found by two reductions and
+// update warps on warp 0's scheduler too 38 us; with one block barrier per
+// column 57 us.
 __global__ void __launch_bounds__(kTileThreads, 1)
 lu_tile_kernel(float2* __restrict__ A, int64_t lda, int w, int j0, int32_t* __restrict__ perm, PanelWs ws,
                float2* __restrict__ Uinv, float2* __restrict__ Linv) {
@@ -1567,69 +1568,105 @@ lu_tile_kernel(float2* __restrict__ A, int64_t lda, int w, int j0, int32_t* __re
   }
 }
 
+// acc (row r of a staged block, columns 2 g + 16 q, 2 g + 16 q + 1, q < 4) += or -= row r of X times
+// M (64 x 64 in shared memory); TRI: M is upper triangular.  CT: the row's threads take the
+// CT-th parts of its columns: q from q0 in steps of CT.
+template <int CT, bool SUB, bool TRI>
+__device__ __forceinline__ void row_times(float2 (&acc)[8 / CT], const float2* x, const float2* M, int g, int q0,
+                                          int w) {
+#pragma unroll
+  for (int seg = 0; seg < 4; ++seg) {
+    const int end = min(16 * seg + 16, w);
+#pragma unroll 4
+    for (int i = 16 * seg; i < end; ++i) {
+      const float2 a = x[i];
+#pragma unroll
+      for (int q = 0; q < 4 / CT; ++q) {
+        if (TRI && CT * q + CT - 1 < seg) continue;   // columns left of this segment's rows
+        const float4 m = *reinterpret_cast<const float4*>(M + i * 64 + 2 * g + 16 * (CT * q + q0));
+        if (SUB) {
+          cfms(acc[2 * q], a, make_float2(m.x, m.y));
+          cfms(acc[2 * q + 1], a, make_float2(m.z, m.w));
+        } else {
+          cfma(acc[2 * q], a, make_float2(m.x, m.y));
+          cfma(acc[2 * q + 1], a, make_float2(m.z, m.w));
+        }
+      }
+    }
+  }
+}
+// 64 columns of RB rows (of `rows`, from r0) into shared memory, zeros beyond w columns
+template <int RB>
+__device__ __forceinline__ void stage_rows(float2* dst, const float2* A, int64_t lda, int r0, int rows, int w,
+                                           bool vec, int tid) {
+  if (vec && w == 64) {
+    for (int idx = tid; idx < RB * 32; idx += 256) {
+      const int r = idx >> 5, k = 2 * (idx & 31);
+      const bool in = r0 + r < rows;
+      cp_async_elem<16>(dst + r * 64 + k, in ? A + (int64_t)(r0 + r) * lda + k : A, in);
+    }
+    return;
+  }
+  for (int idx = tid; idx < RB * 64; idx += 256) {
+    const int r = idx >> 6, k = idx & 63;
+    const bool in = r0 + r < rows && k < w;
+    cp_async_elem<8>(dst + idx, in ? A + (int64_t)(r0 + r) * lda + k : A, in);
+  }
+}
+
 // Rows below the first tile of a 128-wide block (tile pivoting), fused:
 // L21 = A21 U11^-1 on the first panel's w columns, then the second panel's wb
 // columns A22 -= L21 U12 (U12: the first panel's rows of those columns,
-// already solved).  32 rows per CTA, thread = (row, every eighth column).
+// already solved).  RB rows per CTA: 16 while that leaves every SM at most one
+// CTA (n = 2000: 9 us against 15 with 32, one column a load and U11^-1 as a full
+// matrix), else 32.
+template <int RB>
 __global__ void __launch_bounds__(256)
 lu_l21_update_kernel(float2* __restrict__ A, int64_t lda, int rows, int w, int wb, const float2* __restrict__ Uinv,
                      const float2* __restrict__ U12) {
   // A: first row below the tile, first column of the panel; U12: the panel's
   // first row, first column of the second panel
+  constexpr int CT = 32 / RB;
   extern __shared__ __align__(16) unsigned char fused_smem[];
   float2* Ui = reinterpret_cast<float2*>(fused_smem);   // [64][64]
   float2* Us = Ui + 64 * 64;                             // [64][64] U12
-  float2* Ar = Us + 64 * 64;                             // [32][64] A21, then L21
-  float2* Cr = Ar + 32 * 64;                             // [32][64] A22
-  const int tid = threadIdx.x, r0 = blockIdx.x * 32;
+  float2* Ar = Us + 64 * 64;                             // [RB][64] A21, then L21
+  float2* Cr = Ar + RB * 64;                             // [RB][64] A22
+  const int tid = threadIdx.x, r0 = blockIdx.x * RB;
+  const bool vec = (lda & 1) == 0 && ((uintptr_t)A & 15) == 0 && ((uintptr_t)U12 & 15) == 0;
+  stage_rows<RB>(Ar, A, lda, r0, rows, w, vec, tid);
   for (int idx = tid; idx < 64 * 32; idx += 256) cp_async_elem<16>(Ui + 2 * idx, Uinv + 2 * idx, true);
-  for (int idx = tid; idx < 64 * 64; idx += 256) {
-    const int k = idx >> 6, c = idx & 63;
-    const bool in = k < w && c < wb;
-    cp_async_elem<8>(Us + idx, in ? U12 + (int64_t)k * lda + c : U12, in);
-  }
-  for (int idx = tid; idx < 32 * 64; idx += 256) {
-    const int r = idx >> 6, k = idx & 63;
-    const bool ra = r0 + r < rows && k < w, rc = r0 + r < rows && k < wb;
-    cp_async_elem<8>(Ar + idx, ra ? A + (int64_t)(r0 + r) * lda + k : A, ra);
-    cp_async_elem<8>(Cr + idx, rc ? A + (int64_t)(r0 + r) * lda + w + k : A, rc);
-  }
   cp_async_commit();
-  cp_async_wait<0>();
+  stage_rows<64>(Us, U12, lda, 0, w, wb, vec, tid);
+  stage_rows<RB>(Cr, A + w, lda, r0, rows, wb, vec, tid);
+  cp_async_commit();
+  cp_async_wait<1>();
   __syncthreads();
-  const int r = tid >> 3, g = tid & 7;
-  float2 acc[8];
+  const int r = tid / (8 * CT), g = tid & 7, q0 = (tid >> 3) % CT;
+  float2 acc[8 / CT];
 #pragma unroll
-  for (int q = 0; q < 8; ++q) acc[q] = make_float2(0.f, 0.f);
-  for (int i = 0; i < w; ++i) {
-    const float2 a = Ar[r * 64 + i];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) cfma(acc[q], a, Ui[i * 64 + g + 8 * q]);
-  }
+  for (int q = 0; q < 8 / CT; ++q) acc[q] = make_float2(0.f, 0.f);
+  row_times<CT, false, true>(acc, Ar + r * 64, Ui, g, q0, w);
+  cp_async_wait<0>();
   __syncthreads();   // every thread has read its row of A21
 #pragma unroll
-  for (int q = 0; q < 8; ++q) {
-    const int k = g + 8 * q;
+  for (int q = 0; q < 8 / CT; ++q) {
+    const int k = 2 * g + 16 * (CT * (q >> 1) + q0) + (q & 1);
     Ar[r * 64 + k] = acc[q];
     if (r0 + r < rows && k < w) A[(int64_t)(r0 + r) * lda + k] = acc[q];
+    acc[q] = Cr[r * 64 + k];
   }
   __syncthreads();
-#pragma unroll
-  for (int q = 0; q < 8; ++q) acc[q] = Cr[r * 64 + g + 8 * q];
-  for (int k = 0; k < w; ++k) {
-    const float2 l = Ar[r * 64 + k];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) cfms(acc[q], l, Us[k * 64 + g + 8 * q]);
-  }
+  row_times<CT, true, false>(acc, Ar + r * 64, Us, g, q0, w);
   if (r0 + r < rows) {
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int c = g + 8 * q;
+    for (int q = 0; q < 8 / CT; ++q) {
+      const int c = 2 * g + 16 * (CT * (q >> 1) + q0) + (q & 1);
       if (c < wb) A[(int64_t)(r0 + r) * lda + w + c] = acc[q];
     }
   }
 }
-constexpr size_t kL21UpdateSmem = (2 * 64 * 64 + 2 * 32 * 64) * sizeof(float2);
+template <int RB> constexpr size_t l21_update_smem() { return (2 * 64 * 64 + 2 * RB * 64) * sizeof(float2); }
 
 // The interchanges of tile t (rows 64 t .., position q holds tile row
 // perm[64 t + q] - 64 t: rows move only within their tile) on the columns
@@ -1657,17 +1694,19 @@ lu_tile_left_perm_kernel(float2* __restrict__ A, int64_t lda, int n, const int32
   }
 }
 
-// Rows below the tile: A21 <- A21 U11^-1 (w columns), 32 rows per CTA; the
-// operands are staged with asynchronous copies (all in flight at once).
+// Rows below the tile: A21 <- A21 U11^-1 (w columns), RB rows per CTA (as
+// above); the operands are staged with asynchronous copies (all in flight at once).
 // With Lba, one more CTA applies the tile's interchanges (slots) to its rows of
 // the 64 columns at Lba (the block's first panel).
+template <int RB>
 __global__ void __launch_bounds__(256)
 lu_l21_kernel(float2* __restrict__ A, int64_t lda, int rows, int w, const float2* __restrict__ Uinv,
               float2* __restrict__ Lba, const int2* __restrict__ slots) {
   // A: first row below the tile, first column of the panel
+  constexpr int CT = 32 / RB;
   __shared__ __align__(16) float2 Ui[64 * 64];
-  __shared__ __align__(16) float2 Ar[32 * 64];
-  const int tid = threadIdx.x, r0 = blockIdx.x * 32;
+  __shared__ __align__(16) float2 Ar[RB * 64];
+  const int tid = threadIdx.x, r0 = blockIdx.x * RB;
   if (r0 >= rows) {
     for (int idx = tid; idx < 64 * 64; idx += 256) {
       const int q = idx >> 6, k = idx & 63;
@@ -1685,27 +1724,19 @@ lu_l21_kernel(float2* __restrict__ A, int64_t lda, int rows, int w, const float2
     return;
   }
   for (int idx = tid; idx < 64 * 32; idx += 256) cp_async_elem<16>(Ui + 2 * idx, Uinv + 2 * idx, true);
-  for (int idx = tid; idx < 32 * 64; idx += 256) {
-    const int r = idx >> 6, k = idx & 63;
-    const bool in = r0 + r < rows && k < w;
-    cp_async_elem<8>(Ar + idx, in ? A + (int64_t)(r0 + r) * lda + k : A, in);
-  }
+  stage_rows<RB>(Ar, A, lda, r0, rows, w, (lda & 1) == 0 && ((uintptr_t)A & 15) == 0, tid);
   cp_async_commit();
   cp_async_wait<0>();
   __syncthreads();
-  const int r = tid >> 3, g = tid & 7;
-  float2 acc[8];
+  const int r = tid / (8 * CT), g = tid & 7, q0 = (tid >> 3) % CT;
+  float2 acc[8 / CT];
 #pragma unroll
-  for (int q = 0; q < 8; ++q) acc[q] = make_float2(0.f, 0.f);
-  for (int i = 0; i < w; ++i) {
-    const float2 a = Ar[r * 64 + i];
-#pragma unroll
-    for (int q = 0; q < 8; ++q) cfma(acc[q], a, Ui[i * 64 + g + 8 * q]);
-  }
+  for (int q = 0; q < 8 / CT; ++q) acc[q] = make_float2(0.f, 0.f);
+  row_times<CT, false, true>(acc, Ar + r * 64, Ui, g, q0, w);
   if (r0 + r < rows) {
 #pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      const int k = g + 8 * q;
+    for (int q = 0; q < 8 / CT; ++q) {
+      const int k = 2 * g + 16 * (CT * (q >> 1) + q0) + (q & 1);
       if (k < w) A[(int64_t)(r0 + r) * lda + k] = acc[q];
     }
   }
@@ -1921,7 +1952,10 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
     cudaFuncSetAttribute(lu_panel_reg_kernel<T, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)reg_panel_smem(NB, sizeof(V)));
     cudaFuncSetAttribute(lu_tile_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmem);
-    cudaFuncSetAttribute(lu_l21_update_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kL21UpdateSmem);
+    cudaFuncSetAttribute(lu_l21_update_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)l21_update_smem<16>());
+    cudaFuncSetAttribute(lu_l21_update_kernel<32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)l21_update_smem<32>());
   });
   PanelWs ws = panel_ws(work);
   if (cudaMemsetAsync(work, 0, 32, s) != cudaSuccess) return MGT_ERR_CUDA;   // status, nslot
@@ -1954,7 +1988,9 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
         count_launch();
         const int below = n - j0 - w;
         if ((below > 0 && with_l21) || lba) {
-          lu_l21_kernel<<<(below + 31) / 32 + (lba ? 1 : 0), 256, 0, s>>>(
+          const bool few = below <= 16 * sms;   // rows per CTA
+          (few ? lu_l21_kernel<16> : lu_l21_kernel<32>)<<<(below + (few ? 15 : 31)) / (few ? 16 : 32) + (lba ? 1 : 0),
+                                                          256, 0, s>>>(
               A + (int64_t)(j0 + w) * lda + j0, lda, below, w, Ui, lba ? A + (int64_t)j0 * lda + j0 - NB : nullptr,
               panel_ws(work, set).slots);
           count_launch();
@@ -2196,9 +2232,14 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
       if (fuse) {
         if constexpr (sizeof(T) == 4) {
           const float2* Ui = reinterpret_cast<const float2*>((char*)work + LuWsLayout().uinv);
-          lu_l21_update_kernel<<<(n - j1 + 31) / 32, 256, kL21UpdateSmem, s>>>(
-              reinterpret_cast<float2*>(A) + (int64_t)j1 * lda + J0, lda, n - j1, wa, wb, Ui,
-              reinterpret_cast<const float2*>(A) + (int64_t)J0 * lda + j1);
+          float2* below = reinterpret_cast<float2*>(A) + (int64_t)j1 * lda + J0;
+          const float2* U12 = reinterpret_cast<const float2*>(A) + (int64_t)J0 * lda + j1;
+          if (n - j1 <= 16 * sms)
+            lu_l21_update_kernel<16><<<(n - j1 + 15) / 16, 256, l21_update_smem<16>(), s>>>(below, lda, n - j1, wa, wb,
+                                                                                            Ui, U12);
+          else
+            lu_l21_update_kernel<32><<<(n - j1 + 31) / 32, 256, l21_update_smem<32>(), s>>>(below, lda, n - j1, wa, wb,
+                                                                                            Ui, U12);
           count_launch();
         }
       } else {

@@ -537,19 +537,19 @@ __device__ __forceinline__ void tri_partials(const float (&acc)[32], float4* P, 
 // This CTA's 32 rows of the cluster half's sum: row 32 kq + tid / 8, complex columns 4 (tid & 7) .. + 3
 __device__ __forceinline__ void tri_gather(float2 (&s)[4], uint32_t paddr, int half, int kq, int tid) {
   const int row = 32 * kq + (tid >> 3), c4 = 2 * (tid & 7);
-#pragma unroll
-  for (int j = 0; j < 4; ++j) s[j] = make_float2(0.f, 0.f);
+  float4 v[4][2];   // all on their way before the first is used
 #pragma unroll
   for (int q = 0; q < 4; ++q) {
     const uint32_t base = tri_mapa(paddr, (uint32_t)(4 * half + q)) + (uint32_t)row * 256u;
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const float4 v = tri_ld4(base + (uint32_t)(((c4 + j) ^ (row & 15)) * 16));
-      s[2 * j].x += v.x;
-      s[2 * j].y += v.y;
-      s[2 * j + 1].x += v.z;
-      s[2 * j + 1].y += v.w;
-    }
+    for (int j = 0; j < 2; ++j) v[q][j] = tri_ld4(base + (uint32_t)(((c4 + j) ^ (row & 15)) * 16));
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    s[2 * j].x = (v[0][j].x + v[1][j].x) + (v[2][j].x + v[3][j].x);
+    s[2 * j].y = (v[0][j].y + v[1][j].y) + (v[2][j].y + v[3][j].y);
+    s[2 * j + 1].x = (v[0][j].z + v[1][j].z) + (v[2][j].z + v[3][j].z);
+    s[2 * j + 1].y = (v[0][j].w + v[1][j].w) + (v[2][j].w + v[3][j].w);
   }
 }
 
@@ -746,10 +746,12 @@ tri_step_kernel(const float2* __restrict__ F, int64_t ldf, const unsigned char* 
       tri_cluster_sync();
       tri_gather(b, paddr, half, kq, tid);
     }
+    // no CTA leaves while its partial sums are being read
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       if (orow < n && ocol + j < ncols) X[(int64_t)orow * ldx + ocol + j] = b[j];
-    tri_cluster_sync();   // no CTA leaves while its partial sums are being read
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   } else {
     __syncthreads();
   }
