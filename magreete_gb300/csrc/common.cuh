@@ -140,6 +140,31 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
+// Programmatic dependent launch: a kernel launched with launch_early may start
+// while the kernel before it in the stream runs.  early_start lets the next one
+// start likewise and waits until the kernel before has completed and its writes
+// are visible; nothing that a kernel writes may be touched above it.  Saves the
+// 1 to 2 us from one small kernel's last block to the next one's first.
+__device__ __forceinline__ void early_start() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... P, typename... A>
+inline cudaError_t launch_early(bool early, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s,
+                                A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = early ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 // Iteration limit of every device-side spin wait (about a few seconds with
 // the back-off below).  A wait that runs out records MGT_ERR_TIMEOUT in the
 // status word and the kernel returns instead of hanging.

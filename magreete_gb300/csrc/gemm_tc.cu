@@ -164,6 +164,7 @@ cgemm_split3_kernel(const __grid_constant__ CUtensorMap mapAhi, const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  early_start();   // (launched early after the pass that made the operands, or as ever)
   const int first = tbegin + blockIdx.x, stride = gridDim.x;
 
   if (warp == 0 && lane == 0) {
@@ -577,30 +578,31 @@ int tc_split_b(const TcPlan& plan, int N, int K, const float2* B, int64_t ldb, c
 }
 
 static int tc_launch(const TcPlan& plan, const CUtensorMap& cmap, int K, int cx0, int cy0, int aoff, int bcol,
-                     int tiles_n, bool upper, int tbegin, int tend, int* status, cudaStream_t s, int max_ctas) {
+                     int tiles_n, bool upper, int tbegin, int tend, int* status, cudaStream_t s, int max_ctas,
+                     bool early) {
   if (tend <= tbegin) return MGT_OK;
   tc_init_attrs();
   const int kblocks = tc_kcols(plan, K) / (plan.mode == MGT_TC_F16X2 ? tc::Mode<true>::BK : tc::Mode<false>::BK);
   const int ctas = std::min(tend - tbegin, max_ctas > 0 ? max_ctas : tc_num_sms());
   count_launch();
-#define MGT_TC_LAUNCH(F16, ST, CS)                                                                              \
-  tc::cgemm_split3_kernel<F16, ST, CS><<<ctas, tc::THREADS, tc::smem_bytes<ST, CS>(), s>>>(                    \
-      plan.mAhi, plan.mAlo, plan.mBhi, plan.mBlo, cmap, cx0, cy0, aoff, 2 * bcol, tiles_n, upper ? 1 : 0, tbegin,  \
-      tend, kblocks, plan.invA, plan.invB, status)
-  if (plan.mode == MGT_TC_F16X2)
-    MGT_TC_LAUNCH(true, 2, 2);
-  else
-    MGT_TC_LAUNCH(false, 2, 2);
-#undef MGT_TC_LAUNCH
+  auto go = [&](auto kernel) {
+    return launch_early(early, kernel, ctas, tc::THREADS, tc::smem_bytes<2, 2>(), s, plan.mAhi, plan.mAlo, plan.mBhi,
+                        plan.mBlo, cmap, cx0, cy0, aoff, 2 * bcol, tiles_n, upper ? 1 : 0, tbegin, tend, kblocks,
+                        plan.invA, plan.invB, status);
+  };
+  const cudaError_t e = plan.mode == MGT_TC_F16X2 ? go(tc::cgemm_split3_kernel<true, 2, 2>)
+                                                  : go(tc::cgemm_split3_kernel<false, 2, 2>);
+  if (e != cudaSuccess) return MGT_ERR_CUDA;
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }
 
 int tc_gemm(const TcPlan& plan, const CUtensorMap& cmap, int M, int N, int K, int cx0, int cy0, int* status,
-            cudaStream_t s, int max_ctas, int bcol) {
+            cudaStream_t s, int max_ctas, int bcol, bool early) {
   if (M <= 0 || N <= 0 || K <= 0) return MGT_OK;
   if (K > tc::KMAX || M > plan.nmax || bcol < 0 || (int64_t)bcol + N > plan.nmax) return MGT_ERR_UNSUPPORTED;
   const int tiles_n = (2 * N + tc::BN - 1) / tc::BN, tiles_m = (M + tc::BM - 1) / tc::BM;
-  return tc_launch(plan, cmap, K, cx0, cy0, 0, bcol, tiles_n, false, 0, tiles_n * tiles_m, status, s, max_ctas);
+  return tc_launch(plan, cmap, K, cx0, cy0, 0, bcol, tiles_n, false, 0, tiles_n * tiles_m, status, s, max_ctas,
+                   early);
 }
 
 int tc_upper_tiles(int M) {
@@ -613,7 +615,7 @@ int tc_gemm_upper(const TcPlan& plan, const CUtensorMap& cmap, int M, int K, int
   if (M <= 0 || K <= 0) return MGT_OK;
   if (K > tc::KMAX || off < 0 || (int64_t)off + M > plan.nmax) return MGT_ERR_UNSUPPORTED;
   return tc_launch(plan, cmap, K, 2 * c0, c0, off, off, (M + tc::BM - 1) / tc::BM, true, tbegin,
-                   std::min(tend, tc_upper_tiles(M)), status, s, max_ctas);
+                   std::min(tend, tc_upper_tiles(M)), status, s, max_ctas, false);
 }
 
 int gemm_sub_tc(const TcPlan& plan, const CUtensorMap& cmap, int M, int N, int K, const float2* A, int64_t lda,

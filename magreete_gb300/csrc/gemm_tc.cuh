@@ -117,9 +117,11 @@ __device__ __forceinline__ void tc_split_cols(const TcSplitOut& o, const float2*
   if (q == 0) o.invb[col0 + c] = ldexpf(1.f, e);
 }
 
-// bcol: the first column of B (within the split) this launch uses.
+// bcol: the first column of B (within the split) this launch uses.  early: the
+// launch before it in the stream, nothing between, is one that ends the operands
+// and calls early_start.
 int tc_gemm(const TcPlan& plan, const CUtensorMap& cmap, int M, int N, int K, int cx0, int cy0, int* status,
-            cudaStream_t s, int max_ctas = 0, int bcol = 0);
+            cudaStream_t s, int max_ctas = 0, int bcol = 0, bool early = false);
 
 // The 128 x 128 tiles on and above the diagonal of the M x M block of C at row
 // and column c0 (it ends at the matrix's last row and column); the operands

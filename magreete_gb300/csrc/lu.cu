@@ -1367,6 +1367,7 @@ __device__ __forceinline__ void bar_arrive_n(int id) {
 __global__ void __launch_bounds__(kTileThreads, 1)
 lu_tile_kernel(float2* __restrict__ A, int64_t lda, int w, int j0, int32_t* __restrict__ perm, PanelWs ws,
                float2* __restrict__ Uinv, float2* __restrict__ Linv) {
+  early_start();
   // A: the tile's top-left element (row j0, column j0); w <= 64
   extern __shared__ __align__(16) unsigned char tile_smem[];
   float2* T = reinterpret_cast<float2*>(tile_smem);    // [64][kTileLD]: the tile by tile row; then U^-1
@@ -1624,6 +1625,7 @@ template <int RB>
 __global__ void __launch_bounds__(256)
 lu_l21_update_kernel(float2* __restrict__ A, int64_t lda, int rows, int w, int wb, const float2* __restrict__ Uinv,
                      const float2* __restrict__ U12) {
+  early_start();
   // A: first row below the tile, first column of the panel; U12: the panel's
   // first row, first column of the second panel
   constexpr int CT = 32 / RB;
@@ -1702,6 +1704,7 @@ template <int RB>
 __global__ void __launch_bounds__(256)
 lu_l21_kernel(float2* __restrict__ A, int64_t lda, int rows, int w, const float2* __restrict__ Uinv,
               float2* __restrict__ Lba, const int2* __restrict__ slots) {
+  early_start();
   // A: first row below the tile, first column of the panel
   constexpr int CT = 32 / RB;
   __shared__ __align__(16) float2 Ui[64 * 64];
@@ -1747,6 +1750,7 @@ lu_l21_kernel(float2* __restrict__ A, int64_t lda, int rows, int w, const float2
 __global__ void __launch_bounds__(256)
 lu_tile_u12_kernel(float2* __restrict__ A, int64_t lda, int w, int wb, const int2* __restrict__ slots,
                    const float2* __restrict__ Linv) {
+  early_start();
   // A: first row of the tile, first column of the second panel
   __shared__ __align__(16) float2 L[64 * 66];
   __shared__ float2 X[64][4];
@@ -1784,6 +1788,7 @@ template <int CW, bool SPLIT>
 __global__ void __launch_bounds__(256)
 lu_tile_right_kernel(float2* __restrict__ A, int64_t lda, int n, int J0, const int2* __restrict__ slotsA,
                      const int2* __restrict__ slotsB, const float2* __restrict__ Inv, int cblocks, TcSplitOut out) {
+  early_start();
   constexpr int W = 128, LDT = CW + 1, NC = CW / 8, QN = 256 / CW;   // QN threads per column in the split
   extern __shared__ __align__(16) unsigned char tr_smem[];
   float2* LA = reinterpret_cast<float2*>(tr_smem);   // [64][65]: L_AA^-1, L_BA, L_BB^-1
@@ -1918,7 +1923,7 @@ static SideStream* side_stream() {
 // Trailing order from which a symmetric factorisation keeps to the upper half.
 // The panels' chain bounds smaller ones, and each block pays for its transpose:
 // from order 1024 on, n = 3750 takes 3.75 ms against 3.71 with every tile
-// updated; from 4096 on, n = 6000 6.7 against 7.1, 12000 19.1 / 24.2, 21000 57 / 86.
+// updated; from 4096 on, n = 6000 5.9 against 6.4, 12000 17.6 / 22.6, 21000 55 / 83.
 constexpr int kSymMin = 4096;
 
 // A[r][c] = A[c][r] for the columns c0 .. c0 + cols and, in each of their 128-wide
@@ -1926,6 +1931,7 @@ constexpr int kSymMin = 4096;
 // Bound by memory: 32 x 32 tiles through shared memory, whole lines both ways.
 __global__ void __launch_bounds__(256)
 lu_mirror_kernel(float2* __restrict__ A, int64_t lda, int n, int r0, int c0, int cols) {
+  early_start();
   __shared__ float2 t[32][33];
   const int r = r0 + blockIdx.x * 32, c = c0 + blockIdx.y * 32;   // the tile written
   if (r < c0 + ((c - c0) / 128 + 1) * 128) return;
@@ -1966,6 +1972,13 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
   count_launch();
   const int sms = std::min(num_sms(), kMaxPanelBlocks);
   const size_t sm2 = (2 * NB * kSwapCols + NB * NB) * sizeof(V);
+  // Early launches (launch_early) only where this factorisation has the GPU to
+  // itself, as lookahead says, and for blocks that find room beside the side
+  // stream's update: one block, or a block row that needs one CTA an SM at most.
+  // (LU n = 2000 1.72 -> 1.60 ms.  Everywhere, waiting blocks kept others from
+  // starting: a graph of 12 systems 7.3 -> 8.0 ms, n = 12000 23.1 -> 24.4.)
+  const bool early = opt.lookahead != 0;
+  auto early_rows = [&](int rows) { return early && rows <= 16 * sms; };
   // CTAs of the panel kernel for a panel of m rows
   auto panel_ctas = [&](int m) -> int {
     const int64_t min_g_smem = ((int64_t)m * NB * (int64_t)sizeof(V) + kPanelSmemBudget - 1) / kPanelSmemBudget;
@@ -1983,16 +1996,16 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
         float2* Ui = reinterpret_cast<float2*>((char*)work + Lw.uinv);
         // L11^-1 where the fused right-column pass reads the block's diagonal inverses
         float2* Li = reinterpret_cast<float2*>((char*)work + Lw.inv) + (size_t)set * kNBmax * kNBmax;
-        lu_tile_kernel<<<1, kTileThreads, kTileSmem, s>>>(A + (int64_t)j0 * lda + j0, lda, w, j0, perm, panel_ws(work, set),
-                                                  Ui, Li);
+        launch_early(early, lu_tile_kernel, 1, kTileThreads, kTileSmem, s, A + (int64_t)j0 * lda + j0, lda, w, j0, perm,
+                     panel_ws(work, set), Ui, Li);
         count_launch();
         const int below = n - j0 - w;
         if ((below > 0 && with_l21) || lba) {
           const bool few = below <= 16 * sms;   // rows per CTA
-          (few ? lu_l21_kernel<16> : lu_l21_kernel<32>)<<<(below + (few ? 15 : 31)) / (few ? 16 : 32) + (lba ? 1 : 0),
-                                                          256, 0, s>>>(
-              A + (int64_t)(j0 + w) * lda + j0, lda, below, w, Ui, lba ? A + (int64_t)j0 * lda + j0 - NB : nullptr,
-              panel_ws(work, set).slots);
+          launch_early(early_rows(below), few ? lu_l21_kernel<16> : lu_l21_kernel<32>,
+                       (below + (few ? 15 : 31)) / (few ? 16 : 32) + (lba ? 1 : 0), 256, 0, s,
+                       A + (int64_t)(j0 + w) * lda + j0, lda, below, w, Ui,
+                       lba ? A + (int64_t)j0 * lda + j0 - NB : nullptr, panel_ws(work, set).slots);
           count_launch();
         }
         return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
@@ -2220,9 +2233,8 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
     // right-column pass) are swapped with the second panel
     if (fuse) {
       if constexpr (sizeof(T) == 4) {
-        lu_tile_u12_kernel<<<(wb + 3) / 4, 256, 0, s>>>(
-            A + (int64_t)J0 * lda + j1, lda, wa, wb, panel_ws(work, 0).slots,
-            reinterpret_cast<const float2*>((char*)work + LuWsLayout().inv));
+        launch_early(early, lu_tile_u12_kernel, (wb + 3) / 4, 256, 0, s, A + (int64_t)J0 * lda + j1, lda, wa, wb,
+                     panel_ws(work, 0).slots, reinterpret_cast<const float2*>((char*)work + LuWsLayout().inv));
         count_launch();
       }
     } else {
@@ -2234,12 +2246,10 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
           const float2* Ui = reinterpret_cast<const float2*>((char*)work + LuWsLayout().uinv);
           float2* below = reinterpret_cast<float2*>(A) + (int64_t)j1 * lda + J0;
           const float2* U12 = reinterpret_cast<const float2*>(A) + (int64_t)J0 * lda + j1;
-          if (n - j1 <= 16 * sms)
-            lu_l21_update_kernel<16><<<(n - j1 + 15) / 16, 256, l21_update_smem<16>(), s>>>(below, lda, n - j1, wa, wb,
-                                                                                            Ui, U12);
-          else
-            lu_l21_update_kernel<32><<<(n - j1 + 31) / 32, 256, l21_update_smem<32>(), s>>>(below, lda, n - j1, wa, wb,
-                                                                                            Ui, U12);
+          const bool few = n - j1 <= 16 * sms;
+          launch_early(early_rows(n - j1), few ? lu_l21_update_kernel<16> : lu_l21_update_kernel<32>,
+                       (n - j1 + (few ? 15 : 31)) / (few ? 16 : 32), 256,
+                       few ? l21_update_smem<16>() : l21_update_smem<32>(), s, below, lda, n - j1, wa, wb, Ui, U12);
           count_launch();
         }
       } else {
@@ -2270,14 +2280,12 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
         const int blocks = cb + (split ? (right + 7) / 8 : 0);
         const TcSplitOut o = tc_split_out(tc->plan);
         count_launch();
-        if (narrow && split)
-          lu_tile_right_kernel<16, true><<<blocks, 256, tile_right_smem<16>(), s>>>(A, lda, n, J0, sa, sb, Inv, cb, o);
-        else if (narrow)
-          lu_tile_right_kernel<16, false><<<blocks, 256, tile_right_smem<16>(), s>>>(A, lda, n, J0, sa, sb, Inv, cb, o);
-        else if (split)
-          lu_tile_right_kernel<32, true><<<blocks, 256, tile_right_smem<32>(), s>>>(A, lda, n, J0, sa, sb, Inv, cb, o);
-        else
-          lu_tile_right_kernel<32, false><<<blocks, 256, tile_right_smem<32>(), s>>>(A, lda, n, J0, sa, sb, Inv, cb, o);
+        // (after a join of the side stream the pass waits for two things: an ordinary launch)
+        launch_early(early_rows(right) && side == nullptr,
+                     narrow ? (split ? lu_tile_right_kernel<16, true> : lu_tile_right_kernel<16, false>)
+                            : (split ? lu_tile_right_kernel<32, true> : lu_tile_right_kernel<32, false>),
+                     blocks, 256, narrow ? tile_right_smem<16>() : tile_right_smem<32>(), s, A, lda, n, J0, sa, sb, Inv,
+                     cb, o);
         return split;
       }
       if (wb > 0 && opt.fused_right) {
@@ -2308,7 +2316,8 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
       dom_begin(s);
       int e = ready ? MGT_OK : tc_split_a(tc->plan, M, W, L21, lda, s);
       if (e == MGT_OK && !ready) e = tc_split_b(tc->plan, WN, W, U12, lda, s);
-      if (e == MGT_OK) e = tc_gemm(tc->plan, tc->cmap, M, WN, W, 2 * P0, P0, ws.status, s);
+      if (e == MGT_OK) e = tc_gemm(tc->plan, tc->cmap, M, WN, W, 2 * P0, P0, ws.status, s, 0, 0,
+                                    ready && early_rows(M));
       dom_end(s, 8.0 * M * (double)WN * W, sizeof(V) * (2.0 * M * (double)WN + (double)M * W + (double)W * WN));
       if (e != MGT_OK) return e;
       if (cudaEventRecord(side->fork, s) != cudaSuccess || cudaStreamWaitEvent(s2, side->fork, 0) != cudaSuccess)
@@ -2375,7 +2384,8 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
   // Those rows, updated first, stand in for the next block's columns above.
   auto mirror = [&](int r0, int c0, int cols) {
     if constexpr (sizeof(T) == 4) {
-      lu_mirror_kernel<<<dim3((n - r0 + 31) / 32, (cols + 31) / 32), 256, 0, s>>>(A, lda, n, r0, c0, cols);
+      launch_early(false, lu_mirror_kernel, dim3((n - r0 + 31) / 32, (cols + 31) / 32), 256, 0, s, A, lda, n, r0, c0,
+                   cols);
       count_launch();
     }
   };
@@ -2462,7 +2472,7 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
         if constexpr (sizeof(T) == 4) {
           const int M = n - P0;
           dom_begin(s);
-          e = tc_gemm(tc->plan, tc->cmap, M, M, KW, 2 * P0, P0, ws.status, s);
+          e = tc_gemm(tc->plan, tc->cmap, M, M, KW, 2 * P0, P0, ws.status, s, 0, 0, early_rows(M));
           dom_end(s, 8.0 * M * (double)M * KW, sizeof(V) * (2.0 * M * (double)M + 2.0 * (double)M * KW));
         }
       } else {
