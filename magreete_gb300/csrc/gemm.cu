@@ -19,6 +19,7 @@ template <typename T, int RT>
 __global__ void __launch_bounds__(256)
 cgemm_sub_kernel(int M, int N, int K, const cplx<T>* __restrict__ A, int64_t lda,
                  const cplx<T>* __restrict__ B, int64_t ldb, cplx<T>* __restrict__ C, int64_t ldc) {
+  early_start();
   using V = cplx<T>;
   constexpr int GT = 16 * RT;
   __shared__ V As[kGK][GT + 1];
@@ -80,7 +81,8 @@ static int gemm_sub_rt(int M, int N, int K, const cplx<T>* A, int64_t lda, const
   dim3 grid((N + GT - 1) / GT, (M + GT - 1) / GT);
   if (grid.y > 65535) return MGT_ERR_UNSUPPORTED;
   count_launch();
-  cgemm_sub_kernel<T, RT><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, C, ldc);
+  // (complex64 updates run on side streams too, after waits for events: ordinary launches)
+  launch_early(sizeof(T) == 8 && (int64_t)grid.x * grid.y <= 2 * device_sm_count(), cgemm_sub_kernel<T, RT>, grid, 256, 0, s, M, N, K, A, lda, B, ldb, C, ldc);
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }
 

@@ -80,6 +80,12 @@ __device__ __forceinline__ int expo(double v, int off) {
   return max(ex, 1) + off;
 }
 
+// Launched early only while every block is on the GPU at once, two an SM: beyond,
+// the blocks that wait cost the kernel they wait for more than the launch saves
+// (every launch early: n = 5997, 37 columns 59.7 -> 62.2 ms; n = 150, one column,
+// 0.71 -> 0.65).
+static bool early_fits(int64_t blocks) { return blocks <= 2 * device_sm_count(); }
+
 constexpr int kRowSpread = 4;
 // Power of two scaled out of row k of B (see digits_kernel); every lane of a warp calls it.
 __device__ __forceinline__ bool rows_differ(const int* kexp, int K, int lane) {
@@ -157,6 +163,7 @@ __global__ void __launch_bounds__(256)
 digits_kernel(const double2* __restrict__ A, int64_t lda, int M, int ablocks, const double2* __restrict__ B,
               int64_t ldb, int N, int K, const int* __restrict__ kexp, unsigned char* __restrict__ adig,
               int* __restrict__ aexp, unsigned char* __restrict__ bdig, int* __restrict__ bexp, Slabs sl) {
+  early_start();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   // slab blockIdx.y: columns 64 y .. of A, rows 64 y .. of B, its own digits and scales
   A += (int64_t)blockIdx.y * kZK;
@@ -345,6 +352,7 @@ zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aex
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
+  early_start();
 
   if (warp == 0 && lane == 0) {
     // ---------------- producer: whichever copy has a free slot
@@ -575,6 +583,7 @@ __device__ __forceinline__ double2 lower_solve32(const double2* L, int w, double
 __global__ void __launch_bounds__(256)
 zswap_kernel(double2* __restrict__ A, int64_t lda, int n, int j0, int w, ZSlots sl, int lb, int le, int rb, int re,
              int solve, double2* __restrict__ inv, int ldinv) {
+  early_start();
   __shared__ __align__(16) double2 buf[2 * SB][SLAB];
   __shared__ __align__(16) double2 L[SB * (SB + 1)];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -633,6 +642,7 @@ zswap_kernel(double2* __restrict__ A, int64_t lda, int n, int j0, int w, ZSlots 
 __global__ void __launch_bounds__(256)
 zswap_block_kernel(double2* __restrict__ A, int64_t lda, int n, int J0, int wa, int wb, ZSlots sa, ZSlots sb,
                    int nleft, int nright, double2* __restrict__ Inv, int* __restrict__ kexp) {
+  early_start();
   // the moved rows (2 SB x 32), or the inverse's two 32 x 33 factors
   __shared__ __align__(16) unsigned char raw[2 * SB * (SB + 1) * sizeof(double2)];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -746,8 +756,8 @@ int zgemm_digits(const ZGemmPlan& p, const double2* A, int64_t lda, int M, const
   const int ab = (M + BM - 1) / BM * (BM / 32), bb = (N + BNC - 1) / BNC;
   if (ab + bb == 0) return MGT_OK;
   count_launch();
-  digits_kernel<<<ab + bb, 256, 0, s>>>(A, lda, M, ab, B, ldb, N, K, kexp, p.adig, p.aexp, p.bdig, p.bexp,
-                                      Slabs());
+  launch_early(early_fits(ab + bb), digits_kernel, ab + bb, 256, 0, s, A, lda, M, ab, B, ldb, N, K, kexp, p.adig, p.aexp, p.bdig,
+               p.bexp, Slabs());
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }
 
@@ -764,10 +774,10 @@ int zgemm_apply(const ZGemmPlan& p, int arow, int M, int bcol, int N, int K, dou
   if (total > (1 << 30)) return MGT_ERR_UNSUPPORTED;
   const int ctas = (int)std::min<int64_t>(total, max_ctas > 0 ? max_ctas : device_sm_count());
   count_launch();
-  zgemm_kernel<<<ctas, THREADS, smem_bytes(), s>>>(p.adig + (size_t)(arow / BM) * NCH * DIG * D_SLICE, p.aexp + arow,
-                                                   p.bdig + (size_t)(bcol / BNC) * NCH * B_BLOCK, p.bexp + bcol, M, N,
-                                                   (K + KCC - 1) / KCC, ct, (int)total, C, ldc, sub ? 1 : 0, rowmax,
-                                                   status, Slabs());
+  launch_early(total <= 8 * ctas, zgemm_kernel, ctas, THREADS, smem_bytes(), s,
+               p.adig + (size_t)(arow / BM) * NCH * DIG * D_SLICE, p.aexp + arow,
+               p.bdig + (size_t)(bcol / BNC) * NCH * B_BLOCK, p.bexp + bcol, M, N, (K + KCC - 1) / KCC, ct, (int)total, C,
+               ldc, sub ? 1 : 0, rowmax, status, Slabs());
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }
 
@@ -778,6 +788,7 @@ namespace zg {
 // out = E0 - sum over slabs of part
 __global__ void slab_sum_kernel(const double2* __restrict__ part, int slabs, int M, int N,
                                 const double2* __restrict__ E0, int64_t ld0, double2* __restrict__ out, int64_t ldo) {
+  early_start();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)M * N) return;
   const int64_t r = i / N, c = i - r * N;
@@ -830,11 +841,11 @@ int zgemm_wide(const double2* A, int64_t lda, int M, const double2* B, int64_t l
   if (cudaMemsetAsync(b, 0, 256, s) != cudaSuccess) return MGT_ERR_CUDA;   // status
   const int ab = (int)w.rt * (BM / 32);
   count_launch(3);
-  digits_kernel<<<dim3(ab + (unsigned)w.ct, w.slabs), 256, 0, s>>>(A, lda, M, ab, B, ldb, N, K, nullptr, adig, aexp,
+  launch_early(false, digits_kernel, dim3(ab + (unsigned)w.ct, w.slabs), 256, 0, s, A, lda, M, ab, B, ldb, N, K, nullptr, adig, aexp,
                                                                   bdig, bexp, sl);
-  zgemm_kernel<<<(int)std::min<int64_t>(total, device_sm_count()), THREADS, smem_bytes(), s>>>(
+  launch_early(false, zgemm_kernel, (int)std::min<int64_t>(total, device_sm_count()), THREADS, smem_bytes(), s,
       adig, aexp, bdig, bexp, M, N, NCH, (int)w.ct, (int)total, part, N, 0, nullptr, (int*)b, sl);
-  slab_sum_kernel<<<(unsigned)(((int64_t)M * N + 255) / 256), 256, 0, s>>>(part, w.slabs, M, N, E0, ld0, out, ldo);
+  launch_early(false, slab_sum_kernel, (unsigned)(((int64_t)M * N + 255) / 256), 256, 0, s, part, w.slabs, M, N, E0, ld0, out, ldo);
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }
 
@@ -845,7 +856,7 @@ int zswap_panel(double2* A, int64_t lda, int n, int j0, int w, const ZSlots& sl,
   const int blocks = nl + nr + (inv ? 4 : 0);
   if (blocks == 0) return MGT_OK;
   count_launch();
-  zswap_kernel<<<blocks, 256, 0, st>>>(A, lda, n, j0, w, sl, lb, le, rb, re, solve ? 1 : 0, inv, ldinv);
+  launch_early(early_fits(blocks), zswap_kernel, blocks, 256, 0, st, A, lda, n, j0, w, sl, lb, le, rb, re, solve ? 1 : 0, inv, ldinv);
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }
 
@@ -856,7 +867,7 @@ int zswap_block(double2* A, int64_t lda, int n, int J0, int wa, int wb, const ZS
   const int blocks = nleft + nright + (Inv ? 8 : 0);
   if (blocks == 0) return MGT_OK;
   count_launch();
-  zswap_block_kernel<<<blocks, 256, 0, st>>>(A, lda, n, J0, wa, wb, a, b, nleft, nright, Inv, kexp);
+  launch_early(early_fits(blocks), zswap_block_kernel, blocks, 256, 0, st, A, lda, n, J0, wa, wb, a, b, nleft, nright, Inv, kexp);
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }
 

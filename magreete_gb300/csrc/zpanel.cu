@@ -165,6 +165,7 @@ template <int ROWS, bool CLUSTER>
 __global__ void __launch_bounds__(4 * ROWS + 64, 1)
 zpanel_kernel(double2* __restrict__ A, int64_t lda, int m, int w, int j0, int rows_per_cta,
               int32_t* __restrict__ perm, ZPanelWs ws) {
+  early_start();
   constexpr int WARPS = ROWS / 8, THREADS = 4 * ROWS + 64, KR = NB / 4;
   extern __shared__ __align__(16) unsigned char zp_smem[];
   Smem<ROWS>& S = *reinterpret_cast<Smem<ROWS>*>(zp_smem);
@@ -517,13 +518,15 @@ static int launch(double2* P, int64_t lda, int m, int w, int j0, int32_t* perm, 
   cfg.blockDim = dim3(4 * ROWS + 64);
   cfg.dynamicSmemBytes = sizeof(Smem<ROWS>);
   cfg.stream = s;
-  cudaLaunchAttribute at[1];
+  cudaLaunchAttribute at[2];
   if (CLUSTER) {
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = G;
     at[0].val.clusterDim.y = 1;
     at[0].val.clusterDim.z = 1;
-    cfg.numAttrs = 1;
+    at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;   // early_start
+    at[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.numAttrs = 2;
   } else {
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;

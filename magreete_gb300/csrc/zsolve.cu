@@ -76,6 +76,7 @@ template <int CW>
 __global__ void __launch_bounds__(256)
 diag_kernel(const double2* __restrict__ Inv, int upper, double2* __restrict__ X, int64_t ldx, int rb, int ncols,
             int* __restrict__ kexp) {
+  early_start();
   __shared__ double2 xs[CW][TB];
   const int tid = threadIdx.x, row = tid >> 2, q = tid & 3, lane = tid & 31;
   const int c0 = blockIdx.x * CW, nc = min(CW, ncols - c0);
@@ -147,9 +148,9 @@ int zsolve(const double2* F, int64_t ldf, double2* X, int64_t ldx, int n, int nr
     int* ke = kexp + (size_t)step * TB;
     count_launch();
     if (nrhs <= 2 * device_sm_count())
-      diag_kernel<1><<<nrhs, 256, 0, s>>>(iv, upper, Xi, ldx, rb, nrhs, ke);
+      launch_early(true, diag_kernel<1>, nrhs, 256, 0, s, iv, upper, Xi, ldx, rb, nrhs, ke);
     else
-      diag_kernel<4><<<(nrhs + 3) / 4, 256, 0, s>>>(iv, upper, Xi, ldx, rb, nrhs, ke);
+      launch_early(false, diag_kernel<4>, (nrhs + 3) / 4, 256, 0, s, iv, upper, Xi, ldx, rb, nrhs, ke);
     const int q0 = upper ? 0 : r0 + rb, m = upper ? r0 : n - q0;
     if (m <= 0) continue;
     int e = zgemm_digits(plan, F + (int64_t)q0 * ldf + r0, ldf, m, Xi, ldx, nrhs, rb, ke, s);
