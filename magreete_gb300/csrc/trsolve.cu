@@ -23,7 +23,7 @@
 // accumulate in FP32 by weight (h h | h l + l h | l l).
 //
 // Measured, LU solve of 64 columns with the inverses made (ms): n = 2000 0.26,
-// 6000 0.90, 12000 2.14; work items of 64-row blocks claimed by persistent CTAs,
+// 6000 0.85, 12000 2.01; work items of 64-row blocks claimed by persistent CTAs,
 // products on the FP32 pipe: 0.54, 1.66, 3.93.  A step takes 11 us on the chain
 // (two products, each with its exchange of partial sums); from n = 6000 on the
 // block rows beyond take as long or longer (12000: 20 us).
@@ -789,10 +789,12 @@ static int tri_steps(const float2* F, int64_t ldf, const unsigned char* ops, con
     // step i solves block row i (from the end for U) after updating it and all that follow
     const int first = UPPER ? nb - 1 : 0, src = i == 0 ? -1 : UPPER ? nb - i : i - 1;
     const int rest = i == 0 ? 0 : nb - 1 - i;   // block rows beyond
-    // K over the CTAs of a cluster while every CTA of the launch is resident at
-    // once (two per SM); beyond, one CTA takes all of K: a quarter of the sums
-    // to exchange none, at 38 K clocks for 128 rows against 4 x 25 K
-    const bool split = (int64_t)8 * (1 + rest) * ng <= 2 * sms;
+    // K over the CTAs of a cluster while the launch is less than two rounds of
+    // what is resident at once (two CTAs an SM); beyond, one CTA takes all of K
+    // (34 K clocks for 128 rows, no sums to exchange, against 4 x 20 K).  Solves
+    // of 64 columns with the line at 1.3, 2, 2.6, 3.4 and 4.6 CTAs an SM, ms:
+    // n = 6000 0.98, 0.89, 0.86, 0.85, 0.85; 12000 2.23, 2.12, 2.06, 2.01, 2.07.
+    const bool split = (int64_t)8 * (1 + rest) * ng <= 7 * sms / 2;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(8 * (1 + (split ? rest : (2 * rest + 7) / 8)), ng);
     cfg.blockDim = dim3(kTThreads);
