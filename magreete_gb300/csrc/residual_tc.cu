@@ -593,20 +593,31 @@ __global__ void tc_reduce_kernel(const double2* __restrict__ partial, int splits
   R[(int64_t)r * ldr + c] = acc;
 }
 
-// Split of the K range: about four waves of CTAs, at least 8 chunks (4
-// readouts) per split, at most 16 splits and MAX_SPLIT_CHUNKS chunks each,
-// an even number of chunks per split (whole readouts).
+// Split of the K range, an even number of chunks each, at least 8, at most 16
+// splits and MAX_SPLIT_CHUNKS chunks: the one with the shortest estimate, in
+// chunks of 3.4 us -- rounds of CTAs (one an SM) times a CTA's chunks and 2 more
+// for its start and end, and the split sums written and read once at 6.7 TB/s.
+// Against four rounds whatever their fill, 64 columns: n = 2000 116 -> 91 us a
+// residual, 3750 237 -> 216, 6000 512 -> 470; 33 columns, 21000 5.19 -> 4.66 ms.
 static void plan_splits(int rows, int kdim, int ncols, int* splits, int* cps) {
   const int nch = (kdim + KCC - 1) / KCC;
-  const int tiles = ((rows + BM - 1) / BM) * ((ncols + BNC - 1) / BNC);
+  const int ctiles = (ncols + BNC - 1) / BNC;   // the choice depends on whole column tiles only
+  const int64_t tiles = (int64_t)((rows + BM - 1) / BM) * ctiles;
   const int sms = device_sm_count();
-  const int want = (4 * sms + tiles - 1) / tiles;
-  int sp = std::max(1, std::min(want, std::min(16, nch / 8)));
-  sp = std::max(sp, (nch + MAX_SPLIT_CHUNKS - 1) / MAX_SPLIT_CHUNKS);
-  int c = (nch + sp - 1) / sp;
-  if ((c & 1) && c < nch) ++c;
-  *cps = c;
-  *splits = (nch + c - 1) / c;
+  const int lo = (nch + MAX_SPLIT_CHUNKS - 1) / MAX_SPLIT_CHUNKS, hi = std::max(lo, std::min(16, nch / 8));
+  double best = 0.0;
+  for (int sp = lo; sp <= hi; ++sp) {
+    int c = (nch + sp - 1) / sp;
+    if ((c & 1) && c < nch) ++c;
+    const int n = (nch + c - 1) / c;
+    const double rounds = (double)((tiles * n + sms - 1) / sms);
+    const double cost = rounds * (c + 2) + (n > 1 ? 1.4e-6 * n * (double)rows * (ctiles * BNC) : 0.0);
+    if (sp == lo || cost < best) {
+      best = cost;
+      *cps = c;
+      *splits = n;
+    }
+  }
 }
 
 // workspace of one application (the digits of M are the caller's)
@@ -632,7 +643,15 @@ struct TcResWs {
     status = (int*)take(256, 256);
     colexp = (int*)take((size_t)ncols * sizeof(int), 256);
     bdig = (unsigned char*)take((size_t)ctiles * nch * B_BLOCK, 1024);
-    partial = splits > 1 ? (double2*)take((size_t)splits * rows * ncols * sizeof(double2), 256) : nullptr;
+    // room for as many columns or fewer (fewer may take more splits)
+    size_t sums = 0;
+    for (int c = BNC; c < ncols + BNC; c += BNC) {
+      int sp, per;
+      plan_splits(rows, kdim, std::min(c, ncols), &sp, &per);
+      if (sp > 1) sums = std::max(sums, (size_t)sp * rows * std::min(c, ncols));
+    }
+    char* p = take(sums * sizeof(double2), 256);
+    partial = splits > 1 ? (double2*)p : nullptr;
     total = off + 256;
   }
 };

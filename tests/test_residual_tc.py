@@ -184,3 +184,20 @@ def test_tc_residual_extreme_digits(n):
     bound = 4 * (n / 128 + 32) * 2.0 ** -48 + n * 2.0 ** -51
     assert (got.real - re).abs().max().item() <= bound
     assert (got.imag - im).abs().max().item() <= bound
+
+
+@pytest.mark.parametrize("n", [300, 2000, 2400, 6000, 12000])
+def test_workspace_serves_fewer_columns(n):
+    """A workspace for R columns holds an application to any fewer (the split of
+    K, and with it the partial sums, depends on the columns)."""
+    from magreete_gb300 import _lib as L
+    lib = L.load()
+
+    def q(fn, r):
+        nb = ctypes.c_size_t()
+        L.check(fn(n, r, ctypes.byref(nb)))
+        return nb.value
+
+    for fn in (lib.mgt_residual_workspace_bytes, lib.mgt_refine_workspace_bytes, lib.mgt_refine_scratch_bytes):
+        sizes = [q(fn, r) for r in range(1, 200)]
+        assert all(a <= b for a, b in zip(sizes, sizes[1:]))
