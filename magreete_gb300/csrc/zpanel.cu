@@ -20,11 +20,11 @@
 // chosen row and its reciprocal follow as soon as they are ready (a cluster's
 // chosen CTA sends them to the others; through global memory every CTA
 // publishes its own and the chosen one is read).
-// There is no fence, barrier or flag: every 64-bit word of a message carries an
-// 8-bit tag of the column, so a reader that sees the tag has the data.  Messages
-// alternate by column parity; the previous content of a buffer (two columns
-// back) never carries the current tag, and it is overwritten only by a CTA that
-// has every key of the column in between, when nobody reads it any more.
+// There is no fence, barrier or flag: every 64-bit word of a message carries the
+// column's tag (zpanel_msg.cuh), so a reader that sees the tag has the data.
+// Messages alternate by column parity; what a buffer held before never carries
+// the current tag, however long its CTA had no row, and it is overwritten only by
+// a CTA that has every key of the column in between, when nobody reads it any more.
 //   CLUSTER: one thread-block cluster (at most 16 CTAs), messages in
 //     distributed shared memory (tables cleared before a first cluster barrier);
 //   otherwise records in global memory, cleared when a factorisation starts.
@@ -38,6 +38,7 @@
 #include <algorithm>
 
 #include "zpanel.cuh"
+#include "zpanel_msg.cuh"
 #include "diag.cuh"
 
 namespace mgt {
@@ -46,7 +47,6 @@ namespace zp {
 constexpr int NB = kZNB;
 constexpr int LD = NB + 1;
 constexpr int kMaxCluster = 16;
-constexpr int kNoPos = 0x7fffffff;
 
 // |re|+|im| as an ordered integer: bits + 1, 0 for a NaN
 __device__ __forceinline__ unsigned long long pivot_key(double2 v) {
@@ -80,21 +80,22 @@ __device__ __forceinline__ void cluster_sync() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-// Messages of 64-bit words with the column's tag in the top byte.
-constexpr unsigned long long kData = 0x00FFFFFFFFFFFFFFull;
-__device__ __forceinline__ void encode(unsigned long long tag, double2 v, unsigned long long* w) {
-  const unsigned long long x = (unsigned long long)__double_as_longlong(v.x);
-  const unsigned long long y = (unsigned long long)__double_as_longlong(v.y);
-  w[0] = tag | (x >> 8);
-  w[1] = tag | ((x & 255ull) << 48) | (y >> 16);
-  w[2] = tag | (y & 0xFFFFull);
+// Messages of 64-bit words that carry the column's tag.
+using Word = unsigned long long;
+__device__ __forceinline__ void encode(Word tag, double2 v, Word* w) {
+  uint64_t q[3];
+  pack_number(tag, (uint64_t)__double_as_longlong(v.x), (uint64_t)__double_as_longlong(v.y), q);
+#pragma unroll
+  for (int t = 0; t < 3; ++t) w[t] = q[t];
 }
-__device__ __forceinline__ double2 decode(const unsigned long long* w) {
-  return make_double2(__longlong_as_double((long long)(((w[0] & kData) << 8) | ((w[1] >> 48) & 255ull))),
-                      __longlong_as_double((long long)(((w[1] & 0xFFFFFFFFFFFFull) << 16) | (w[2] & 0xFFFFull))));
+__device__ __forceinline__ double2 decode(const Word* w) {
+  const uint64_t q[3] = {w[0], w[1], w[2]};
+  uint64_t x, y;
+  unpack_number(q, &x, &y);
+  return make_double2(__longlong_as_double((long long)x), __longlong_as_double((long long)y));
 }
-__device__ __forceinline__ bool tagged(unsigned long long tag, const unsigned long long* w) {
-  return !(((w[0] ^ tag) | (w[1] ^ tag) | (w[2] ^ tag)) >> 56);
+__device__ __forceinline__ bool tagged(Word tag, const Word* w) {
+  return has_tag(tag, w[0]) && has_tag(tag, w[1]) && has_tag(tag, w[2]);
 }
 // Row message, laid out so that a warp reads it in few sectors: per column the
 // first two words, then the third ones, then the reciprocal's three words.
@@ -202,7 +203,7 @@ zpanel_kernel(double2* __restrict__ A, int64_t lda, int m, int w, int j0, int ro
   bool pending = false;                          // its columns beyond the next one still to be updated
   for (int c = 0; c < w; ++c) {
     const int buf = c & 1, u = c & 3, live = KR - j;
-    const unsigned long long tag = (unsigned long long)(((j0 + c) & 127) + 1) << 56;
+    const unsigned long long tag = column_tag(j0 + c);
     // ---- the warps' candidates
     int who = -1;
     if (worker) {
@@ -284,16 +285,16 @@ zpanel_kernel(double2* __restrict__ A, int64_t lda, int m, int w, int j0, int ro
       }
     } else {
       // ---- exchange warp: publish the key, gather all keys, fetch the chosen row
-      const unsigned long long k0 = tag | (ckey >> 8);
-      const unsigned long long k1 = tag | ((ckey & 255ull) << 32) | (unsigned long long)(unsigned)cpos;
+      uint64_t kw[2];
+      pack_key(tag, ckey, cpos, kw);
       if constexpr (CLUSTER) {
         if (lane < G) {
-          st_cluster2(map_rank(saddr(&S.keys[buf][bid][0]), (uint32_t)lane), k0, k1);
+          st_cluster2(map_rank(saddr(&S.keys[buf][bid][0]), (uint32_t)lane), kw[0], kw[1]);
         }
       } else if (lane == 0) {
         Mail to;
         to.g = keys_of(buf);
-        to.put2(2 * bid, k0, k1);
+        to.put2(2 * bid, kw[0], kw[1]);
       }
       unsigned seen = 0, it = 0;
       const int per = (G + 31) / 32;
@@ -316,10 +317,11 @@ zpanel_kernel(double2* __restrict__ A, int64_t lda, int m, int w, int j0, int ro
             from.g = keys_of(buf);
             from.get2(2 * q, h0, h1);
           }
-          if (((h0 ^ tag) | (h1 ^ tag)) >> 56) continue;
+          if (!has_tag(tag, h0) || !has_tag(tag, h1)) continue;
           seen |= 1u << t;
-          const unsigned long long k2 = ((h0 & kData) << 8) | ((h1 >> 32) & 255ull);
-          const int p2 = (int)(unsigned)h1;
+          uint64_t k2;
+          int p2;
+          unpack_key(h0, h1, &k2, &p2);
           if (p2 != kNoPos && (bp == kNoPos || k2 > bk || (k2 == bk && p2 < bp))) { bk = k2; bp = p2; bb = q; }
         }
         if (__all_sync(0xffffffffu, seen == want)) break;
@@ -544,7 +546,7 @@ static int launch(double2* P, int64_t lda, int m, int w, int j0, int32_t* perm, 
 int zpanel_factor(double2* P, int64_t lda, int m, int w, int j0, int32_t* perm, const ZPanelWs& ws, int rows_target,
                   int max_ctas, bool cooperative, bool allow_cluster, cudaStream_t s) {
   using namespace zp;
-  if (m <= 0 || w <= 0 || w > NB) return MGT_ERR_UNSUPPORTED;
+  if (m <= 0 || w <= 0 || w > NB || m >= kNoPos || j0 + w > kMaxColumns) return MGT_ERR_UNSUPPORTED;
   const int c64 = max_cluster<64>();
   max_cluster<128>();   // sets its kernels' attributes
   const int cap = std::max(1, std::min(max_ctas, ws.max_ctas));
