@@ -1218,8 +1218,9 @@ lu_block_right_kernel(cplx<T>* __restrict__ A, int64_t lda, int n, int J0, int w
 }
 
 // perm = identity; the factorisation epoch moves on by one; `words` 64-bit words
-// at a distance of `stride` are cleared: the panel records' flags, or the
-// messages of the complex128 panel (the short column tags of both rely on it)
+// at a distance of `stride` are cleared: the panel records' flags (complex64:
+// its short column tags rely on it), or the whole records (complex128: flags
+// and zpanel.cu's messages share them)
 __global__ void lu_start_kernel(int32_t* perm, int n, unsigned long long* epoch, unsigned char* records, int words,
                                 size_t stride) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -1967,8 +1968,9 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
   if (cudaMemsetAsync(work, 0, 32, s) != cudaSuccess) return MGT_ERR_CUDA;   // status, nslot
   const bool zpanel = sizeof(T) == 8 && NB == kZNB && opt.panel_reg == 1;
   lu_start_kernel<<<std::max((n + 255) / 256, zpanel ? 64 : 1), 256, 0, s>>>(
-      perm, n, ws.epoch, ws.records, zpanel ? (int)zpanel_words(kMaxPanelBlocks) : 2 * kMaxPanelBlocks,
+      perm, n, ws.epoch, ws.records, zpanel ? (int)(2 * kMaxPanelBlocks * kRecBytes / 8) : 2 * kMaxPanelBlocks,
       zpanel ? 8 : kRecBytes);
+  bool records_clear = zpanel;   // no panel of another kernel has written where zpanel.cu's messages lie
   count_launch();
   const int sms = std::min(num_sms(), kMaxPanelBlocks);
   const size_t sm2 = (2 * NB * kSwapCols + NB * NB) * sizeof(V);
@@ -2018,9 +2020,15 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
         const ZPanelWs zw{pw.status, pw.nslot, pw.slots, reinterpret_cast<unsigned long long*>(pw.records),
                           kMaxPanelBlocks};
         const int cap = opt.panel_max_ctas > 0 ? std::min(opt.panel_max_ctas, sms) : sms;
+        // taller panels went to the kernel below: its records are no messages
+        if (!records_clear && zpanel_fits(m, cap)) {
+          if (cudaMemsetAsync(pw.records, 0, zpanel_words(kMaxPanelBlocks) * 8, s) != cudaSuccess) return MGT_ERR_CUDA;
+          records_clear = true;
+        }
         const int e = zpanel_factor(A + (int64_t)j0 * lda + j0, lda, m, w, j0, perm, zw, kZPanelRows, cap,
                                     opt.cooperative != 0, opt.panel_cluster != 0, s);
         if (e != MGT_ERR_UNSUPPORTED) return e;
+        records_clear = false;
       }
     }
     const int G = panel_ctas(m);

@@ -17,6 +17,9 @@ struct ZPanelWs {
   int max_ctas;
 };
 
+// Whether a panel of m rows fits `max_ctas` CTAs of at most 128 rows.
+inline bool zpanel_fits(int m, int max_ctas) { return m <= 128 * (max_ctas > 1 ? max_ctas : 1); }
+
 // Factors columns [0, w) (w <= 32) of the m-row panel at P in place, with partial pivoting
 // (LAPACK's rule); MGT_ERR_UNSUPPORTED where the panel does not fit (nothing is launched).
 int zpanel_factor(double2* P, int64_t lda, int m, int w, int j0, int32_t* perm, const ZPanelWs& ws, int rows_target,

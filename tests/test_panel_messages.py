@@ -86,3 +86,44 @@ def test_panels_of_varying_grids(n):
     assert int(outs[1].perm[0]) == n - 1 and int(outs[1].perm[1]) == 0
     assert torch.equal(outs[0].perm, outs[1].perm)
     assert torch.equal(outs[0].lu, outs[1].lu)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,ctas", [(1100, 8), (2112, 8)])
+@pytest.mark.parametrize("scale", [1.0, 1e6, 1e-290])
+def test_panels_of_two_kernels(n, ctas, scale):
+    """Panels too tall for the CTAs allowed go to the shared-memory kernel, which
+    leaves raw rows where the others' messages lie.  The workspace comes
+    from a factorisation with the same sequence numbers, and its flags are not
+    taken for this one's either: the factors have the bits of the
+    shared-memory kernel's for every panel."""
+    import ctypes
+    import torch
+    from magreete_gb300 import _lib as L
+    from magreete_gb300 import engine as E
+    lib = L.load()
+    gen = torch.Generator(device="cuda").manual_seed(n)
+    mats = [scale * torch.randn(n, n, dtype=torch.complex128, device="cuda", generator=gen) for _ in range(2)]
+    nb = ctypes.c_size_t()
+    L.check(lib.mgt_lu_workspace_bytes(L.MGT_C128, n, ctypes.byref(nb)))
+    work = torch.zeros(nb.value, dtype=torch.uint8, device="cuda")
+
+    def factor(A, **options):
+        lu, perm = A.clone(), torch.empty(n, dtype=torch.int32, device="cuda")
+        opt = L.LuOptions(**options)
+        L.check(lib.mgt_lu_factor_ex(L.MGT_C128, E._ptr(lu), n, n, E._ptr(perm), E._ptr(work), nb.value,
+                                     ctypes.byref(opt), E._stream()))
+        return lu, perm
+
+    epoch = work[40:48].clone()
+    factor(mats[0], panel_max_ctas=ctas)
+    torch.cuda.synchronize()
+    work[40:48] = epoch          # the next call counts as the last one did
+    lu, perm = factor(mats[1], panel_max_ctas=ctas)
+    try:
+        lib.mgt_set_tuning(L.MGT_TUNE_PANEL_REGISTERS, 0)
+        ref = E.lu_factor(mats[1].clone())
+    finally:
+        lib.mgt_set_tuning(L.MGT_TUNE_PANEL_REGISTERS, 1)
+    assert torch.equal(perm, ref.perm)
+    assert torch.equal(lu, ref.lu)
