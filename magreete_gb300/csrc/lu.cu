@@ -1238,12 +1238,13 @@ struct TcLU {
   TcPlan plan;
   CUtensorMap cmap;   // the whole matrix being factored
 };
+constexpr int kZStats = 2 * kZK + 32;
 // complex128: operand digits of the tensor-core products, inverse of a block's diagonal
 struct ZLU {
   ZGemmPlan plan;
   double2* inv;       // 64 x 64
-  int* kexp;          // per block: 64 row exponents of A12, 64 of U12
-  size_t kexp_bytes;
+  int* stats;         // per block kZStats: largest exponent fields of 64 rows of A12, of U12, and of the inverse
+  size_t stats_bytes;
 };
 static int trailing_update(const TcLU* tc, int M, int N, int K, const double2* A, int64_t lda, const double2* B,
                            int64_t ldb, double2* C, int64_t ldc, int, int*, cudaStream_t s, int) {
@@ -2089,7 +2090,7 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
     if constexpr (sizeof(T) == 8 && NB == kZNB) {
       const PanelWs pw = panel_ws(work, set);
       zswap_panel(A, lda, n, j0, w, ZSlots{pw.slots, pw.nslot}, left_begin, left_end, right_begin, right_end,
-                  do_trsm != 0, nullptr, 0, st);
+                  do_trsm != 0, nullptr, 0, nullptr, st);
     } else {
       const int nleft = left_end > left_begin ? (left_end - left_begin + kSwapCols - 1) / kSwapCols : 0;
       const int nright = right_end > right_begin ? (right_end - right_begin + kSwapCols - 1) / kSwapCols : 0;
@@ -2156,30 +2157,34 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
     if (zlu) {
       const PanelWs p0 = panel_ws(work, 0), p1 = panel_ws(work, 1);
       const ZSlots s0{p0.slots, p0.nslot}, s1{p1.slots, p1.nslot};
-      if (cudaMemsetAsync(zlu->kexp, 0, zlu->kexp_bytes, s) != cudaSuccess) return MGT_ERR_CUDA;
+      if (cudaMemsetAsync(zlu->stats, 0, zlu->stats_bytes, s) != cudaSuccess) return MGT_ERR_CUDA;
       for (int J0 = 0; J0 < n; J0 += kZK) {
         const int W = std::min(kZK, n - J0), wa = std::min(NB, W), wb = W - wa, j1 = J0 + wa, P0 = J0 + W;
         const int right = n - P0;
         double2* inv = right > 0 ? zlu->inv : nullptr;
-        int* ke = zlu->kexp + 2 * J0;
+        int* st = zlu->stats + J0 / kZK * kZStats;   // fields of the rows of A12 and of U12, of the inverse
+        int *a12 = st, *u12 = st + kZK, *im = st + 2 * kZK;
         int e = panel_only(J0, wa, 0);
         if (e == MGT_OK && wb > 0) {
-          e = zswap_panel(A, lda, n, J0, wa, s0, 0, 0, j1, P0, true, inv, kZK, s);
+          e = zswap_panel(A, lda, n, J0, wa, s0, 0, 0, j1, P0, true, inv, kZK, im, s);
           if (e == MGT_OK) e = update(j1, j1, J0, wa, n - j1, wb, false);
           if (e == MGT_OK) e = panel_only(j1, wb, 1);
-          if (e == MGT_OK) e = zswap_panel(A, lda, n, j1, wb, s1, J0, j1, 0, 0, false, nullptr, 0, s);
+          if (e == MGT_OK) e = zswap_panel(A, lda, n, j1, wb, s1, J0, j1, 0, 0, false, nullptr, 0, nullptr, s);
         }
-        if (e == MGT_OK) e = zswap_block(A, lda, n, J0, wa, wb, s0, s1, inv, ke, s);
+        if (e == MGT_OK) e = zswap_block(A, lda, n, J0, wa, wb, s0, s1, inv, im, a12, s);
         if (e == MGT_OK && right > 0) {
+          V* A11 = A + (int64_t)J0 * lda + J0;
           V* A12 = A + (int64_t)J0 * lda + P0;
           V* A21 = A + (int64_t)P0 * lda + J0;
-          e = zgemm_digits(zlu->plan, inv, kZK, kZK, A12, lda, right, kZK, ke, s);
-          if (e == MGT_OK) e = zgemm_apply(zlu->plan, 0, kZK, 0, right, kZK, A12, lda, false, ke + kZK, ws.status, s);
-          if (e == MGT_OK) e = zgemm_digits(zlu->plan, A21, lda, right, A12, lda, right, kZK, ke + kZK, s);
+          const ZRows ra{ZRows::MAX, a12, im}, ru{ZRows::MAX, u12, nullptr};
+          e = zgemm_digits(zlu->plan, inv, kZK, kZK, A12, lda, right, kZK, ra, s);
+          if (e == MGT_OK)
+            e = zgemm_apply(zlu->plan, A11, lda, kZK, A12, lda, right, kZK, A12, lda, ZOut::SOLVE, u12, ws.status, s);
+          if (e == MGT_OK) e = zgemm_digits(zlu->plan, A21, lda, right, A12, lda, right, kZK, ru, s);
           dom_begin(s);
           if (e == MGT_OK)
-            e = zgemm_apply(zlu->plan, 0, right, 0, right, kZK, A + (int64_t)P0 * lda + P0, lda, true, nullptr,
-                            ws.status, s);
+            e = zgemm_apply(zlu->plan, A21, lda, right, A12, lda, right, kZK, A + (int64_t)P0 * lda + P0, lda,
+                            ZOut::SUB, nullptr, ws.status, s);
           dom_end(s, 8.0 * right * (double)right * kZK,
                   sizeof(V) * (2.0 * right * (double)right + 2.0 * (double)right * kZK));
         }
@@ -2661,10 +2666,10 @@ static size_t tc_region_offset() { return (LuWsLayout().total + 1023) & ~size_t(
 // no-allocation entry point has no room for the digits, and up to this order
 // both entry points give the same bits.
 constexpr int64_t kZMinN = 768;
-// complex128 tensor-core region: the inverse of a block's diagonal, row exponents, the digits
-static size_t z_kexp_bytes(int64_t n) { return (size_t)((n + kZK - 1) / kZK) * 2 * kZK * sizeof(int); }
+// complex128 tensor-core region: the inverse of a block's diagonal, sizes of rows, the digits
+static size_t z_stats_bytes(int64_t n) { return (size_t)((n + kZK - 1) / kZK) * kZStats * sizeof(int); }
 static size_t z_region_bytes(int64_t n) {
-  return kZK * kZK * sizeof(double2) + z_kexp_bytes(n) + zgemm_bytes(n, n);
+  return kZK * kZK * sizeof(double2) + z_stats_bytes(n) + zgemm_bytes(n, n);
 }
 
 extern "C" int mgt_lu_workspace_bytes(int dtype, int64_t n, size_t* bytes) {
@@ -2688,9 +2693,9 @@ extern "C" int mgt_lu_factor_ex(int dtype, void* A, int64_t n, int64_t lda, int3
     if (n >= kZMinN && work_bytes >= tc_region_offset() + z_region_bytes(n)) {
       ZLU z;
       z.inv = (double2*)((char*)work + tc_region_offset());
-      z.kexp = (int*)(z.inv + kZK * kZK);
-      z.kexp_bytes = z_kexp_bytes(n);
-      z.plan.init((char*)z.kexp + z.kexp_bytes, n, n);
+      z.stats = (int*)(z.inv + kZK * kZK);
+      z.stats_bytes = z_stats_bytes(n);
+      z.plan.init((char*)z.stats + z.stats_bytes, n, n);
       return lu_factor_impl<double, 32>((double2*)A, (int)n, lda, perm, work, s, opt, nullptr, &z);
     }
     return lu_factor_impl<double, 32>((double2*)A, (int)n, lda, perm, work, s, opt);

@@ -58,6 +58,7 @@ constexpr int THREADS = (EPI0 + NEPI + NCONV) * 32;
 constexpr int EPI_COLS = BN / (NEPI / 4);
 constexpr long long BIAS = 0x0080808080808080LL;
 constexpr int kNonFinite = 0x40000000;
+constexpr int kPlainExp = 0x50000000;   // instead of row exponents: the product goes to the FP64 pipe
 constexpr int FIX = 54;
 static_assert(TMEM_COLS == 512, "all of TMEM");
 
@@ -86,22 +87,54 @@ __device__ __forceinline__ int expo(double v, int off) {
 // 0.71 -> 0.65).
 static bool early_fits(int64_t blocks) { return blocks <= 2 * device_sm_count(); }
 
-constexpr int kRowSpread = 4;
-// Power of two scaled out of row k of B (see digits_kernel); every lane of a warp calls it.
-__device__ __forceinline__ bool rows_differ(const int* kexp, int K, int lane) {
-  int lo = 1 << 20, hi = -1;
-  for (int k = lane; k < K; k += 32) {
-    const int e = kexp[k];
-    if (e > 0 && e < 2047) {
-      lo = min(lo, e);
-      hi = max(hi, e);
-    }
+// What to do with B's rows (ZRows); every lane of a warp calls it, every warp gets the same.
+enum RowMode { kAsIs = 0, kShift = 1, kFp64 = 2 };
+constexpr int kRowSpread = 4, kHalfSpread = 12, kShapeSpread = 6, kInvLimit = 1023 + 4;
+__device__ __forceinline__ int row_mean(int4 s) {
+  const int count = s.w + (int)((unsigned)s.z >> 31);   // a negative sum has borrowed from it
+  return count ? 1023 + __float2int_rn(__fdividef((float)s.z, (float)count)) : 0;
+}
+// sh: the powers of two moved from rows lane and lane + 32 of B to A's columns.
+template <int KIND>
+__device__ __forceinline__ int row_mode(const ZRows& rows, int K, int lane, int (&sh)[2]) {
+  sh[0] = sh[1] = 0;
+  if (KIND == ZRows::NONE) return kAsIs;
+  int4 st[2];   // every load on its way at once
+  int inv = 0;
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int k = min(lane + 32 * i, K - 1);
+    if (KIND == ZRows::MEAN) st[i] = __ldg(reinterpret_cast<const int4*>(rows.stats) + k);
+    else st[i].x = __ldg(rows.stats + k);
+  }
+  if (KIND == ZRows::MAX && rows.inv) inv = __ldg(rows.inv);
+  int lo = 1 << 20, hi = -1, slo = 1 << 20, shi = -1;   // of the sizes, and of largest less mean
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    if (st[i].x <= 0) continue;   // zero (or not finite)
+    const int e = KIND == ZRows::MEAN ? row_mean(st[i]) : st[i].x;
+    lo = min(lo, e);
+    hi = max(hi, e);
+    slo = min(slo, st[i].x - e);
+    shi = max(shi, st[i].x - e);
   }
   lo = __reduce_min_sync(0xffffffffu, lo);
   hi = __reduce_max_sync(0xffffffffu, hi);
-  return hi - lo > kRowSpread;
+  (void)inv;
+  if (hi - lo <= kRowSpread) return kAsIs;
+  if (KIND == ZRows::MAX) {
+    if (hi - lo > kHalfSpread) return kFp64;
+  } else {
+    slo = __reduce_min_sync(0xffffffffu, slo);
+    shi = __reduce_max_sync(0xffffffffu, shi);
+    if (shi - slo > kShapeSpread) return kFp64;
+  }
+#pragma unroll
+  for (int i = 0; i < 2; ++i)
+    if (st[i].x > 0 && lane + 32 * i < K)
+      sh[i] = KIND == ZRows::MEAN ? row_mean(st[i]) - 1023 : (st[i].x - 1023) >> 1;
+  return kShift;
 }
-__device__ __forceinline__ int row_scale(int e) { return (e <= 0 || e >= 2047) ? 0 : e - 1023; }
 
 // Larger exponent field of both parts; 0 for zeros, infinities and NaN.
 __device__ __forceinline__ int field(double2 v) {
@@ -154,14 +187,12 @@ struct Slabs {
 // of A each, the others 32 columns of B.  A: byte slices (row tile, chunk,
 // digit) at half the width of the swizzled FP16 operand; B: the swizzled FP16
 // operand itself (block (column tile, chunk): rows s 64 + 2 j, + 1).  Zeros
-// beyond the operand.  K <= 64.  kexp (or null): the largest exponent field of
-// row k of B's whole row (0: zero row).  Where the rows' sizes differ by more
-// than 2^4, column k of A is scaled up and row k of B down by that power of
-// two, so that rows of B of very different size (a badly row-scaled matrix)
-// do not share one column scale; a well-scaled operand is left as it is.
+// beyond the operand.  K <= 64.  br: powers of two moved from B's rows to A's
+// columns (ZRows; none where the product goes to the FP64 pipe).
+template <int KIND>
 __global__ void __launch_bounds__(256)
 digits_kernel(const double2* __restrict__ A, int64_t lda, int M, int ablocks, const double2* __restrict__ B,
-              int64_t ldb, int N, int K, const int* __restrict__ kexp, unsigned char* __restrict__ adig,
+              int64_t ldb, int N, int K, ZRows br, unsigned char* __restrict__ adig,
               int* __restrict__ aexp, unsigned char* __restrict__ bdig, int* __restrict__ bexp, Slabs sl) {
   early_start();
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -173,26 +204,27 @@ digits_kernel(const double2* __restrict__ A, int64_t lda, int M, int ablocks, co
   bdig += blockIdx.y * sl.bdig;
   bexp += blockIdx.y * sl.bexp;
   K = min(kZK, K - (int)blockIdx.y * kZK);
-  const bool rows = kexp && rows_differ(kexp, K, lane);
+  int sh[NCH];
+  // (kFp64: the row exponents say so, and nothing made of the digits is used)
+  const int mode = row_mode<KIND>(br, K, lane, sh);
   if ((int)blockIdx.x < ablocks) {
     for (int q = 0; q < 4; ++q) {
       const int row = blockIdx.x * 32 + warp * 4 + q;
       double2 v[NCH];
-      int off[NCH], em = kZeroExp;
+      int em = kZeroExp;
 #pragma unroll
       for (int c = 0; c < NCH; ++c) {
         const int k = c * KCC + lane;
-        off[c] = (rows && k < K) ? row_scale(kexp[k]) : 0;
         v[c] = (row < M && k < K) ? A[(int64_t)row * lda + k] : make_double2(0.0, 0.0);
-        em = max(em, max(expo(v[c].x, off[c]), expo(v[c].y, off[c])));
+        em = max(em, max(expo(v[c].x, sh[c]), expo(v[c].y, sh[c])));
       }
       em = __reduce_max_sync(0xffffffffu, em);
-      if (lane == 0 && row < M) aexp[row] = em == kBadExp ? kNonFinite : em - 1022;
+      if (lane == 0 && row < M) aexp[row] = mode == kFp64 ? kPlainExp : em == kBadExp ? kNonFinite : em - 1022;
       const int rt = row / BM, rho = row % BM;
       const uint32_t at = (uint32_t)rho * 64u + ((uint32_t)((lane >> 2) ^ (rho & 7)) << 3) + (uint32_t)(lane & 3) * 2u;
 #pragma unroll
       for (int c = 0; c < NCH; ++c) {
-        const long long yr = fixed54(v[c].x, off[c], em) + BIAS, yi = fixed54(v[c].y, off[c], em) + BIAS;
+        const long long yr = fixed54(v[c].x, sh[c], em) + BIAS, yi = fixed54(v[c].y, sh[c], em) + BIAS;
         unsigned char* blk = adig + ((size_t)rt * NCH + c) * DIG * D_SLICE + at;
 #pragma unroll
         for (int s = 0; s < DIG; ++s) {
@@ -211,7 +243,7 @@ digits_kernel(const double2* __restrict__ A, int64_t lda, int M, int ablocks, co
 #pragma unroll
   for (int i = 0; i < kZK / 8; ++i) {
     const int k = warp * (kZK / 8) + i;
-    off[i] = (rows && k < K) ? -row_scale(kexp[k]) : 0;
+    off[i] = KIND == ZRows::NONE ? 0 : -__shfl_sync(0xffffffffu, warp < 4 ? sh[0] : sh[1], k & 31);
     v[i] = (k < K && j < N) ? B[(int64_t)k * ldb + j] : make_double2(0.0, 0.0);
     em = max(em, max(expo(v[i].x, off[i]), expo(v[i].y, off[i])));
   }
@@ -304,11 +336,101 @@ __device__ __forceinline__ void issue_digit(uint32_t tmem, uint64_t ad, uint64_t
   }
 }
 
+// The same on the FP64 pipe (600 K clocks a tile of 128 x 32), by the whole CTA:
+// thread = (column, every 16th row), K staged 16 at a time.  Calls, so that the
+// kernel's registers are those of the way above.
+struct Plain {
+  const double2 *A, *B;
+  int64_t lda, ldb;
+  int K;
+  ZOut out;
+};
+__device__ __noinline__ void plain_tiles(const Plain& p, unsigned char* smem, int M, int N, int ctiles,
+                                         int total_tiles, double2* C, int64_t ldc, int* rowmax) {
+  double2 (*As)[17] = reinterpret_cast<double2 (*)[17]>(smem);                                // [BM][16]
+  double2 (*Bs)[BNC] = reinterpret_cast<double2 (*)[BNC]>(smem + BM * 17 * sizeof(double2));  // [16][BNC]
+  const int tid = threadIdx.x, tx = tid & 31, ty = tid >> 5;
+  for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
+    const int row0 = (t / ctiles) * BM, col0 = (t % ctiles) * BNC;
+    double2 acc[BM / 16];
+#pragma unroll
+    for (int i = 0; i < BM / 16; ++i) acc[i] = make_double2(0.0, 0.0);
+    for (int k0 = 0; k0 < p.K; k0 += 16) {
+      for (int i = tid; i < BM * 16; i += THREADS) {
+        const int r = i >> 4, k = k0 + (i & 15);
+        As[r][i & 15] = row0 + r < M && k < p.K ? p.A[(int64_t)(row0 + r) * p.lda + k] : make_double2(0.0, 0.0);
+      }
+      Bs[ty][tx] = k0 + ty < p.K && col0 + tx < N ? p.B[(int64_t)(k0 + ty) * p.ldb + col0 + tx] : make_double2(0.0, 0.0);
+      __syncthreads();
+#pragma unroll 4
+      for (int k = 0; k < 16; ++k) {
+        const double2 b = Bs[k][tx];
+#pragma unroll
+        for (int i = 0; i < BM / 16; ++i) cfma(acc[i], As[ty + 16 * i][k], b);
+      }
+      __syncthreads();
+    }
+#pragma unroll
+    for (int i = 0; i < BM / 16; ++i) {
+      const int row = row0 + ty + 16 * i;
+      if (row < M && col0 + tx < N) {
+        double2* c = C + (int64_t)row * ldc + col0 + tx;
+        const double2 v = p.out == ZOut::SUB ? csub(*c, acc[i]) : acc[i];
+        *c = v;
+        if (rowmax) atomicMax(rowmax + row, field(v));
+      }
+    }
+  }
+}
+// C = L^-1 C by substitution, 64 rows: two columns per warp, lane = rows lane and lane + 32
+__device__ __noinline__ void plain_solve(const Plain& p, unsigned char* smem, int N, int total_tiles, double2* C,
+                                         int64_t ldc, int* rowmax) {
+  double2 (*L)[kZK + 1] = reinterpret_cast<double2 (*)[kZK + 1]>(smem);
+  double2 (*X)[BNC + 1] = reinterpret_cast<double2 (*)[BNC + 1]>(smem + kZK * (kZK + 1) * sizeof(double2));
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  for (int i = tid; i < kZK * kZK; i += THREADS) {
+    const int r = i / kZK, k = i % kZK;
+    L[r][k] = k < r ? p.A[(int64_t)r * p.lda + k] : make_double2(0.0, 0.0);
+  }
+  for (int t = blockIdx.x; t < total_tiles; t += gridDim.x) {
+    const int col0 = t * BNC;
+    for (int i = tid; i < kZK * BNC; i += THREADS) {
+      const int r = i / BNC, c = i % BNC;
+      X[r][c] = col0 + c < N ? C[(int64_t)r * ldc + col0 + c] : make_double2(0.0, 0.0);
+    }
+    __syncthreads();
+    for (int c = warp; c < BNC; c += THREADS / 32) {
+      double2 x0 = X[lane][c], x1 = X[lane + 32][c];
+      for (int k = 0; k < kZK - 1; ++k) {
+        const double2 s = k < 32 ? x0 : x1;
+        double2 xk;
+        xk.x = __shfl_sync(0xffffffffu, s.x, k & 31);
+        xk.y = __shfl_sync(0xffffffffu, s.y, k & 31);
+        if (k < 31 && lane > k) cfms(x0, L[lane][k], xk);
+        if (lane + 32 > k) cfms(x1, L[lane + 32][k], xk);
+      }
+      X[lane][c] = x0;
+      X[lane + 32][c] = x1;
+    }
+    __syncthreads();
+    for (int i = tid; i < kZK * BNC; i += THREADS) {
+      const int r = i / BNC, c = i % BNC;   // a warp holds one row
+      const bool in = col0 + c < N;
+      if (in) C[(int64_t)r * ldc + col0 + c] = X[r][c];
+      const int em = __reduce_max_sync(0xffffffffu, in ? field(X[r][c]) : 0);
+      if (rowmax && c == 0 && em > 0) atomicMax(rowmax + r, em);
+    }
+    __syncthreads();
+  }
+}
+
 __global__ void __launch_bounds__(THREADS, 1)
 zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aexp,
              const unsigned char* __restrict__ bdig, const int* __restrict__ bexp, int M, int N, int nch, int ctiles,
-             int total_tiles, double2* C, int64_t ldc, int sub, int* __restrict__ rowmax, int* status, Slabs sl) {
+             int total_tiles, double2* C, int64_t ldc, Plain p64, int* __restrict__ rowmax, int* status,
+             Slabs sl) {
   using namespace tc;
+  const bool sub = p64.out == ZOut::SUB;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   unsigned char* base = (unsigned char*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   unsigned char* aring = base;
@@ -326,6 +448,7 @@ zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aex
   uint64_t* done = tempty + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
   volatile int* abort = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  int* fp64 = reinterpret_cast<int*>(tmem_slot + 2);   // the digits' kernel marked the product
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int first = blockIdx.x, stride = gridDim.x;
@@ -381,6 +504,7 @@ zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aex
       if (progress) idle = 0;
       else if (++idle >= kProducerLimit) { *abort = 1; break; }
     }
+    *fp64 = p64.A && *aexp == kPlainExp;   // (read here, where nothing waits for it)
     // copies in flight land before the CTA may exit
     for (int j = max(0, ib - 2); j < ib; ++j) mbar_wait_plain(&full_b[j & 1], (j >> 1) & 1);
     for (int j = max(0, q - DSLOTS); j < q; ++j) mbar_wait_plain(&full_d[j % DSLOTS], (j / DSLOTS) & 1);
@@ -422,7 +546,7 @@ zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aex
       const int tt = first + lt * stride, slab = tt / sl.tiles, t = tt - slab * sl.tiles;
       const int row = (t / ctiles) * BM + r, col0 = (t % ctiles) * BNC + part * (EPI_COLS / 2);
       double2* crow = C + slab * sl.c + (int64_t)row * ldc + col0;
-      const int ncol = row < M ? min(EPI_COLS / 2, N - col0) : 0;
+      int ncol = row < M ? min(EPI_COLS / 2, N - col0) : 0;
       if (sub && ncol > 0) {
         asm volatile("prefetch.global.L2 [%0];" ::"l"(crow));
         asm volatile("prefetch.global.L2 [%0];" ::"l"(crow + (ncol - 1)));
@@ -466,6 +590,7 @@ zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aex
       int em = 0;
       const int ebmax = __reduce_max_sync(0xffffffffu, lane < NC ? ebl : INT_MIN);
       const int ebmin = __reduce_min_sync(0xffffffffu, lane < NC ? ebl : INT_MAX);
+      if (ea == kPlainExp) ncol = 0;   // C stays as it is
       const bool plain = ncol == NC && ea != kNonFinite && ebmax < 1 << 20 && abs(ea + ebmax - FIX) <= 900 &&
                          abs(ea + ebmin - FIX) <= 900;
       if (__all_sync(0xffffffffu, plain)) {
@@ -555,6 +680,11 @@ zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aex
   tc_fence_before();
   __syncthreads();
   if (threadIdx.x == 0 && *abort) atomicExch(status, MGT_ERR_TIMEOUT);
+  if (*fp64 && !*abort) {
+    // every copy has landed, every product is done (the epilogue has waited for the last tile's)
+    if (p64.out == ZOut::SOLVE) plain_solve(p64, base, N, total_tiles, C, ldc, rowmax);
+    else plain_tiles(p64, base, M, N, ctiles, total_tiles, C, ldc, rowmax);
+  }
   if (warp == 0) {
     if (lane == 0) mbar_wait_plain(done, 0);
     __syncwarp();
@@ -582,7 +712,7 @@ __device__ __forceinline__ double2 lower_solve32(const double2* L, int w, double
 // Blocks: 8-column slabs of [lb, le), then of [rb, re), then (inv) four blocks of L11^-1's columns.
 __global__ void __launch_bounds__(256)
 zswap_kernel(double2* __restrict__ A, int64_t lda, int n, int j0, int w, ZSlots sl, int lb, int le, int rb, int re,
-             int solve, double2* __restrict__ inv, int ldinv) {
+             int solve, double2* __restrict__ inv, int ldinv, int* __restrict__ invmax) {
   early_start();
   __shared__ __align__(16) double2 buf[2 * SB][SLAB];
   __shared__ __align__(16) double2 L[SB * (SB + 1)];
@@ -603,6 +733,8 @@ zswap_kernel(double2* __restrict__ A, int64_t lda, int n, int j0, int w, ZSlots 
     const int col = (b - nleft - nright) * 8 + warp;
     const double2 x = lower_solve32(L, w, make_double2(lane == col ? 1.0 : 0.0, 0.0), lane);
     inv[(int64_t)lane * ldinv + col] = x;
+    const int em = __reduce_max_sync(0xffffffffu, field(x));
+    if (lane == 0) atomicMax(invmax, em);
     return;
   }
   const int c0 = right ? rb + (b - nleft) * SLAB : lb + b * SLAB;
@@ -641,7 +773,7 @@ zswap_kernel(double2* __restrict__ A, int64_t lda, int n, int j0, int w, ZSlots 
 // rows right of it.
 __global__ void __launch_bounds__(256)
 zswap_block_kernel(double2* __restrict__ A, int64_t lda, int n, int J0, int wa, int wb, ZSlots sa, ZSlots sb,
-                   int nleft, int nright, double2* __restrict__ Inv, int* __restrict__ kexp) {
+                   int nleft, int nright, double2* __restrict__ Inv, int* __restrict__ invmax, int* __restrict__ kexp) {
   early_start();
   // the moved rows (2 SB x 32), or the inverse's two 32 x 33 factors
   __shared__ __align__(16) unsigned char raw[2 * SB * (SB + 1) * sizeof(double2)];
@@ -678,6 +810,8 @@ zswap_block_kernel(double2* __restrict__ A, int64_t lda, int n, int J0, int wa, 
     x = lower_solve32(Lb, wb, x, lane);
     Inv[(int64_t)(SB + lane) * kZK + col] = x;
     if (col >= SB) Inv[(int64_t)lane * kZK + col] = make_double2(0.0, 0.0);
+    const int em = __reduce_max_sync(0xffffffffu, field(x));
+    if (lane == 0) atomicMax(invmax, em);
     return;
   }
   double2* buf = reinterpret_cast<double2*>(raw);   // [2 SB][32]
@@ -747,7 +881,7 @@ void ZGemmPlan::init(void* work, int64_t r, int64_t c) {
 }
 
 int zgemm_digits(const ZGemmPlan& p, const double2* A, int64_t lda, int M, const double2* B, int64_t ldb, int N, int K,
-                 const int* kexp, cudaStream_t s) {
+                 const ZRows& rows, cudaStream_t s) {
   using namespace zg;
   if (!A) M = 0;
   if (!B) N = 0;
@@ -756,28 +890,28 @@ int zgemm_digits(const ZGemmPlan& p, const double2* A, int64_t lda, int M, const
   const int ab = (M + BM - 1) / BM * (BM / 32), bb = (N + BNC - 1) / BNC;
   if (ab + bb == 0) return MGT_OK;
   count_launch();
-  launch_early(early_fits(ab + bb), digits_kernel, ab + bb, 256, 0, s, A, lda, M, ab, B, ldb, N, K, kexp, p.adig, p.aexp, p.bdig,
-               p.bexp, Slabs());
+  launch_early(early_fits(ab + bb),
+               rows.kind == ZRows::MEAN  ? digits_kernel<ZRows::MEAN>
+               : rows.kind == ZRows::MAX ? digits_kernel<ZRows::MAX>
+                                         : digits_kernel<ZRows::NONE>,
+               ab + bb, 256, 0, s, A, lda, M, ab, B, ldb, N, K, rows, p.adig, p.aexp,
+               p.bdig, p.bexp, Slabs());
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }
 
-int zgemm_apply(const ZGemmPlan& p, int arow, int M, int bcol, int N, int K, double2* C, int64_t ldc, bool sub,
-                int* rowmax, int* status, cudaStream_t s, int max_ctas) {
+int zgemm_apply(const ZGemmPlan& p, const double2* A, int64_t lda, int M, const double2* B, int64_t ldb, int N, int K,
+                double2* C, int64_t ldc, ZOut out, int* rowmax, int* status, cudaStream_t s) {
   using namespace zg;
   if (M <= 0 || N <= 0) return MGT_OK;
-  if (K <= 0 || K > kZK || arow % BM || bcol % BNC || arow < 0 || bcol < 0 || (int64_t)arow + M > p.rows ||
-      (int64_t)bcol + N > p.cols)
-    return MGT_ERR_ARG;
+  if (K <= 0 || K > kZK || M > p.rows || N > p.cols || (out == ZOut::SOLVE && (M != kZK || K != kZK))) return MGT_ERR_ARG;
   set_attributes();
   const int rt = (M + BM - 1) / BM, ct = (N + BNC - 1) / BNC;
   const int64_t total = (int64_t)rt * ct;
   if (total > (1 << 30)) return MGT_ERR_UNSUPPORTED;
-  const int ctas = (int)std::min<int64_t>(total, max_ctas > 0 ? max_ctas : device_sm_count());
+  const int ctas = (int)std::min<int64_t>(total, device_sm_count());
   count_launch();
-  launch_early(total <= 8 * ctas, zgemm_kernel, ctas, THREADS, smem_bytes(), s,
-               p.adig + (size_t)(arow / BM) * NCH * DIG * D_SLICE, p.aexp + arow,
-               p.bdig + (size_t)(bcol / BNC) * NCH * B_BLOCK, p.bexp + bcol, M, N, (K + KCC - 1) / KCC, ct, (int)total, C,
-               ldc, sub ? 1 : 0, rowmax, status, Slabs());
+  launch_early(total <= 8 * ctas, zgemm_kernel, ctas, THREADS, smem_bytes(), s, p.adig, p.aexp, p.bdig, p.bexp, M, N,
+               (K + KCC - 1) / KCC, ct, (int)total, C, ldc, Plain{A, B, lda, ldb, K, out}, rowmax, status, Slabs());
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }
 
@@ -841,33 +975,34 @@ int zgemm_wide(const double2* A, int64_t lda, int M, const double2* B, int64_t l
   if (cudaMemsetAsync(b, 0, 256, s) != cudaSuccess) return MGT_ERR_CUDA;   // status
   const int ab = (int)w.rt * (BM / 32);
   count_launch(3);
-  launch_early(false, digits_kernel, dim3(ab + (unsigned)w.ct, w.slabs), 256, 0, s, A, lda, M, ab, B, ldb, N, K, nullptr, adig, aexp,
+  launch_early(false, digits_kernel<ZRows::NONE>, dim3(ab + (unsigned)w.ct, w.slabs), 256, 0, s, A, lda, M, ab, B, ldb, N, K, ZRows(), adig, aexp,
                                                                   bdig, bexp, sl);
   launch_early(false, zgemm_kernel, (int)std::min<int64_t>(total, device_sm_count()), THREADS, smem_bytes(), s,
-      adig, aexp, bdig, bexp, M, N, NCH, (int)w.ct, (int)total, part, N, 0, nullptr, (int*)b, sl);
+      adig, aexp, bdig, bexp, M, N, NCH, (int)w.ct, (int)total, part, N,
+      Plain{nullptr, nullptr, 0, 0, 0, ZOut::SET}, nullptr, (int*)b, sl);
   launch_early(false, slab_sum_kernel, (unsigned)(((int64_t)M * N + 255) / 256), 256, 0, s, part, w.slabs, M, N, E0, ld0, out, ldo);
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }
 
 int zswap_panel(double2* A, int64_t lda, int n, int j0, int w, const ZSlots& sl, int lb, int le, int rb, int re,
-                bool solve, double2* inv, int ldinv, cudaStream_t st) {
+                bool solve, double2* inv, int ldinv, int* invmax, cudaStream_t st) {
   using namespace zg;
   const int nl = le > lb ? (le - lb + SLAB - 1) / SLAB : 0, nr = re > rb ? (re - rb + SLAB - 1) / SLAB : 0;
   const int blocks = nl + nr + (inv ? 4 : 0);
   if (blocks == 0) return MGT_OK;
   count_launch();
-  launch_early(early_fits(blocks), zswap_kernel, blocks, 256, 0, st, A, lda, n, j0, w, sl, lb, le, rb, re, solve ? 1 : 0, inv, ldinv);
+  launch_early(early_fits(blocks), zswap_kernel, blocks, 256, 0, st, A, lda, n, j0, w, sl, lb, le, rb, re, solve ? 1 : 0, inv, ldinv, invmax);
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }
 
 int zswap_block(double2* A, int64_t lda, int n, int J0, int wa, int wb, const ZSlots& a, const ZSlots& b,
-                double2* Inv, int* kexp, cudaStream_t st) {
+                double2* Inv, int* invmax, int* kexp, cudaStream_t st) {
   using namespace zg;
   const int nleft = (J0 + 31) / 32, nright = (n - J0 - wa - wb + 31) / 32;
   const int blocks = nleft + nright + (Inv ? 8 : 0);
   if (blocks == 0) return MGT_OK;
   count_launch();
-  launch_early(early_fits(blocks), zswap_block_kernel, blocks, 256, 0, st, A, lda, n, J0, wa, wb, a, b, nleft, nright, Inv, kexp);
+  launch_early(early_fits(blocks), zswap_block_kernel, blocks, 256, 0, st, A, lda, n, J0, wa, wb, a, b, nleft, nright, Inv, invmax, kexp);
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }
 

@@ -4,8 +4,8 @@
 // Per block row i: X_i = Inv_i X_i (the block's inverted diagonal, FP64), then
 // every remaining row takes X_r -= F_(r, i) X_i as one tensor-core product of
 // FP64 accuracy (zgemm_tc.cu).  Three launches per block row: the diagonal
-// product (which also records the size of each of its rows, the scaling of the
-// product's K), the digits of the factor's block column and of X_i, and the
+// product (which also records the sizes of its rows, for the scaling of the
+// product's K: ZRows), the digits of the factor's block column and of X_i, and the
 // product.  The chain of block rows is what bounds a solve of few columns:
 // about 23 us per block row, where block-to-block flags with FP64 products of
 // 64 x 64 blocks (19 clocks per FP64 warp instruction and SM) took 130 us.
@@ -71,14 +71,15 @@ inverse_kernel(const double2* __restrict__ F, int64_t ldf, int n, double2* __res
 }
 
 // X_i = Inv X_i on CW columns per CTA; thread = (row, a quarter of K), its part
-// of Inv's row in registers.  kexp[row]: largest exponent field of the row.
+// of Inv's row in registers.  stats: 16 bytes a row, as ZRows::MEAN reads them
+// (nonzero finite entries).
 template <int CW>
 __global__ void __launch_bounds__(256)
 diag_kernel(const double2* __restrict__ Inv, int upper, double2* __restrict__ X, int64_t ldx, int rb, int ncols,
-            int* __restrict__ kexp) {
+            int* __restrict__ stats) {
   early_start();
   __shared__ double2 xs[CW][TB];
-  const int tid = threadIdx.x, row = tid >> 2, q = tid & 3, lane = tid & 31;
+  const int tid = threadIdx.x, row = tid >> 2, q = tid & 3;
   const int c0 = blockIdx.x * CW, nc = min(CW, ncols - c0);
   for (int e = tid; e < CW * TB; e += 256) {
     const int r = e / CW, c = e % CW;
@@ -91,7 +92,7 @@ diag_kernel(const double2* __restrict__ Inv, int upper, double2* __restrict__ X,
   // only the triangle's part of K, by the warp's eight rows
   const int wr0 = (tid >> 5) * 8;
   const int tb = upper ? wr0 / 4 : 0, te = upper ? TB / 4 : wr0 / 4 + 2;
-  int em = 0;
+  int em = 0, sum = 0, count = 0;
   for (int c = 0; c < nc; ++c) {
     double2 acc = make_double2(0.0, 0.0);
 #pragma unroll
@@ -104,18 +105,25 @@ diag_kernel(const double2* __restrict__ Inv, int upper, double2* __restrict__ X,
     }
     if (q == 0 && row < rb) {
       X[(int64_t)row * ldx + c0 + c] = acc;
-      em = max(em, max((__double2hiint(acc.x) >> 20) & 0x7ff, (__double2hiint(acc.y) >> 20) & 0x7ff));
+      const int ex = (__double2hiint(acc.x) >> 20) & 0x7ff, ey = (__double2hiint(acc.y) >> 20) & 0x7ff;
+      const int f = max(ex == 2047 ? 0 : ex, ey == 2047 ? 0 : ey);
+      em = max(em, f);
+      sum += f ? f - 1023 : 0;
+      count += f ? 1 : 0;
     }
   }
-  (void)lane;
-  if (q == 0 && row < rb && em > 0) atomicMax(kexp + row, em);
+  if (q == 0 && row < rb && count > 0) {
+    atomicMax(stats + 4 * row, em);
+    atomicAdd(reinterpret_cast<unsigned long long*>(stats + 4 * row + 2),
+              (unsigned long long)(((long long)count << 32) + sum));
+  }
 }
 
 struct Ws {
-  size_t status = 0, kexp = 256, inv, plan, total;
+  size_t status = 0, stats = 256, inv, plan, total;   // stats: 4 TB ints per block row and triangle
   Ws(int64_t n, int64_t nrhs) {
     const int64_t nb = (n + TB - 1) / TB;
-    inv = (kexp + (size_t)(2 * nb * TB) * sizeof(int) + 255) & ~size_t(255);
+    inv = (stats + (size_t)(2 * nb * 4 * TB) * sizeof(int) + 255) & ~size_t(255);
     plan = inv + (size_t)(2 * nb) * TB * TB * sizeof(double2);
     total = plan + zgemm_bytes(n, nrhs);
   }
@@ -133,11 +141,11 @@ int zsolve(const double2* F, int64_t ldf, double2* X, int64_t ldx, int n, int nr
   const Ws L(n, nrhs);
   const int nb = (n + TB - 1) / TB;
   int* status = (int*)((char*)work + L.status);
-  int* kexp = (int*)((char*)work + L.kexp);
+  int* stats = (int*)((char*)work + L.stats);
   double2* inv = (double2*)((char*)work + L.inv);
   ZGemmPlan plan;
   plan.init((char*)work + L.plan, n, nrhs);
-  if (cudaMemsetAsync(work, 0, L.inv, s) != cudaSuccess) return MGT_ERR_CUDA;   // status, row exponents
+  if (cudaMemsetAsync(work, 0, L.inv, s) != cudaSuccess) return MGT_ERR_CUDA;   // status, sizes of rows
   count_launch();
   inverse_kernel<<<dim3(nb, 8, 2), 256, smem, s>>>(F, ldf, n, inv);
   for (int step = 0; step < 2 * nb; ++step) {
@@ -145,16 +153,19 @@ int zsolve(const double2* F, int64_t ldf, double2* X, int64_t ldx, int n, int nr
     const int i = upper ? 2 * nb - 1 - step : step, r0 = i * TB, rb = std::min(TB, n - r0);
     double2* Xi = X + (int64_t)r0 * ldx;
     const double2* iv = inv + (size_t)(upper ? nb + i : i) * TB * TB;
-    int* ke = kexp + (size_t)step * TB;
+    int* st = stats + (size_t)step * 4 * TB;
     count_launch();
     if (nrhs <= 2 * device_sm_count())
-      launch_early(true, diag_kernel<1>, nrhs, 256, 0, s, iv, upper, Xi, ldx, rb, nrhs, ke);
+      launch_early(true, diag_kernel<1>, nrhs, 256, 0, s, iv, upper, Xi, ldx, rb, nrhs, st);
     else
-      launch_early(false, diag_kernel<4>, (nrhs + 3) / 4, 256, 0, s, iv, upper, Xi, ldx, rb, nrhs, ke);
+      launch_early(false, diag_kernel<4>, (nrhs + 3) / 4, 256, 0, s, iv, upper, Xi, ldx, rb, nrhs, st);
     const int q0 = upper ? 0 : r0 + rb, m = upper ? r0 : n - q0;
     if (m <= 0) continue;
-    int e = zgemm_digits(plan, F + (int64_t)q0 * ldf + r0, ldf, m, Xi, ldx, nrhs, rb, ke, s);
-    if (e == MGT_OK) e = zgemm_apply(plan, 0, m, 0, nrhs, rb, X + (int64_t)q0 * ldx, ldx, true, nullptr, status, s);
+    const ZRows rows{ZRows::MEAN, st, nullptr};
+    const double2* Fi = F + (int64_t)q0 * ldf + r0;
+    int e = zgemm_digits(plan, Fi, ldf, m, Xi, ldx, nrhs, rb, rows, s);
+    if (e == MGT_OK)
+      e = zgemm_apply(plan, Fi, ldf, m, Xi, ldx, nrhs, rb, X + (int64_t)q0 * ldx, ldx, ZOut::SUB, nullptr, status, s);
     if (e != MGT_OK) return e;
   }
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
