@@ -120,7 +120,7 @@ __device__ __forceinline__ int row_mode(const ZRows& rows, int K, int lane, int 
   }
   lo = __reduce_min_sync(0xffffffffu, lo);
   hi = __reduce_max_sync(0xffffffffu, hi);
-  (void)inv;
+  if (KIND == ZRows::MAX && inv >= kInvLimit) return kFp64;
   if (hi - lo <= kRowSpread) return kAsIs;
   if (KIND == ZRows::MAX) {
     if (hi - lo > kHalfSpread) return kFp64;

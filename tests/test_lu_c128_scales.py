@@ -51,7 +51,8 @@ def _matrix(name):
     return A
 
 
-@pytest.mark.parametrize("name", ["large entries", "blocks", "rows and columns", "pairs"])
+@pytest.mark.parametrize("name", ["large entries", "blocks", "rows and columns", "pairs", "ill-conditioned L 0.5",
+                                  "ill-conditioned L 0.9"])
 def test_columns_of_the_factors(name):
     from magreete_gb300 import engine as E
     A = _matrix(name)
