@@ -203,6 +203,7 @@ digits_kernel(const double2* __restrict__ A, int64_t lda, int M, int ablocks, co
   aexp += blockIdx.y * sl.aexp;
   bdig += blockIdx.y * sl.bdig;
   bexp += blockIdx.y * sl.bexp;
+  if (KIND == ZRows::MEAN) br.stats += (size_t)blockIdx.y * kZK * 4;
   K = min(kZK, K - (int)blockIdx.y * kZK);
   int sh[NCH];
   // (kFp64: the row exponents say so, and nothing made of the digits is used)
@@ -919,22 +920,53 @@ int zgemm_apply(const ZGemmPlan& p, const double2* A, int64_t lda, int M, const 
 
 namespace zg {
 
-// out = E0 - sum over slabs of part
+// Sizes of B's rows (ZRows::MEAN), one warp per row.
+__global__ void __launch_bounds__(256)
+row_stats_kernel(const double2* __restrict__ B, int64_t ldb, int K, int N, int4* __restrict__ stats) {
+  const int k = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (k >= K) return;
+  int em = 0, sum = 0, count = 0;
+  for (int c = lane; c < N; c += 32) {
+    const int f = field(B[(int64_t)k * ldb + c]);
+    em = max(em, f);
+    sum += f ? f - 1023 : 0;
+    count += f ? 1 : 0;
+  }
+  em = __reduce_max_sync(0xffffffffu, em);
+  sum = __reduce_add_sync(0xffffffffu, sum);
+  count = __reduce_add_sync(0xffffffffu, count);
+  const long long both = ((long long)count << 32) + sum;
+  if (lane == 0) stats[k] = make_int4(em, 0, (int)both, (int)(both >> 32));
+}
+
+// out = E0 - sum over slabs of part; a slab that the digits' kernel left to the
+// FP64 pipe (its row exponents say so) is multiplied out here.
 __global__ void slab_sum_kernel(const double2* __restrict__ part, int slabs, int M, int N,
-                                const double2* __restrict__ E0, int64_t ld0, double2* __restrict__ out, int64_t ldo) {
+                                const double2* __restrict__ E0, int64_t ld0, double2* __restrict__ out, int64_t ldo,
+                                const int* __restrict__ aexp, size_t aexp_stride, const double2* __restrict__ A,
+                                int64_t lda, const double2* __restrict__ B, int64_t ldb, int K) {
   early_start();
   const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= (int64_t)M * N) return;
   const int64_t r = i / N, c = i - r * N;
   double2 s = make_double2(0.0, 0.0);
-  for (int q = 0; q < slabs; ++q) s = cadd(s, part[(int64_t)q * M * N + i]);
+  for (int q = 0; q < slabs; ++q) {
+    double2 p;
+    if (__ldg(aexp + q * aexp_stride) == kPlainExp) {
+      p = make_double2(0.0, 0.0);
+      for (int k = q * kZK; k < min(K, (q + 1) * kZK); ++k) cfma(p, A[r * lda + k], B[k * ldb + c]);
+    } else {
+      p = part[(int64_t)q * M * N + i];
+    }
+    s = cadd(s, p);
+  }
   const double2 e = E0 ? E0[r * ld0 + c] : make_double2(0.0, 0.0);
   out[r * ldo + c] = csub(e, s);
 }
 
 struct Wide {
   int slabs;
-  size_t rt, ct, adig, bdig, aexp, bexp, part, total;
+  size_t rt, ct, adig, bdig, aexp, bexp, stats, part, total;
   Wide(int64_t M, int64_t N, int64_t K) {
     slabs = (int)((K + kZK - 1) / kZK);
     rt = (size_t)((M + BM - 1) / BM);
@@ -943,7 +975,8 @@ struct Wide {
     bdig = adig + up(slabs * rt * NCH * DIG * D_SLICE, 1024);
     aexp = bdig + up(slabs * ct * NCH * B_BLOCK, 1024);
     bexp = aexp + up(slabs * rt * BM * sizeof(int), 256);
-    part = bexp + up(slabs * ct * BNC * sizeof(int), 256);
+    stats = bexp + up(slabs * ct * BNC * sizeof(int), 256);
+    part = stats + (size_t)slabs * kZK * sizeof(int4);
     total = part + (size_t)slabs * M * N * sizeof(double2) + 1024;
   }
 };
@@ -974,13 +1007,17 @@ int zgemm_wide(const double2* A, int64_t lda, int M, const double2* B, int64_t l
   set_attributes();
   if (cudaMemsetAsync(b, 0, 256, s) != cudaSuccess) return MGT_ERR_CUDA;   // status
   const int ab = (int)w.rt * (BM / 32);
-  count_launch(3);
-  launch_early(false, digits_kernel<ZRows::NONE>, dim3(ab + (unsigned)w.ct, w.slabs), 256, 0, s, A, lda, M, ab, B, ldb, N, K, ZRows(), adig, aexp,
+  int4* stats = (int4*)(b + w.stats);
+  count_launch(4);
+  launch_early(false, row_stats_kernel, (K + 7) / 8, 256, 0, s, B, ldb, K, N, stats);
+  const ZRows rows{ZRows::MEAN, (const int*)stats, nullptr};
+  launch_early(false, digits_kernel<ZRows::MEAN>, dim3(ab + (unsigned)w.ct, w.slabs), 256, 0, s, A, lda, M, ab, B, ldb, N, K, rows, adig, aexp,
                                                                   bdig, bexp, sl);
   launch_early(false, zgemm_kernel, (int)std::min<int64_t>(total, device_sm_count()), THREADS, smem_bytes(), s,
       adig, aexp, bdig, bexp, M, N, NCH, (int)w.ct, (int)total, part, N,
       Plain{nullptr, nullptr, 0, 0, 0, ZOut::SET}, nullptr, (int*)b, sl);
-  launch_early(false, slab_sum_kernel, (unsigned)(((int64_t)M * N + 255) / 256), 256, 0, s, part, w.slabs, M, N, E0, ld0, out, ldo);
+  launch_early(false, slab_sum_kernel, (unsigned)(((int64_t)M * N + 255) / 256), 256, 0, s, part, w.slabs, M, N, E0, ld0, out, ldo,
+               aexp, sl.aexp, A, lda, B, ldb, K);
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }
 

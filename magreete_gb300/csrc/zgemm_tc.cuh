@@ -33,7 +33,7 @@ size_t zgemm_bytes(int64_t rows, int64_t cols);
 //     of the engine's systems spread by 2^2 to 2^8, Poisson clouds at the upper
 //     end; pairs of scatterers at 1e-4 of their wavelength by 2^30, where
 //     moving whole exponents lost 1e9 of a column's accuracy.)
-//   MEAN (the triangular solves; stats: 16 bytes a row -- the largest field, 4 unused
+//   MEAN (the solves and the propagation; stats: 16 bytes a row -- the largest field, 4 unused
 //     bytes, and in 64 bits the sum of the fields less 1023 plus 2^32 for each nonzero entry).  Right-hand sides may have single
 //     large entries, so that a row's mean says what meets A's column: spreads of
 //     the means up to 2^4: as they are; beyond, where the rows are alike but for
@@ -56,7 +56,7 @@ int zgemm_apply(const ZGemmPlan& p, const double2* A, int64_t lda, int M, const 
                 double2* C, int64_t ldc, ZOut out, int* rowmax, int* status, cudaStream_t s);
 
 // out (M x N) = E0 - A B for any K (E0 may be null: zero), in a workspace of zgemm_wide_bytes: every 64
-// columns of K have their own scales, their products are summed in FP64.  The status word is the first int
+// columns of K have their own scales (and ZRows::MEAN of their own), their products are summed in FP64.  The status word is the first int
 // of the workspace's first 1024-byte boundary.
 size_t zgemm_wide_bytes(int64_t M, int64_t N, int64_t K);
 int zgemm_wide(const double2* A, int64_t lda, int M, const double2* B, int64_t ldb, int N, int K, const double2* E0,
