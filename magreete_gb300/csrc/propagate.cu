@@ -235,21 +235,25 @@ static bool prop_tc_ok(int64_t nt, int64_t ns, int64_t nrhs, int d) {
   return residual_tc_supported(prop_chunk_targets(nt, ns, d) * d, (int64_t)d * ns, nrhs);
 }
 // Plain method: FP64 multiply-adds of the matrix-free kernel (its column tiles are 16, 32 or 64 wide) above
-// which the assembled way is faster.  The FP64 pipes do 254 a clock; the assembled way takes two launches per
-// 64 columns of K, about 20 us.
+// which the assembled way is faster.  The FP64 pipes do 254 a clock; the assembled way takes four launches
+// (20 us) and 18.4 K clocks an SM for a tile of 128 rows x 32 columns of each 64 of K, however few rows it
+// holds: a handful of detectors before very many scatterers stay with the matrix-free kernel.
 constexpr double kPropTcMinFma = 6e7;
+constexpr int64_t kPropMaxTargets = 65535 * 4;   // rows of points of one assembly launch
 static bool prop_z_pays(int64_t nt, int64_t ns, int64_t nrhs, int d) {
-  return 4.0 * d * d * (double)nt * (double)ns * (double)((nrhs + 15) / 16 * 16) >= kPropTcMinFma &&
-         (int64_t)d * nt <= (1 << 28) && nrhs <= (1 << 16);
+  const double fma = 4.0 * d * d * (double)nt * (double)ns * (double)((nrhs + 15) / 16 * 16);
+  const int64_t slabs = (d * ns + kZK - 1) / kZK;
+  const double tiles = (double)slabs * (double)((d * nt + 127) / 128) * (double)((nrhs + 31) / 32);
+  return fma >= kPropTcMinFma && tiles * 18.4e3 / sm_count() < fma / 254 && slabs <= 65535 && nrhs <= (1 << 16) &&
+         (int64_t)d * nt <= (1 << 28);
 }
 // targets per chunk: rows, their digits and the partial products within about 1 GiB each
 static int64_t prop_z_targets(int64_t nt, int64_t ns, int64_t nrhs, int d) {
   const int64_t slabs = (d * ns + kZK - 1) / kZK;
   const int64_t per = std::max((int64_t)d * d * ns * 16, (int64_t)d * slabs * nrhs * 16);
-  return std::max<int64_t>(1, std::min<int64_t>(nt, (int64_t)kPropChunkBytes / per));
+  return std::max<int64_t>(1, std::min<int64_t>({nt, (int64_t)kPropChunkBytes / per, kPropMaxTargets}));
 }
 static size_t prop_z_bytes(int64_t nt, int64_t ns, int64_t nrhs, int d) {
-  if (!prop_z_pays(nt, ns, nrhs, d)) return 0;
   const int64_t ct = prop_z_targets(nt, ns, nrhs, d);
   return (size_t)ct * d * d * ns * sizeof(double2) + zgemm_wide_bytes(ct * d, nrhs, (int64_t)d * ns) + 1024;
 }
@@ -283,7 +287,7 @@ extern "C" int mgt_propagate_workspace_bytes(int kind, int64_t n_targets, int64_
   // double-float copy of Ek plus one chunk of assembled propagator rows
   *bytes = std::max({(size_t)nsplit * n_targets * d * std::min<int64_t>(nrhs, kPCols) * sizeof(double2),
                      prop_df_bytes(n_targets, n_sources, nrhs, d), prop_tc_bytes(n_targets, n_sources, nrhs, d),
-                     prop_z_bytes(n_targets, n_sources, nrhs, d)});
+                     prop_z_pays(n_targets, n_sources, nrhs, d) ? prop_z_bytes(n_targets, n_sources, nrhs, d) : 0});
   return MGT_OK;
 }
 
