@@ -83,6 +83,7 @@ SIGNATURES = {
     "mgt_refine_start": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _i64, _vp, _sz, _vp]),
     "mgt_refine_correct": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _i64, _vp, _sz, _vp]),
     "mgt_refine_norms": (_i32, [_vp, _i64, _i64, _vp, _i64, _vp, _i64, _i64, _vp, _sz, _vp, _vp]),
+    "mgt_propagate_workspace_bytes_for": (_i32, [_i32, _i32, _i64, _i64, _i64, ctypes.POINTER(_sz)]),
     "mgt_propagate_workspace_bytes": (_i32, [_i32, _i64, _i64, _i64, ctypes.POINTER(_sz)]),
     "mgt_propagate": (_i32, [_i32, _i32, _vp, _i64, _vp, _i64, _f64, _f64, _f64, _i32, _f64, _vp, _i64, _vp, _i64,
                              _vp, _i64, _i64, _vp, _sz, _vp]),

@@ -277,17 +277,34 @@ static int kind_dim_d(int kind, int* dim) {
 
 using namespace mgt;
 
+// partial sums of the matrix-free kernel
+static size_t prop_free_bytes(int64_t nt, int64_t ns, int64_t nrhs, int d) {
+  return (size_t)choose_splits(nt, ns) * nt * d * std::min<int64_t>(nrhs, kPCols) * sizeof(double2);
+}
+
+extern "C" int mgt_propagate_workspace_bytes_for(int kind, int dtype, int64_t n_targets, int64_t n_sources,
+                                                 int64_t nrhs, size_t* bytes) {
+  int dim;
+  const int d = kind_dim_d(kind, &dim);
+  if (!bytes || d == 0 || (dtype != MGT_C128 && dtype != MGT_CDF) || n_targets <= 0 || n_sources <= 0 || nrhs <= 0)
+    return MGT_ERR_ARG;
+  if (dtype == MGT_C128)
+    *bytes = prop_z_pays(n_targets, n_sources, nrhs, d) ? prop_z_bytes(n_targets, n_sources, nrhs, d)
+                                                        : prop_free_bytes(n_targets, n_sources, nrhs, d);
+  else
+    *bytes = prop_tc_ok(n_targets, n_sources, nrhs, d) ? prop_tc_bytes(n_targets, n_sources, nrhs, d)
+                                                       : prop_df_bytes(n_targets, n_sources, nrhs, d);
+  return MGT_OK;
+}
+
 extern "C" int mgt_propagate_workspace_bytes(int kind, int64_t n_targets, int64_t n_sources, int64_t nrhs,
                                              size_t* bytes) {
-  int dim;
-  int d = kind_dim_d(kind, &dim);
-  if (!bytes || d == 0 || n_targets <= 0 || n_sources <= 0 || nrhs <= 0) return MGT_ERR_ARG;
-  int nsplit = choose_splits(n_targets, n_sources);
-  // the larger of the two methods' needs: FP64 partial sums, or the
-  // double-float copy of Ek plus one chunk of assembled propagator rows
-  *bytes = std::max({(size_t)nsplit * n_targets * d * std::min<int64_t>(nrhs, kPCols) * sizeof(double2),
-                     prop_df_bytes(n_targets, n_sources, nrhs, d), prop_tc_bytes(n_targets, n_sources, nrhs, d),
-                     prop_z_pays(n_targets, n_sources, nrhs, d) ? prop_z_bytes(n_targets, n_sources, nrhs, d) : 0});
+  if (!bytes) return MGT_ERR_ARG;
+  size_t plain = 0, mixed = 0;
+  const int e = mgt_propagate_workspace_bytes_for(kind, MGT_C128, n_targets, n_sources, nrhs, &plain);
+  if (e != MGT_OK) return e;
+  mgt_propagate_workspace_bytes_for(kind, MGT_CDF, n_targets, n_sources, nrhs, &mixed);
+  *bytes = std::max(plain, mixed);
   return MGT_OK;
 }
 
@@ -303,11 +320,13 @@ extern "C" int mgt_propagate(int kind, int dtype, const double* targets, int64_t
   if (ld_ek < nrhs || ld_out < nrhs || (E0 && ld_e0 < nrhs)) return MGT_ERR_ARG;
   if (n_targets > (1 << 28) || n_sources > (1 << 28)) return MGT_ERR_UNSUPPORTED;
   size_t need = 0;
-  mgt_propagate_workspace_bytes(kind, n_targets, n_sources, nrhs, &need);
-  if (work_bytes < need) return MGT_ERR_WORKSPACE;
+  mgt_propagate_workspace_bytes_for(kind, dtype, n_targets, n_sources, nrhs, &need);
+  // a workspace too small for the plain method's assembled way may serve the matrix-free kernel
+  if (work_bytes < need && (dtype != MGT_C128 || work_bytes < prop_free_bytes(n_targets, n_sources, nrhs, d)))
+    return MGT_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
   const int nt = (int)n_targets, ns = (int)n_sources;
-  if (dtype == MGT_C128 && prop_z_pays(nt, ns, nrhs, d)) {
+  if (dtype == MGT_C128 && prop_z_pays(nt, ns, nrhs, d) && work_bytes >= need) {
     const int64_t ct = prop_z_targets(nt, ns, nrhs, d);
     double2* Gc = (double2*)work;
     void* zw = (char*)work + (size_t)ct * d * d * ns * sizeof(double2);

@@ -435,7 +435,8 @@ class SystemFactorization:
 # ------------------------------------------------------------------ propagate
 
 def propagate(kind, targets, sources, k0, coef, Ek, E0=None, regularize=False, radius=0.0, precision="fp64"):
-    """coef * G(targets, sources) @ Ek + E0, matrix-free.  Ek (d*S, R),
+    """coef * G(targets, sources) @ Ek + E0 (rows of G in chunks of at most 1 GiB;
+    small calls of the plain method without storing them).  Ek (d*S, R),
     E0 (d*T, R) or None.  Returns (d*T, R) complex128."""
     lib = L.load()
     dim, d = KIND_DIMS[kind]
@@ -445,12 +446,12 @@ def propagate(kind, targets, sources, k0, coef, Ek, E0=None, regularize=False, r
     if E0 is not None:
         E0 = E0.reshape(d * T, R).to(torch.complex128).contiguous()
     out = torch.empty((d * T, R), dtype=torch.complex128, device=targets.device)
+    code = L.MGT_C128 if precision == "fp64" else L.MGT_CDF
     nb = ctypes.c_size_t()
-    L.check(lib.mgt_propagate_workspace_bytes(KIND_CODE[kind], T, S, R, ctypes.byref(nb)),
-            "mgt_propagate_workspace_bytes")
+    L.check(lib.mgt_propagate_workspace_bytes_for(KIND_CODE[kind], code, T, S, R, ctypes.byref(nb)),
+            "mgt_propagate_workspace_bytes_for")
     work = workspace(nb.value, targets.device)
     coef = complex(coef)
-    code = L.MGT_C128 if precision == "fp64" else L.MGT_CDF
     L.check(lib.mgt_propagate(KIND_CODE[kind], code, _ptr(targets), T, _ptr(sources), S, float(k0), coef.real,
                               coef.imag, int(bool(regularize)), float(radius), _ptr(Ek), R, _ptr(E0), R,
                               _ptr(out), R, R, _ptr(work), work.numel(), _stream()), "mgt_propagate")

@@ -2,9 +2,9 @@
 
 A request (``workloads.Problem``) is one coupled-dipole solve: incident
 fields at the scatterers and detectors, system assembly, LU, (refined)
-solve for all right-hand sides, and matrix-free propagation to the
-detectors -- the ``generate_source`` -> ``solve`` -> ``propagate`` sequence
-the reference driver runs per frequency (magreete.py:371-400).
+solve for all right-hand sides, and propagation to the detectors -- the
+``generate_source`` -> ``solve`` -> ``propagate`` sequence the reference
+driver runs per frequency (magreete.py:371-400).
 
 ``Server`` keeps several requests in flight on one GPU: each of ``slots``
 worker threads owns a CUDA stream and takes the oldest waiting request as
@@ -19,12 +19,14 @@ from __future__ import annotations
 
 import collections
 import concurrent.futures as cf
+import ctypes
 import dataclasses
 import threading
 import time
 
 import torch
 
+from . import _lib as L
 from . import engine as E
 from . import selfterm
 from . import sources as S
@@ -73,29 +75,32 @@ def solve_problem(prob, precision="mixed", pts=None, det=None, tol=E.DEFAULT_TOL
     return Result(X, Ed, it, rr if rr is not None else float("nan"), reused_factorization=factorization is not None)
 
 
+def _query(fn, *args):
+    nb = ctypes.c_size_t()
+    L.check(fn(*args, ctypes.byref(nb)), "workspace query")
+    return nb.value
+
+
 def matrix_bytes(prob, precision="mixed"):
-    """Device bytes a request holds at its peak: the matrix copies (24 B / entry
-    mixed: complex64 LU + double-float residual copy; 16 B fp64), the
-    tensor-core split buffers of the LU's update (12 KB per row: K up to 256,
-    sized for fp32 splits), the triangular solves' inverted diagonal blocks (12 KB
-    per row, rows rounded up to 256), the right-hand-side blocks and
-    the propagation workspace (double-float propagator rows, at most 1 GiB at
-    a time, and the double-float copy of the fields), the split-K partial sums
-    of the residual (at most 16 splits) and the digits of the tensor-core
-    residual: the right-hand sides' (56 KB per 32 rows and 32 right-hand
-    sides) and, in the mixed method, the matrix's (14 B per entry, rows padded
-    to 128) and the propagator rows' (14 B per entry of a chunk)."""
-    n, R = prob.n, prob.nrhs
-    per = 16 if precision == "fp64" else 24
+    """Device bytes a request holds at its peak, from the library's own workspace
+    queries (host only): the matrix copies (24 B an entry mixed: complex64 LU and
+    double-float residual copy; 16 B fp64), the LU's workspace, the
+    refinement's or the triangular solves', the propagation's in this precision, and
+    the blocks of fields."""
+    lib = L.load()
+    n, R = prob.n, max(1, prob.nrhs)
+    if precision == "fp64":
+        per, code, prop_code = 16, L.MGT_C128, L.MGT_C128
+        solve = _query(lib.mgt_lu_solve_workspace_bytes, code, n, R)
+    else:
+        per, code, prop_code = 24, L.MGT_C64, L.MGT_CDF
+        solve = _query(lib.mgt_refine_workspace_bytes, n, R)
+    need = per * n * n + _query(lib.mgt_lu_workspace_bytes, code, n) + solve + 8 * 16 * n * R + (64 << 20)
     T = prob.detectors.shape[0] if prob.detectors is not None else 0
-    chunk = min(1 << 30, 16 * prob.d * n * T)
-    prop = chunk + 16 * n * R + (chunk * 14 // 16 if precision != "fp64" else 0)
-    partial = 16 * 16 * n * max(R, 64)
-    digits = 57344 * -(-n // 32) * -(-R // 32)
-    if precision != "fp64":
-        digits += 14 * (-(-n // 128) * 128) * (-(-n // 32) * 32)
-    split = 12288 * n + 12288 * (-(-n // 256) * 256)
-    return per * n * n + split + 8 * 16 * n * R + prop + partial + digits + (64 << 20)
+    if T:
+        need += _query(lib.mgt_propagate_workspace_bytes_for, E.KIND_CODE[prob.kind], prop_code, T, n // prob.d, R)
+        need += 4 * 16 * prob.d * T * R
+    return need
 
 
 def serve_sequential(problems, precision="mixed", device_inputs=None, start=None):
