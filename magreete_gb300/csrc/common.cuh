@@ -165,6 +165,10 @@ inline cudaError_t launch_early(bool early, void (*kernel)(P...), dim3 grid, dim
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
 }
 
+// Byte offset of the two status words (error, info) in every workspace that has
+// them: mgt_workspace_status reads them there.
+constexpr size_t kStatusOffset = 8;
+
 // Iteration limit of every device-side spin wait (about a few seconds with
 // the back-off below).  A wait that runs out records MGT_ERR_TIMEOUT in the
 // status word and the kernel returns instead of hanging.

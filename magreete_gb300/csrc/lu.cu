@@ -41,7 +41,7 @@ constexpr size_t kRecBytes = (kRecHeader + 2 * kNBmax * sizeof(double2) + 127) &
 
 // Workspace layout (byte offsets), identical for both element types.
 struct LuWsLayout {
-  size_t status = 8;      // 2 x i32: error, info
+  size_t status = kStatusOffset;   // 2 x i32: error, info
   size_t nslot = 16;      // 2 x i32: slots written by the last panel of each slot set
   size_t epoch = 40;      // u64: factorisation counter (bumped on the device, never cleared)
   size_t slots = 64;      // 2 sets x 2*NBmax x int2 (pos, src)

@@ -255,7 +255,7 @@ static int64_t prop_z_targets(int64_t nt, int64_t ns, int64_t nrhs, int d) {
 }
 static size_t prop_z_bytes(int64_t nt, int64_t ns, int64_t nrhs, int d) {
   const int64_t ct = prop_z_targets(nt, ns, nrhs, d);
-  return (size_t)ct * d * d * ns * sizeof(double2) + zgemm_wide_bytes(ct * d, nrhs, (int64_t)d * ns) + 1024;
+  return 256 + (size_t)ct * d * d * ns * sizeof(double2) + zgemm_wide_bytes(ct * d, nrhs, (int64_t)d * ns) + 1024;
 }
 static size_t prop_tc_bytes(int64_t nt, int64_t ns, int64_t nrhs, int d) {
   if (!prop_tc_ok(nt, ns, nrhs, d)) return 0;
@@ -328,8 +328,11 @@ extern "C" int mgt_propagate(int kind, int dtype, const double* targets, int64_t
   const int nt = (int)n_targets, ns = (int)n_sources;
   if (dtype == MGT_C128 && prop_z_pays(nt, ns, nrhs, d) && work_bytes >= need) {
     const int64_t ct = prop_z_targets(nt, ns, nrhs, d);
-    double2* Gc = (double2*)work;
-    void* zw = (char*)work + (size_t)ct * d * d * ns * sizeof(double2);
+    // status words | rows | digits and partial products
+    int* status = (int*)((char*)work + kStatusOffset);
+    if (cudaMemsetAsync(work, 0, 256, st) != cudaSuccess) return MGT_ERR_CUDA;
+    double2* Gc = (double2*)((char*)work + 256);
+    void* zw = (char*)(Gc + (size_t)ct * d * d * ns);
     const double2 mcoef = make_double2(-coef_re, -coef_im);
     const int kd = d * ns;
     int e = MGT_OK;
@@ -340,7 +343,7 @@ extern "C" int mgt_propagate(int kind, int dtype, const double* targets, int64_t
       if (e == MGT_OK)
         e = zgemm_wide(Gc, kd, tc * d, (const double2*)Ek, ld_ek, (int)nrhs, kd,
                        E0 ? (const double2*)E0 + t0 * d * ld_e0 : nullptr, ld_e0, (double2*)out + t0 * d * ld_out,
-                       ld_out, zw, st);
+                       ld_out, zw, status, st);
     }
     return e;
   }

@@ -10,6 +10,13 @@ namespace mgt {
 namespace tc {
 
 constexpr uint32_t kWaitLimit = 1u << 22;
+// of the waits that may give up (mbar_wait); a build with 0 takes every such path
+// (copies and MMAs in flight are waited for all the same: mbar_wait_plain)
+#ifdef MGT_ROLE_WAIT_LIMIT
+constexpr uint32_t kRoleWaitLimit = MGT_ROLE_WAIT_LIMIT;
+#else
+constexpr uint32_t kRoleWaitLimit = kWaitLimit;
+#endif
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
@@ -46,7 +53,7 @@ __device__ __forceinline__ bool mbar_wait_plain(uint64_t* bar, uint32_t parity) 
 }
 // Bounded wait: false if the CTA aborted or the limit ran out (then abort is set).
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort) {
-  for (uint32_t it = 0; it < kWaitLimit; ++it) {
+  for (uint32_t it = 0; it < kRoleWaitLimit; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
     if (*abort) return false;
   }

@@ -654,14 +654,22 @@ tri_step_kernel(const float2* __restrict__ F, int64_t ldf, const unsigned char* 
     tc_fence_before();
     __syncthreads();
     if (tid == 0) {
-      if (inverse && !mbar_wait_plain(&bar_inv, 0)) abort_flag = 1;
+      // a wait that runs out: noted, and once more, so that nothing is left in flight
+      if (inverse && !mbar_wait(&bar_inv, 0, &abort_flag)) mbar_wait_plain(&bar_inv, 0);
       tc_fence_after();
       tri_issue(tmem, abuf, bbuf);
       mma_commit(&bar);
     }
-    if (!mbar_wait_plain(&bar, phase)) abort_flag = 1;
+    if (!mbar_wait(&bar, phase, &abort_flag)) mbar_wait_plain(&bar, phase);
     phase ^= 1;
     tc_fence_after();
+  };
+  // the products of a CTA whose wait ran out are NaN, and so are the block rows made of them
+  auto poison = [&]() {
+    if (*(volatile int*)&abort_flag) {
+#pragma unroll
+      for (int j = 0; j < 32; ++j) acc[j] = __int_as_float(0x7FC00000);
+    }
   };
   auto load_inverse = [&]() {
     if (tid == 0) {
@@ -681,6 +689,7 @@ tri_step_kernel(const float2* __restrict__ F, int64_t ldf, const unsigned char* 
       product(false);
       if (!alone && cl == 0) load_inverse();   // the tile's products are done
       tri_read(acc, tmem, rexp, cexp, warp, lane);
+      poison();
       tc_fence_before();
       if (!alone || q == 3) break;
       __syncthreads();   // the exponents and tensor memory are read
@@ -740,6 +749,7 @@ tri_step_kernel(const float2* __restrict__ F, int64_t ldf, const unsigned char* 
 #pragma unroll
       for (int j = 0; j < 32; ++j) acc[j] = 0.f;
       tri_read(acc, tmem, rexp, cexp, warp, lane);
+      poison();
       tc_fence_before();
       __syncthreads();
       tri_partials(acc, P, warp, lane);
@@ -762,7 +772,7 @@ tri_step_kernel(const float2* __restrict__ F, int64_t ldf, const unsigned char* 
   }
 }
 
-// Workspace of a solve: the status words (at byte 128); the inverted diagonal
+// Workspace of a solve: the status words; the inverted diagonal
 // blocks of L and of U; those of ill-conditioned blocks after the Newton step;
 // the operands and their row exponents; the blocks' row sums and condition
 // numbers.
@@ -834,7 +844,7 @@ int tri_solve(const float2* F, int64_t ldf, float2* X, int64_t ldx, int n, int n
     cudaFuncSetAttribute(tri_step_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTSmem);
     cudaFuncSetAttribute(tri_step_kernel<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTSmem);
   });
-  int* status = (int*)((char*)work + 128);
+  int* status = (int*)((char*)work + kStatusOffset);
   if (cudaMemsetAsync(status, 0, 2 * sizeof(int), s) != cudaSuccess) return MGT_ERR_CUDA;
   const int nb = (n + kTD - 1) / kTD;
   const TriWs L(n);

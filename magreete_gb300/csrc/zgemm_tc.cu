@@ -29,8 +29,8 @@
 //                output is left (an FP64 conversion costs as much as the subtraction)
 //   warps 10-15: converters: byte digits -> FP16 operand slices
 // The MMAs of the next tile run while the epilogue finishes the last one.
-// Every wait is bounded; on expiry MGT_ERR_TIMEOUT is recorded, the issued work
-// drained and TMEM freed.
+// Every wait is bounded; on expiry MGT_ERR_TIMEOUT is recorded, the CTA's tiles
+// become NaN, the issued work is drained and TMEM freed.
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -425,6 +425,19 @@ __device__ __noinline__ void plain_solve(const Plain& p, unsigned char* smem, in
   }
 }
 
+// NaN in the place of the CTA's tiles, after a wait that ran out
+__device__ __noinline__ void poison_tiles(int M, int N, int ctiles, int total_tiles, double2* C, int64_t ldc,
+                                          const Slabs& sl) {
+  const double nan = __longlong_as_double(0x7FF8000000000000LL);
+  for (int tt = blockIdx.x; tt < total_tiles; tt += gridDim.x) {
+    const int slab = tt / sl.tiles, t = tt - slab * sl.tiles;
+    for (int i = threadIdx.x; i < BM * BNC; i += THREADS) {
+      const int row = (t / ctiles) * BM + i / BNC, col = (t % ctiles) * BNC + i % BNC;
+      if (row < M && col < N) C[slab * sl.c + (int64_t)row * ldc + col] = make_double2(nan, nan);
+    }
+  }
+}
+
 __global__ void __launch_bounds__(THREADS, 1)
 zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aexp,
              const unsigned char* __restrict__ bdig, const int* __restrict__ bexp, int M, int N, int nch, int ctiles,
@@ -552,7 +565,7 @@ zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aex
         asm volatile("prefetch.global.L2 [%0];" ::"l"(crow));
         asm volatile("prefetch.global.L2 [%0];" ::"l"(crow + (ncol - 1)));
       }
-      if (!mbar_wait(tfull, lt & 1, abort)) break;
+      if (!__all_sync(0xffffffffu, mbar_wait(tfull, lt & 1, abort))) break;   // (the warp leaves as one)
       tc_fence_after();
       long long acc[EPI_COLS];
 #pragma unroll
@@ -660,18 +673,19 @@ zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aex
     const int nq = nblk * DIG;
     for (int q = 0; q < nq; ++q) {
       const int ds = q % DSLOTS, as = q % ASLOTS;
-      if (!mbar_wait(&full_d[ds], (q / DSLOTS) & 1, abort)) break;
-      if (q >= ASLOTS && !mbar_wait(&empty_a[as], ((q / ASLOTS) - 1) & 1, abort)) break;
+      const bool ok = mbar_wait(&full_d[ds], (q / DSLOTS) & 1, abort) &&
+                      (q < ASLOTS || mbar_wait(&empty_a[as], ((q / ASLOTS) - 1) & 1, abort));
       const unsigned char* src = dring + ds * D_SLICE;
       unsigned char* dst = aring + as * A_SLICE;
-      for (int u = ctid; u < (int)(D_SLICE / 8); u += NCONV * 32) {
-        const uint32_t off = (uint32_t)u * 8u;
-        const uint2 v = *reinterpret_cast<const uint2*>(src + off);
-        const uint2 w0 = widen4(v.x), w1 = widen4(v.y);
-        *reinterpret_cast<uint4*>(dst + 2 * off) = make_uint4(w0.x, w0.y, w1.x, w1.y);
-      }
+      if (ok)
+        for (int u = ctid; u < (int)(D_SLICE / 8); u += NCONV * 32) {
+          const uint32_t off = (uint32_t)u * 8u;
+          const uint2 v = *reinterpret_cast<const uint2*>(src + off);
+          const uint2 w0 = widen4(v.x), w1 = widen4(v.y);
+          *reinterpret_cast<uint4*>(dst + 2 * off) = make_uint4(w0.x, w0.y, w1.x, w1.y);
+        }
       fence_async_smem();
-      __syncwarp();
+      if (!__all_sync(0xffffffffu, ok)) break;   // (the warp leaves as one)
       if (lane == 0) {
         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&full_a[as])) : "memory");
         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&empty_d[ds])) : "memory");
@@ -681,7 +695,9 @@ zgemm_kernel(const unsigned char* __restrict__ adig, const int* __restrict__ aex
   tc_fence_before();
   __syncthreads();
   if (threadIdx.x == 0 && *abort) atomicExch(status, MGT_ERR_TIMEOUT);
-  if (*fp64 && !*abort) {
+  if (*abort) {
+    poison_tiles(M, N, ctiles, total_tiles, C, ldc, sl);
+  } else if (*fp64) {
     // every copy has landed, every product is done (the epilogue has waited for the last tile's)
     if (p64.out == ZOut::SOLVE) plain_solve(p64, base, N, total_tiles, C, ldc, rowmax);
     else plain_tiles(p64, base, M, N, ctiles, total_tiles, C, ldc, rowmax);
@@ -971,7 +987,7 @@ struct Wide {
     slabs = (int)((K + kZK - 1) / kZK);
     rt = (size_t)((M + BM - 1) / BM);
     ct = (size_t)((N + BNC - 1) / BNC);
-    adig = 1024;
+    adig = 0;
     bdig = adig + up(slabs * rt * NCH * DIG * D_SLICE, 1024);
     aexp = bdig + up(slabs * ct * NCH * B_BLOCK, 1024);
     bexp = aexp + up(slabs * rt * BM * sizeof(int), 256);
@@ -986,7 +1002,7 @@ struct Wide {
 size_t zgemm_wide_bytes(int64_t M, int64_t N, int64_t K) { return zg::Wide(M, N, K).total; }
 
 int zgemm_wide(const double2* A, int64_t lda, int M, const double2* B, int64_t ldb, int N, int K, const double2* E0,
-               int64_t ld0, double2* out, int64_t ldo, void* work, cudaStream_t s) {
+               int64_t ld0, double2* out, int64_t ldo, void* work, int* status, cudaStream_t s) {
   using namespace zg;
   const Wide w(M, N, K);
   char* b = (char*)up((size_t)work, 1024);
@@ -1005,7 +1021,6 @@ int zgemm_wide(const double2* A, int64_t lda, int M, const double2* B, int64_t l
   sl.c = (size_t)M * N;
   sl.tiles = (int)(w.rt * w.ct);
   set_attributes();
-  if (cudaMemsetAsync(b, 0, 256, s) != cudaSuccess) return MGT_ERR_CUDA;   // status
   const int ab = (int)w.rt * (BM / 32);
   int4* stats = (int4*)(b + w.stats);
   count_launch(4);
@@ -1015,7 +1030,7 @@ int zgemm_wide(const double2* A, int64_t lda, int M, const double2* B, int64_t l
                                                                   bdig, bexp, sl);
   launch_early(false, zgemm_kernel, (int)std::min<int64_t>(total, device_sm_count()), THREADS, smem_bytes(), s,
       adig, aexp, bdig, bexp, M, N, NCH, (int)w.ct, (int)total, part, N,
-      Plain{nullptr, nullptr, 0, 0, 0, ZOut::SET}, nullptr, (int*)b, sl);
+      Plain{nullptr, nullptr, 0, 0, 0, ZOut::SET}, nullptr, status, sl);
   launch_early(false, slab_sum_kernel, (unsigned)(((int64_t)M * N + 255) / 256), 256, 0, s, part, w.slabs, M, N, E0, ld0, out, ldo,
                aexp, sl.aexp, A, lda, B, ldb, K);
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;

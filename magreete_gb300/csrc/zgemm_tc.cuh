@@ -56,11 +56,10 @@ int zgemm_apply(const ZGemmPlan& p, const double2* A, int64_t lda, int M, const 
                 double2* C, int64_t ldc, ZOut out, int* rowmax, int* status, cudaStream_t s);
 
 // out (M x N) = E0 - A B for any K (E0 may be null: zero), in a workspace of zgemm_wide_bytes: every 64
-// columns of K have their own scales (and ZRows::MEAN of their own), their products are summed in FP64.  The status word is the first int
-// of the workspace's first 1024-byte boundary.
+// columns of K have their own scales (and ZRows::MEAN of their own), their products are summed in FP64.
 size_t zgemm_wide_bytes(int64_t M, int64_t N, int64_t K);
 int zgemm_wide(const double2* A, int64_t lda, int M, const double2* B, int64_t ldb, int N, int K, const double2* E0,
-               int64_t ld0, double2* out, int64_t ldo, void* work, cudaStream_t s);
+               int64_t ld0, double2* out, int64_t ldo, void* work, int* status, cudaStream_t s);
 
 // ---- blocked complex128 LU: interchanges and block inverses
 struct ZSlots {
@@ -78,7 +77,7 @@ int zswap_panel(double2* A, int64_t lda, int n, int j0, int w, const ZSlots& s, 
 int zswap_block(double2* A, int64_t lda, int n, int J0, int wa, int wb, const ZSlots& a, const ZSlots& b,
                 double2* Inv, int* invmax, int* kexp, cudaStream_t st);
 
-// ---- triangular solves X = U^-1 L^-1 X in place (zsolve.cu); the status word is the first int of work
+// ---- triangular solves X = U^-1 L^-1 X in place (zsolve.cu); status words where mgt_workspace_status reads them
 size_t zsolve_workspace_bytes(int64_t n, int64_t nrhs);
 int zsolve(const double2* F, int64_t ldf, double2* X, int64_t ldx, int n, int nrhs, void* work, cudaStream_t s);
 

@@ -120,7 +120,7 @@ diag_kernel(const double2* __restrict__ Inv, int upper, double2* __restrict__ X,
 }
 
 struct Ws {
-  size_t status = 0, stats = 256, inv, plan, total;   // stats: 4 TB ints per block row and triangle
+  size_t status = kStatusOffset, stats = 256, inv, plan, total;   // stats: 4 TB ints per block row and triangle
   Ws(int64_t n, int64_t nrhs) {
     const int64_t nb = (n + TB - 1) / TB;
     inv = (stats + (size_t)(2 * nb * 4 * TB) * sizeof(int) + 255) & ~size_t(255);
