@@ -351,8 +351,9 @@ struct RefineWs {
     }
     return residual_impl(M, ldm, X, ldx, B, ldb, Rr, nr, n, nr, Xs, part, part_elems, s);
   }
-  // device status word of the tensor-core residual (MGT_OK or MGT_ERR_TIMEOUT), or null
+  // device status words (MGT_OK or MGT_ERR_TIMEOUT): of the tensor-core residual, or null; of the triangular solves
   int* status() const { return tc ? (int*)tcw : nullptr; }
+  int* tri_status() const { return (int*)((char*)tri + kStatusOffset); }
 };
 
 }  // namespace mgt
@@ -469,6 +470,13 @@ static int solve_refined(const void* M, int64_t ldm, const void* prepared, const
     if (cudaStreamSynchronize(s) != cudaSuccess) return MGT_ERR_CUDA;
     if (dev_status != MGT_OK) return dev_status;
     rel = h[0] > 0 ? sqrt(h[1] / h[0]) : sqrt(h[1]);
+    if (rel != rel) {
+      // a solve step whose wait ran out leaves NaN and says so (read only here: the copy costs a correction 5 us)
+      if (cudaMemcpyAsync(&dev_status, w.tri_status(), sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+          cudaStreamSynchronize(s) != cudaSuccess)
+        return MGT_ERR_CUDA;
+      if (dev_status != MGT_OK) return dev_status;
+    }
     if (rel <= tol || it >= max_iter) break;
     if (it > 0 && !(rel < 0.9 * prev)) break;  // stagnation or divergence
     prev = rel;

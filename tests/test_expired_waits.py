@@ -48,7 +48,7 @@ def lib(tmp_path_factory):
     subprocess.run([build.nvcc_path()] + build.ARCH +
                    ["-O2", "-std=c++17", "-shared", "-Xcompiler", "-fPIC", "-I", build.INCLUDE, "-I", build.CSRC,
                     "--expt-relaxed-constexpr", "-DMGT_ROLE_WAIT_LIMIT=0", "--threads", "5"] + src +
-                   ["-o", out, "-lcuda"], check=True)
+                   ["-o", out], check=True)
     lib = ctypes.CDLL(out)
     lib.t_bytes.restype = ctypes.c_size_t
     lib.t_bytes.argtypes = [ctypes.c_int] + [ctypes.c_int64] * 3
@@ -90,4 +90,42 @@ def test_solves(lib, complex64):
     fn = lib.t_trisolve if complex64 else lib.t_zsolve
     assert fn(_p(F), _p(X), n, R, _p(work)) == 0
     assert _status(work) == L.MGT_ERR_TIMEOUT
+    assert not torch.isfinite(torch.view_as_real(X)).any()
+
+
+def test_refined_solve(tmp_path):
+    """A refined solve whose triangular solves ran out of waiting says so, instead of
+    not having converged: the library with its solve steps alone built that way."""
+    import glob
+    from magreete_gb300 import _lib as L
+    from magreete_gb300 import build
+    from magreete_gb300 import engine as E
+    # the other files as the library has them, their objects where the build left them
+    others = [f for f in glob.glob(os.path.join(build.CSRC, "*.cu")) if os.path.basename(f) != "trsolve.cu"]
+    objects = [os.path.join(build.BUILD, os.path.basename(f) + ".o") for f in others]
+    for src, obj in zip(others, objects):
+        if not os.path.exists(obj):
+            subprocess.run([build.nvcc_path()] + build.ARCH + ["-O3", "-std=c++17", "-Xcompiler", "-fPIC", "-I",
+                            build.INCLUDE, "--expt-relaxed-constexpr", "-c", src, "-o", str(tmp_path / os.path.basename(obj))],
+                           check=True)
+            objects[objects.index(obj)] = str(tmp_path / os.path.basename(obj))
+    out = str(tmp_path / "libexpired_steps.so")
+    subprocess.run([build.nvcc_path()] + build.ARCH +
+                   ["-O2", "-std=c++17", "-shared", "-Xcompiler", "-fPIC", "-I", build.INCLUDE, "-I", build.CSRC,
+                    "--expt-relaxed-constexpr", "-DMGT_ROLE_WAIT_LIMIT=0", os.path.join(build.CSRC, "trsolve.cu")] +
+                   objects + ["-o", out], check=True)
+    lib = ctypes.CDLL(out)
+    lib.mgt_solve_refined.argtypes = L.SIGNATURES["mgt_solve_refined"][1]
+    n, R = 600, 5
+    pts = torch.rand(n, 3, dtype=torch.float64, generator=torch.Generator().manual_seed(1)).cuda()
+    Mdf, M32 = E.assemble_system("3d_scalar", pts, 9.0, 0.05, 0.0, ("cdf", "c64"))
+    f = E.lu_factor(M32)
+    B = torch.randn(n, R, dtype=torch.complex128).cuda()
+    X = torch.zeros_like(B)
+    nb = ctypes.c_size_t()
+    L.check(L.load().mgt_refine_workspace_bytes(n, R, ctypes.byref(nb)))
+    work = torch.zeros(nb.value, dtype=torch.uint8, device="cuda")
+    st = lib.mgt_solve_refined(E._ptr(Mdf), n, E._ptr(f.lu), f.lu.stride(0), E._ptr(f.perm), n, E._ptr(B), R, E._ptr(X),
+                               R, R, 1e-10, 10, E._ptr(work), nb.value, None, None, E._stream())
+    assert st == L.MGT_ERR_TIMEOUT
     assert not torch.isfinite(torch.view_as_real(X)).any()
