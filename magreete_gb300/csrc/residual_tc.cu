@@ -338,7 +338,7 @@ residual_tc_kernel(const unsigned char* __restrict__ D, int rows, const int* __r
     const uint32_t tbase = tmem + ((uint32_t)(qd * 32) << 16) + (uint32_t)(part * EPI_COLS);
     bool ok = true;
     for (int ro = 0; ro < nread; ++ro) {
-      if (!mbar_wait(tfull, ro & 1, abort)) { ok = false; break; }
+      if (!__all_sync(0xffffffffu, mbar_wait(tfull, ro & 1, abort))) { ok = false; break; }
       tc_fence_after();
       // a fresh copy per readout keeps the 28 TMEM addresses from being
       // hoisted out of the loop into registers
@@ -420,7 +420,8 @@ residual_tc_kernel(const unsigned char* __restrict__ D, int rows, const int* __r
       return true;
     };
     bool ok = nq > 0 && fetch(0);
-    for (int q = 0; ok && q < nq; ++q) {
+    // (a warp leaves as one: its lanes wait for each other below)
+    for (int q = 0; q < nq && __all_sync(0xffffffffu, ok); ++q) {
       uint32_t w[32];
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
@@ -442,7 +443,7 @@ residual_tc_kernel(const unsigned char* __restrict__ D, int rows, const int* __r
       if (q + 1 < nq) ok = fetch(q + 1);   // on its way while this slice waits for its place
       const int as = q % ASLOTS;
       if (q >= ASLOTS) {
-        if (!mbar_wait(&empty_a[as], ((q / ASLOTS) - 1) & 1, abort)) break;
+        if (!__all_sync(0xffffffffu, mbar_wait(&empty_a[as], ((q / ASLOTS) - 1) & 1, abort))) break;
         tc_fence_after();
       }
       tmem_st16(abase + (uint32_t)as * A_COLS, w);
