@@ -17,10 +17,14 @@
 // conversion are done before it waits for X_i.
 //
 // Products on the tensor cores: both operands scaled by a power of two (each
-// row of the factor's tile, each right-hand side) and split into two fp16
-// parts, x = h + 2^-11 l, each rounded to nearest, so that h and l keep the
-// full 22 bits down to 2^-28 of the largest value; the four part products
-// accumulate in FP32 by weight (h h | h l + l h | l l).
+// row of the factor's tile, each right-hand side) to just below 2^15 and split
+// into two fp16 parts, x = h + 2^-11 l, each rounded to nearest, so that h and
+// l keep the full 22 bits down to 2^-28 of the largest value (2^-50 of it
+// absolutely); the four part products accumulate in FP32 by weight
+// (h h | h l + l h | l l).  Where the rows of the right-hand sides differ by more
+// than 2^13 in their means, as they do for column-scaled factors, large values
+// of one operand meet small ones of the other and that is not enough: such a
+// product of 64 columns of K is made on the FP32 pipe (kTSpread).
 //
 // Measured, LU solve of 64 columns with the inverses made (ms): n = 2000 0.26,
 // 6000 0.85, 12000 2.01; work items of 64-row blocks claimed by persistent CTAs,
@@ -387,10 +391,10 @@ __device__ __forceinline__ void tri_cluster_sync() {
 __device__ __forceinline__ uint32_t tri_swz(int row, int kr) {
   return (uint32_t)row * 128u + (uint32_t)((((kr >> 3) ^ (row & 7)) << 4) + (kr & 7) * 2);
 }
-// exponent e, |e| <= 126, with |x| 2^-e < 4 for every |x| up to the one with bits mx, which
-// stays at 2^-1 or above where it is normal (0 for zero and non-finite maxima)
+// exponent e, |e| <= 126, with |x| 2^-e < 2^15 for every |x| up to the one with bits mx, which
+// stays at 2^14 or above where e allows (0 for zero and non-finite maxima)
 __device__ __forceinline__ int tri_exp(unsigned mx) {
-  return mx == 0u || mx >= 0x7F800000u ? 0 : min(max((int)(mx >> 23), 1) - 126, 126);
+  return mx == 0u || mx >= 0x7F800000u ? 0 : max((int)(mx >> 23) - 141, -126);
 }
 __device__ __forceinline__ float tri_pow2(int e) { return __int_as_float((127 + e) << 23); }   // |e| <= 126
 // (x, y) times sc as h + 2^-11 l, two fp16 pairs: the difference is exact
@@ -440,11 +444,20 @@ __device__ __forceinline__ void tri_store_tile(const float2 (&v)[16][2], unsigne
 
 // The B operand from 64 x 32 values, this thread's rows 8 warp .. + 7 of column
 // lane: rows 2c and 2c + 1 of B'^T hold (re, -im) and (im, re) of column c.
+// rmean: the means of the rows' exponents over nonzero finite values (0: none).
 __device__ __forceinline__ void tri_store_rhs(const float2 (&x)[8], unsigned char* bbuf, unsigned* cmax, int* cexp,
-                                              int warp, int lane) {
+                                              int* rmean, int warp, int lane) {
   unsigned mx = 0;
+  unsigned sum = 0;   // of row lane: exponents, and 2^16 for each
 #pragma unroll
-  for (int i = 0; i < 8; ++i) mx = max(mx, max(__float_as_uint(fabsf(x[i].x)), __float_as_uint(fabsf(x[i].y))));
+  for (int i = 0; i < 8; ++i) {
+    const unsigned m = max(__float_as_uint(fabsf(x[i].x)), __float_as_uint(fabsf(x[i].y)));
+    mx = max(mx, m);
+    const unsigned si = __reduce_add_sync(0xffffffffu, m - 0x00800000u < 0x7F000000u ? 0x10000u + (m >> 23) : 0u);
+    if (lane == i) sum = si;
+  }
+  if (lane < 8)
+    rmean[8 * warp + lane] = sum ? __float2int_rn(__fdividef((float)(sum & 0xFFFFu), (float)(sum >> 16))) : 0;
   cmax[warp * 32 + lane] = mx;
   __syncthreads();
 #pragma unroll
@@ -471,6 +484,43 @@ __device__ __forceinline__ void tri_store_rhs(const float2 (&x)[8], unsigned cha
     *reinterpret_cast<uint4*>(base + tri_swz(2 * lane + 1, kr)) = make_uint4(h1[0], h1[1], h1[2], h1[3]);
     *reinterpret_cast<uint4*>(base + tri_swz(64 + 2 * lane, kr)) = make_uint4(l0[0], l0[1], l0[2], l0[3]);
     *reinterpret_cast<uint4*>(base + tri_swz(64 + 2 * lane + 1, kr)) = make_uint4(l1[0], l1[1], l1[2], l1[3]);
+  }
+}
+// Whether the FP32 pipe takes a product: the means differ by more than kTSpread
+// (up to there the error of a product is at most 2^-50 2^13 of the sum of its
+// terms' sizes, well within FP32's; a single large right-hand side leaves the
+// means as they are), or a row of the factor is so near the ends of FP32's range
+// that tri_read's sums of up to 2^38 would leave it on the way.
+constexpr int kTSpread = 13;
+__device__ __forceinline__ bool tri_rows_differ(const int* rmean, const int* rexp, int lane) {
+  bool ends = false;
+#pragma unroll
+  for (int i = 0; i < 4; ++i) ends = ends || abs(rexp[lane + 32 * i]) > 88;
+  const int m0 = rmean[lane], m1 = rmean[lane + 32];
+  const int hi = __reduce_max_sync(0xffffffffu, max(m0, m1));
+  const int lo = __reduce_min_sync(0xffffffffu, min(m0 ? m0 : 255, m1 ? m1 : 255));
+  return hi - lo > kTSpread || __any_sync(0xffffffffu, ends);
+}
+
+// acc (laid out as tri_read's) += the 128 x 64 tile at A (rows < rn, columns < cn) times the 64 x 32 values
+// xs, on the FP32 pipe
+__device__ __noinline__ void tri_plain(float* acc, const float2* __restrict__ A, int64_t lda, int rn, int cn,
+                                       const float2* xs, int warp, int lane) {
+  const int row = 32 * (warp & 3) + lane, c0 = 16 * (warp >> 2);
+  if (row >= rn) return;
+  const float2* a = A + (int64_t)row * lda;
+  float2 s[16];
+#pragma unroll
+  for (int c = 0; c < 16; ++c) s[c] = make_float2(0.f, 0.f);
+  for (int k = 0; k < min(kTK, cn); ++k) {
+    const float2 t = a[k];
+#pragma unroll
+    for (int c = 0; c < 16; ++c) cfma(s[c], t, xs[k * kTC + c0 + c]);
+  }
+#pragma unroll
+  for (int c = 0; c < 16; ++c) {
+    acc[2 * c] += s[c].x;
+    acc[2 * c + 1] += s[c].y;
   }
 }
 
@@ -573,7 +623,8 @@ tri_operand_kernel(const float2* __restrict__ Inv, const float2* __restrict__ re
 template <bool UPPER, bool SPLIT>
 __global__ void __launch_bounds__(kTThreads, 2)
 tri_step_kernel(const float2* __restrict__ F, int64_t ldf, const unsigned char* __restrict__ ops,
-                const int* __restrict__ exps, float2* X, int64_t ldx, int n, int ncols, int src, int first,
+                const int* __restrict__ exps, const float2* __restrict__ inv, const float2* __restrict__ refined,
+                const float* __restrict__ cond, float2* X, int64_t ldx, int n, int ncols, int src, int first,
                 int* status) {
   using namespace tc;
   extern __shared__ __align__(1024) unsigned char smem_raw[];
@@ -582,6 +633,7 @@ tri_step_kernel(const float2* __restrict__ F, int64_t ldf, const unsigned char* 
   float2* fresh = reinterpret_cast<float2*>(bbuf + 2 * kTSlice);   // 32 rows x 32 columns
   __shared__ int rexp[128], cexp[kTC];
   __shared__ unsigned cmax[8 * 32];
+  __shared__ int rmean[kTK];
   __shared__ uint64_t bar, bar_inv;
   __shared__ uint32_t tmem_slot;
   __shared__ int abort_flag;
@@ -647,9 +699,10 @@ tri_step_kernel(const float2* __restrict__ F, int64_t ldf, const unsigned char* 
   float acc[32];
 #pragma unroll
   for (int j = 0; j < 32; ++j) acc[j] = 0.f;
-  // acc += (the tile in abuf) x (the right-hand sides in x)
-  auto product = [&](bool inverse) {
-    tri_store_rhs(x, bbuf, cmax, cexp, warp, lane);
+  // (the tile in abuf: the factor's columns from k0 on, or the inverse's) x (the right-hand sides in x), in tensor
+  // memory; or true, and acc += it
+  auto product = [&](bool inverse, int k0) -> bool {
+    tri_store_rhs(x, bbuf, cmax, cexp, rmean, warp, lane);
     fence_async_smem();
     tc_fence_before();
     __syncthreads();
@@ -660,9 +713,28 @@ tri_step_kernel(const float2* __restrict__ F, int64_t ldf, const unsigned char* 
       tri_issue(tmem, abuf, bbuf);
       mma_commit(&bar);
     }
+    const bool differ = tri_rows_differ(rmean, rexp, lane);   // (beside the products)
     if (!mbar_wait(&bar, phase, &abort_flag)) mbar_wait_plain(&bar, phase);
     phase ^= 1;
     tc_fence_after();
+    if (differ) {
+      float2* xs = reinterpret_cast<float2*>(bbuf);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) xs[(8 * warp + i) * kTC + lane] = x[i];
+      __syncthreads();
+      float part[32];
+#pragma unroll
+      for (int j = 0; j < 32; ++j) part[j] = acc[j];
+      if (inverse)
+        tri_plain(part,
+                  (cond[next] <= kTCond ? inv : refined) + (int64_t)next * kTD * kTD + (int64_t)half * 128 * kTD + kq * kTK,
+                  kTD, 128, kTK, xs, warp, lane);
+      else
+        tri_plain(part, F + (int64_t)row0 * ldf + k0, ldf, n - row0, n - k0, xs, warp, lane);
+#pragma unroll
+      for (int j = 0; j < 32; ++j) acc[j] = part[j];
+    }
+    return differ;
   };
   // the products of a CTA whose wait ran out are NaN, and so are the block rows made of them
   auto poison = [&]() {
@@ -686,9 +758,9 @@ tri_step_kernel(const float2* __restrict__ F, int64_t ldf, const unsigned char* 
         const int k = k0 + 8 * warp + i;
         x[i] = k < n && cg + lane < ncols ? ldcg(X + (int64_t)k * ldx + cg + lane) : make_float2(0.f, 0.f);
       }
-      product(false);
+      const bool made = product(false, k0);
       if (!alone && cl == 0) load_inverse();   // the tile's products are done
-      tri_read(acc, tmem, rexp, cexp, warp, lane);
+      if (!made) tri_read(acc, tmem, rexp, cexp, warp, lane);
       poison();
       tc_fence_before();
       if (!alone || q == 3) break;
@@ -745,10 +817,9 @@ tri_step_kernel(const float2* __restrict__ F, int64_t ldf, const unsigned char* 
                             (uint32_t)((8 * (warp & 3) * kTC + lane) * 8);
 #pragma unroll
       for (int i = 0; i < 8; ++i) x[i] = tri_ld2(from + (uint32_t)(i * kTC * 8));
-      product(true);
 #pragma unroll
       for (int j = 0; j < 32; ++j) acc[j] = 0.f;
-      tri_read(acc, tmem, rexp, cexp, warp, lane);
+      if (!product(true, 0)) tri_read(acc, tmem, rexp, cexp, warp, lane);
       poison();
       tc_fence_before();
       __syncthreads();
@@ -792,8 +863,9 @@ struct TriWs {
 size_t tri_solve_workspace_bytes(int64_t n) { return TriWs(n).total; }
 
 template <bool UPPER>
-static int tri_steps(const float2* F, int64_t ldf, const unsigned char* ops, const int* exps, float2* X, int64_t ldx,
-                     int n, int nrhs, int* status, cudaStream_t s) {
+static int tri_steps(const float2* F, int64_t ldf, const unsigned char* ops, const int* exps, const float2* inv,
+                     const float2* refined, const float* cond, float2* X, int64_t ldx, int n, int nrhs, int* status,
+                     cudaStream_t s) {
   const int nb = (n + kTD - 1) / kTD, ng = (nrhs + kTC - 1) / kTC, sms = device_sm_count();
   for (int i = 0; i < nb; ++i) {
     // step i solves block row i (from the end for U) after updating it and all that follow
@@ -821,7 +893,7 @@ static int tri_steps(const float2* F, int64_t ldf, const unsigned char* ops, con
     cfg.numAttrs = UPPER || i > 0 ? 2 : 1;
     count_launch();
     if (cudaLaunchKernelEx(&cfg, split ? tri_step_kernel<UPPER, true> : tri_step_kernel<UPPER, false>, F, ldf, ops, exps,
-                           X, ldx, n, nrhs, src, first, status) != cudaSuccess)
+                           inv, refined, cond, X, ldx, n, nrhs, src, first, status) != cudaSuccess)
       return MGT_ERR_CUDA;
   }
   return MGT_OK;
@@ -863,10 +935,11 @@ int tri_solve(const float2* F, int64_t ldf, float2* X, int64_t ldx, int n, int n
     tri_newton_kernel<<<dim3(nb * 16, 2), 512, kTNewtonSmem, s>>>(F, ldf, n, nb, inv, cond, refined);
     tri_operand_kernel<<<nb * 16, kTThreads, 0, s>>>(inv, refined, cond, ops, exps);
   }
-  int e = tri_steps<false>(F, ldf, ops, exps, X, ldx, n, nrhs, status, s);
+  const size_t upper = (size_t)nb * kTD * kTD;
+  int e = tri_steps<false>(F, ldf, ops, exps, inv, refined, cond, X, ldx, n, nrhs, status, s);
   if (e == MGT_OK)
-    e = tri_steps<true>(F, ldf, ops + (size_t)nb * 8 * 4 * kTSlice, exps + (size_t)nb * 8 * 128, X, ldx, n, nrhs,
-                        status, s);
+    e = tri_steps<true>(F, ldf, ops + (size_t)nb * 8 * 4 * kTSlice, exps + (size_t)nb * 8 * 128, inv + upper,
+                        refined + upper, cond + nb, X, ldx, n, nrhs, status, s);
   if (e != MGT_OK) return e;
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }
