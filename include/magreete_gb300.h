@@ -265,9 +265,15 @@ int mgt_solve_refined(const void* M, int64_t ldm, const void* LU, int64_t ldlu,
  * to mgt_refine_prepare, for any nrhs): everything else is in `work`, of
  * mgt_refine_scratch_bytes(n, nrhs) bytes, so that right-hand sides wider than
  * the prepared workspace was sized for are solved in one block.  `prepared`
- * is only read.
+ * is only read.  Every `group` columns (mgt_solve_prepared: 64) are held to tol
+ * by themselves, as if solved one group at a time; rel_res is that of all columns
+ * where each group meets tol, else the largest of a group.
  */
 int mgt_refine_scratch_bytes(int64_t n, int64_t nrhs, size_t* bytes);
+int mgt_solve_prepared_groups(const void* prepared, const void* LU, int64_t ldlu, const int32_t* perm, int64_t n,
+                              const void* B, int64_t ldb, void* X, int64_t ldx, int64_t nrhs, int64_t group,
+                              double tol, int max_iter, void* work, size_t work_bytes, int* iters, double* rel_res,
+                              void* stream);
 int mgt_solve_prepared(const void* prepared, const void* LU, int64_t ldlu, const int32_t* perm, int64_t n,
                        const void* B, int64_t ldb, void* X, int64_t ldx, int64_t nrhs, double tol, int max_iter,
                        void* work, size_t work_bytes, int* iters, double* rel_res, void* stream);

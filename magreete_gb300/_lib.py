@@ -80,6 +80,8 @@ SIGNATURES = {
     "mgt_refine_scratch_bytes": (_i32, [_i64, _i64, ctypes.POINTER(_sz)]),
     "mgt_solve_prepared": (_i32, [_vp, _vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _i64, _f64, _i32, _vp, _sz,
                                   ctypes.POINTER(_i32), ctypes.POINTER(_f64), _vp]),
+    "mgt_solve_prepared_groups": (_i32, [_vp, _vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _i64, _i64, _f64, _i32, _vp,
+                                         _sz, ctypes.POINTER(_i32), ctypes.POINTER(_f64), _vp]),
     "mgt_refine_start": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _i64, _vp, _sz, _vp]),
     "mgt_refine_correct": (_i32, [_vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _vp, _i64, _i64, _vp, _sz, _vp]),
     "mgt_refine_norms": (_i32, [_vp, _i64, _i64, _vp, _i64, _vp, _i64, _i64, _vp, _sz, _vp, _vp]),

@@ -7,7 +7,10 @@
 // recovers FP64 accuracy: x += LU^-1 (b - M x), with the residual formed in
 // double-float arithmetic from a double-float copy of M.
 #include <algorithm>
+#include <limits>
+#include <memory>
 #include <mutex>
+#include <new>
 
 #include "common.cuh"
 #include "df.cuh"
@@ -123,7 +126,11 @@ __global__ void c64_into_c128_kernel(const float2* __restrict__ Y, int64_t ldy, 
 }
 
 // out[slot] += sum |X|^2 (slot 0 or 1); FP64 accumulation per thread, then atomics
-__global__ void sumsq_kernel(const double2* __restrict__ X, int64_t ldx, int n, int ncols, double* out) {
+// out[g] += ||X_g||_F^2 of each group g (blockIdx.y) of `group` columns
+__global__ void sumsq_kernel(const double2* __restrict__ X, int64_t ldx, int n, int ncols, int group, double* out) {
+  X += (int64_t)blockIdx.y * group;
+  ncols = min(group, ncols - (int)blockIdx.y * group);
+  out += blockIdx.y;
   double s = 0.0;
   int64_t total = (int64_t)n * ncols;
   for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total;
@@ -142,6 +149,14 @@ __global__ void sumsq_kernel(const double2* __restrict__ X, int64_t ldx, int n, 
     for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += red[w];
     atomicAdd(out, t);
   }
+}
+
+static void launch_sumsq(const double2* X, int64_t ldx, int n, int ncols, int group, double* out, cudaStream_t s) {
+  const int groups = (ncols + group - 1) / group;
+  const int64_t blocks = ((int64_t)n * std::min(group, ncols) + 255) / 256;
+  count_launch();
+  sumsq_kernel<<<dim3((unsigned)std::min<int64_t>(std::max(1, 1024 / groups), blocks), groups), 256, 0, s>>>(
+      X, ldx, n, ncols, group, out);
 }
 
 template <int RT>
@@ -285,7 +300,7 @@ struct RefineWs {
   double2* Rr;    // n x nrhs residual
   float2* R32;    // n x nrhs complex64 residual / right-hand side
   float2* D32;    // n x nrhs complex64 correction
-  double* norms;  // [0] = ||B||^2, [1] = ||R||^2
+  double* norms;  // ||B||^2 of each group of columns, then ||R||^2 (at most a group per column)
   void* tri;      // triangular solves: inverted diagonal blocks
   double2* part;  // (double-float residual) split-K partial sums
   int64_t part_elems;
@@ -319,7 +334,7 @@ struct RefineWs {
     Rr = (double2*)take(n * r * sizeof(double2));
     R32 = (float2*)take(n * r * sizeof(float2));
     D32 = (float2*)take(n * r * sizeof(float2));
-    norms = (double*)take(2 * sizeof(double));
+    norms = (double*)take(2 * r * sizeof(double));
     tri = take(tri_solve_workspace_bytes(n));
     Xs = nullptr;
     part = nullptr;
@@ -429,10 +444,10 @@ extern "C" int mgt_refine_workspace_bytes(int64_t n, int64_t nrhs, size_t* bytes
 
 static int solve_refined(const void* M, int64_t ldm, const void* prepared, const void* LU, int64_t ldlu,
                          const int32_t* perm, int64_t n, const void* B, int64_t ldb, void* X, int64_t ldx,
-                         int64_t nrhs, double tol, int max_iter, void* work, size_t work_bytes, int* iters,
-                         double* rel_res, void* stream) {
+                         int64_t nrhs, int64_t group, double tol, int max_iter, void* work, size_t work_bytes,
+                         int* iters, double* rel_res, void* stream) {
   if (!LU || !perm || !B || !X || !work || n <= 0 || nrhs <= 0 || (M && ldm < n) || ldlu < n || ldb < nrhs ||
-      ldx < nrhs || max_iter < 0)
+      ldx < nrhs || max_iter < 0 || group <= 0)
     return MGT_ERR_ARG;
   RefineWs w(work, n, nrhs, prepared);
   if (!M && !w.tc) return MGT_ERR_ARG;   // prepared digits exist only for the tensor-core residual
@@ -443,10 +458,14 @@ static int solve_refined(const void* M, int64_t ldm, const void* prepared, const
   const unsigned eg = (unsigned)((tot + 255) / 256);
   const double2* Bd = (const double2*)B;
   double2* Xd = (double2*)X;
-  double h[2];
-  if (cudaMemsetAsync(w.norms, 0, 2 * sizeof(double), s) != cudaSuccess) return MGT_ERR_CUDA;
-  count_launch();
-  sumsq_kernel<<<std::min<int64_t>(1024, (tot + 255) / 256), 256, 0, s>>>(Bd, ldb, nn, nr, w.norms);
+  // every group of columns is held to tol by itself, so that a group of small
+  // right-hand sides is not lost beside larger ones
+  const int gc = (int)std::max(std::min(group, nrhs), (nrhs + 65534) / 65535), ng = (nr + gc - 1) / gc;
+  const std::unique_ptr<double[]> host(new (std::nothrow) double[3 * (size_t)ng]);
+  if (!host) return MGT_ERR_CUDA;
+  double *h = host.get(), *prev = h + 2 * ng;   // ||B||^2, ||R||^2; the last relative residuals
+  if (cudaMemsetAsync(w.norms, 0, ng * sizeof(double), s) != cudaSuccess) return MGT_ERR_CUDA;
+  launch_sumsq(Bd, ldb, nn, nr, gc, w.norms, s);
   // x0 = LU^-1 b in complex64
   count_launch();
   c128_to_c64_kernel<<<eg, 256, 0, s>>>(Bd, ldb, w.R32, nr, nn, nr);
@@ -454,32 +473,49 @@ static int solve_refined(const void* M, int64_t ldm, const void* prepared, const
   if (e != MGT_OK) return e;
   count_launch();
   c64_into_c128_kernel<<<eg, 256, 0, s>>>(w.D32, nr, Xd, ldx, nn, nr, 1);
-  double prev = 0.0, rel = 0.0;
+  double rel = 0.0;
   int it = 0;
   int dev_status = MGT_OK;
+  bool met = false;
   for (;; ++it) {
     e = w.residual((const float4*)M, ldm, Xd, ldx, Bd, ldb, nn, nr, it > 0 || !M, s);
     if (e != MGT_OK) return e;
-    if (cudaMemsetAsync(w.norms + 1, 0, sizeof(double), s) != cudaSuccess) return MGT_ERR_CUDA;
-    count_launch();
-    sumsq_kernel<<<std::min<int64_t>(1024, (tot + 255) / 256), 256, 0, s>>>(w.Rr, nr, nn, nr, w.norms + 1);
-    if (cudaMemcpyAsync(h, w.norms, 2 * sizeof(double), cudaMemcpyDeviceToHost, s) != cudaSuccess) return MGT_ERR_CUDA;
+    if (cudaMemsetAsync(w.norms + ng, 0, ng * sizeof(double), s) != cudaSuccess) return MGT_ERR_CUDA;
+    launch_sumsq(w.Rr, nr, nn, nr, gc, w.norms + ng, s);
+    if (cudaMemcpyAsync(h, w.norms, 2 * ng * sizeof(double), cudaMemcpyDeviceToHost, s) != cudaSuccess)
+      return MGT_ERR_CUDA;
     if (w.status() &&
         cudaMemcpyAsync(&dev_status, w.status(), sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess)
       return MGT_ERR_CUDA;
     if (cudaStreamSynchronize(s) != cudaSuccess) return MGT_ERR_CUDA;
     if (dev_status != MGT_OK) return dev_status;
-    rel = h[0] > 0 ? sqrt(h[1] / h[0]) : sqrt(h[1]);
-    if (rel != rel) {
+    // rel: of all columns where every group meets tol, else of the worst group
+    double b2 = 0.0, r2 = 0.0, worst = 0.0;
+    bool better = false, bad = false;
+    met = true;
+    for (int g = 0; g < ng; ++g) {
+      const double r = h[g] > 0 ? sqrt(h[ng + g] / h[g]) : sqrt(h[ng + g]);
+      b2 += h[g];
+      r2 += h[ng + g];
+      if (r != r) bad = true;
+      if (!(r <= tol)) {
+        met = false;
+        if (it == 0 || r < 0.9 * prev[g]) better = true;
+      }
+      if (!(r <= worst)) worst = r;
+      prev[g] = r;
+    }
+    rel = !met ? worst : b2 > 0 ? sqrt(r2 / b2) : sqrt(r2);
+    if (bad) {
+      rel = std::numeric_limits<double>::quiet_NaN();
       // a solve step whose wait ran out leaves NaN and says so (read only here: the copy costs a correction 5 us)
       if (cudaMemcpyAsync(&dev_status, w.tri_status(), sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
           cudaStreamSynchronize(s) != cudaSuccess)
         return MGT_ERR_CUDA;
       if (dev_status != MGT_OK) return dev_status;
     }
-    if (rel <= tol || it >= max_iter) break;
-    if (it > 0 && !(rel < 0.9 * prev)) break;  // stagnation or divergence
-    prev = rel;
+    if (met || it >= max_iter) break;
+    if (!better) break;   // stagnation or divergence of every group that is left
     count_launch();
     c128_to_c64_kernel<<<eg, 256, 0, s>>>(w.Rr, nr, w.R32, nr, nn, nr);
     e = lu_solve_c64((const float2*)LU, nn, ldlu, perm, w.R32, w.D32, nr, w.tri, true, s);
@@ -490,14 +526,14 @@ static int solve_refined(const void* M, int64_t ldm, const void* prepared, const
   if (iters) *iters = it;
   if (rel_res) *rel_res = rel;
   if (cudaGetLastError() != cudaSuccess) return MGT_ERR_CUDA;
-  return (rel <= tol && rel == rel) ? MGT_OK : MGT_ERR_NOT_CONVERGED;
+  return met ? MGT_OK : MGT_ERR_NOT_CONVERGED;
 }
 
 extern "C" int mgt_solve_refined(const void* M, int64_t ldm, const void* LU, int64_t ldlu, const int32_t* perm,
                                  int64_t n, const void* B, int64_t ldb, void* X, int64_t ldx, int64_t nrhs,
                                  double tol, int max_iter, void* work, size_t work_bytes, int* iters,
                                  double* rel_res, void* stream) {
-  return solve_refined(M, ldm, nullptr, LU, ldlu, perm, n, B, ldb, X, ldx, nrhs, tol, max_iter, work, work_bytes,
+  return solve_refined(M, ldm, nullptr, LU, ldlu, perm, n, B, ldb, X, ldx, nrhs, nrhs, tol, max_iter, work, work_bytes,
                        iters, rel_res, stream);
 }
 
@@ -508,13 +544,21 @@ extern "C" int mgt_refine_scratch_bytes(int64_t n, int64_t nrhs, size_t* bytes) 
   return MGT_OK;
 }
 
+extern "C" int mgt_solve_prepared_groups(const void* prepared, const void* LU, int64_t ldlu, const int32_t* perm,
+                                         int64_t n, const void* B, int64_t ldb, void* X, int64_t ldx, int64_t nrhs,
+                                         int64_t group, double tol, int max_iter, void* work, size_t work_bytes,
+                                         int* iters, double* rel_res, void* stream) {
+  if (!prepared) return MGT_ERR_ARG;
+  return solve_refined(nullptr, 0, prepared, LU, ldlu, perm, n, B, ldb, X, ldx, nrhs, group, tol, max_iter, work,
+                       work_bytes, iters, rel_res, stream);
+}
+
 extern "C" int mgt_solve_prepared(const void* prepared, const void* LU, int64_t ldlu, const int32_t* perm, int64_t n,
                                   const void* B, int64_t ldb, void* X, int64_t ldx, int64_t nrhs, double tol,
                                   int max_iter, void* work, size_t work_bytes, int* iters, double* rel_res,
                                   void* stream) {
-  if (!prepared) return MGT_ERR_ARG;
-  return solve_refined(nullptr, 0, prepared, LU, ldlu, perm, n, B, ldb, X, ldx, nrhs, tol, max_iter, work, work_bytes,
-                       iters, rel_res, stream);
+  return mgt_solve_prepared_groups(prepared, LU, ldlu, perm, n, B, ldb, X, ldx, nrhs, 64, tol, max_iter, work,
+                                   work_bytes, iters, rel_res, stream);
 }
 
 // ---------------------------------------------------------------- DOS dots
@@ -616,9 +660,7 @@ extern "C" int mgt_refine_norms(const void* M, int64_t ldm, int64_t n, const voi
   int e = w.residual((const float4*)M, ldm, (const double2*)X, ldx, (const double2*)B, ldb, nn, nr, !M, s);
   if (e != MGT_OK) return e;
   if (cudaMemsetAsync(norms_dev, 0, 2 * sizeof(double), s) != cudaSuccess) return MGT_ERR_CUDA;
-  count_launch(2);
-  sumsq_kernel<<<(unsigned)std::min<int64_t>(1024, (tot + 255) / 256), 256, 0, s>>>((const double2*)B, ldb, nn, nr,
-                                                                                   norms_dev);
-  sumsq_kernel<<<(unsigned)std::min<int64_t>(1024, (tot + 255) / 256), 256, 0, s>>>(w.Rr, nr, nn, nr, norms_dev + 1);
+  launch_sumsq((const double2*)B, ldb, nn, nr, nr, norms_dev, s);
+  launch_sumsq(w.Rr, nr, nn, nr, nr, norms_dev + 1, s);
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }

@@ -227,8 +227,10 @@ class RefineContext:
 def solve_refined(M, f, B, tol=DEFAULT_TOL, max_iter=DEFAULT_MAX_ITER, require=True):
     """Refined solve of M X = B (B complex128 n x R) with complex64 factors f.
     M: the double-float matrix, or a RefineContext (right-hand sides wider
-    than it was prepared for are solved in blocks of up to WIDE_NRHS columns).  Returns
-    (X, iterations, rel_residual)."""
+    than it was prepared for are solved in blocks of up to WIDE_NRHS columns,
+    in which every max_nrhs columns are held to tol by themselves).  Returns (X,
+    iterations, rel_residual): the relative residual of all columns, or the
+    largest of a block or group that did not reach tol."""
     if isinstance(M, RefineContext):
         if M.work is None:
             return solve_refined(M.Mdf, f, B, tol, max_iter, require)
@@ -272,26 +274,30 @@ def _solve_prepared(ctx, f, B, tol, max_iter, require):
         nbytes = ctypes.c_size_t()
         L.check(lib.mgt_refine_scratch_bytes(n, width, ctypes.byref(nbytes)), "mgt_refine_scratch_bytes")
         work = workspace(nbytes.value, B.device)
-    its, sq = [], 0.0
+    its, sq, missed = [], 0.0, 0.0
     for c0 in range(0, R, width):
         Bc = B if width >= R else B[:, c0:c0 + width].contiguous()
         Xc = X if width >= R else torch.empty_like(Bc)
         rc = Bc.shape[1]
         it = ctypes.c_int(0)
         rr = ctypes.c_double(0.0)
-        args = (_ptr(f.lu), f.lu.stride(0), _ptr(f.perm), n, _ptr(Bc), rc, _ptr(Xc), rc, rc, float(tol), int(max_iter),
-                _ptr(work), work.numel(), ctypes.byref(it), ctypes.byref(rr), _stream())
+        args = (_ptr(f.lu), f.lu.stride(0), _ptr(f.perm), n, _ptr(Bc), rc, _ptr(Xc), rc, rc)
+        rest = (float(tol), int(max_iter), _ptr(work), work.numel(), ctypes.byref(it), ctypes.byref(rr), _stream())
         if work is ctx.work:
-            st = lib.mgt_solve_refined(None, n, *args)
+            st = lib.mgt_solve_refined(None, n, *args, *rest)
         else:
-            st = lib.mgt_solve_prepared(_ptr(ctx.work), *args)
-        if not (st == L.MGT_ERR_NOT_CONVERGED and not require):
+            st = lib.mgt_solve_prepared_groups(_ptr(ctx.work), *args, ctx.max_nrhs, *rest)
+        if st == L.MGT_ERR_NOT_CONVERGED and not require:
+            missed = max(missed, rr.value) if rr.value == rr.value else float("inf")
+        else:
             L.check(st, f"mgt_solve_refined (iterations {it.value}, relative residual {rr.value:.3e})")
         its.append(it.value)
         if rc == R:
             return X, it.value, rr.value
         X[:, c0:c0 + rc] = Xc
         sq += (rr.value * torch.linalg.norm(Bc).item()) ** 2
+    if missed > 0:
+        return X, max(its), missed
     nb = torch.linalg.norm(B).item()
     return X, max(its), (sq ** 0.5 / nb if nb > 0 else sq ** 0.5)
 
