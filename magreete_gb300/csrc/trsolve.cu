@@ -936,10 +936,15 @@ int tri_solve(const float2* F, int64_t ldf, float2* X, int64_t ldx, int n, int n
     tri_operand_kernel<<<nb * 16, kTThreads, 0, s>>>(inv, refined, cond, ops, exps);
   }
   const size_t upper = (size_t)nb * kTD * kTD;
-  int e = tri_steps<false>(F, ldf, ops, exps, inv, refined, cond, X, ldx, n, nrhs, status, s);
-  if (e == MGT_OK)
-    e = tri_steps<true>(F, ldf, ops + (size_t)nb * 8 * 4 * kTSlice, exps + (size_t)nb * 8 * 128, inv + upper,
-                        refined + upper, cond + nb, X, ldx, n, nrhs, status, s);
+  int e = MGT_OK;
+  constexpr int kCols = 65535 * kTC;   // columns of one launch
+  for (int64_t c0 = 0; c0 < nrhs && e == MGT_OK; c0 += kCols) {
+    const int nc = (int)std::min<int64_t>(kCols, nrhs - c0);
+    e = tri_steps<false>(F, ldf, ops, exps, inv, refined, cond, X + c0, ldx, n, nc, status, s);
+    if (e == MGT_OK)
+      e = tri_steps<true>(F, ldf, ops + (size_t)nb * 8 * 4 * kTSlice, exps + (size_t)nb * 8 * 128, inv + upper,
+                          refined + upper, cond + nb, X + c0, ldx, n, nc, status, s);
+  }
   if (e != MGT_OK) return e;
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
 }

@@ -119,13 +119,18 @@ diag_kernel(const double2* __restrict__ Inv, int upper, double2* __restrict__ X,
   }
 }
 
+// Columns solved together: the digits of a block row of right-hand sides take 3.5 KB a
+// column, and from some thousand columns on the chain of block rows is no longer
+// what a solve waits for.
+constexpr int64_t kCols = 16384;
+
 struct Ws {
   size_t status = kStatusOffset, stats = 256, inv, plan, total;   // stats: 4 TB ints per block row and triangle
   Ws(int64_t n, int64_t nrhs) {
     const int64_t nb = (n + TB - 1) / TB;
     inv = (stats + (size_t)(2 * nb * 4 * TB) * sizeof(int) + 255) & ~size_t(255);
     plan = inv + (size_t)(2 * nb) * TB * TB * sizeof(double2);
-    total = plan + zgemm_bytes(n, nrhs);
+    total = plan + zgemm_bytes(n, std::min(nrhs, kCols));
   }
 };
 
@@ -133,21 +138,11 @@ struct Ws {
 
 size_t zsolve_workspace_bytes(int64_t n, int64_t nrhs) { return zs::Ws(n, nrhs).total; }
 
-int zsolve(const double2* F, int64_t ldf, double2* X, int64_t ldx, int n, int nrhs, void* work, cudaStream_t s) {
+// X = U^-1 L^-1 X for at most kCols columns; stats: zeros
+static int solve_columns(const double2* F, int64_t ldf, double2* X, int64_t ldx, int n, int nrhs, const double2* inv,
+                         int* stats, int* status, const ZGemmPlan& plan, cudaStream_t s) {
   using namespace zs;
-  static OncePerDevice once;
-  const size_t smem = (size_t)TB * LD * sizeof(double2);
-  once([smem] { cudaFuncSetAttribute(inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); });
-  const Ws L(n, nrhs);
   const int nb = (n + TB - 1) / TB;
-  int* status = (int*)((char*)work + L.status);
-  int* stats = (int*)((char*)work + L.stats);
-  double2* inv = (double2*)((char*)work + L.inv);
-  ZGemmPlan plan;
-  plan.init((char*)work + L.plan, n, nrhs);
-  if (cudaMemsetAsync(work, 0, L.inv, s) != cudaSuccess) return MGT_ERR_CUDA;   // status, sizes of rows
-  count_launch();
-  inverse_kernel<<<dim3(nb, 8, 2), 256, smem, s>>>(F, ldf, n, inv);
   for (int step = 0; step < 2 * nb; ++step) {
     const bool upper = step >= nb;
     const int i = upper ? 2 * nb - 1 - step : step, r0 = i * TB, rb = std::min(TB, n - r0);
@@ -166,6 +161,29 @@ int zsolve(const double2* F, int64_t ldf, double2* X, int64_t ldx, int n, int nr
     int e = zgemm_digits(plan, Fi, ldf, m, Xi, ldx, nrhs, rb, rows, s);
     if (e == MGT_OK)
       e = zgemm_apply(plan, Fi, ldf, m, Xi, ldx, nrhs, rb, X + (int64_t)q0 * ldx, ldx, ZOut::SUB, nullptr, status, s);
+    if (e != MGT_OK) return e;
+  }
+  return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
+}
+
+int zsolve(const double2* F, int64_t ldf, double2* X, int64_t ldx, int n, int nrhs, void* work, cudaStream_t s) {
+  using namespace zs;
+  static OncePerDevice once;
+  const size_t smem = (size_t)TB * LD * sizeof(double2);
+  once([smem] { cudaFuncSetAttribute(inverse_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem); });
+  const Ws L(n, nrhs);
+  const int nb = (n + TB - 1) / TB;
+  int* status = (int*)((char*)work + L.status);
+  int* stats = (int*)((char*)work + L.stats);
+  double2* inv = (double2*)((char*)work + L.inv);
+  ZGemmPlan plan;
+  plan.init((char*)work + L.plan, n, std::min<int64_t>(nrhs, kCols));
+  if (cudaMemsetAsync(work, 0, L.inv, s) != cudaSuccess) return MGT_ERR_CUDA;   // status, sizes of rows
+  count_launch();
+  inverse_kernel<<<dim3(nb, 8, 2), 256, smem, s>>>(F, ldf, n, inv);
+  for (int64_t c0 = 0; c0 < nrhs; c0 += kCols) {
+    if (c0 > 0 && cudaMemsetAsync(stats, 0, L.inv - L.stats, s) != cudaSuccess) return MGT_ERR_CUDA;
+    const int e = solve_columns(F, ldf, X + c0, ldx, n, (int)std::min<int64_t>(kCols, nrhs - c0), inv, stats, status, plan, s);
     if (e != MGT_OK) return e;
   }
   return cudaGetLastError() == cudaSuccess ? MGT_OK : MGT_ERR_CUDA;
