@@ -338,7 +338,10 @@ int mgt_column_dots(const void* A, int64_t lda, const void* B, int64_t ldb, int6
  * Tuning knobs of the LU (no counterpart in the reference), process-wide:
  *   MGT_TUNE_PANEL_ROWS  rows of the panel each CTA of the panel kernel aims
  *                        for (32..4096, default 256; the shared-memory limit
- *                        can raise the CTA count further)
+ *                        can raise the CTA count further).  complex128: at the
+ *                        default 32 where the panel is a cluster, a cooperative
+ *                        launch or bounded by PANEL_MAX_CTAS; another value
+ *                        applies as it is
  *   MGT_TUNE_OUTER_BLOCK outer block width of the complex64 tensor-core LU,
  *                        64 or 128 (default 128: two inner panels per block)
  *   MGT_TUNE_PANEL_MAX_CTAS  upper bound on the panel kernel's CTAs (0: one per SM)
@@ -347,9 +350,11 @@ int mgt_column_dots(const void* A, int64_t lda, const void* B, int64_t ldb, int6
  *                        where the caller keeps the CTAs of all panels that may
  *                        run at once within the SM count (every panel CTA
  *                        then finds an SM and no panel waits on another)
- *   MGT_TUNE_PANEL_REGISTERS  panels with at most 256 rows per CTA keep one row
- *                        per thread in registers: 1 (default) for complex64,
- *                        2 for both types, 0 never (rows in shared memory)
+ *   MGT_TUNE_PANEL_REGISTERS  panels keep their rows in registers: 1 (default)
+ *                        complex64 one row a thread (at most 256 rows per CTA),
+ *                        complex128 one row over four threads (at most 128);
+ *                        2: one row a thread for both types; 0: never (rows in
+ *                        shared memory)
  *   MGT_TUNE_TC_PRECISION  split-product scheme of the complex64 tensor-core
  *                        update: MGT_TC_F16X2 (default; operands scaled by
  *                        powers of two, split into two fp16, kind::f16) or
@@ -364,10 +369,11 @@ int mgt_column_dots(const void* A, int64_t lda, const void* B, int64_t ldb, int6
  *                        panels' interchanges, solves with the inverted 64 x 64
  *                        diagonal blocks); 0: two swap passes and a pre-update
  *                        pass with substitution
- *   MGT_TUNE_PANEL_CLUSTER 1 (default): complex64 register panels of at most 16
- *                        CTAs (8 where the device schedules no larger cluster)
- *                        run as one thread-block cluster and exchange pivots
- *                        through distributed shared memory; 0: through L2
+ *   MGT_TUNE_PANEL_CLUSTER 1 (default): register panels of at most 16 CTAs (8
+ *                        where the device schedules no larger cluster; 64 rows
+ *                        a CTA in complex128) run as one thread-block cluster
+ *                        and exchange pivots through distributed shared
+ *                        memory; 0: through L2
  *   MGT_TUNE_SYM_ASSEMBLY 1 (default): mgt_assemble_system evaluates each pair
  *                        of points once and writes both mirror-image blocks
  *                        (bitwise the same matrix); 0: every block evaluated

@@ -2021,13 +2021,20 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
         const ZPanelWs zw{pw.status, pw.nslot, pw.slots, reinterpret_cast<unsigned long long*>(pw.records),
                           kMaxPanelBlocks};
         const int cap = opt.panel_max_ctas > 0 ? std::min(opt.panel_max_ctas, sms) : sms;
+        // rows per CTA: the caller's, else kZPanelRows.  A plain launch whose CTAs wait for one
+        // another needs the count that the caller reckons with: panel_rows', or at most
+        // panel_max_ctas; with neither given the kernel below keeps to 256 rows a CTA
+        // (a cluster's CTAs are placed together and need no such care)
+        const bool asked = opt.panel_rows != kPanelRowsTarget;
+        const int rows = asked ? opt.panel_rows : kZPanelRows;
+        const bool wide = opt.cooperative != 0 || asked || opt.panel_max_ctas > 0;
         // taller panels went to the kernel below: its records are no messages
-        if (!records_clear && zpanel_fits(m, cap)) {
+        if (!records_clear && zpanel_fits(m, rows, cap)) {
           if (cudaMemsetAsync(pw.records, 0, zpanel_words(kMaxPanelBlocks) * 8, s) != cudaSuccess) return MGT_ERR_CUDA;
           records_clear = true;
         }
-        const int e = zpanel_factor(A + (int64_t)j0 * lda + j0, lda, m, w, j0, perm, zw, kZPanelRows, cap,
-                                    opt.cooperative != 0, opt.panel_cluster != 0, s);
+        const int e = zpanel_factor(A + (int64_t)j0 * lda + j0, lda, m, w, j0, perm, zw, rows, cap,
+                                    opt.cooperative != 0, opt.panel_cluster != 0, wide, s);
         if (e != MGT_ERR_UNSUPPORTED) return e;
         records_clear = false;
       }

@@ -544,12 +544,13 @@ static int launch(double2* P, int64_t lda, int m, int w, int j0, int32_t* perm, 
 }  // namespace zp
 
 int zpanel_factor(double2* P, int64_t lda, int m, int w, int j0, int32_t* perm, const ZPanelWs& ws, int rows_target,
-                  int max_ctas, bool cooperative, bool allow_cluster, cudaStream_t s) {
+                  int max_ctas, bool cooperative, bool allow_cluster, bool allow_wide, cudaStream_t s) {
   using namespace zp;
   if (m <= 0 || w <= 0 || w > NB || m >= kNoPos || j0 + w > kMaxColumns) return MGT_ERR_UNSUPPORTED;
   const int c64 = max_cluster<64>();
   max_cluster<128>();   // sets its kernels' attributes
   const int cap = std::max(1, std::min(max_ctas, ws.max_ctas));
+  if (!zpanel_fits(m, rows_target, cap)) return MGT_ERR_UNSUPPORTED;
   // Up to 64 rows a CTA one cluster is fastest (1000 rows: 3.4 us a column against 4.5 through global
   // memory); with 128 rows its 16 SMs' FP64 pipes take longer than the wider exchange (5.6 against 4.8).
   if (allow_cluster) {
@@ -560,6 +561,7 @@ int zpanel_factor(double2* P, int64_t lda, int m, int w, int j0, int32_t* perm, 
         return launch<64, true>(P, lda, m, w, j0, perm, ws, (m + rpc - 1) / rpc, rpc, cooperative, s);
     }
   }
+  if (!allow_wide) return MGT_ERR_UNSUPPORTED;
   int G = std::min(cap, (m + rows_target - 1) / rows_target);
   const int rpc = (m + G - 1) / G;
   G = (m + rpc - 1) / rpc;

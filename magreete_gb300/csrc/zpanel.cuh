@@ -17,12 +17,15 @@ struct ZPanelWs {
   int max_ctas;
 };
 
-// Whether a panel of m rows fits `max_ctas` CTAs of at most 128 rows.
-inline bool zpanel_fits(int m, int max_ctas) { return m <= 128 * (max_ctas > 1 ? max_ctas : 1); }
+// Whether a panel of m rows fits `max_ctas` CTAs of about rows_target, at most 128, rows.
+inline bool zpanel_fits(int m, int rows_target, int max_ctas) {
+  return rows_target <= 128 && m <= 128 * (max_ctas > 1 ? max_ctas : 1);
+}
 
 // Factors columns [0, w) (w <= 32) of the m-row panel at P in place, with partial pivoting
 // (LAPACK's rule); MGT_ERR_UNSUPPORTED where the panel does not fit (nothing is launched).
+// allow_cluster, allow_wide: as one cluster; as CTAs that exchange through global memory.
 int zpanel_factor(double2* P, int64_t lda, int m, int w, int j0, int32_t* perm, const ZPanelWs& ws, int rows_target,
-                  int max_ctas, bool cooperative, bool allow_cluster, cudaStream_t s);
+                  int max_ctas, bool cooperative, bool allow_cluster, bool allow_wide, cudaStream_t s);
 
 }  // namespace mgt
