@@ -94,6 +94,12 @@ __device__ inline float cabs1(float2 a) { return fabsf(a.x) + fabsf(a.y); }
 // FP64 instruction that is predicated off still takes its time.
 __device__ __noinline__ inline double2 crecip_scaled(double2 z) {
   const int ex = max((__double2hiint(z.x) >> 20) & 0x7ff, (__double2hiint(z.y) >> 20) & 0x7ff);
+  if (ex == 2047) {
+    // zero for one infinite part, NaN for two and for a NaN, as Smith's division has it
+    const bool swap = fabs(z.x) < fabs(z.y);
+    const double a = swap ? z.y : z.x, b = swap ? z.x : z.y, r = b / a, inv = 1.0 / (a + b * r);
+    return swap ? make_double2(r * inv, -inv) : make_double2(inv, -r * inv);
+  }
   // 2^-(exponent of the larger part), in two factors so that neither overflows
   const int h = (1023 - ex) / 2, k = 1023 - ex - h;
   const double s1 = __hiloint2double((1023 + h) << 20, 0), s2 = __hiloint2double((1023 + k) << 20, 0);
