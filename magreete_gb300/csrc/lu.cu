@@ -2309,9 +2309,9 @@ static int lu_factor_impl(cplx<T>* A, int n, int64_t lda, int32_t* perm, void* w
         return split;
       }
       if (wb > 0 && opt.fused_right) {
+        // (partial pivoting: with tile pivoting a block with columns to its right is 128 wide)
         V* Inv = reinterpret_cast<V*>((char*)work + LuWsLayout().inv);
-        // tile pivoting: the tile kernels left both diagonal blocks' inverses there
-        if (opt.pivoting != MGT_PIVOT_TILE) lower_block_inverses(A + (int64_t)J0 * lda + J0, lda, W, Inv, s);
+        lower_block_inverses(A + (int64_t)J0 * lda + J0, lda, W, Inv, s);
         lu_block_right_kernel<T, NB><<<(right + kSwapCols - 1) / kSwapCols, 256, block_right_smem<NB>(sizeof(V)), s>>>(
             A, lda, n, J0, wa, wb, J0 + W, panel_ws(work, 0), panel_ws(work, 1), Inv);
         count_launch();

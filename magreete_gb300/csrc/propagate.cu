@@ -1,4 +1,4 @@
-// K5: matrix-free propagation to detectors.
+// K5: propagation to detectors.
 //
 // out[m*d+a, r] = coef * sum_j sum_b G_ab(t_m - s_j) Ek[j*d+b, r] + E0[m*d+a, r]
 //
@@ -35,35 +35,15 @@ constexpr int kPT = 16;      // detectors per CTA
 constexpr int kPJ = 8;       // sources per chunk
 constexpr int kPCols = 64;   // right-hand-side columns per launch
 
-template <bool DF> struct Acc;
-template <> struct Acc<false> {
-  using S = double2;   // staged operand
-  using A = double2;   // accumulator
-  __device__ static S from(double2 v) { return v; }
-  __device__ static A zero() { return make_double2(0.0, 0.0); }
-  __device__ static void mac(A& acc, S a, S b) { cfma(acc, a, b); }
-  __device__ static double2 out(A a) { return a; }
-};
-template <> struct Acc<true> {
-  using S = float4;
-  using A = float4;
-  __device__ static S from(double2 v) { return df_split(v); }
-  __device__ static A zero() { return make_float4(0.f, 0.f, 0.f, 0.f); }
-  __device__ static void mac(A& acc, S a, S b) { df_cmac(acc, a, b); }
-  __device__ static double2 out(A a) { return df_join(a); }
-};
-
-template <int KIND, int RT, bool DF>
+template <int KIND, int RT>
 __global__ void __launch_bounds__(256)
 propagate_partial_kernel(const double* __restrict__ tgt, int nt, const double* __restrict__ src, int ns, double k0,
                          bool regularize, double radius, const double2* __restrict__ Ek, int64_t ld_ek, int ncols,
                          int src_per_split, double2* __restrict__ partial) {
   constexpr int d = Kind<KIND>::d, dim = Kind<KIND>::dim;
   constexpr int ROWS = kPT * d, KC = kPJ * d;
-  using P = Acc<DF>;
-  using S = typename P::S;
-  __shared__ S Gs[ROWS][KC + 1];
-  __shared__ S Es[KC][16 * RT];
+  __shared__ double2 Gs[ROWS][KC + 1];
+  __shared__ double2 Es[KC][16 * RT];
   __shared__ double tpos[kPT][dim];
   const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   const int t0 = blockIdx.x * kPT;
@@ -72,11 +52,11 @@ propagate_partial_kernel(const double* __restrict__ tgt, int nt, const double* _
     int tt = tid / dim, c = tid - tt * dim;
     tpos[tt][c] = (t0 + tt < nt) ? tgt[(int64_t)(t0 + tt) * dim + c] : 0.0;
   }
-  typename P::A acc[d][RT];
+  double2 acc[d][RT];
 #pragma unroll
   for (int i = 0; i < d; ++i)
 #pragma unroll
-    for (int j = 0; j < RT; ++j) acc[i][j] = P::zero();
+    for (int j = 0; j < RT; ++j) acc[i][j] = make_double2(0.0, 0.0);
   __syncthreads();
   for (int sj0 = sbeg; sj0 < send; sj0 += kPJ) {
     if (tid < kPT * kPJ) {
@@ -98,26 +78,26 @@ propagate_partial_kernel(const double* __restrict__ tgt, int nt, const double* _
 #pragma unroll
       for (int a = 0; a < d; ++a)
 #pragma unroll
-        for (int b = 0; b < d; ++b) Gs[tt * d + a][jj * d + b] = P::from(g[a * d + b]);
+        for (int b = 0; b < d; ++b) Gs[tt * d + a][jj * d + b] = g[a * d + b];
     }
     for (int idx = tid; idx < KC * 16 * RT; idx += 256) {
       int kk = idx / (16 * RT), c = idx - kk * (16 * RT);
       int64_t row = (int64_t)sj0 * d + kk;
       double2 v = make_double2(0.0, 0.0);
       if (row < (int64_t)send * d && c < ncols) v = Ek[row * ld_ek + c];
-      Es[kk][c] = P::from(v);
+      Es[kk][c] = v;
     }
     __syncthreads();
 #pragma unroll 4
     for (int kk = 0; kk < KC; ++kk) {
-      S a[d];
+      double2 a[d];
 #pragma unroll
       for (int i = 0; i < d; ++i) a[i] = Gs[ty + 16 * i][kk];
 #pragma unroll
       for (int j = 0; j < RT; ++j) {
-        S x = Es[kk][tx + 16 * j];
+        const double2 x = Es[kk][tx + 16 * j];
 #pragma unroll
-        for (int i = 0; i < d; ++i) P::mac(acc[i][j], a[i], x);
+        for (int i = 0; i < d; ++i) cfma(acc[i][j], a[i], x);
       }
     }
     __syncthreads();
@@ -131,7 +111,7 @@ propagate_partial_kernel(const double* __restrict__ tgt, int nt, const double* _
 #pragma unroll
     for (int j = 0; j < RT; ++j) {
       int c = tx + 16 * j;
-      if (c < ncols) part[row * ncols + c] = P::out(acc[i][j]);
+      if (c < ncols) part[row * ncols + c] = acc[i][j];
     }
   }
 }
@@ -167,36 +147,35 @@ static int choose_splits(int64_t nt, int64_t ns) {
   return (int)std::max<int64_t>(1, std::min<int64_t>({want, maxs, 64}));
 }
 
-template <int KIND, int RT, bool DF>
+template <int KIND, int RT>
 static void launch_partial(dim3 grid, const double* t, int nt, const double* s, int ns, double k0, bool reg,
                            double radius, const double2* Ek, int64_t ld_ek, int ncols, int sps, double2* part,
                            cudaStream_t st) {
   count_launch();
   prepare_green<KIND>(st);
-  propagate_partial_kernel<KIND, RT, DF><<<grid, 256, 0, st>>>(t, nt, s, ns, k0, reg, radius, Ek, ld_ek,
+  propagate_partial_kernel<KIND, RT><<<grid, 256, 0, st>>>(t, nt, s, ns, k0, reg, radius, Ek, ld_ek,
                                                               ncols, sps, part);
 }
 
-template <int KIND, bool DF>
+template <int KIND>
 static void launch_partial_rt(int rt, dim3 grid, const double* t, int nt, const double* s, int ns, double k0,
                               bool reg, double radius, const double2* Ek, int64_t ld_ek, int ncols, int sps,
                               double2* part, cudaStream_t st) {
   switch (rt) {
-    case 1: launch_partial<KIND, 1, DF>(grid, t, nt, s, ns, k0, reg, radius, Ek, ld_ek, ncols, sps, part, st); break;
-    case 2: launch_partial<KIND, 2, DF>(grid, t, nt, s, ns, k0, reg, radius, Ek, ld_ek, ncols, sps, part, st); break;
-    default: launch_partial<KIND, 4, DF>(grid, t, nt, s, ns, k0, reg, radius, Ek, ld_ek, ncols, sps, part, st); break;
+    case 1: launch_partial<KIND, 1>(grid, t, nt, s, ns, k0, reg, radius, Ek, ld_ek, ncols, sps, part, st); break;
+    case 2: launch_partial<KIND, 2>(grid, t, nt, s, ns, k0, reg, radius, Ek, ld_ek, ncols, sps, part, st); break;
+    default: launch_partial<KIND, 4>(grid, t, nt, s, ns, k0, reg, radius, Ek, ld_ek, ncols, sps, part, st); break;
   }
 }
 
-template <bool DF>
 static void launch_partial_kind(int kind, int rt, dim3 grid, const double* t, int nt, const double* s, int ns,
                                 double k0, bool reg, double radius, const double2* Ek, int64_t ld_ek, int ncols,
                                 int sps, double2* part, cudaStream_t st) {
   switch (kind) {
-    case MGT_2D_VECTOR: launch_partial_rt<MGT_2D_VECTOR, DF>(rt, grid, t, nt, s, ns, k0, reg, radius, Ek, ld_ek, ncols, sps, part, st); break;
-    case MGT_2D_SCALAR: launch_partial_rt<MGT_2D_SCALAR, DF>(rt, grid, t, nt, s, ns, k0, reg, radius, Ek, ld_ek, ncols, sps, part, st); break;
-    case MGT_3D_VECTOR: launch_partial_rt<MGT_3D_VECTOR, DF>(rt, grid, t, nt, s, ns, k0, reg, radius, Ek, ld_ek, ncols, sps, part, st); break;
-    default: launch_partial_rt<MGT_3D_SCALAR, DF>(rt, grid, t, nt, s, ns, k0, reg, radius, Ek, ld_ek, ncols, sps, part, st); break;
+    case MGT_2D_VECTOR: launch_partial_rt<MGT_2D_VECTOR>(rt, grid, t, nt, s, ns, k0, reg, radius, Ek, ld_ek, ncols, sps, part, st); break;
+    case MGT_2D_SCALAR: launch_partial_rt<MGT_2D_SCALAR>(rt, grid, t, nt, s, ns, k0, reg, radius, Ek, ld_ek, ncols, sps, part, st); break;
+    case MGT_3D_VECTOR: launch_partial_rt<MGT_3D_VECTOR>(rt, grid, t, nt, s, ns, k0, reg, radius, Ek, ld_ek, ncols, sps, part, st); break;
+    default: launch_partial_rt<MGT_3D_SCALAR>(rt, grid, t, nt, s, ns, k0, reg, radius, Ek, ld_ek, ncols, sps, part, st); break;
   }
 }
 
@@ -402,12 +381,8 @@ extern "C" int mgt_propagate(int kind, int dtype, const double* targets, int64_t
     int rt = (nc + 15) / 16;
     if (rt == 3) rt = 4;
     dim3 grid(tiles, nsplit);
-    if (dtype == MGT_CDF)
-      launch_partial_kind<true>(kind, rt, grid, targets, nt, sources, ns, k0, regularize != 0, radius, ek + c0, ld_ek,
-                                nc, sps, part, st);
-    else
-      launch_partial_kind<false>(kind, rt, grid, targets, nt, sources, ns, k0, regularize != 0, radius, ek + c0,
-                                 ld_ek, nc, sps, part, st);
+    launch_partial_kind(kind, rt, grid, targets, nt, sources, ns, k0, regularize != 0, radius, ek + c0, ld_ek, nc, sps,
+                        part, st);
     int64_t nrows = (int64_t)nt * d;
     int64_t tot = nrows * nc;
     count_launch();

@@ -44,7 +44,7 @@
 // MMA operand's 128-byte-swizzled K-major rows at half width, so that
 // widening byte k of a slice to fp16 lands at byte 2k of the operand.
 // residual_tc_kernel: one CTA per (32 complex right-hand sides) x (128 rows)
-// x (a range of K in chunks), 512 threads:
+// x (a range of K in chunks), 448 threads:
 //   warp 0      : TMEM allocation (7 levels x 64 columns); bulk copies: per chunk the right-hand sides' digit block
 //                 (bdigits_kernel, 56 KB, 2 stages) and the seven 8 KB digit
 //                 slices of M (10-slice ring), whichever has a free slot

@@ -871,8 +871,8 @@ static int tri_steps(const float2* F, int64_t ldf, const unsigned char* ops, con
     // step i solves block row i (from the end for U) after updating it and all that follow
     const int first = UPPER ? nb - 1 : 0, src = i == 0 ? -1 : UPPER ? nb - i : i - 1;
     const int rest = i == 0 ? 0 : nb - 1 - i;   // block rows beyond
-    // K over the CTAs of a cluster while the launch is less than two rounds of
-    // what is resident at once (two CTAs an SM); beyond, one CTA takes all of K
+    // K over the CTAs of a cluster while the launch is at most 1.75 rounds of
+    // what is resident at once (two CTAs an SM, 3.5 in all); beyond, one CTA takes all of K
     // (34 K clocks for 128 rows, no sums to exchange, against 4 x 20 K).  Solves
     // of 64 columns with the line at 1.3, 2, 2.6, 3.4 and 4.6 CTAs an SM, ms:
     // n = 6000 0.98, 0.89, 0.86, 0.85, 0.85; 12000 2.23, 2.12, 2.06, 2.01, 2.07.
