@@ -4,8 +4,8 @@ The MAGreeTe driver images |E| and its longitudinal / transverse parts on a
 ``ngridx x ngridy`` grid (magreete.py:570-741).  It splits the grid into
 batches and calls ``propagate`` once per batch and per plotted angle, because
 the reference builds the dense (grid x scatterers) Green's matrix in host
-memory.  ``propagate`` here is matrix-free on the GPU (propagator rows are
-built in chunks of at most 1 GiB), so the whole grid and every plotted angle
+memory.  ``propagate`` here builds propagator rows on the GPU in chunks of at
+most 1 GiB (none for small calls), so the whole grid and every plotted angle
 go in ONE call, with the angles as right-hand-side columns.
 
     pts = grid_points(2, 301, 301, L, window_width)
