@@ -312,8 +312,8 @@ int mgt_refine_norms(const void* M, int64_t ldm, int64_t n, const void* B, int64
  * reference's G is NaN come out NaN; the host applies the reference's
  * row fix-up.  E0 may be NULL (treated as zero).
  */
-/* workspace of one dtype's method; mgt_propagate_workspace_bytes: of either.  MGT_C128 also accepts less
- * (the matrix-free kernel's partial sums) and then runs matrix-free. */
+/* workspace of one dtype's method; mgt_propagate_workspace_bytes: of either.  MGT_C128 also accepts
+ * less: it then takes smaller chunks of targets, or runs matrix-free where only that kernel's partial sums fit. */
 int mgt_propagate_workspace_bytes_for(int kind, int dtype, int64_t n_targets, int64_t n_sources, int64_t nrhs,
                                       size_t* bytes);
 int mgt_propagate_workspace_bytes(int kind, int64_t n_targets, int64_t n_sources, int64_t nrhs,

@@ -232,8 +232,7 @@ static int64_t prop_z_targets(int64_t nt, int64_t ns, int64_t nrhs, int d) {
   const int64_t per = std::max((int64_t)d * d * ns * 16, (int64_t)d * slabs * nrhs * 16);
   return std::max<int64_t>(1, std::min<int64_t>({nt, (int64_t)kPropChunkBytes / per, kPropMaxTargets}));
 }
-static size_t prop_z_bytes(int64_t nt, int64_t ns, int64_t nrhs, int d) {
-  const int64_t ct = prop_z_targets(nt, ns, nrhs, d);
+static size_t prop_z_bytes(int64_t ct, int64_t ns, int64_t nrhs, int d) {
   return 256 + (size_t)ct * d * d * ns * sizeof(double2) + zgemm_wide_bytes(ct * d, nrhs, (int64_t)d * ns) + 1024;
 }
 static size_t prop_tc_bytes(int64_t nt, int64_t ns, int64_t nrhs, int d) {
@@ -268,8 +267,9 @@ extern "C" int mgt_propagate_workspace_bytes_for(int kind, int dtype, int64_t n_
   if (!bytes || d == 0 || (dtype != MGT_C128 && dtype != MGT_CDF) || n_targets <= 0 || n_sources <= 0 || nrhs <= 0)
     return MGT_ERR_ARG;
   if (dtype == MGT_C128)
-    *bytes = prop_z_pays(n_targets, n_sources, nrhs, d) ? prop_z_bytes(n_targets, n_sources, nrhs, d)
-                                                        : prop_free_bytes(n_targets, n_sources, nrhs, d);
+    *bytes = prop_z_pays(n_targets, n_sources, nrhs, d)
+                 ? prop_z_bytes(prop_z_targets(n_targets, n_sources, nrhs, d), n_sources, nrhs, d)
+                 : prop_free_bytes(n_targets, n_sources, nrhs, d);
   else
     *bytes = prop_tc_ok(n_targets, n_sources, nrhs, d) ? prop_tc_bytes(n_targets, n_sources, nrhs, d)
                                                        : prop_df_bytes(n_targets, n_sources, nrhs, d);
@@ -300,13 +300,18 @@ extern "C" int mgt_propagate(int kind, int dtype, const double* targets, int64_t
   if (n_targets > (1 << 28) || n_sources > (1 << 28)) return MGT_ERR_UNSUPPORTED;
   size_t need = 0;
   mgt_propagate_workspace_bytes_for(kind, dtype, n_targets, n_sources, nrhs, &need);
-  // a workspace too small for the plain method's assembled way may serve the matrix-free kernel
-  if (work_bytes < need && (dtype != MGT_C128 || work_bytes < prop_free_bytes(n_targets, n_sources, nrhs, d)))
+  // The plain method in a smaller workspace: chunks of fewer targets, at least 128 rows each; the
+  // matrix-free kernel in one that has no room for those
+  int64_t ct = 0;
+  if (dtype == MGT_C128 && prop_z_pays(n_targets, n_sources, nrhs, d)) {
+    ct = prop_z_targets(n_targets, n_sources, nrhs, d);
+    while (ct > 0 && work_bytes < prop_z_bytes(ct, n_sources, nrhs, d)) ct = ct * d >= 256 ? ct / 2 : 0;
+  }
+  if (ct == 0 && work_bytes < (dtype == MGT_C128 ? prop_free_bytes(n_targets, n_sources, nrhs, d) : need))
     return MGT_ERR_WORKSPACE;
   cudaStream_t st = (cudaStream_t)stream;
   const int nt = (int)n_targets, ns = (int)n_sources;
-  if (dtype == MGT_C128 && prop_z_pays(nt, ns, nrhs, d) && work_bytes >= need) {
-    const int64_t ct = prop_z_targets(nt, ns, nrhs, d);
+  if (ct > 0) {
     // status words | rows | digits and partial products
     int* status = (int*)((char*)work + kStatusOffset);
     if (cudaMemsetAsync(work, 0, 256, st) != cudaSuccess) return MGT_ERR_CUDA;

@@ -440,6 +440,18 @@ class SystemFactorization:
 
 # ------------------------------------------------------------------ propagate
 
+def _propagation_workspace(nbytes, device, precision):
+    """The workspace asked for, or what the device still has of it for the plain
+    method, which takes its chunks to fit (down to 32 MB)."""
+    while True:
+        try:
+            return workspace(nbytes, device)
+        except torch.cuda.OutOfMemoryError:
+            nbytes //= 4
+            if precision != "fp64" or nbytes < 32 << 20:
+                raise
+
+
 def propagate(kind, targets, sources, k0, coef, Ek, E0=None, regularize=False, radius=0.0, precision="fp64"):
     """coef * G(targets, sources) @ Ek + E0 (rows of G in chunks of at most 1 GiB;
     small calls of the plain method without storing them).  Ek (d*S, R),
@@ -456,7 +468,7 @@ def propagate(kind, targets, sources, k0, coef, Ek, E0=None, regularize=False, r
     nb = ctypes.c_size_t()
     L.check(lib.mgt_propagate_workspace_bytes_for(KIND_CODE[kind], code, T, S, R, ctypes.byref(nb)),
             "mgt_propagate_workspace_bytes_for")
-    work = workspace(nb.value, targets.device)
+    work = _propagation_workspace(nb.value, targets.device, precision)
     coef = complex(coef)
     L.check(lib.mgt_propagate(KIND_CODE[kind], code, _ptr(targets), T, _ptr(sources), S, float(k0), coef.real,
                               coef.imag, int(bool(regularize)), float(radius), _ptr(Ek), R, _ptr(E0), R,
