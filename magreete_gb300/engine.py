@@ -269,11 +269,16 @@ def _solve_prepared(ctx, f, B, tol, max_iter, require):
     X = torch.empty_like(B)
     width, work = ctx.max_nrhs, ctx.work
     if R > width:
-        # blocks of equal width, in a workspace of their own
-        width = max(width, -(-R // -(-R // WIDE_NRHS)))
+        # blocks of equal width, in a workspace of their own (the context's, and its
+        # width, where the device has no room for it)
+        wide = max(width, -(-R // -(-R // WIDE_NRHS)))
         nbytes = ctypes.c_size_t()
-        L.check(lib.mgt_refine_scratch_bytes(n, width, ctypes.byref(nbytes)), "mgt_refine_scratch_bytes")
-        work = workspace(nbytes.value, B.device)
+        L.check(lib.mgt_refine_scratch_bytes(n, wide, ctypes.byref(nbytes)), "mgt_refine_scratch_bytes")
+        try:
+            work = workspace(nbytes.value, B.device)
+            width = wide
+        except torch.cuda.OutOfMemoryError:
+            pass
     its, sq, missed = [], 0.0, 0.0
     for c0 in range(0, R, width):
         Bc = B if width >= R else B[:, c0:c0 + width].contiguous()

@@ -51,3 +51,24 @@ def test_a_group_that_misses_the_tolerance():
         E.solve_refined(ctx, f, B, tol=1e-30)
     X, _, rr = E.solve_refined(ctx, f, B, tol=1e-11)
     assert rr <= 1e-11 and not X[:, 16:32].any()
+
+
+def test_no_room_for_a_wide_block(monkeypatch):
+    """Where the device has no room for a wide block's workspace the columns are
+    solved in blocks of the context's width, in its own."""
+    from magreete_gb300 import engine as E
+    Mdf, M32 = _system(300)
+    B = torch.randn(600, 200, dtype=torch.complex128, generator=torch.Generator().manual_seed(2)).cuda()
+    f = E.mixed_factor(M32, lambda: None)
+    ctx = E.RefineContext(Mdf, 32)
+    X0, _, r0 = E.solve_refined(ctx, f, B)
+    calls = []
+
+    def full(nbytes, device):
+        calls.append(nbytes)
+        raise torch.cuda.OutOfMemoryError("no room")
+
+    monkeypatch.setattr(E, "workspace", full)
+    X1, _, r1 = E.solve_refined(ctx, f, B)
+    assert len(calls) == 1 and r0 <= 1e-10 and r1 <= 1e-10
+    assert (torch.linalg.norm(X1 - X0) / torch.linalg.norm(X0)).item() < 1e-8
