@@ -172,10 +172,11 @@ int mgt_lu_factor_static(int dtype, void* A, int64_t n, int64_t lda, int32_t* pe
 /*
  * Solve A X = B with the factors of mgt_lu_factor (the ?getrs half of
  * ?gesv): X = U^-1 L^-1 P B for nrhs columns.  B is not modified.  With a
- * workspace of mgt_lu_solve_workspace_bytes(dtype, n, nrhs) bytes each
- * triangle is two launches (inverse of the 64 x 64 diagonal blocks, then one
- * persistent flag-ordered solve over block rows and 16-column groups); with
- * work == NULL the solve launches two kernels per 64-row block instead.
+ * workspace of mgt_lu_solve_workspace_bytes(dtype, n, nrhs) bytes the diagonal
+ * blocks are inverted first and the products run on the tensor cores:
+ * complex64 one launch per 256-row block and triangle, complex128 three per
+ * 64-row block.  With work == NULL two kernels per 64-row block on the FP32 /
+ * FP64 pipes instead.  A wait that runs out leaves NaN in what depends on it.
  */
 int mgt_lu_solve_workspace_bytes(int dtype, int64_t n, int64_t nrhs, size_t* bytes);
 int mgt_lu_solve(int dtype, const void* LU, int64_t n, int64_t lda, const int32_t* perm,
